@@ -76,6 +76,16 @@ def host_lib():
         _host.reef_sched_error.restype = C.c_char_p
         _host.reef_sched_avg_preempt_latency.restype = C.c_int64
         _host.reef_sched_avg_kernel_sel_latency.restype = C.c_int64
+        # declared argument types for the per-request calls: plain ints and bytes go in without a ctypes object each
+        for pre in ("reef_executor_", "reef_sched_"):
+            mid = [] if pre == "reef_executor_" else [C.c_uint32]
+            getattr(_host, pre + "get_data_size").argtypes = [C.c_void_p] + mid + [C.c_char_p, C.c_void_p]
+        _host.reef_executor_set_input.argtypes = [C.c_void_p, C.c_char_p, C.c_void_p, C.c_size_t]
+        _host.reef_executor_get_output.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t]
+        _host.reef_sched_set_input.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_size_t, C.c_char_p]
+        _host.reef_sched_get_output.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.c_size_t, C.c_char_p]
+        _host.reef_sched_new_task.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p]
+        _host.reef_sched_wait_task.argtypes = [C.c_void_p, C.c_uint32]
     return _host
 
 
@@ -142,7 +152,7 @@ def launch_count() -> int:
 
 
 def _buf(a: np.ndarray):
-    return a.ctypes.data_as(C.c_void_p)
+    return C.c_void_p(a.ctypes.data)
 
 
 class HybridExecutor:
@@ -150,6 +160,7 @@ class HybridExecutor:
 
     def __init__(self, device: int = 0):
         self._h = C.c_void_p()
+        self._out_bytes = {}
         self._lib = host_lib()
         _check(self._lib.reef_executor_create(C.c_int(device), C.byref(self._h)), "reef_executor_create")
 
@@ -168,6 +179,7 @@ class HybridExecutor:
         return (self._lib.reef_executor_error(self._h) or b"").decode()
 
     def load_model_from_file(self, json_path: str, profile_path: str | None = None):
+        self._out_bytes.clear()
         rc = self._lib.reef_executor_load(self._h, json_path.encode(), (profile_path or "").encode())
         _check(rc, "load_hybrid_model_from_file", self._err())
 
@@ -186,13 +198,16 @@ class HybridExecutor:
 
     def set_input(self, name: str, value: np.ndarray):
         v = np.ascontiguousarray(value)
-        _check(self._lib.reef_executor_set_input(self._h, name.encode(), _buf(v), C.c_size_t(v.nbytes)),
-               f"set_input({name})")
+        rc = self._lib.reef_executor_set_input(self._h, name.encode(), v.ctypes.data, v.nbytes)
+        if rc != SUCC:
+            _check(rc, f"set_input({name})")
 
     def get_output(self, dtype=np.float32) -> np.ndarray:
-        n = self.get_data_size("output")
+        n = self._out_bytes.get("output")
+        if n is None:      # fixed by the loaded model
+            n = self._out_bytes["output"] = self.get_data_size("output")
         out = np.empty(n // np.dtype(dtype).itemsize, dtype=dtype)
-        _check(self._lib.reef_executor_get_output(self._h, _buf(out), C.c_size_t(out.nbytes)), "get_output")
+        _check(self._lib.reef_executor_get_output(self._h, out.ctypes.data, out.nbytes), "get_output")
         return out
 
     def get_data(self, idx: int, nbytes: int, dtype=np.float32) -> np.ndarray:
@@ -202,7 +217,9 @@ class HybridExecutor:
         return out
 
     def execute(self):
-        _check(self._lib.reef_executor_execute(self._h), "execute", self._err())
+        rc = self._lib.reef_executor_execute(self._h)
+        if rc != SUCC:
+            _check(rc, "execute", self._err())
 
     def execute_to(self, idx: int):
         _check(self._lib.reef_executor_execute_to(self._h, C.c_int(idx)), "execute_to", self._err())
@@ -214,7 +231,9 @@ class HybridExecutor:
         _check(self._lib.reef_executor_execute_preemptable(self._h), "execute_preemptale", self._err())
 
     def execute_graph(self):
-        _check(self._lib.reef_executor_execute_graph(self._h), "execute_graph", self._err())
+        rc = self._lib.reef_executor_execute_graph(self._h)
+        if rc != SUCC:
+            _check(rc, "execute_graph", self._err())
 
     def execute_dispatch(self):
         _check(self._lib.reef_executor_execute_dispatch(self._h), "execute_dispatch", self._err())
@@ -317,6 +336,7 @@ class REEFScheduler:
 
     def __init__(self, mode: int = 3, device: int = 0):
         self._h = C.c_void_p()
+        self._out_bytes = {}
         self._lib = host_lib()
         _check(self._lib.reef_sched_create(C.c_int(mode), C.c_int(device), C.byref(self._h)), "REEFScheduler")
 
@@ -361,28 +381,27 @@ class REEFScheduler:
 
     def set_input(self, mid: int, data: np.ndarray, name: str = "data"):
         v = np.ascontiguousarray(data)
-        _check(self._lib.reef_sched_set_input(self._h, C.c_uint32(mid), _buf(v), C.c_size_t(v.nbytes), name.encode()),
-               "set_input")
+        _check(self._lib.reef_sched_set_input(self._h, mid, v.ctypes.data, v.nbytes, name.encode()), "set_input")
 
     def get_output(self, mid: int, name: str = "output", dtype=np.float32) -> np.ndarray:
-        n = self.get_data_size(mid, name)
+        n = self._out_bytes.get((mid, name))
+        if n is None:      # fixed by the loaded model; model ids are never reused
+            n = self._out_bytes[(mid, name)] = self.get_data_size(mid, name)
         out = np.empty(n // np.dtype(dtype).itemsize, dtype=dtype)
-        _check(self._lib.reef_sched_get_output(self._h, C.c_uint32(mid), _buf(out), C.c_size_t(out.nbytes),
-                                               name.encode()), "get_output")
+        _check(self._lib.reef_sched_get_output(self._h, mid, out.ctypes.data, out.nbytes, name.encode()), "get_output")
         return out
 
     def get_output_into(self, mid: int, out: np.ndarray, name: str = "output"):
         """Copy the named tensor into ``out`` (a contiguous array of exactly the tensor's size in bytes)."""
-        _check(self._lib.reef_sched_get_output(self._h, C.c_uint32(mid), _buf(out), C.c_size_t(out.nbytes),
-                                               name.encode()), "get_output")
+        _check(self._lib.reef_sched_get_output(self._h, mid, out.ctypes.data, out.nbytes, name.encode()), "get_output")
 
     def new_task(self, mid: int) -> int:
         tid = C.c_uint32()
-        _check(self._lib.reef_sched_new_task(self._h, C.c_uint32(mid), C.byref(tid)), "new_task")
+        _check(self._lib.reef_sched_new_task(self._h, mid, C.byref(tid)), "new_task")
         return tid.value
 
     def wait_task(self, tid: int):
-        _check(self._lib.reef_sched_wait_task(self._h, C.c_uint32(tid)), "wait_task")
+        _check(self._lib.reef_sched_wait_task(self._h, tid), "wait_task")
 
     def inject_launch_failures(self, mid: int, n: int):
         """Host-side failure injection: the next ``n`` kernel launches of model ``mid`` return an error."""

@@ -49,14 +49,14 @@ reef_status reef_gpu_init(int device) {
     if (t_device == device) return REEF_SUCC;   // this thread is already bound
     CK(cudaSetDevice(device));
     CK(cudaFree(0));
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) {
-        set_error("libreef_cuda is built for sm_100a only; device is sm_" + std::to_string(prop.major) +
-                  std::to_string(prop.minor));
+    int major = 0, minor = 0;   // (single attributes: cudaGetDeviceProperties gathers everything and takes milliseconds)
+    CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major != 10) {
+        set_error("libreef_cuda is built for sm_100a only; device is sm_" + std::to_string(major) + std::to_string(minor));
         return REEF_FAIL;
     }
-    g_num_sms = prop.multiProcessorCount;
+    CK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, device));
     t_device = device;
     return REEF_SUCC;
 }

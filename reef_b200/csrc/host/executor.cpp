@@ -1,5 +1,7 @@
 #include "executor.h"
 
+#include <emmintrin.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -8,10 +10,17 @@ namespace reef {
 namespace executor {
 
 static const size_t kAlign = 256;
+// Requests up to this size go through the pinned staging area / output mirror (beyond it the copies themselves, at
+// 20 GB/s and more, dwarf what staging saves, and an executor should not pin that much host memory).
+static const size_t kHostBufferMax = 4u << 20;
+static const size_t kMirrorKernelMax = 512u << 10;
 
 ExecutorBase::ExecutorBase() {}
 
 ExecutorBase::~ExecutorBase() {
+    wait_input();
+    if (input_ev) reef_event_destroy(input_ev);
+    if (host_buf) reef_host_free_pinned(host_buf);
     if (arena) reef_free(arena);
     if (own_module && base_mod) reef_module_close(base_mod);
 }
@@ -108,7 +117,11 @@ Status ExecutorBase::init_executor_base(const char* json_file_path, GPUModule_t 
     GPU_RETURN_STATUS(reef_malloc(&arena, total));
     GPU_RETURN_STATUS(reef_memset(arena, 0, total));
     storage.clear();
-    for (size_t i = 0; i < model->storage.size(); i++) storage.push_back(arena + offs[i]);
+    storage_idx.clear();
+    for (size_t i = 0; i < model->storage.size(); i++) {
+        storage.push_back(arena + offs[i]);
+        storage_idx.emplace(model->storage[i].name, i);
+    }
 
     // 4. positional args -> pointers to the storage slots
     raw_args.clear();
@@ -128,6 +141,69 @@ Status ExecutorBase::init_executor_base(const char* json_file_path, GPUModule_t 
         }
     }
     if (s == nullptr) GPU_RETURN_STATUS(reef_stream_create(&s, 0));
+    return init_host_buffers();
+}
+
+// Pinned host side of a request.  The staging area fits the model's first argument (its input; other inputs are no
+// larger in practice, and a larger one takes the direct path), the mirror the "output" tensor.  A small output (class
+// probabilities) is stored through the mapped pointer by a copy kernel behind the last layer, about 4 us in the pass;
+// a copy-engine transfer with its own wait afterwards takes 9 us (17 us from pageable memory).  Beyond kMirrorKernelMax
+// the copy engine does it as part of the pass: a copy node costs more to start (393 KB: 18 us against 11 us for the
+// kernel), but the kernel's stores over PCIe fall behind it on a megabyte (1.2 MB: 46 us against 36 us).
+Status ExecutorBase::init_host_buffers() {
+    if (!model->args.empty() && model->args[0] < model->storage.size()) {
+        const size_t bytes = storage_bytes(model->args[0]);
+        if (bytes <= kHostBufferMax) stage_bytes = align_up(bytes, kAlign);
+    }
+    size_t out = 0, out_bytes = 0;
+    if (find_storage_idx("output", out) == Status::Succ && storage_bytes(out) <= kHostBufferMax) {
+        out_bytes = storage_bytes(out);
+        if (out_bytes <= kMirrorKernelMax) {
+            const std::string name = "fused_nn_batch_flatten__n" + std::to_string(out_bytes / 4);
+            GPU_RETURN_STATUS(reef_module_get_kernel(base_mod, name.c_str(), &mirror_kernel));
+            GPU_RETURN_STATUS(reef_kernel_plan(name.c_str(), mirror_dims, &mirror_smem, nullptr));
+        }
+    }
+    if (stage_bytes + out_bytes == 0) return Status::Succ;
+    GPU_RETURN_STATUS(reef_host_alloc_pinned((void**)&host_buf, stage_bytes + out_bytes));
+    GPU_RETURN_STATUS(reef_event_create_untimed(&input_ev));
+    if (out_bytes) {
+        mirror = host_buf + stage_bytes;
+        mirror_args[0] = (GPUDevicePtr_t)mirror;
+        mirror_args[1] = storage[out];
+        mirror_bytes = out_bytes;
+    }
+    return Status::Succ;
+}
+
+Status ExecutorBase::launch_output_mirror(GPUStream_t stream) {
+    if (!mirror) return Status::Succ;
+    if (mirror_kernel) {
+        void* args[2] = {&mirror_args[0], &mirror_args[1]};
+        GPU_RETURN_STATUS(reef_launch(mirror_kernel, mirror_dims, mirror_smem, stream, args));
+    } else {
+        GPU_RETURN_STATUS(reef_memcpy_d2h_async(mirror, mirror_args[1], mirror_bytes, stream));
+    }
+    mirror_fresh.store(true, std::memory_order_relaxed);
+    return Status::Succ;
+}
+
+Status ExecutorBase::order_input(GPUStream_t stream) {
+    if (!input_pending.load(std::memory_order_acquire)) return Status::Succ;
+    if (stream != input_stream) {
+        int pending = 1;
+        GPU_RETURN_STATUS(reef_event_query(input_ev, &pending));
+        if (pending) GPU_RETURN_STATUS(reef_stream_wait_event(stream, input_ev));
+    }
+    input_pending.store(false, std::memory_order_release);
+    return Status::Succ;
+}
+
+// host wait for the staged copy (before the staging area is written again, read back or freed)
+Status ExecutorBase::wait_input() {
+    if (input_stream == nullptr) return Status::Succ;
+    GPU_RETURN_STATUS(reef_event_sync(input_ev));
+    input_pending.store(false, std::memory_order_release);
     return Status::Succ;
 }
 
@@ -142,8 +218,9 @@ Status ExecutorBase::load_param_from_file(const char* param_file_path) {
             err_ = "param " + model->storage[i].name + " is larger than its storage entry";
             RETURN_STATUS(Status::OutOfRange);
         }
-        GPU_RETURN_STATUS(reef_memcpy_h2d(storage[i], blob->data, bytes));
+        GPU_RETURN_STATUS(reef_memcpy_h2d_async(storage[i], blob->data, bytes, s));
     }
+    GPU_RETURN_STATUS(reef_stream_sync(s));   // the mapping goes away with `params`
     return Status::Succ;
 }
 
@@ -164,11 +241,54 @@ Status ExecutorBase::set_input(const std::string& key, const void* value, size_t
     return set_input((int)idx, value, len);
 }
 
+// A staged input of this size or more goes out in two pieces, so that the copy engine works on the first half while
+// the host writes the second (each further piece costs the host the 2 us of an asynchronous copy call).
+static const size_t kStageSplit = 128u << 10;
+// Host copy into the staging area.  Large pieces bypass the caches (streaming stores): lines left dirty in a core's
+// cache are snooped by the copy engine, and the next request's memcpy into them ran at half speed (602 KB: 26 us
+// against 21 us).  The staging area and the pieces are 64-byte aligned.
+static void stage_copy(unsigned char* dst, const unsigned char* src, size_t n) {
+    if (n < (64u << 10)) {
+        memcpy(dst, src, n);
+        return;
+    }
+    size_t i = 0;
+    for (; i + 64 <= n; i += 64) {
+        const __m128i a = _mm_loadu_si128((const __m128i*)(src + i)), b = _mm_loadu_si128((const __m128i*)(src + i + 16));
+        const __m128i c = _mm_loadu_si128((const __m128i*)(src + i + 32)), d = _mm_loadu_si128((const __m128i*)(src + i + 48));
+        _mm_stream_si128((__m128i*)(dst + i), a);
+        _mm_stream_si128((__m128i*)(dst + i + 16), b);
+        _mm_stream_si128((__m128i*)(dst + i + 32), c);
+        _mm_stream_si128((__m128i*)(dst + i + 48), d);
+    }
+    memcpy(dst + i, src + i, n - i);
+    _mm_sfence();
+}
+
 Status ExecutorBase::set_input(int idx, const void* value, size_t len) {
     if (idx < 0 || (size_t)idx >= storage.size()) return Status::OutOfRange;
     size_t bytes = storage_bytes(idx);
     if (len < bytes) return Status::OutOfRange;
-    GPU_RETURN_STATUS(reef_memcpy_h2d(storage[idx], value, bytes));
+    if (storage[idx] == mirror_args[1]) drop_output_mirror();
+    RETURN_STATUS(wait_input());
+    if (bytes > stage_bytes) {
+        GPU_RETURN_STATUS(reef_memcpy_h2d(storage[idx], value, bytes));
+        return Status::Succ;
+    }
+    // The caller's bytes are in the staging area when this returns; the copy engine follows on the executor's stream,
+    // and whatever launches kernels next is ordered behind it (order_input).  A 224x224 image (602 KB): 50 us for a
+    // copy from pageable memory that waits for its end, 34 us until this returns, and the tail of the copy travels
+    // beside the launch.
+    const unsigned char* src = (const unsigned char*)value;
+    const size_t piece = bytes < kStageSplit ? bytes : align_up(bytes / 2, kAlign);
+    for (size_t off = 0; off < bytes; off += piece) {
+        const size_t n = std::min(piece, bytes - off);
+        stage_copy(host_buf + off, src + off, n);
+        GPU_RETURN_STATUS(reef_memcpy_h2d_async(storage[idx] + off, host_buf + off, n, s));
+    }
+    GPU_RETURN_STATUS(reef_event_record(input_ev, s));
+    input_stream = s;
+    input_pending.store(true, std::memory_order_release);
     return Status::Succ;
 }
 
@@ -177,6 +297,8 @@ Status ExecutorBase::set_input_async(const std::string& key, const void* value, 
     if (find_storage_idx(key, idx) != Status::Succ) return Status::NotFound;
     size_t bytes = storage_bytes(idx);
     if (len < bytes) return Status::OutOfRange;
+    if (storage[idx] == mirror_args[1]) drop_output_mirror();
+    RETURN_STATUS(order_input(stream));
     GPU_RETURN_STATUS(reef_memcpy_h2d_async(storage[idx], value, bytes, stream));
     return Status::Succ;
 }
@@ -186,13 +308,17 @@ Status ExecutorBase::get_output(std::vector<float>& out) {
     if (find_storage_idx("output", idx) != Status::Succ) return Status::NotFound;
     if (Model::get_stype_size(model->storage[idx].stype) != sizeof(float)) return Status::Fail;
     out.resize(model->storage[idx].size);
-    return get_data((int)idx, (void*)out.data(), out.size() * sizeof(float));
+    return get_output((void*)out.data(), out.size() * sizeof(float));
 }
 
 Status ExecutorBase::get_output(void* out, size_t len) {
     size_t idx;
     if (find_storage_idx("output", idx) != Status::Succ) return Status::NotFound;
     if (len < storage_bytes(idx)) return Status::Fail;
+    if (mirror_fresh.load(std::memory_order_relaxed)) {
+        memcpy(out, mirror, storage_bytes(idx));
+        return Status::Succ;
+    }
     return get_data((int)idx, out, len);
 }
 
@@ -209,17 +335,16 @@ Status ExecutorBase::get_data(int idx, void* out, size_t len) {
     if (idx < 0 || (size_t)idx >= storage.size()) return Status::OutOfRange;
     size_t bytes = storage_bytes(idx);
     if (len < bytes) return Status::Fail;
+    RETURN_STATUS(wait_input());
     GPU_RETURN_STATUS(reef_memcpy_d2h(out, storage[idx], bytes));
     return Status::Succ;
 }
 
 Status ExecutorBase::find_storage_idx(const std::string& name, size_t& idx) {
-    for (size_t i = 0; i < storage.size(); i++)
-        if (model->storage[i].name == name) {
-            idx = i;
-            return Status::Succ;
-        }
-    return Status::NotFound;
+    auto it = storage_idx.find(name);
+    if (it == storage_idx.end()) return Status::NotFound;
+    idx = it->second;
+    return Status::Succ;
 }
 
 size_t ExecutorBase::num_kernels() const { return model ? model->kernels.size() : 0; }
@@ -231,7 +356,9 @@ Status ExecutorBase::execute(GPUStream_t stream) { return execute_to((int)num_ke
 Status ExecutorBase::execute_to(int idx, GPUStream_t stream) {
     if (stream == nullptr) stream = s;
     if (idx < 0 || (size_t)idx > num_kernels()) return Status::OutOfRange;
+    drop_output_mirror();
     for (int i = 0; i < idx; i++) RETURN_STATUS(launch_kernel(i, stream));
+    if ((size_t)idx == num_kernels()) RETURN_STATUS(launch_output_mirror(stream));
     GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
 }
@@ -239,6 +366,7 @@ Status ExecutorBase::execute_to(int idx, GPUStream_t stream) {
 Status ExecutorBase::execute_kernel(int idx, GPUStream_t stream) {
     if (stream == nullptr) stream = s;
     if (idx < 0 || (size_t)idx >= num_kernels()) return Status::OutOfRange;
+    drop_output_mirror();
     RETURN_STATUS(launch_kernel(idx, stream));
     GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
@@ -250,6 +378,7 @@ Status ExecutorBase::launch_kernel(int i, GPUStream_t stream) {
         err_ = "injected launch failure at kernel " + std::to_string(i);
         return Status::Fail;
     }
+    RETURN_STATUS(order_input(stream));
     int rc = reef_launch(kernels[i], model->kernels[i].launch_params, kernel_smem[i], stream, raw_args[i].data());
     if (rc != REEF_SUCC) err_ = reef_last_error();
     GPU_RETURN_STATUS(rc);
@@ -327,7 +456,9 @@ Status HybridExecutor::set_preempt_flag(GPUDevicePtr_t flag) {
 
 Status HybridExecutor::execute_preemptale(GPUStream_t stream) {
     if (stream == nullptr) stream = s;
+    drop_output_mirror();
     for (size_t i = 0; i < num_kernels(); i++) RETURN_STATUS(launch_preempt_kernel((int)i, stream));
+    RETURN_STATUS(launch_output_mirror(stream));
     GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
 }
@@ -360,6 +491,7 @@ Status HybridExecutor::launch_preempt_kernel(int i, GPUStream_t stream) {
         err_ = "injected launch failure at kernel " + std::to_string(i);
         return Status::Fail;
     }
+    RETURN_STATUS(order_input(stream));
     int rc = reef_launch_be(kernels[i], model->kernels[i].launch_params, kernel_smem[i], stream, preempt_flag,
                             task_slot_base + (size_t)i * 4, raw_args[i].data());
     if (rc != REEF_SUCC) err_ = reef_last_error();
@@ -370,6 +502,12 @@ Status HybridExecutor::launch_preempt_kernel(int i, GPUStream_t stream) {
 Status HybridExecutor::launch_dispatch(int rt_idx, HybridExecutor* be, int be_idx, int be_block_offset,
                                        int be_block_num, int sm_partition, int occupancy, GPUStream_t stream,
                                        GPUStream_t be_stream) {
+    drop_output_mirror();
+    RETURN_STATUS(order_input(stream));
+    if (be) {
+        be->drop_output_mirror();
+        RETURN_STATUS(be->order_input(be_stream ? be_stream : stream));
+    }
     int rc = reef_dispatch(kernels[rt_idx], raw_args[rt_idx].data(), be ? be->kernels[be_idx] : nullptr,
                            be ? be->raw_args[be_idx].data() : nullptr, be_block_offset, be_block_num, sm_partition,
                            occupancy, be ? be->task_slot_base + (size_t)be_idx * 4 : 0, dispatch_ctrl,
@@ -380,6 +518,7 @@ Status HybridExecutor::launch_dispatch(int rt_idx, HybridExecutor* be, int be_id
 }
 
 Status HybridExecutor::launch_pad_piece(int idx, int block_offset, int block_num, int occupancy, GPUStream_t stream) {
+    RETURN_STATUS(order_input(stream));
     int rc = reef_dispatch(nullptr, nullptr, kernels[idx], raw_args[idx].data(), block_offset, block_num, 0, occupancy,
                            task_slot_base + (size_t)idx * 4, dispatch_ctrl, dispatch_ctrl, stream, stream);
     if (rc != REEF_SUCC) err_ = reef_last_error();
@@ -389,6 +528,7 @@ Status HybridExecutor::launch_pad_piece(int idx, int block_offset, int block_num
 
 Status HybridExecutor::build_pad_segments() {
     if (!pad_segments.empty()) return Status::Succ;
+    RETURN_STATUS(wait_input());   // a wait on another stream's event must not be captured
     GPUStream_t cap = nullptr;
     GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
     const int n = (int)num_kernels();
@@ -422,6 +562,7 @@ Status HybridExecutor::build_pad_segments() {
 
 Status HybridExecutor::launch_pad_segment(int seg, GPUStream_t stream) {
     if (seg < 0 || seg >= (int)pad_segments.size()) RETURN_STATUS(Status::OutOfRange);
+    RETURN_STATUS(order_input(stream));
     GPU_RETURN_STATUS(reef_graph_launch(pad_segments[seg], stream));
     return Status::Succ;
 }
@@ -463,6 +604,7 @@ Status HybridExecutor::build_chains(int clusters) {
 
 // the schedule in order: a chain launch for every run that has one, a plain launch for every other kernel
 Status HybridExecutor::launch_schedule(GPUStream_t stream, bool use_chains) {
+    RETURN_STATUS(order_input(stream));
     size_t ci = 0;
     for (size_t i = 0; i < num_kernels();) {
         if (use_chains && ci < chains.size() && chains[ci].begin == (int)i) {
@@ -485,6 +627,7 @@ Status HybridExecutor::launch_schedule(GPUStream_t stream, bool use_chains) {
 Status HybridExecutor::launch_preempt_chain(int k, int clusters, GPUStream_t stream, int* next) {
     const int ci = chain_of(k);
     if (ci < 0) RETURN_STATUS(Status::OutOfRange);
+    RETURN_STATUS(order_input(stream));
     int rc = reef_chain_launch_be(chains[ci].handle, stream, k - chains[ci].begin, preempt_flag, clusters);
     if (rc != REEF_SUCC) {
         err_ = reef_last_error();
@@ -496,6 +639,7 @@ Status HybridExecutor::launch_preempt_chain(int k, int clusters, GPUStream_t str
 
 Status HybridExecutor::execute_preemptable_chained(int clusters, GPUStream_t stream) {
     if (stream == nullptr) stream = s;
+    drop_output_mirror();
     const int n = (int)num_kernels();
     for (int i = 0; i < n;) {
         if (chain_of(i) >= 0) {
@@ -529,6 +673,7 @@ Status HybridExecutor::execute_preempt_resume_chained(int delay_us, int clusters
     GPU_RETURN_STATUS(reef_stream_create(&flag_stream, 1));
     const int n = (int)num_kernels();
     int from = 0, rounds = 0;
+    drop_output_mirror();
     if (first_incomplete) *first_incomplete = -1;
     GPU_RETURN_STATUS(reef_write32_async(flag_stream, preempt_flag, 0));
     GPU_RETURN_STATUS(reef_stream_sync(flag_stream));
@@ -589,7 +734,9 @@ Status HybridExecutor::execute_preempt_resume_chained(int delay_us, int clusters
 
 Status HybridExecutor::execute_chained(GPUStream_t stream) {
     if (stream == nullptr) stream = s;
+    drop_output_mirror();
     RETURN_STATUS(launch_schedule(stream, true));
+    RETURN_STATUS(launch_output_mirror(stream));
     GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
 }
@@ -600,11 +747,22 @@ Status HybridExecutor::execute_graph(GPUStream_t stream) {
         err_ = "injected graph launch failure";
         return Status::Fail;
     }
-    if (graph == nullptr || graph_stream != stream) {
+    drop_output_mirror();
+    RETURN_STATUS(order_input(stream));   // before a capture begins: the wait is no part of the graph
+    if (graph_stream != stream) {
+        // The first pass on a stream launches kernel by kernel: capturing and instantiating a graph takes milliseconds,
+        // which a request should not wait for before it is known that more of them follow.
         if (graph) reef_graph_destroy(graph);
         graph = nullptr;
+        RETURN_STATUS(launch_schedule(stream, true));
+        RETURN_STATUS(launch_output_mirror(stream));
+        graph_stream = stream;
+        return Status::Succ;
+    }
+    if (graph == nullptr) {
         GPU_RETURN_STATUS(reef_graph_begin(stream));
         Status st = launch_schedule(stream, true);
+        if (st == Status::Succ) st = launch_output_mirror(stream);
         int rc = reef_graph_end(stream, &graph);
         if (st != Status::Succ || rc != REEF_SUCC) {
             // a launch failed while capturing: what was captured is a partial graph and must never be replayed
@@ -614,9 +772,17 @@ Status HybridExecutor::execute_graph(GPUStream_t stream) {
             graph_stream = nullptr;
             return st != Status::Succ ? st : Status::Fail;
         }
-        graph_stream = stream;
     }
     GPU_RETURN_STATUS(reef_graph_launch(graph, stream));
+    if (mirror) mirror_fresh.store(true, std::memory_order_relaxed);   // the graph ends with the copy
+    return Status::Succ;
+}
+
+Status HybridExecutor::execute(GPUStream_t stream) {
+    if (stream == nullptr) stream = s;
+    if (!chains.empty()) return execute_to((int)num_kernels(), stream);   // chains are execute_graph's and execute_chained's
+    RETURN_STATUS(execute_graph(stream));
+    GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
 }
 
@@ -641,6 +807,7 @@ Status HybridExecutor::execute_preempt_resume(int delay_us, int* restarts, int* 
     GPU_RETURN_STATUS(reef_stream_create(&flag_stream, 1));
     const int n = (int)num_kernels();
     int from = 0, rounds = 0;
+    drop_output_mirror();
     if (first_incomplete) *first_incomplete = -1;
     if (first_count) *first_count = -1;
     GPU_RETURN_STATUS(reef_write32_async(flag_stream, preempt_flag, 0));
@@ -681,6 +848,7 @@ Status HybridExecutor::profile_kernels(int iters, float* us) {
     // (weights of the other layers have cycled through L2 since its last run).  The stream is held by
     // a short delay kernel while the host queues the pass, so event gaps hold no launch latency.
     const size_t n = num_kernels();
+    drop_output_mirror();
     std::vector<reef_event_t> ev(n + 1);
     for (auto& e : ev) GPU_RETURN_STATUS(reef_event_create(&e));
     std::vector<double> sum(n, 0.0);
@@ -707,6 +875,8 @@ Status HybridExecutor::profile_kernels(int iters, float* us) {
 
 Status HybridExecutor::profile_wave(int idx, int occupancy, int iters, float* us) {
     if (idx < 0 || (size_t)idx >= num_kernels() || occupancy < 1) return Status::OutOfRange;
+    drop_output_mirror();
+    RETURN_STATUS(order_input(s));
     int num_sms = 0;
     GPU_RETURN_STATUS(reef_device_num_sms(&num_sms));
     int blocks = std::min(trans_args[idx].block_num, num_sms * occupancy);
@@ -738,6 +908,7 @@ Status HybridExecutor::profile_wave(int idx, int occupancy, int iters, float* us
 
 Status HybridExecutor::measure_profile(int iters, ModelProfile* out) {
     if (iters < 1) iters = 1;
+    drop_output_mirror();
     reef_event_t a, b;
     GPU_RETURN_STATUS(reef_event_create(&a));
     GPU_RETURN_STATUS(reef_event_create(&b));

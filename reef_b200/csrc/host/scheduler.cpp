@@ -698,7 +698,7 @@ void REEFScheduler::execute_rt_task(std::shared_ptr<Task>& task) {
             }
             if (reef_stream_sync(rt_queue->stream) != REEF_SUCC) ok = false;
             if (ok) task->model->add_alone_sample((double)ns_since(t0));
-        } else if (exe.execute(rt_queue->stream) != Status::Succ) {
+        } else if (exe.execute_to((int)exe.num_kernels(), rt_queue->stream) != Status::Succ) {
             err_ = "real-time launch failed: " + exe.error();
             ok = false;
         }
@@ -731,6 +731,7 @@ void REEFScheduler::advance_padded(Task* be_task, TaskQueue* q, int blocks, bool
     if (side_launch) {
         // its last blocks are on the best-effort stream: the task completes when that stream has drained,
         // which the best-effort branch of the loop sees through the window
+        be_exe.launch_output_mirror(q->stream);   // (a refused launch leaves get_output to copy for itself)
         reef_event_t ev;
         if (!q->free_events.empty()) {
             ev = q->free_events.back();
@@ -1216,6 +1217,7 @@ void REEFScheduler::execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr
         } else {
             reef_event_create_untimed(&ev);
         }
+        if (k == num_kernels - 1) exe.launch_output_mirror(tqueue->stream);
         reef_event_record(ev, tqueue->stream);
         tqueue->inflight.push_back(InFlight{ev, k});
         task->launch_offset = k + 1;

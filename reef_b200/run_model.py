@@ -2,7 +2,7 @@
 
     python -m reef_b200.run_model --model resnet152 [--variant _fp32] [--mode raw|graph|be|dispatch|chain] [--iters 20]
 
-``raw`` launches the kernels of <model>.json one by one (the reference's ExecutorBase::execute,
+``raw`` launches the kernels of <model>.json one by one (the reference's ExecutorBase::execute_to,
 src/reef/executor/executor_base.cpp:196-223), ``graph`` replays a CUDA graph of them, ``be`` uses the
 best-effort flavour (preempt flag + completion counters), ``dispatch`` sends every kernel through the
 dynamic-kernel-padding entry point without a partner, ``chain`` runs every run of consecutive tensor-core layers as
@@ -46,7 +46,7 @@ def main():
             e.set_input(name, rng.normal(0, 1, n // 4).astype(np.float32))
     if a.mode == "chain":
         print("chains:", e.build_chains(a.clusters), "first:", e.chain_info(0))
-    run = {"chain": e.execute_chained, "raw": e.execute, "graph": e.execute_graph, "be": e.execute_preemptable, "dispatch": e.execute_dispatch}[a.mode]
+    run = {"chain": e.execute_chained, "raw": lambda: e.execute_to(e.num_kernels()), "graph": e.execute_graph, "be": e.execute_preemptable, "dispatch": e.execute_dispatch}[a.mode]
     t0 = time.perf_counter()
     for _ in range(a.iters):
         run()

@@ -1,0 +1,57 @@
+"""Requests through host memory: staged input, output mirror, graph replay behind the first pass.  A one-kernel model that
+copies its input makes every byte of the way visible; sizes straddle the two-piece split of the staging copy, the limit
+between the mirror's copy kernel and the copy engine, and the limit of the pinned buffers."""
+
+import numpy as np
+import pytest
+
+from reef_b200 import capi
+from reef_b200.resources.graph import Graph, kname
+
+pytestmark = pytest.mark.gpu
+
+KB = 256            # floats per KB
+SIZES = [1, 3, 128 * KB - 1, 128 * KB, 128 * KB + 5, 512 * KB, 512 * KB + 1, 4096 * KB, 4096 * KB + 3]
+
+
+def copy_model(tmp_path, n):
+    g = Graph("copy")
+    data = g.input("data", n)
+    g.kernel(kname("fused_nn_batch_flatten", n=n), [g.add_storage("output", n), data])
+    return g.write(str(tmp_path), capi.plan_fn)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_executor_request(tmp_path, n):
+    base = copy_model(tmp_path, n)
+    e = capi.HybridExecutor(0)
+    e.load_model_from_file(base + ".json", base + ".profile.json")
+    rng = np.random.default_rng(n)
+    for run in (e.execute, e.execute_graph, e.execute_preemptable, e.execute_dispatch, lambda: e.execute_to(1)):
+        for _ in range(3):      # plain launches, capture, replay
+            x = rng.normal(0, 1, n).astype(np.float32)
+            e.set_input("data", np.zeros(n, np.float32))
+            e.set_input("data", x)      # the second input waits for the first one's copy
+            run()
+            assert np.array_equal(e.get_output(), x)
+    e.set_input("data", x + 1)
+    assert np.array_equal(e.get_output(), x), "a new input alone leaves the last output"
+    assert np.array_equal(e.get_data(0, 4 * n), x + 1)
+    e.close()
+
+
+@pytest.mark.parametrize("kind", [capi.REEFScheduler.RealTimeQueue, capi.REEFScheduler.BestEffortQueue])
+@pytest.mark.parametrize("n", [3, 128 * KB + 5, 512 * KB + 1, 4096 * KB + 3])
+def test_scheduler_request(tmp_path, kind, n):
+    base = copy_model(tmp_path, n)
+    s = capi.REEFScheduler(capi.REEFScheduler.REEF, 0)
+    mid = s.load_model_files(base + ".json", base + ".profile.json")
+    s.bind_model_queue(s.create_queue(kind), mid)
+    s.run()
+    rng = np.random.default_rng(n)
+    for _ in range(4):
+        x = rng.normal(0, 1, n).astype(np.float32)
+        s.set_input(mid, x)
+        s.wait_task(s.new_task(mid))
+        assert np.array_equal(s.get_output(mid), x)
+    s.close()
