@@ -393,6 +393,7 @@ HybridExecutor::~HybridExecutor() {
     for (auto& c : chains) reef_chain_destroy(c.handle);
     if (graph) reef_graph_destroy(graph);
     for (auto g : pad_segments) reef_graph_destroy(g);
+    for (auto g : be_segments) reef_graph_destroy(g);
     if (own_flag && preempt_flag) reef_free(preempt_flag);
     if (task_slot_base) reef_free(task_slot_base);
     if (dispatch_ctrl) reef_free(dispatch_ctrl);
@@ -558,6 +559,62 @@ Status HybridExecutor::build_pad_segments() {
         pad_segments.clear();
     }
     return st;
+}
+
+Status HybridExecutor::build_be_segments() {
+    if (!be_segments.empty()) return Status::Succ;
+    RETURN_STATUS(wait_input());
+    GPUStream_t cap = nullptr;
+    GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
+    const int n = (int)num_kernels();
+    Status st = Status::Succ;
+    for (int k0 = 0; k0 < n && st == Status::Succ; k0 += kBeSegment) {
+        if (reef_graph_begin(cap) != REEF_SUCC) {
+            st = Status::Fail;
+            break;
+        }
+        const int k1 = std::min(n, k0 + kBeSegment);
+        for (int k = k0; k < k1 && st == Status::Succ; k++) st = launch_preempt_kernel(k, cap);
+        if (st == Status::Succ && k1 == n) st = launch_output_mirror(cap);
+        reef_graph_t g = nullptr;
+        if (reef_graph_end(cap, &g) != REEF_SUCC) {
+            err_ = reef_last_error();
+            st = Status::Fail;
+        }
+        if (st == Status::Succ) be_segments.push_back(g);
+        else if (g) reef_graph_destroy(g);
+    }
+    reef_stream_destroy(cap);
+    drop_output_mirror();
+    if (st != Status::Succ) {
+        for (auto g : be_segments) reef_graph_destroy(g);
+        be_segments.clear();
+    }
+    return st;
+}
+
+// Best-effort kernels from k on: a whole segment where k stands at a segment boundary, else (a task resumed in the middle
+// of a segment, or `single`) kernel k alone.  *last = the last kernel launched.
+Status HybridExecutor::launch_preempt_segment(int k, GPUStream_t stream, bool single, int* last) {
+    const int n = (int)num_kernels();
+    if (single || be_segments.empty() || k % kBeSegment != 0) {
+        *last = k;
+        RETURN_STATUS(launch_preempt_kernel(k, stream));
+        if (k == n - 1) RETURN_STATUS(launch_output_mirror(stream));
+        return Status::Succ;
+    }
+    if (fail_launches > 0) {
+        fail_launches--;
+        err_ = "injected launch failure at kernel " + std::to_string(k);
+        return Status::Fail;
+    }
+    RETURN_STATUS(order_input(stream));
+    *last = std::min(n, k + kBeSegment) - 1;
+    int rc = reef_graph_launch(be_segments[k / kBeSegment], stream);
+    if (rc != REEF_SUCC) err_ = reef_last_error();
+    GPU_RETURN_STATUS(rc);
+    if (*last == n - 1 && mirror) mirror_fresh.store(true, std::memory_order_relaxed);
+    return Status::Succ;
 }
 
 Status HybridExecutor::launch_pad_segment(int seg, GPUStream_t stream) {

@@ -161,6 +161,11 @@ public:
     Status build_pad_segments();
     bool has_pad_segments() const { return !pad_segments.empty(); }
     Status launch_pad_segment(int seg, GPUStream_t stream);
+    // Best-effort segments: the same cut into runs of kBeSegment kernels for the best-effort flavour (every kernel still
+    // polls the flag and counts into its slot).  A task at full speed is fed one graph launch and one event per run.
+    static const int kBeSegment = 8;
+    Status build_be_segments();
+    Status launch_preempt_segment(int kernel_offset, GPUStream_t stream, bool single, int* last);
     bool has_tensor_core_kernels() const { return has_tc; }
     // Persistent chains: every run of two or more consecutive tensor-core convolution / matmul kernels of the
     // schedule becomes ONE persistent kernel (reef_chain_create) with `clusters` 8-CTA clusters (0 = the library's
@@ -233,6 +238,7 @@ protected:
     std::shared_ptr<ModelProfile> model_profile;
     reef_graph_t graph = nullptr;
     std::vector<reef_graph_t> pad_segments;
+    std::vector<reef_graph_t> be_segments;
     GPUStream_t graph_stream = nullptr;
     struct Chain {
         int begin, end;          // kernels [begin, end) of the schedule

@@ -260,6 +260,9 @@ private:
     uint32_t dkp_next_queue = 0;
     int rt_grace_us = 30;
     bool rt_recent = false;
+    bool rt_expected() const;
+    uint64_t rt_pause_ns[4] = {0, 0, 0, 0};   // from a real-time task's end to the next one's start, the last four
+    static const int kRtActiveMs = 20;   // real-time clients count as active this long after their last request
     std::chrono::steady_clock::time_point last_rt_finish;
     int pad_depth = 3;
     int pad_overcommit = 100;

@@ -55,3 +55,35 @@ def test_scheduler_request(tmp_path, kind, n):
         s.wait_task(s.new_task(mid))
         assert np.array_equal(s.get_output(mid), x)
     s.close()
+
+
+@pytest.mark.parametrize("kernels", [1, 7, 8, 9, 16, 17])
+def test_best_effort_segments(tmp_path, kernels):
+    """Schedules shorter than, equal to and just beyond a segment of the best-effort window, with the GPU to themselves
+    (whole segments) and while a real-time client is active (single kernels, resumed anywhere in a segment)."""
+    n = 5000
+    g = Graph("copies")
+    src = g.input("data", n)
+    for i in range(kernels):
+        dst = g.add_storage("output" if i == kernels - 1 else "null", n)
+        g.kernel(kname("fused_nn_batch_flatten", n=n), [dst, src])
+        src = dst
+    base = g.write(str(tmp_path), capi.plan_fn)
+    s = capi.REEFScheduler(capi.REEFScheduler.REEF, 0)
+    be = s.load_model_files(base + ".json", base + ".profile.json")
+    rt = s.load_model_files(base + ".json", base + ".profile.json")
+    s.bind_model_queue(s.create_queue(capi.REEFScheduler.BestEffortQueue), be)
+    s.bind_model_queue(s.create_queue(capi.REEFScheduler.RealTimeQueue), rt)
+    s.run()
+    rng = np.random.default_rng(kernels)
+    for i in range(12):
+        x, y = rng.normal(0, 1, (2, n)).astype(np.float32)
+        s.set_input(be, x)
+        t = s.new_task(be)
+        if i >= 4:
+            s.set_input(rt, y)
+            s.wait_task(s.new_task(rt))
+            assert np.array_equal(s.get_output(rt), y)
+        s.wait_task(t)
+        assert np.array_equal(s.get_output(be), x)
+    s.close()
