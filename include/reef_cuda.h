@@ -92,6 +92,12 @@ REEF_API reef_status reef_stream_wait_event(reef_stream_t s, reef_event_t e);
  * hipModuleLaunchKernel per layer, executor_base.cpp:196-223). */
 REEF_API reef_status reef_graph_begin(reef_stream_t s);
 REEF_API reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g);
+/* The same with the order of the captured launches relaxed to what they need: launch j waits for launch i only where
+ * from[e] == i and to[e] == j for some e (indices in capture order, from < to), so that independent branches of a model
+ * run side by side.  An edge between two kernels is a programmatic one (the later kernel's prologue overlaps the earlier
+ * kernel, as between neighbours of the captured stream); every kernel of this library waits for its predecessors before
+ * it touches memory, so an order that follows from other edges needs none of its own. */
+REEF_API reef_status reef_graph_end_relaxed(reef_stream_t s, const int* from, const int* to, size_t num_edges, reef_graph_t* g);
 REEF_API reef_status reef_graph_launch(reef_graph_t g, reef_stream_t s);
 REEF_API reef_status reef_graph_destroy(reef_graph_t g);
 
@@ -125,6 +131,11 @@ REEF_API reef_status reef_kernel_prepare(reef_kernel_t k, void** args);
  * index); here the loader refuses a json whose storage entry is smaller than what the shape in the kernel name
  * makes the kernel touch. */
 REEF_API reef_status reef_kernel_arg_bytes(reef_kernel_t k, size_t* bytes, int n);
+
+/* What a launch does with the buffer behind positional argument `arg`: *writes != 0 for an output, and the channels
+ * [*c0, *c1) of every *stride it touches (stride 0: the whole buffer).  Two accesses of one buffer with the same stride
+ * and disjoint channels do not meet: the branches of a concatenation write side by side. */
+REEF_API reef_status reef_kernel_arg_use(reef_kernel_t k, int arg, int* writes, int* c0, int* c1, int* stride);
 
 /* GPUConfig::KernelResource + calculate_occupancy (reference: hip_impl.h:62-74, hip_impl.cpp:34-74). */
 typedef struct {

@@ -423,10 +423,7 @@ reef_status reef_graph_begin(reef_stream_t s) {
     CK(cudaStreamBeginCapture((cudaStream_t)s, cudaStreamCaptureModeThreadLocal));
     return REEF_SUCC;
 }
-reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g) {
-    *g = nullptr;
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamEndCapture((cudaStream_t)s, &graph));
+static reef_status graph_instantiate(cudaGraph_t graph, reef_graph_t* g) {
     cudaGraphExec_t exec;
     cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
     if (e != cudaSuccess) {
@@ -442,6 +439,75 @@ reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g) {
     }
     *g = (reef_graph_t)h;
     return REEF_SUCC;
+}
+reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g) {
+    *g = nullptr;
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamEndCapture((cudaStream_t)s, &graph));
+    return graph_instantiate(graph, g);
+}
+// The captured chain of nodes in order, its edges replaced by the given ones.
+static reef_status graph_relax(cudaGraph_t graph, const int* from, const int* to, size_t num_edges) {
+    size_t n = 0, roots = 1;
+    CK(cudaGraphGetNodes(graph, nullptr, &n));
+    if (n < 2) return REEF_SUCC;
+    std::vector<cudaGraphNode_t> order(n), a, b;
+    std::vector<cudaGraphEdgeData> edge;
+    CK(cudaGraphGetRootNodes(graph, order.data(), &roots));
+    if (roots != 1) {
+        set_error("reef_graph_end_relaxed: the capture is not a chain of launches");
+        return REEF_FAIL;
+    }
+    for (size_t i = 0; i + 1 < n; i++) {
+        cudaGraphEdgeData e;
+        size_t next = 1;
+        CK(cudaGraphNodeGetDependentNodes_v2(order[i], &order[i + 1], &e, &next));
+        if (next != 1) {
+            set_error("reef_graph_end_relaxed: the capture is not a chain of launches");
+            return REEF_FAIL;
+        }
+        a.push_back(order[i]);
+        b.push_back(order[i + 1]);
+        edge.push_back(e);
+    }
+    CK(cudaGraphRemoveDependencies_v2(graph, a.data(), b.data(), edge.data(), n - 1));
+    std::vector<char> kernel(n);
+    for (size_t i = 0; i < n; i++) {
+        cudaGraphNodeType t;
+        CK(cudaGraphNodeGetType(order[i], &t));
+        kernel[i] = t == cudaGraphNodeTypeKernel;
+    }
+    a.clear();
+    b.clear();
+    edge.clear();
+    for (size_t e = 0; e < num_edges; e++) {
+        if (from[e] < 0 || from[e] >= to[e] || (size_t)to[e] >= n) {
+            set_error("reef_graph_end_relaxed: edge outside the captured launches");
+            return REEF_OUT_OF_RANGE;
+        }
+        cudaGraphEdgeData d;
+        memset(&d, 0, sizeof(d));
+        if (kernel[from[e]] && kernel[to[e]]) {
+            d.from_port = cudaGraphKernelNodePortProgrammatic;
+            d.type = cudaGraphDependencyTypeProgrammatic;
+        }
+        a.push_back(order[from[e]]);
+        b.push_back(order[to[e]]);
+        edge.push_back(d);
+    }
+    if (num_edges) CK(cudaGraphAddDependencies_v2(graph, a.data(), b.data(), edge.data(), num_edges));
+    return REEF_SUCC;
+}
+reef_status reef_graph_end_relaxed(reef_stream_t s, const int* from, const int* to, size_t num_edges, reef_graph_t* g) {
+    *g = nullptr;
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamEndCapture((cudaStream_t)s, &graph));
+    reef_status rc = graph_relax(graph, from, to, num_edges);
+    if (rc != REEF_SUCC) {
+        cudaGraphDestroy(graph);
+        return rc;
+    }
+    return graph_instantiate(graph, g);
 }
 reef_status reef_graph_launch(reef_graph_t g, reef_stream_t s) {
     reef_graph_s* h = (reef_graph_s*)g;
@@ -512,6 +578,15 @@ reef_status reef_kernel_prepare(reef_kernel_t k, void** args) {
 reef_status reef_kernel_arg_bytes(reef_kernel_t k, size_t* bytes, int n) {
     if (!k || !bytes || n < k->spec.nargs) return REEF_OUT_OF_RANGE;
     for (int i = 0; i < k->spec.nargs; i++) bytes[i] = k->spec.arg_bytes[i];
+    return REEF_SUCC;
+}
+reef_status reef_kernel_arg_use(reef_kernel_t k, int arg, int* writes, int* c0, int* c1, int* stride) {
+    if (!k || arg < 0 || arg >= k->spec.nargs) return REEF_OUT_OF_RANGE;
+    const ArgUse u = arg_use(k->spec, arg);
+    *writes = u.writes;
+    *c0 = u.c0;
+    *c1 = u.c1;
+    *stride = u.stride;
     return REEF_SUCC;
 }
 reef_status reef_kernel_attrs(reef_kernel_t k, reef_kernel_attrs_t* out) {

@@ -564,6 +564,8 @@ Status HybridExecutor::build_pad_segments() {
 Status HybridExecutor::build_be_segments() {
     if (!be_segments.empty()) return Status::Succ;
     RETURN_STATUS(wait_input());
+    std::vector<int> from, to;
+    RETURN_STATUS(schedule_edges(&from, &to));
     GPUStream_t cap = nullptr;
     GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
     const int n = (int)num_kernels();
@@ -576,8 +578,15 @@ Status HybridExecutor::build_be_segments() {
         const int k1 = std::min(n, k0 + kBeSegment);
         for (int k = k0; k < k1 && st == Status::Succ; k++) st = launch_preempt_kernel(k, cap);
         if (st == Status::Succ && k1 == n) st = launch_output_mirror(cap);
+        // branches side by side inside a segment, too; the segments follow one another on the stream
+        std::vector<int> seg_from, seg_to;
+        for (size_t e = 0; e < from.size(); e++)
+            if (from[e] >= k0 && to[e] < k1 + (k1 == n ? 1 : 0)) {
+                seg_from.push_back(from[e] - k0);
+                seg_to.push_back(to[e] - k0);
+            }
         reef_graph_t g = nullptr;
-        if (reef_graph_end(cap, &g) != REEF_SUCC) {
+        if (reef_graph_end_relaxed(cap, seg_from.data(), seg_to.data(), seg_from.size(), &g) != REEF_SUCC) {
             err_ = reef_last_error();
             st = Status::Fail;
         }
@@ -798,6 +807,45 @@ Status HybridExecutor::execute_chained(GPUStream_t stream) {
     return Status::Succ;
 }
 
+// Launch j needs an edge from launch i < j where they meet in a storage entry that one of them writes, unless it already
+// follows from other edges.  The predecessors of j are gone through from the latest to the earliest, and one that is
+// reachable from an edge already taken is skipped: what remains is the least set of edges with the schedule's order.
+Status HybridExecutor::schedule_edges(std::vector<int>* from, std::vector<int>* to) {
+    struct Use {
+        int launch, writes, c0, c1, stride;
+    };
+    const size_t n = num_kernels(), words = (n + 64) / 64;
+    std::vector<std::vector<Use>> uses(storage.size());
+    std::vector<std::vector<uint64_t>> before(n + 1, std::vector<uint64_t>(words, 0));   // launches each one is ordered behind
+    auto meet = [](const Use& a, const Use& b) {
+        return (a.writes || b.writes) && (a.stride == 0 || a.stride != b.stride || (a.c0 < b.c1 && b.c0 < a.c1));
+    };
+    size_t out = 0;
+    const bool mirrored = mirror != nullptr && find_storage_idx("output", out) == Status::Succ;
+    for (size_t j = 0; j < n + (mirrored ? 1 : 0); j++) {
+        std::vector<char> pred(j, 0);
+        const size_t nargs = j < n ? model->kernels[j].args.size() : 1;
+        std::vector<std::pair<size_t, Use>> mine;
+        for (size_t k = 0; k < nargs; k++) {
+            Use u{(int)j, 0, 0, 0, 0};
+            const size_t idx = j < n ? model->kernels[j].args[k] : out;
+            if (j < n) GPU_RETURN_STATUS(reef_kernel_arg_use(kernels[j], (int)k, &u.writes, &u.c0, &u.c1, &u.stride));
+            for (const Use& v : uses[idx])
+                if (meet(u, v)) pred[v.launch] = 1;
+            mine.push_back({idx, u});
+        }
+        for (auto& m : mine) uses[m.first].push_back(m.second);
+        for (size_t i = j; i-- > 0;) {
+            if (!pred[i] || (before[j][i / 64] >> (i % 64) & 1)) continue;
+            from->push_back((int)i);
+            to->push_back((int)j);
+            for (size_t w = 0; w < words; w++) before[j][w] |= before[i][w];
+            before[j][i / 64] |= 1ull << (i % 64);
+        }
+    }
+    return Status::Succ;
+}
+
 Status HybridExecutor::execute_graph(GPUStream_t stream) {
     if (fail_launches > 0 && graph != nullptr && graph_stream == stream) {   // injected failure of a graph replay
         fail_launches--;
@@ -820,7 +868,9 @@ Status HybridExecutor::execute_graph(GPUStream_t stream) {
         GPU_RETURN_STATUS(reef_graph_begin(stream));
         Status st = launch_schedule(stream, true);
         if (st == Status::Succ) st = launch_output_mirror(stream);
-        int rc = reef_graph_end(stream, &graph);
+        std::vector<int> from, to;
+        const bool relaxed = st == Status::Succ && chains.empty() && schedule_edges(&from, &to) == Status::Succ;
+        int rc = relaxed ? reef_graph_end_relaxed(stream, from.data(), to.data(), from.size(), &graph) : reef_graph_end(stream, &graph);
         if (st != Status::Succ || rc != REEF_SUCC) {
             // a launch failed while capturing: what was captured is a partial graph and must never be replayed
             if (rc != REEF_SUCC && st == Status::Succ) err_ = reef_last_error();

@@ -246,6 +246,9 @@ protected:
     };
     std::vector<Chain> chains;
     Status launch_schedule(GPUStream_t stream, bool use_chains);
+    // which launches of the schedule (and, as number num_kernels(), of the output mirror behind it) have to wait for
+    // which others
+    Status schedule_edges(std::vector<int>* from, std::vector<int>* to);
 };
 
 }  // namespace executor

@@ -489,6 +489,50 @@ static void fill_arg_bytes(KernelSpec* s) {
     }
 }
 
+ArgUse arg_use(const KernelSpec& s, int arg) {
+    const KTask& t = s.task;
+    int out = 0, out2 = -1;
+    ArgUse u = {0, 0, 0, 0};
+    auto slice = [&](int c0, int c, int stride) {
+        if (c < stride) { u.c0 = c0; u.c1 = c0 + c; u.stride = stride; }
+    };
+    switch (t.family) {
+        case F_MOCK_ADD:
+        case F_MOCK_MUL:
+        case F_DENSE:
+            out = 2;
+            break;
+        case F_BIAS_RELU:
+            if (arg == 1) slice(t.p.elt.ioff, t.p.elt.c, t.p.elt.ics);
+            break;
+        case F_GLOBAL_AVG_POOL:
+        case F_SOFTMAX:
+            out = 1;
+            break;
+        case F_MAX_POOL:
+        case F_AVG_POOL:
+            out = 1;
+            if (arg == 0) slice(t.p.pool.ioff, t.p.pool.c, t.p.pool.ics);
+            if (arg == 1) slice(t.p.pool.ooff, t.p.pool.c, t.p.pool.ocs);
+            break;
+        case F_ATTENTION:
+        case F_ATTENTION_TC:
+            out = s.nargs - 1;
+            break;
+        case F_CONV_SIMT:
+        case F_CONV_TC:
+            out = 2;
+            out2 = t.p.conv.i_out2;
+            if (arg == 0 && !t.p.conv.nchw) slice(t.p.conv.ioff, t.p.conv.ci, t.p.conv.ics);
+            if (arg == 2) slice(t.p.conv.ooff, t.p.conv.co, t.p.conv.ocs);
+            break;
+        default:
+            break;   // the other families write their first argument
+    }
+    u.writes = arg == out || arg == out2;
+    return u;
+}
+
 int plan_kernel(const char* name, KernelSpec* s) {
     int rc = build_spec(name, s);
     if (rc != REEF_SUCC) return rc;

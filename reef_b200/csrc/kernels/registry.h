@@ -44,6 +44,10 @@ void set_error(const std::string& s);
 const char* last_error();
 
 int plan_kernel(const char* name, KernelSpec* out);
+struct ArgUse {
+    int writes, c0, c1, stride;   // channels [c0, c1) of every `stride`, stride 0 = the whole buffer
+};
+ArgUse arg_use(const KernelSpec& s, int arg);
 int launch_plain(const KernelSpec& s, const uint32_t dims[6], uint32_t smem, cudaStream_t st, void** args);
 int launch_be(const KernelSpec& s, const uint32_t dims[6], uint32_t smem, cudaStream_t st, const int* flag,
               int* slot, void** args);

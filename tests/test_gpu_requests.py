@@ -87,3 +87,33 @@ def test_best_effort_segments(tmp_path, kernels):
         s.wait_task(t)
         assert np.array_equal(s.get_output(be), x)
     s.close()
+
+
+@pytest.mark.parametrize("model", ["inception_v3_139", "densenet121_64", "resnet50_64", "bert_tiny"])
+def test_branches_side_by_side(gen, model):
+    """Graphs run the independent branches of a model at the same time: bit for bit what the launches in order give, for
+    the graph of a whole pass and for best-effort segments."""
+    base = gen(model)
+    e = capi.HybridExecutor(0)
+    e.load_model_from_file(base + ".json", base + ".profile.json")
+    e.load_param_from_file(base + ".param")
+    s = capi.REEFScheduler(capi.REEFScheduler.REEF, 0)
+    mid = s.load_model_files(base + ".json", base + ".profile.json", base + ".param")
+    s.bind_model_queue(s.create_queue(capi.REEFScheduler.BestEffortQueue), mid)
+    s.run()
+    name = "input0" if model.startswith("bert") else "data"
+    rng = np.random.default_rng(5)
+    for _ in range(4):
+        n = e.get_data_size(name)
+        x = rng.integers(0, 1000, n // 8) if name == "input0" else rng.normal(0, 1, n // 4).astype(np.float32)
+        e.set_input(name, x)
+        e.execute_to(e.num_kernels())
+        want = e.get_output()
+        e.execute_graph()
+        assert np.array_equal(e.get_output(), want)
+        s.set_input(mid, x, name)
+        s.wait_task(s.new_task(mid))
+        assert np.array_equal(s.get_output(mid), want)
+    assert capi.device_error() == 0
+    s.close()
+    e.close()
