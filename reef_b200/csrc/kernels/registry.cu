@@ -84,6 +84,18 @@ static bool parse_name(const std::string& name, std::string* op, Attrs* attrs) {
 
 static int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+static void plan_conv_simt(KernelSpec* s) {
+    ConvP& p = s->task.p.conv;
+    ConvSimtTile w = conv_simt_tile(p.ptot, p.co, p.ktot);
+    if (!conv_simt_fast(p)) w.tc = 32;   // the element-wise loader's tile
+    p.tile_c = w.tc;
+    p.kgroups = w.kg;
+    p.tiles_p = ceil_div(p.ptot, CTP * 8 / w.kg);
+    p.tiles_c = ceil_div(p.co, w.tc);
+    s->task.nblocks = p.tiles_p * p.tiles_c;
+    s->dyn_smem = kConvSimtSmem;
+}
+
 // Build the device task + launch plan for a name.  Returns REEF_SUCC / REEF_NOT_FOUND.
 static int build_spec(const std::string& name, KernelSpec* s) {
     std::string op;
@@ -296,10 +308,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
             return REEF_SUCC;
         }
         t.family = F_CONV_SIMT;
-        p.tiles_p = ceil_div(p.ptot, CBM);
-        p.tiles_c = ceil_div(p.co, CBN);
-        t.nblocks = p.tiles_p * p.tiles_c;
-        s->dyn_smem = kConvSimtSmem;
+        plan_conv_simt(s);
         return REEF_SUCC;
     }
     // reef_conv2d_add_preact: conv + residual written to `out`, and relu(out + bias2) written to `out2` by the
@@ -352,7 +361,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         p.ptot = p.ho * p.wo;
         if (p.ho <= 0 || p.wo <= 0) goto bad;
         if ((p.co | p.ocs | p.ooff) & 3) goto bad;
-        if (!p.nchw && (p.ci % CBK) == 0 && ((p.ics | p.ioff) & 3)) goto bad;
+        if (!p.nchw && (p.ci % 16) == 0 && ((p.ics | p.ioff) & 3)) goto bad;
         s->nargs = nargs;
         // algorithmic work counts the real input channels (cr: the 3-channel model input is padded to 4)
         const double cr = (double)a.get("cr", p.ci);
@@ -367,10 +376,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         }
         if (impl == 0) {
             t.family = F_CONV_SIMT;
-            p.tiles_p = ceil_div(p.ptot, CBM);
-            p.tiles_c = ceil_div(p.co, CBN);
-            t.nblocks = p.tiles_p * p.tiles_c;
-            s->dyn_smem = kConvSimtSmem;
+            plan_conv_simt(s);
             return REEF_SUCC;
         }
         if (impl == 1) {
@@ -573,7 +579,8 @@ __device__ __forceinline__ bool run_body(const KTask& t, int vb, unsigned char* 
     return true;
 }
 
-__device__ __forceinline__ bool run_any(const KTask& t, int vb, unsigned char* smem, const int* flag) {
+// (not inlined: the dispatcher calls it for either kind, and two copies of every body spilled)
+__device__ __noinline__ bool run_any(const KTask& t, int vb, unsigned char* smem, const int* flag) {
     switch (t.family) {
         case F_MOCK_ADD: return run_body<F_MOCK_ADD>(t, vb, smem, flag);
         case F_MOCK_MUL: return run_body<F_MOCK_MUL>(t, vb, smem, flag);
@@ -622,8 +629,11 @@ __device__ __forceinline__ void preempt_stamp_leave() {
     atomicMax(&w[1], t);
 }
 
+// Two blocks per SM where the body's registers would otherwise leave room for one.
+constexpr int min_blocks(int family) { return family == F_CONV_SIMT ? 2 : 1; }
+
 template <int F>
-__global__ void __launch_bounds__(kThreads) k_plain(const __grid_constant__ KTask t) {
+__global__ void __launch_bounds__(kThreads, min_blocks(F)) k_plain(const __grid_constant__ KTask t) {
     pdl_prologue();
     run_body<F>(t, blockIdx.x, reef_dyn_smem, nullptr);
 }
@@ -632,7 +642,7 @@ __global__ void __launch_bounds__(kThreads) k_plain(const __grid_constant__ KTas
 // the preempt flag is up; bodies poll it again at their loop heads; a block that ran to the end
 // (all of its stores issued, fenced) adds one to the kernel's completion counter.
 template <int F>
-__global__ void __launch_bounds__(kThreads) k_be(const __grid_constant__ KTask t, const int* __restrict__ flag,
+__global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_constant__ KTask t, const int* __restrict__ flag,
                                                  int* __restrict__ task_slot) {
     pdl_prologue();
     // ONE thread reads the flag and the block takes one decision: were every thread to read it for itself, a flag
@@ -667,7 +677,7 @@ __device__ __forceinline__ int next_ticket(int* counter, int* s_slot) {
     return *s_slot;
 }
 
-__global__ void __launch_bounds__(kThreads) k_dispatch(const __grid_constant__ KTask rt, const __grid_constant__ KTask be,
+__global__ void __launch_bounds__(kThreads, 2) k_dispatch(const __grid_constant__ KTask rt, const __grid_constant__ KTask be,
                                                        int be_off, int be_num, int sm_partition,
                                                        int* __restrict__ be_slot, int* __restrict__ ctrl) {
     __shared__ int s_ticket;
@@ -826,10 +836,13 @@ static void prepare_carveout() {
         cudaFuncSetAttribute(be_fn(f), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     }
     cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    // the GEMV's copy ring takes more than the 48 KB a kernel gets without asking (also when the dispatcher hosts it)
+    // the GEMV's and the fp32 convolution's rings take more than the 48 KB a kernel gets without asking (also when the
+    // dispatcher hosts them)
+    cudaFuncSetAttribute(plain_fn(F_CONV_SIMT), cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSimtSmem);
+    cudaFuncSetAttribute(be_fn(F_CONV_SIMT), cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSimtSmem);
     cudaFuncSetAttribute(plain_fn(F_DENSE), cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
     cudaFuncSetAttribute(be_fn(F_DENSE), cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
-    cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
+    cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem > kConvSimtSmem ? kDenseSmem : kConvSimtSmem);
     int* w = nullptr;
     tc_error_word(&w);   // the device error word exists before any launch can be part of a stream capture
     cudaGetLastError();

@@ -48,6 +48,7 @@ struct ConvP {
     int ics, ioff, ocs, ooff, nchw;
     int ktot, ptot;          // K = kh*kw*ci, P = ho*wo
     int tiles_p, tiles_c;    // tile grid: pixels x out-channels
+    int tile_c, kgroups;     // fp32 variant: channels of a warp tile (32 or 16), warps sharing a tile's K
     int ep;                  // EP_* bits
     int i_res, i_bias, i_gamma, i_beta;   // positions in the arg list, -1 when absent
     int round_tf32;          // tensor-core variant: store activations rounded to the nearest TF32 value
