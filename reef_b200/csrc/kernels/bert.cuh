@@ -4,6 +4,7 @@
 // (reference: resource/bert/bert.cu:3-12,159-204,273-395).  Here each is one kernel; the dense projections
 // run on the tensor-core GEMM with bias / GELU / residual fused in its epilogue (conv_tc.cuh).
 #pragma once
+#include "bf16_split.cuh"
 #include "simple.cuh"
 
 namespace reef {
@@ -91,121 +92,254 @@ __device__ __forceinline__ bool body_layernorm(const KTask& t, int vb, unsigned 
 // scores = Q K^T / sqrt(d); mask[j] == 0 -> -inf; row softmax (max-subtracted, online over key chunks);
 // ctx = P V   (reference: bert.cu:22-157 batch_matmul_4/5, :289-311 divide + transposes, :381-387 where,
 // softmax :3-12,159-165,327-336,389-395).  args: qkv, [mask], out.  d == 64.
-// One logical block = one head x 16 query rows (S = 128: 96 blocks); a warp owns 2 rows and works on both at
-// once, so every shared-memory operand feeds two multiply-adds.  Keys/values are staged through shared memory
-// 64 at a time (128-bit global loads); for the scores a lane owns two keys, for P*V two output dimensions.
-constexpr int kAttRows = 16;
-constexpr int kAttChunk = 64;
+// fp32 throughout: both products run on the tensor cores with exactly split operands (bf16_split.cuh), every 16 positions
+// of a sum added to the fp32 result with rounding.  One logical block = one head x 16 query rows; its eight warps divide
+// the keys (a range of whole 16s each) and keep their own running maximum, sum and context, merged at the end in warp
+// order.  A lane's four K positions are consecutive dimensions in the first product; in the second it holds eight
+// consecutive dimensions of four keys, which are its columns of all eight 8-column tiles at once: operands are read with
+// 128-bit loads either way.  The query fragments are split once per block.
+//
+// Two forms.  What bounds a pass that fits the SMs at once (up to 148 blocks) is its latency: keys and values go from L2
+// straight into registers (250 of them, one block per SM), the next loads travelling during either product.  Beyond that
+// what counts is how many warps hide the chains of dependent multiplications behind each other (2 us per 16 keys with one
+// block on an SM): keys and values are staged through shared memory by cp.async and two blocks share an SM.
+// Measured, 12 heads: 128 tokens 8.6 (fp32 instructions) / 7.8 (TF32, tcgen05) -> 5.7 us, 384 tokens 30.9 -> 15.4 us, 512
+// tokens 75 -> 28.8 us; error against fp64 0.3-0.5 of the fp32 instructions'.
+constexpr int kAttChunk = 16;                              // keys a warp takes at a time
 constexpr int kAttD = 64;
-constexpr int kAttSmem = (2 * kAttChunk * (kAttD + 1) + 8 * 2 * kAttD + 8 * 2 * kAttChunk) * 4;   // 41.3 KB
-__device__ __forceinline__ bool body_attention(const KTask& t, int vb, unsigned char* smem_raw, const int* flag) {
+constexpr int kAttRowStride = kAttD + 4;
+constexpr int kAttRows = 16;
+constexpr int kAttMergeBytes = 8 * kAttRows * kAttRowStride * 4;        // contexts of the eight warps
+constexpr int kAttStageBytes = 8 * 3 * kAttChunk * kAttD * 4;           // per warp two key buffers and one of values
+constexpr int kAttFixedBytes = 4 * 3 * 32 * 16 + 2 * 8 * kAttRows * 4;  // query fragments, maxima and sums
+__host__ inline bool att_staged(int s, int heads) { return heads * ((s + kAttRows - 1) / kAttRows) > 148; }
+__host__ inline int att_smem(bool staged) { return kAttFixedBytes + (staged ? kAttStageBytes : kAttMergeBytes); }   // 103 / 41 KB
+// 16-byte chunks of a staged row of keys / values are exchanged so that the eight lanes of a 128-bit load's quarter (two
+// rows x four chunks of keys; four rows x two chunks of values) meet different banks
+__device__ __forceinline__ int att_swz_k(int row) { return (row & 1) << 2; }
+__device__ __forceinline__ int att_swz_v(int row) { return ((row >> 1) & 1) | (((row >> 2) & 1) << 2); }
+template <bool STAGED>
+__device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned char* smem_raw, const int* flag) {
+    constexpr int ROWS = kAttRows;
     const int S = t.p.raw[0], heads = t.p.raw[1], has_mask = t.p.raw[3];
     const int H = heads * kAttD;
     const float* qkv = (const float*)t.a[0];
     const float* mask = has_mask ? (const float*)t.a[1] : nullptr;
     float* out = (float*)t.a[has_mask ? 2 : 1];
-    float* Ks = reinterpret_cast<float*>(smem_raw);            // [64][65]
-    float* Vs = Ks + kAttChunk * (kAttD + 1);                  // [64][65]
-    float* Qs = Vs + kAttChunk * (kAttD + 1);                  // [8 warps][2 rows][64]
-    float* Ps = Qs + 8 * 2 * kAttD;                            // [8 warps][2 rows][64]: probabilities of the rows in work
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rblocks = (S + kAttRows - 1) / kAttRows;
-    const int head = vb / rblocks, r0 = (vb - head * rblocks) * kAttRows + warp * 2;
-    const float scale = rsqrtf((float)kAttD);
+    uint4* Qs = reinterpret_cast<uint4*>(smem_raw);                       // [k step][h, m, l][lane]: A fragments
+    float* ml = reinterpret_cast<float*>(Qs + 4 * 3 * 32);                // [warp][row]: maximum, then [warp][row]: sum
+    float* part = ml + 2 * 8 * ROWS;                                      // [warp][row][dimension], over the stages
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const int rblocks = (S + ROWS - 1) / ROWS;
+    const int head = vb / rblocks, row0 = (vb - head * rblocks) * ROWS;
+    const float scale = 0.125f;                                           // 1 / sqrt(64)
     const float ninf = -__int_as_float(0x7f800000);
-    // this warp's 2 query rows -> shared (read back as 128-bit broadcasts)
-    for (int r = 0; r < 2; r++) {
-        const int row = r0 + r;
-        for (int c = lane; c < kAttD; c += 32)
-            Qs[(warp * 2 + r) * kAttD + c] = row < S ? qkv[(size_t)row * 3 * H + head * kAttD + c] : 0.f;
-    }
-    float m[2], l[2], acc[2][2];
-#pragma unroll
-    for (int r = 0; r < 2; r++) { m[r] = ninf; l[r] = 0.f; acc[r][0] = acc[r][1] = 0.f; }
-
-    for (int k0 = 0; k0 < S; k0 += kAttChunk) {
-        // the barrier says the previous chunk is fully consumed; in the best-effort flavour it also carries the
-        // loop-head poll of the preempt flag (an OR over the block, so that all threads take the same exit)
-        if (flag != nullptr) {
-            if (__syncthreads_or(ld_flag(flag))) return false;
-        } else {
-            __syncthreads();
-        }
-        for (int i = threadIdx.x; i < kAttChunk * (kAttD / 4); i += kThreads) {
-            const int j = i / (kAttD / 4), c = (i - j * (kAttD / 4)) * 4, key = k0 + j;
-            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-            if (key < S) {
-                kv = *reinterpret_cast<const float4*>(qkv + (size_t)key * 3 * H + H + head * kAttD + c);
-                vv = *reinterpret_cast<const float4*>(qkv + (size_t)key * 3 * H + 2 * H + head * kAttD + c);
-            }
-            float* kd = Ks + j * (kAttD + 1) + c;
-            float* vd = Vs + j * (kAttD + 1) + c;
-            kd[0] = kv.x; kd[1] = kv.y; kd[2] = kv.z; kd[3] = kv.w;
-            vd[0] = vv.x; vd[1] = vv.y; vd[2] = vv.z; vd[3] = vv.w;
-        }
-        __syncthreads();
-        // scores of both rows against keys lane and 32 + lane
-        const float4* qa = reinterpret_cast<const float4*>(Qs + (warp * 2 + 0) * kAttD);
-        const float4* qb = reinterpret_cast<const float4*>(Qs + (warp * 2 + 1) * kAttD);
-        const float* ka = Ks + lane * (kAttD + 1);
-        const float* kb = Ks + (32 + lane) * (kAttD + 1);
-        float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f;    // s[row][key group]
-#pragma unroll 4
-        for (int c4 = 0; c4 < kAttD / 4; c4++) {
-            const float4 a = qa[c4], b = qb[c4];
-            const float x0 = ka[4 * c4], x1 = ka[4 * c4 + 1], x2 = ka[4 * c4 + 2], x3 = ka[4 * c4 + 3];
-            const float y0 = kb[4 * c4], y1 = kb[4 * c4 + 1], y2 = kb[4 * c4 + 2], y3 = kb[4 * c4 + 3];
-            s00 = fmaf(a.x, x0, s00); s00 = fmaf(a.y, x1, s00); s00 = fmaf(a.z, x2, s00); s00 = fmaf(a.w, x3, s00);
-            s01 = fmaf(a.x, y0, s01); s01 = fmaf(a.y, y1, s01); s01 = fmaf(a.z, y2, s01); s01 = fmaf(a.w, y3, s01);
-            s10 = fmaf(b.x, x0, s10); s10 = fmaf(b.y, x1, s10); s10 = fmaf(b.z, x2, s10); s10 = fmaf(b.w, x3, s10);
-            s11 = fmaf(b.x, y0, s11); s11 = fmaf(b.y, y1, s11); s11 = fmaf(b.z, y2, s11); s11 = fmaf(b.w, y3, s11);
-        }
-        const bool dead0 = (k0 + lane >= S) || (mask && mask[min(k0 + lane, S - 1)] == 0.f);
-        const bool dead1 = (k0 + 32 + lane >= S) || (mask && mask[min(k0 + 32 + lane, S - 1)] == 0.f);
-        float sc[2][2] = {{dead0 ? ninf : s00 * scale, dead1 ? ninf : s01 * scale},
-                          {dead0 ? ninf : s10 * scale, dead1 ? ninf : s11 * scale}};
-        float corr[2];
-        float* pr = Ps + warp * 2 * kAttChunk;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const float cmax = warp_max(fmaxf(sc[r][0], sc[r][1]));
-            const float mnew = fmaxf(m[r], cmax);
-            corr[r] = (mnew == ninf) ? 1.f : expf(m[r] - mnew);
-            const float p0 = (sc[r][0] == ninf) ? 0.f : expf(sc[r][0] - mnew);
-            const float p1 = (sc[r][1] == ninf) ? 0.f : expf(sc[r][1] - mnew);
-            l[r] = l[r] * corr[r] + warp_sum(p0 + p1);
-            m[r] = mnew;
-            pr[r * kAttChunk + lane] = p0;
-            pr[r * kAttChunk + 32 + lane] = p1;
-        }
-        __syncwarp();
-        float a00 = acc[0][0] * corr[0], a01 = acc[0][1] * corr[0], a10 = acc[1][0] * corr[1], a11 = acc[1][1] * corr[1];
-        const float4* pa = reinterpret_cast<const float4*>(pr);
-        const float4* pb = reinterpret_cast<const float4*>(pr + kAttChunk);
-#pragma unroll 4
-        for (int j4 = 0; j4 < kAttChunk / 4; j4++) {
-            const float4 u = pa[j4], w = pb[j4];
-            const float* v = Vs + (4 * j4) * (kAttD + 1) + lane;
-            const float v00 = v[0], v01 = v[32], v10 = v[kAttD + 1], v11 = v[kAttD + 1 + 32];
-            const float v20 = v[2 * (kAttD + 1)], v21 = v[2 * (kAttD + 1) + 32], v30 = v[3 * (kAttD + 1)], v31 = v[3 * (kAttD + 1) + 32];
-            a00 = fmaf(u.x, v00, a00); a00 = fmaf(u.y, v10, a00); a00 = fmaf(u.z, v20, a00); a00 = fmaf(u.w, v30, a00);
-            a01 = fmaf(u.x, v01, a01); a01 = fmaf(u.y, v11, a01); a01 = fmaf(u.z, v21, a01); a01 = fmaf(u.w, v31, a01);
-            a10 = fmaf(w.x, v00, a10); a10 = fmaf(w.y, v10, a10); a10 = fmaf(w.z, v20, a10); a10 = fmaf(w.w, v30, a10);
-            a11 = fmaf(w.x, v01, a11); a11 = fmaf(w.y, v11, a11); a11 = fmaf(w.z, v21, a11); a11 = fmaf(w.w, v31, a11);
-        }
-        acc[0][0] = a00; acc[0][1] = a01; acc[1][0] = a10; acc[1][1] = a11;
-        __syncwarp();
-    }
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const int row = r0 + r;
-        if (row < S) {
-            const float inv = 1.0f / l[r];
-            out[(size_t)row * H + head * kAttD + lane] = acc[r][0] * inv;
-            out[(size_t)row * H + head * kAttD + 32 + lane] = acc[r][1] * inv;
-        }
+    const float* base = qkv + head * kAttD;
+    __syncthreads();                           // a persistent caller's previous block is out of shared memory
+    if (warp < 4) {
+        const int ks = warp, row = row0 + g;
+        const float4 x = *reinterpret_cast<const float4*>(base + (size_t)min(row, S - 1) * 3 * H + ks * 16 + c * 4);
+        const float4 y = *reinterpret_cast<const float4*>(base + (size_t)min(row + 8, S - 1) * 3 * H + ks * 16 + c * 4);
+        const Bf16Triple a0 = bf16_split(x.x, x.y), a1 = bf16_split(y.x, y.y), a2 = bf16_split(x.z, x.w), a3 = bf16_split(y.z, y.w);
+        Qs[(warp * 3 + 0) * 32 + lane] = make_uint4(a0.h, a1.h, a2.h, a3.h);
+        Qs[(warp * 3 + 1) * 32 + lane] = make_uint4(a0.m, a1.m, a2.m, a3.m);
+        Qs[(warp * 3 + 2) * 32 + lane] = make_uint4(a0.l, a1.l, a2.l, a3.l);
     }
     __syncthreads();
+
+    const int range = ((S + 7) / 8 + 15) / 16 * 16;
+    const int k_begin = warp * range, k_end = min(S, k_begin + range);
+    float m[2] = {ninf, ninf}, l[2] = {0.f, 0.f}, ctx[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++) ctx[j][0] = ctx[j][1] = ctx[j][2] = ctx[j][3] = 0.f;
+    // keys k0 .. k0 + 15 of K: tile j, k step ks; of V: keys 2 c, 2 c + 1, 2 c + 8, 2 c + 9, dimensions 8 g .. 8 g + 7 (keys
+    // beyond the sequence repeat the last one: their probability is zero)
+    float4 kf[2][4];
+    float vf[4][8];
+    auto load_k = [&](int k0) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float* src = base + (size_t)min(k0 + 8 * j + g, S - 1) * 3 * H + H + c * 4;
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) kf[j][ks] = *reinterpret_cast<const float4*>(src + ks * 16);
+        }
+    };
+    // staged form: K buffers 0 and 1, V buffer, 16 rows of 256 bytes each
+    float* mine = part + warp * 3 * kAttChunk * kAttD;
+    const uint32_t mine_s = (uint32_t)__cvta_generic_to_shared(mine);
+    auto stage = [&](int k0, int which, uint32_t dst, bool values) {   // which: 1 keys, 2 values of the token row
+        if (k0 < k_end) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int row = 2 * i + (lane >> 4), chunk = lane & 15;
+                const float* src = base + (size_t)min(k0 + row, S - 1) * 3 * H + which * H + chunk * 4;
+                const uint32_t d = dst + row * 256 + ((chunk ^ (values ? att_swz_v(row) : att_swz_k(row))) << 4);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    bool stopped = false;
+    if (STAGED) {
+        stage(k_begin, 1, mine_s, false);
+        stage(k_begin, 2, mine_s + 8192, true);
+    } else if (k_begin < k_end) {
+        load_k(k_begin);
+    }
+    int buf = 0;
+#pragma unroll 1
+    for (int k0 = k_begin; k0 < k_end; k0 += kAttChunk) {
+        // best-effort flavour: loop-head poll of the preempt flag
+        if (flag != nullptr && __any_sync(0xffffffffu, ld_flag(flag))) {
+            stopped = true;
+            break;
+        }
+        if (STAGED) {
+            stage(k0 + kAttChunk, 1, mine_s + (buf ^ 1) * 4096, false);
+            asm volatile("cp.async.wait_group 2;" ::: "memory");       // this step's keys (behind them: values, next keys)
+            __syncwarp();
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float* src = base + (size_t)min(k0 + 2 * c + (u & 1) + 8 * (u >> 1), S - 1) * 3 * H + 2 * H + 8 * g;
+                *reinterpret_cast<float4*>(&vf[u][0]) = *reinterpret_cast<const float4*>(src);
+                *reinterpret_cast<float4*>(&vf[u][4]) = *reinterpret_cast<const float4*>(src + 4);
+            }
+        }
+        // ---- scores; s[j][e]: row g + 8 (e / 2), key k0 + 8 j + 2 c + e % 2 ----
+        float s[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++) {
+            if (STAGED) {
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    kf[j][ks] = *reinterpret_cast<const float4*>(mine + buf * 1024 + (8 * j + g) * 64 + ((4 * ks + c) ^ att_swz_k(g)) * 4);
+            }
+            const Bf16Triple b0[2] = {bf16_split(kf[0][ks].x, kf[0][ks].y), bf16_split(kf[1][ks].x, kf[1][ks].y)};
+            const Bf16Triple b1[2] = {bf16_split(kf[0][ks].z, kf[0][ks].w), bf16_split(kf[1][ks].z, kf[1][ks].w)};
+            const uint4 qh = Qs[(ks * 3 + 0) * 32 + lane], qm = Qs[(ks * 3 + 1) * 32 + lane], ql = Qs[(ks * 3 + 2) * 32 + lane];
+            const Bf16Triple a[4] = {{qh.x, qm.x, ql.x}, {qh.y, qm.y, ql.y}, {qh.z, qm.z, ql.z}, {qh.w, qm.w, ql.w}};
+            float d[2][4];
+            mma_split(d, a, b0, b1);
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[j][e] += d[j][e];
+        }
+        if (!STAGED) load_k(k0 + kAttChunk);
+        // ---- mask, running maximum, probabilities ----
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int key = k0 + 8 * j + 2 * c + e;
+                const bool dead = key >= k_end || (mask && mask[key] == 0.f);
+                s[j][e] = dead ? ninf : s[j][e] * scale;
+                s[j][2 + e] = dead ? ninf : s[j][2 + e] * scale;
+            }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            float top = fmaxf(fmaxf(s[0][2 * r], s[0][2 * r + 1]), fmaxf(s[1][2 * r], s[1][2 * r + 1]));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            const float mnew = fmaxf(m[r], top);
+            const float corr = mnew == ninf ? 1.f : expf(m[r] - mnew);
+            m[r] = mnew;
+            float add = 0.f;
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 2 * r; e < 2 * r + 2; e++) {
+                    s[j][e] = s[j][e] == ninf ? 0.f : expf(s[j][e] - mnew);
+                    add += s[j][e];
+                }
+            l[r] = l[r] * corr + add;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                ctx[j][2 * r] *= corr;
+                ctx[j][2 * r + 1] *= corr;
+            }
+        }
+        Bf16Triple p[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) p[q] = bf16_split(s[q >> 1][2 * (q & 1)], s[q >> 1][2 * (q & 1) + 1]);
+        // ---- context: column g of tile j = dimension 8 g + j ----
+        if (STAGED) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");       // this step's values
+            __syncwarp();
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < 8; j0 += 4) {
+            if (STAGED) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int row = 2 * c + (u & 1) + 8 * (u >> 1);
+                    *reinterpret_cast<float4*>(&vf[u][j0]) = *reinterpret_cast<const float4*>(mine + 2048 + row * 64 + ((2 * g + j0 / 4) ^ att_swz_v(row)) * 4);
+                }
+            }
+            Bf16Triple b0[4], b1[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                b0[j] = bf16_split(vf[0][j0 + j], vf[1][j0 + j]);
+                b1[j] = bf16_split(vf[2][j0 + j], vf[3][j0 + j]);
+            }
+            float d[4][4];
+            mma_split(d, p, b0, b1);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) ctx[j0 + j][e] += d[j][e];
+        }
+        if (STAGED) {
+            __syncwarp();                                               // every lane has read this step's values
+            stage(k0 + kAttChunk, 2, mine_s + 8192, true);
+            buf ^= 1;
+        }
+    }
+    if (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (__syncthreads_or(stopped)) return false;
+
+    // ---- the eight warps' parts meet: lane (g, c) holds dimensions 16 c .. 16 c + 15 of its rows ----
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        float sum = l[r];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const int row = g + 8 * r;
+        if (c == 0) {
+            ml[warp * ROWS + row] = m[r];
+            ml[(8 + warp) * ROWS + row] = sum;
+        }
+        float* dst = part + (warp * ROWS + row) * kAttRowStride + 16 * c;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                *reinterpret_cast<float4*>(dst + 8 * h + 4 * q) =
+                    make_float4(ctx[4 * q][2 * r + h], ctx[4 * q + 1][2 * r + h], ctx[4 * q + 2][2 * r + h], ctx[4 * q + 3][2 * r + h]);
+    }
+    __syncthreads();
+    const int row = threadIdx.x >> 4, d0 = (threadIdx.x & 15) * 4;
+    float top = ninf;
+#pragma unroll
+    for (int w = 0; w < 8; w++) top = fmaxf(top, ml[w * ROWS + row]);
+    float sum = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {          // fixed order: deterministic
+        const float mw = ml[w * ROWS + row];
+        const float f = mw == ninf ? 0.f : expf(mw - top);
+        sum = fmaf(f, ml[(8 + w) * ROWS + row], sum);
+        const float4 x = *reinterpret_cast<const float4*>(part + (w * ROWS + row) * kAttRowStride + d0);
+        o.x = fmaf(f, x.x, o.x); o.y = fmaf(f, x.y, o.y); o.z = fmaf(f, x.z, o.z); o.w = fmaf(f, x.w, o.w);
+    }
+    if (row0 + row < S) {
+        const float inv = 1.0f / sum;
+        o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+        *reinterpret_cast<float4*>(out + (size_t)(row0 + row) * H + head * kAttD + d0) = o;
+    }
     return true;
 }
 

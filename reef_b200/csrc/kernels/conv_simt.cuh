@@ -11,12 +11,10 @@
 // What bounds it: 128 fp32 multiply-adds per clock and SM fed from shared memory at one word per lane and clock, so that
 // CUDA cores reach their rate only on tiles of 8x8 outputs per thread — and at batch 1 there are far too few of those (a
 // 13x13 layer of 256 channels is 12 tiles of 64x64, which left 136 SMs idle: 133 us; small tiles by fp32 instructions,
-// 20 us).  The products therefore go to the tensor cores without giving up a bit of the operands: an fp32 value is the
-// exact sum of three bf16 values (8 + 8 + 8 significand bits), a product of two values the sum of nine bf16 products, each
-// of them exact in fp32.  Six are computed (mma.sync m16n8k16, fp32 accumulators); the three left out together stay below
-// 2^-26 of |a b|, under half of what one fp32 rounding loses.  Accumulators are fp32: the large products are added up over
-// 32 K positions and then to the running sum with a rounding addition (the tensor core truncates), the small ones in
-// accumulators of their own.  Against fp64 the result is as close as a chain of fp32 fused multiply-adds, or closer.
+// 20 us).  The products therefore go to the tensor cores with exactly split operands (bf16_split.cuh, mma.sync m16n8k16).
+// Accumulators are fp32: the large products are added up over 32 K positions and then to the running sum with a rounding
+// addition (the tensor core truncates), the small ones in accumulators of their own.  Against fp64 the result is as close
+// as a chain of fp32 fused multiply-adds, or closer.
 //
 // Work split: the eight warps of a block share one K loop.  A WARP computes a tile of 16 pixels x 32 or 16 channels over
 // every KG-th K slice, KG = 1, 2, 4 or 8 warps sharing a tile and 8/KG tiles (neighbouring pixels) making a block.  Warps
@@ -26,6 +24,7 @@
 // Measured, 3x3 256 -> 256 at 13x13: 133 -> 13.6 us; 3x3 512 -> 512 at 7x7: 261 -> 18.3 us; ResNet-50 at 193x193, a request:
 // 3.39 -> 0.64 ms.
 #pragma once
+#include "bf16_split.cuh"
 #include "task.cuh"
 
 namespace reef {
@@ -63,27 +62,6 @@ __host__ inline ConvSimtTile conv_simt_tile(int ptot, int co, int ktot) {
 __host__ __device__ inline bool conv_simt_fast(const ConvP& p) {
     return !p.nchw && ((p.ci | p.ics | p.ioff) & 3) == 0 && p.kh <= 31 && p.kw <= 31;
 }
-// x = the exact sum of three bf16 values, two values of x at a time (first in the lower half)
-struct Bf16Triple {
-    uint32_t h, m, l;
-};
-__device__ __forceinline__ Bf16Triple bf16_split(float x, float y) {
-    Bf16Triple r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.h) : "f"(y), "f"(x));
-    x -= __uint_as_float(r.h << 16);
-    y -= __uint_as_float(r.h & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.m) : "f"(y), "f"(x));
-    x -= __uint_as_float(r.m << 16);
-    y -= __uint_as_float(r.m & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.l) : "f"(y), "f"(x));
-    return r;
-}
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // bit t: position first + t lies inside [0, n), for the t < taps <= 31
 __device__ __forceinline__ int taps_inside(int first, int n, int taps) {
     const unsigned below = (1u << max(0, min(taps, n - first))) - 1u, before = (1u << max(0, min(31, -first))) - 1u;

@@ -5,6 +5,7 @@
 // src/reef/executor/hybrid_executor.cpp:153-163, src/reef/server/scheduler.cpp:613-649).
 #include "registry.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -272,7 +273,8 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         }
         t.family = F_ATTENTION;
         t.nblocks = heads * ceil_div(sN, kAttRows);
-        s->dyn_smem = kAttSmem;
+        if (att_staged(sN, heads)) t.family = F_ATTENTION_STAGED;
+        s->dyn_smem = (uint32_t)att_smem(att_staged(sN, heads));
         return REEF_SUCC;
     }
     if (op.rfind("reef_matmul_nt", 0) == 0) {
@@ -468,6 +470,7 @@ static void fill_arg_bytes(KernelSpec* s) {
             break;
         }
         case F_ATTENTION:
+        case F_ATTENTION_STAGED:
         case F_ATTENTION_TC: {
             const double sN = t.p.raw[0], H = (double)t.p.raw[1] * t.p.raw[2];
             int i = 0;
@@ -522,6 +525,7 @@ ArgUse arg_use(const KernelSpec& s, int arg) {
             if (arg == 1) slice(t.p.pool.ooff, t.p.pool.c, t.p.pool.ocs);
             break;
         case F_ATTENTION:
+        case F_ATTENTION_STAGED:
         case F_ATTENTION_TC:
             out = s.nargs - 1;
             break;
@@ -575,7 +579,8 @@ __device__ __forceinline__ bool run_body(const KTask& t, int vb, unsigned char* 
     if (F == F_SOFTMAX) return body_softmax(t, vb, smem, flag);
     if (F == F_EMBEDDING) return body_embedding(t, vb, smem, flag);
     if (F == F_LAYERNORM) return body_layernorm(t, vb, smem, flag);
-    if (F == F_ATTENTION) return body_attention(t, vb, smem, flag);
+    if (F == F_ATTENTION) return attention_rows<false>(t, vb, smem, flag);
+    if (F == F_ATTENTION_STAGED) return attention_rows<true>(t, vb, smem, flag);
     return true;
 }
 
@@ -597,7 +602,8 @@ __device__ __noinline__ bool run_any(const KTask& t, int vb, unsigned char* smem
         case F_SOFTMAX: return run_body<F_SOFTMAX>(t, vb, smem, flag);
         case F_EMBEDDING: return run_body<F_EMBEDDING>(t, vb, smem, flag);
         case F_LAYERNORM: return run_body<F_LAYERNORM>(t, vb, smem, flag);
-        case F_ATTENTION: return run_body<F_ATTENTION>(t, vb, smem, flag);
+        case F_ATTENTION:           // (the staged form for either: the dispatcher has 128 registers; same results bit for bit)
+        case F_ATTENTION_STAGED: return run_body<F_ATTENTION_STAGED>(t, vb, smem, flag);
         default: return true;
     }
 }
@@ -630,7 +636,7 @@ __device__ __forceinline__ void preempt_stamp_leave() {
 }
 
 // Two blocks per SM where the body's registers would otherwise leave room for one.
-constexpr int min_blocks(int family) { return family == F_CONV_SIMT ? 2 : 1; }
+constexpr int min_blocks(int family) { return family == F_CONV_SIMT || family == F_ATTENTION_STAGED ? 2 : 1; }
 
 template <int F>
 __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_plain(const __grid_constant__ KTask t) {
@@ -803,7 +809,7 @@ void add_launches(unsigned long long n) { g_launches.fetch_add(n, std::memory_or
 
 #define FOR_EACH_FAMILY(X)                                                                      \
     X(F_MOCK_ADD) X(F_MOCK_MUL) X(F_FUSED_ADD_NCHW) X(F_BIAS_RELU) X(F_CONV_SIMT) X(F_MAX_POOL) \
-    X(F_AVG_POOL) X(F_GLOBAL_AVG_POOL) X(F_COPY) X(F_DENSE) X(F_SOFTMAX) X(F_EMBEDDING) X(F_LAYERNORM) X(F_ATTENTION) \
+    X(F_AVG_POOL) X(F_GLOBAL_AVG_POOL) X(F_COPY) X(F_DENSE) X(F_SOFTMAX) X(F_EMBEDDING) X(F_LAYERNORM) X(F_ATTENTION) X(F_ATTENTION_STAGED) \
     X(F_NCHW_TO_NHWC4) X(F_IM2COL_NCHW)
 
 static const void* plain_fn(int family) {
@@ -836,13 +842,16 @@ static void prepare_carveout() {
         cudaFuncSetAttribute(be_fn(f), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     }
     cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(plain_fn(F_ATTENTION_STAGED), cudaFuncAttributeMaxDynamicSharedMemorySize, att_smem(true));
+    cudaFuncSetAttribute(be_fn(F_ATTENTION_STAGED), cudaFuncAttributeMaxDynamicSharedMemorySize, att_smem(true));
     // the GEMV's and the fp32 convolution's rings take more than the 48 KB a kernel gets without asking (also when the
     // dispatcher hosts them)
     cudaFuncSetAttribute(plain_fn(F_CONV_SIMT), cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSimtSmem);
     cudaFuncSetAttribute(be_fn(F_CONV_SIMT), cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSimtSmem);
     cudaFuncSetAttribute(plain_fn(F_DENSE), cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
     cudaFuncSetAttribute(be_fn(F_DENSE), cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
-    cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem > kConvSimtSmem ? kDenseSmem : kConvSimtSmem);
+    cudaFuncSetAttribute((const void*)k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         std::max(att_smem(true), std::max(kDenseSmem, kConvSimtSmem)));
     int* w = nullptr;
     tc_error_word(&w);   // the device error word exists before any launch can be part of a stream capture
     cudaGetLastError();
@@ -981,6 +990,9 @@ int launch_be(const KernelSpec& s, const uint32_t dims[6], uint32_t smem, cudaSt
     return check_cuda(e, "cudaLaunchKernel(be)");
 }
 
+// dynamic shared memory of a kernel's blocks inside the dispatcher
+static uint32_t hosted_smem(const KernelSpec& s) { return s.task.family == F_ATTENTION ? (uint32_t)att_smem(true) : s.dyn_smem; }
+
 // One padded step.  Two shapes:
 //  * both kernels are logical-block families and no separate best-effort stream is given: ONE persistent
 //    dispatcher grid on `st` runs the real-time blocks and the best-effort blocks (SM-partitioned);
@@ -1007,13 +1019,13 @@ int launch_dispatch(const KernelSpec* rt, void** rt_args, const KernelSpec* be, 
         uint32_t smem = 0;
         if (rt != nullptr) {
             fill_args(*rt, rt_args, &trt);
-            smem = rt->dyn_smem;
+            smem = hosted_smem(*rt);
         } else {
             memset(&trt, 0, sizeof(trt));   // nblocks = 0: the real-time phase ends at once
         }
         if (be_num > 0) {
             fill_args(*be, be_args, &tbe);
-            if (be->dyn_smem > smem) smem = be->dyn_smem;
+            smem = std::max(smem, hosted_smem(*be));
         } else {
             memset(&tbe, 0, sizeof(tbe));
         }
@@ -1038,7 +1050,7 @@ int launch_dispatch(const KernelSpec* rt, void** rt_args, const KernelSpec* be, 
             int grid = num_sms * occupancy;
             if (grid > trt.nblocks) grid = trt.nblocks;
             void* kargs[] = {&trt, &tbe, &zero, &zero, &part, (void*)&null_slot, (void*)&ctrl};
-            cudaError_t e = cudaLaunchKernel((const void*)k_dispatch, dim3(grid), dim3(kThreads), kargs, rt->dyn_smem, st);
+            cudaError_t e = cudaLaunchKernel((const void*)k_dispatch, dim3(grid), dim3(kThreads), kargs, hosted_smem(*rt), st);
             count_launch();
             rc = check_cuda(e, "cudaLaunchKernel(dispatch rt)");
         }
@@ -1067,7 +1079,7 @@ int launch_dispatch(const KernelSpec* rt, void** rt_args, const KernelSpec* be, 
             return REEF_FAIL;
         }
         void* kargs[] = {&trt, &tbe, &be_off, &be_num, &part, (void*)&be_slot, (void*)&ctrl2};
-        cudaError_t e = cudaLaunchKernel((const void*)k_dispatch, dim3(grid), dim3(kThreads), kargs, be->dyn_smem, bs);
+        cudaError_t e = cudaLaunchKernel((const void*)k_dispatch, dim3(grid), dim3(kThreads), kargs, hosted_smem(*be), bs);
         count_launch();
         return check_cuda(e, "cudaLaunchKernel(dispatch be)");
     }
@@ -1124,13 +1136,13 @@ int launch_dispatch_static(const KernelSpec* rt, void** rt_args, const KernelSpe
     uint32_t smem = 0;
     if (rt != nullptr) {
         fill_args(*rt, rt_args, &trt);
-        smem = rt->dyn_smem;
+        smem = hosted_smem(*rt);
     } else {
         memset(&trt, 0, sizeof(trt));
     }
     if (be_num > 0) {
         fill_args(*be, be_args, &tbe);
-        if (be->dyn_smem > smem) smem = be->dyn_smem;
+        smem = std::max(smem, hosted_smem(*be));
     } else {
         memset(&tbe, 0, sizeof(tbe));
     }

@@ -32,6 +32,7 @@ enum Family : int {
     F_EMBEDDING,
     F_LAYERNORM,
     F_ATTENTION,
+    F_ATTENTION_STAGED,
     F_NCHW_TO_NHWC4,
     F_IM2COL_NCHW,
     F_COUNT,

@@ -80,8 +80,11 @@ def build_bert(*, name: str = "bert_base", layers: int = 12, hidden: int = 768, 
     for li in range(layers):
         att_attrs = dict(s=seq, heads=heads, d=hidden // heads)
         att_tc = False
-        if conv_impl != "simt":
-            try:   # both attention products on the tensor cores where the registry has the shape (<= 128 tokens)
+        # The exact-fp32 attention is the faster one while its blocks (16 query rows of a head each) fit the 148 SMs at once
+        # (12 heads of 128 tokens: 5.7 us against 7.8 us); with more heads than that the TF32 kernel's single block per
+        # head is, where the registry has the shape (<= 128 tokens).
+        if conv_impl != "simt" and heads * (-(-seq // 16)) > 148:
+            try:
                 capi.kernel_plan(kname("reef_attention", **att_attrs, v=1))
                 att_attrs["v"] = 1
                 att_tc = True
