@@ -3,7 +3,7 @@
 // GEMM view (implicit, no im2col buffer):  D[co][pixel] = sum_k W[co][k] * X[pixel][k]
 //   A = weights  OHWI = [Cout][kh*kw*Cin]  : K-major, M = Cout  -> TMEM lanes (128 per tile)
 //   B = activations NHWC                    : K-major per filter tap, N = pixels -> TMEM columns
-// Both operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a 4-stage shared-memory
+// Both operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a shared-memory
 // ring; a K block is 32 channels of one filter tap = one 128-byte row per pixel / per output channel.
 // Zero padding, ragged tiles and strides are folded into the tensor maps (out-of-bounds boxes read
 // zeros; a stride-s conv uses up to s*s maps over the s-strided sub-lattices of the input).
@@ -15,9 +15,13 @@
 // distributed shared memory in rank order 0..S-1 — a fixed order, so results are bit-reproducible (no
 // float atomics, no global scratch, no counters to reset when a best-effort run is preempted and re-run).
 //
-// One thread issues TMA, one thread issues tcgen05.mma, all eight warps run the epilogue
-// (tcgen05.ld -> +residual -> +bias | *gamma+beta -> ReLU -> coalesced 128-byte stores, one output
-// channel per lane).  Every mbarrier wait is bounded: on expiry the kernel records an error word,
+// One warp issues TMA, one warp issues tcgen05.mma, all eight warps run the epilogue
+// (tcgen05.ld -> +residual -> +bias | *gamma+beta -> ReLU -> coalesced 512-byte rows, four output
+// channels per lane).  What bounds it: a launch of a few microseconds is a chain of latencies (hand-over from
+// the previous grid 1.7 us, first K block 0.3 us, cluster barrier 0.6 us, rows 1 us) around a main loop that
+// takes about 57 bytes a clock into an SM.  Issue by whole warps and the remote-load epilogue took the replay
+// of ResNet-152 from 827 to 760 us, Inception-v3's from 377 to 338 us, BERT's (128 tokens) from 593 to 560 us.
+// Every mbarrier wait is bounded: on expiry the kernel records an error word,
 // skips further waits, still joins every cluster barrier, frees its TMEM and returns.
 #pragma once
 #include <cuda.h>
@@ -34,10 +38,12 @@ enum : int { TC_EP_RES = 1, TC_EP_BIAS = 2, TC_EP_GB = 4, TC_EP_RELU = 8, TC_EP_
 
 // Branch-free form of (+residual) (+bias | *gamma+beta) (ReLU): r = 0, sc = 1, sh = 0, lo = -inf stand in for
 // the absent terms (v + 0 and fma(v, 1, b) are exact, so this equals the conditional form bit for bit).
-// exact-erf GELU (reference: resource/bert/bert.cu:167-173).  Not inlined on purpose: inlined, the compiler turned
+// exact-erf GELU (reference: resource/bert/bert.cu:167-173).  Not inlined here on purpose: inlined, the compiler turned
 // the uniform `if (gelu)` of the epilogue into straight-line code and every layer paid for erff on each element
-// (0.5 us per launch on the row-finishing loop).
-static __device__ __noinline__ float tc_gelu(float v) { return v * (0.5f * erff(v * 0.70710678118654752440f) + 0.5f); }
+// (0.5 us per launch on the row-finishing loop).  Where a whole loop is for GELU layers (tc_finish_rows) it is inlined:
+// the calls made BERT's 768 -> 3072 matmul at 384 tokens spend 8 us on finishing its rows.
+__device__ __forceinline__ float tc_gelu_inline(float v) { return v * (0.5f * erff(v * 0.70710678118654752440f) + 0.5f); }
+static __device__ __noinline__ float tc_gelu(float v) { return tc_gelu_inline(v); }
 
 __device__ __forceinline__ float tc_epilogue(float v, float r, float sc, float sh, float lo, bool rnd, bool gelu = false) {
     if (gelu) {
@@ -54,6 +60,15 @@ __device__ __forceinline__ float tc_epilogue(float v, float r, float sc, float s
         v = __uint_as_float(u);
     }
     return v;
+}
+
+__device__ __forceinline__ float4 tc_round4(float4 o) {
+    uint32_t u;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.x)); o.x = __uint_as_float(u);
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.y)); o.y = __uint_as_float(u);
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.z)); o.z = __uint_as_float(u);
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.w)); o.w = __uint_as_float(u);
+    return o;
 }
 
 // the same on the 4 channels of a lane at once: one uniform branch per pixel row instead of one per element
@@ -100,16 +115,65 @@ __device__ __forceinline__ void tc_stamp(const TcParams& P, int slot) {
 __device__ __forceinline__ void tc_stamp(const TcParams&, int) {}
 #endif
 
+// Finishes the pixel rows [jb, je) this CTA owns: row jb + i of the accumulator is summed over the staged tiles of the
+// cluster's ranks 0..S-1 in rank order (a fixed order: bit-reproducible), read from distributed shared memory; then the
+// epilogue, and a 512-byte row is stored.  A warp takes every 8th row and RB of them at a time, RB * SMAX 128-bit loads per
+// lane in flight (16: the kernel is built for two CTAs per SM, so a thread has 128 registers).
+template <int RB, int SMAX, bool GELU>
+__device__ __forceinline__ void tc_finish_rows(const TcParams& P, uint32_t stage, int S, int jb, int je, int warp, int cbase, int co, int pix0,
+                                               float4 sc, float4 sh, float lo, bool rnd, bool has_res, float4 b2, const float4* rpre) {
+    uint32_t src[SMAX];
+#pragma unroll
+    for (int q = 0; q < SMAX; q++) {
+        const uint32_t own = stage + (uint32_t)(jb * TC_BM + cbase) * 4u;
+        src[q] = SMAX == 1 ? own : mapa_shared(own, (uint32_t)(q < S ? q : 0));
+    }
+    for (int jbase = warp; jbase < je - jb; jbase += 8 * RB) {
+        float4 part[RB][SMAX], rv[RB];
+#pragma unroll
+        for (int u = 0; u < RB; u++) {
+            const int jr = jbase + 8 * u;   // row within this CTA's share
+            rv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (jr < je - jb) {
+#pragma unroll
+                for (int q = 0; q < SMAX; q++)
+                    if (q < S) part[u][q] = SMAX == 1 ? ld_smem_v4(src[q] + (uint32_t)jr * TC_BM * 4u) : ld_dsmem_v4(src[q] + (uint32_t)jr * TC_BM * 4u);
+                if (has_res) rv[u] = (u < 2 && jbase == warp) ? rpre[u & 1] : ld_activation(P.res + (size_t)(pix0 + jb + jr) * P.co + co);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < RB; u++) {
+            const int jr = jbase + 8 * u;
+            if (jr < je - jb) {
+                float4 v = part[u][0];
+#pragma unroll
+                for (int q = 1; q < SMAX; q++)   // fixed rank order: deterministic sum
+                    if (q < S) { v.x += part[u][q].x; v.y += part[u][q].y; v.z += part[u][q].z; v.w += part[u][q].w; }
+                float4 o;
+                if (GELU) {
+                    o.x = tc_gelu_inline(v.x + sh.x) + rv[u].x; o.y = tc_gelu_inline(v.y + sh.y) + rv[u].y;
+                    o.z = tc_gelu_inline(v.z + sh.z) + rv[u].z; o.w = tc_gelu_inline(v.w + sh.w) + rv[u].w;
+                    if (rnd) o = tc_round4(o);
+                } else {
+                    o = tc_epilogue4(v, rv[u], sc, sh, lo, rnd, false);
+                }
+                *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + jb + jr) * P.ocs + P.ooff + co) = o;
+                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.co + co) = tc_preact(o, b2, rnd);
+            }
+        }
+    }
+}
+
 // Finishes the pixel rows [jb, je) a cluster rank owns after a K split: sums the partials of ranks 0..S-1 in
 // rank order (a fixed order: bit-reproducible), applies the epilogue and stores 512-byte rows.  RB rows per warp
 // are in flight at a time, RB * SMAX 128-bit loads per lane (16: the kernel is built for two CTAs per SM, so
 // a thread has 128 registers).
-// CG: the residual was written earlier in the SAME launch (persistent chain kernel): it is read at L2 (ld.global.cg),
-// never through the non-coherent path, and there is no early prefetch.
-template <int RB, int SMAX, bool CG = false>
+// The persistent chain kernel's form (partials already in this CTA's shared memory).  The residual was written earlier in
+// the SAME launch: it is read at L2 (ld.global.cg), never through the non-coherent path.
+template <int RB, int SMAX>
 __device__ __forceinline__ void tc_finish_split(const TcParams& P, const float* stage, const float* recv, int S, int split,
                                                 int jb, int je, int warp, int cbase, int co, int pix0, float4 sc, float4 sh,
-                                                float lo, bool rnd, bool gelu, bool has_res, float4 b2, const float4* rpre) {
+                                                float lo, bool rnd, bool gelu, bool has_res, float4 b2) {
     const float* src[SMAX];
 #pragma unroll
     for (int q = 0; q < SMAX; q++)
@@ -125,11 +189,7 @@ __device__ __forceinline__ void tc_finish_split(const TcParams& P, const float* 
 #pragma unroll
                 for (int q = 0; q < SMAX; q++)
                     if (q < S) part[u][q] = *reinterpret_cast<const float4*>(src[q] + (size_t)jr * TC_BM);
-                if (has_res) {
-                    const float4* rp = reinterpret_cast<const float4*>(P.res + (size_t)(pix0 + jb + jr) * P.co + co);
-                    if (CG) rv[u] = __ldcg(rp);
-                    else rv[u] = (u < 2 && jbase == warp) ? rpre[u & 1] : __ldg(rp);
-                }
+                if (has_res) rv[u] = __ldcg(reinterpret_cast<const float4*>(P.res + (size_t)(pix0 + jb + jr) * P.co + co));
             }
         }
 #pragma unroll
@@ -166,12 +226,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     const uint32_t ctrl = base + (uint32_t)P.region_bytes;
     const int NS = P.stages;   // ring depth of this launch (<= TC_MAX_STAGES)
     const uint32_t bar_full = ctrl, bar_empty = ctrl + 8 * TC_MAX_STAGES, bar_acc = ctrl + 16 * TC_MAX_STAGES;
-    const uint32_t bar_red = bar_acc + 8;
     volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + P.region_bytes + 16 * TC_MAX_STAGES + 16);
     volatile uint32_t* s_flags = s_tmem + 1;    // [0] abort (preempt flag seen by this CTA), [1] wait expired,
                                                 //  [2] K blocks whose loads were issued when the producer stopped
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be warp-uniform)
     // best-effort flavour: the poll at block entry is issued first, so that its latency hides behind the set-up
     int flag0 = 0;
     if (BE && tid == 0) flag0 = *reinterpret_cast<const volatile int*>(P.preempt_flag);
@@ -191,7 +251,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_acc, 1);
-        mbar_init(bar_red, 1);
         s_flags[0] = (uint32_t)(flag0 != 0);
         s_flags[1] = 0;
         s_flags[2] = 0;
@@ -212,59 +271,58 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     const uint32_t tmem = *s_tmem;
     if (tid == 0) tc_stamp(P, 1);   // set-up done (barriers, TMEM)
 
-    // K-split exchange barrier: armed now, so that peers may send as soon as their own tile is staged.  The
-    // cluster barrier below (cheap here: all CTAs of a cluster start together, and it overlaps the first loads'
-    // latency) guarantees every peer's barrier is initialised and armed before any remote completion.
     // spatial tiles: tile_n -> (row group ty, row piece tx); tx > 0 only where a row is wider than a tile
     const int tile_y = P.xsplit > 1 ? tile_n / P.xsplit : tile_n, tile_x = P.xsplit > 1 ? tile_n - tile_y * P.xsplit : 0;
     const int pix0 = P.spatial ? tile_y * P.rows * P.wo + tile_x * P.xw : tile_n * P.n_valid;
     const int n_lim = min(P.n_valid, P.ptot - pix0);   // columns of this tile that are real pixels
     const int cpc = (n_lim + S - 1) / S;               // pixel rows one rank finishes
     const int jb = min(split * cpc, n_lim), je = min(jb + cpc, n_lim);
-    if (S > 1 && tid == 0) mbar_expect_tx(bar_red, (uint32_t)((S - 1) * (je - jb) * TC_BM * 4));
     // best-effort flavour: what this CTA saw at entry.  Nothing is loaded then; the cluster agrees at its first barrier.
     const bool abort0 = BE && s_flags[0] != 0;
 
     {
         const int m0 = tile_m * TC_BM;
         // ---------------- TMA producer, part 1: fill the ring (no waits) ----------------
+        // Warp 0 refills the ring and warp 1 issues the multiplications as whole warps: control flow, addresses and
+        // descriptors are warp-uniform (uniform registers), one elected lane executes each instruction.  As code of a
+        // single thread every instruction had its operands moved into uniform registers first: 540 cycles per K block in
+        // the multiplication loop, whatever the tile's width.
         const uint32_t tx = TC_A_BYTES + (uint32_t)P.b_bytes;
         const int first = nkb < NS ? nkb : NS;
-        // tap and channel block of a K block (2^32/1 does not fit the magic: one channel block per tap is a copy)
-        auto tap_of = [&](int kb) { return P.cblocks == 1 ? kb : (int)__umulhi((unsigned)kb, P.cb_magic); };
-        auto load_a = [&](int i, int s) {   // weights: 32 channels of one tap for this tile's 128 output channels
-            const int kb = kb_begin + i, tap = tap_of(kb), cb = kb - tap * P.cblocks;
-            tma_load_3d(base + s * stage_bytes, &P.tm_w, bar_full + 8 * s, cb * TC_BK, tap, m0);
+        // filter tap and channel block of the next K block to refill, carried along (2^32 / 1 does not fit the magic: one
+        // channel block per tap is a copy)
+        int tap = P.cblocks == 1 ? kb_begin + first : (int)__umulhi((unsigned)(kb_begin + first), P.cb_magic);
+        int cb = kb_begin + first - tap * P.cblocks;
+        auto next_kb = [&]() {
+            if (++cb == P.cblocks) { cb = 0; tap++; }
         };
-        auto load_b = [&](int i, int s) {
-            const uint32_t st = base + s * stage_bytes;
-            const int kb = kb_begin + i;
+        // weights: 32 channels of one tap for this tile's 128 output channels
+        auto load_a = [&](int s) { tma_load_3d(base + s * stage_bytes, &P.tm_w, bar_full + 8 * s, cb * TC_BK, tap, m0); };
+        auto load_b = [&](int s) {
+            const uint32_t dst = base + s * stage_bytes + TC_A_BYTES;
             // the per-tap sub-lattice and offsets come from a host table
-            const int tap = tap_of(kb), cb = kb - tap * P.cblocks;
             if (P.spatial) {
-                tma_load_3d(st + TC_A_BYTES, &P.tm_x[P.tap_map[tap]], bar_full + 8 * s, cb * TC_BK,
-                            tile_x * P.xw + P.tap_qx[tap], tile_y * P.rows + P.tap_qy[tap]);
+                tma_load_3d(dst, &P.tm_x[P.tap_map[tap]], bar_full + 8 * s, cb * TC_BK, tile_x * P.xw + P.tap_qx[tap],
+                            tile_y * P.rows + P.tap_qy[tap]);
             } else {
-                tma_load_2d(st + TC_A_BYTES, &P.tm_x[0], bar_full + 8 * s, cb * TC_BK, tile_n * P.n_valid);
+                tma_load_2d(dst, &P.tm_x[0], bar_full + 8 * s, cb * TC_BK, tile_n * P.n_valid);
             }
         };
         if (warp == 0) {
-            // one lane per stage: issuing a load costs a few hundred cycles of address arithmetic and
-            // descriptor traffic, so the ring is filled by up to eight lanes at once.  Weights do not depend
-            // on the previous kernel: they are requested before the dependency wait, activations after it.
-            // coordinates of this lane's activation load: worked out before the dependency wait, so that after it
-            // only the copy instruction itself is left on the critical path
+            // The first loads: one lane per stage.  Weights do not depend on the previous kernel and are requested before
+            // the dependency wait, activations after it, their coordinates worked out before it, so that only the copy
+            // instruction itself is left on the critical path (30 cycles a lane; 90 with the coordinates in line).
             const CUtensorMap* bmap = &P.tm_x[0];
             int bc0 = 0, bc1 = tile_n * P.n_valid, bc2 = 0;
             if (lane < first && !abort0) {
+                const int kb = kb_begin + lane, t = P.cblocks == 1 ? kb : (int)__umulhi((unsigned)kb, P.cb_magic);
+                bc0 = (kb - t * P.cblocks) * TC_BK;
                 mbar_expect_tx(bar_full + 8 * lane, tx);
-                load_a(lane, lane);
-                const int kb = kb_begin + lane, tap = tap_of(kb);
-                bc0 = (kb - tap * P.cblocks) * TC_BK;
+                tma_load_3d(base + lane * stage_bytes, &P.tm_w, bar_full + 8 * lane, bc0, t, m0);
                 if (P.spatial) {
-                    bmap = &P.tm_x[P.tap_map[tap]];
-                    bc1 = tile_x * P.xw + P.tap_qx[tap];
-                    bc2 = tile_y * P.rows + P.tap_qy[tap];
+                    bmap = &P.tm_x[P.tap_map[t]];
+                    bc1 = tile_x * P.xw + P.tap_qx[t];
+                    bc2 = tile_y * P.rows + P.tap_qy[t];
                 }
             }
             asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -278,6 +336,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 if (P.spatial) tma_load_3d(bdst, bmap, bar_full + 8 * lane, bc0, bc1, bc2);
                 else tma_load_2d(bdst, bmap, bar_full + 8 * lane, bc0, bc1);
             }
+            __syncwarp();
             if (lane == 0) tc_stamp(P, 2);   // ring filled (loads issued)
         }
         __syncwarp();
@@ -303,10 +362,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         const bool rnd = (P.ep & TC_EP_ROUND) != 0;
         const bool gelu = (P.ep & TC_EP_GELU) != 0;
 
-        if (warp == 0 && lane == 0) {
+        if (warp == 0) {
             // ---------------- TMA producer, part 2: refill stages as the MMAs release them ----------------
             // (stage index and phase parity are carried along: a division by the runtime ring depth per K block
-            // is dozens of cycles on this single thread's critical path)
+            // is dozens of cycles on this critical path)
             bool ok = true;
             int s = first == NS ? 0 : first;      // first < NS only when nkb < NS, and then this loop does not run
             uint32_t par = 0;                      // parity of the "empty" phase awaited: ((i / NS) - 1) & 1
@@ -316,76 +375,85 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // running one is resident early (programmatic dependent launch) and made its entry poll long before its
             // predecessor finished, possibly before the flag went up.  Its first loads are out (their barriers were
             // armed for both operands, so the activation loads had to follow the weight loads); it issues no more, and
-            // the MMA thread only waits for those to land.
-            if (BE && !stop && *reinterpret_cast<const volatile int*>(P.preempt_flag) != 0) stop = true;
+            // the MMA warp only waits for those to land.
+            if (BE && !stop) stop = __any_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(P.preempt_flag) != 0);
             for (int i = first; i < nkb && ok && !stop; i++) {
                 // loop-head poll of the preempt flag (every 4th K block): the load is issued before the wait for a
                 // free stage and looked at after it, so its latency hides behind the wait
                 int f = 0;
                 if (BE && (i & 3) == 0) f = *reinterpret_cast<const volatile int*>(P.preempt_flag);
-                ok = mbar_wait(bar_empty + 8 * s, par);
+                ok = mbar_wait_warp(bar_empty + 8 * s, par);
                 if (!ok) break;
-                if (BE && f != 0) { stop = true; break; }
-                mbar_expect_tx(bar_full + 8 * s, tx);
-                load_a(i, s);
-                load_b(i, s);
+                if (BE && __any_sync(0xffffffffu, f != 0)) { stop = true; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(bar_full + 8 * s, tx);
+                    load_a(s);
+                    load_b(s);
+                }
+                next_kb();
                 issued++;
                 if (++s == NS) { s = 0; par ^= 1u; }
             }
-            if (BE && stop) {
+            if (BE && stop && lane == 0) {
                 s_flags[2] = (uint32_t)issued;     // first how far the loads got, then the request to stop
                 __threadfence_block();
                 s_flags[0] = 1;
             }
-            if (!ok) s_flags[1] = 1;
-        } else if (warp == 1 && lane == 0) {
+            if (!ok && lane == 0) s_flags[1] = 1;
+        } else if (warp == 1) {
             // ---------------- MMA issuer ----------------
-            bool ok = true;
+            bool ok = true, halted = false;
             const uint32_t idesc = umma_idesc_tf32(P.n_mma);
 #ifdef REEF_DEBUG_AIDS
-            const bool tr = P.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
+            const bool tr = lane == 0 && P.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
 #endif
             int s = 0;
             uint32_t par = 0;
-            for (int i = 0; i < nkb && ok; i++) {
-                const uint32_t st = base + s * stage_bytes;
+            uint64_t da = umma_desc_sw128(base);
+            for (int i = 0; i < nkb; i++) {
                 if (BE) {
-                    const int w = mbar_wait_abortable(bar_full + 8 * s, par, &s_flags[0]);
+                    const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0]);
                     if (w == 2) {
                         // The producer stopped.  Loads it had issued may still be in flight: they must have landed
                         // before this CTA leaves or reuses its shared memory, so their barriers are awaited (bounded)
                         // without multiplying.
                         __threadfence_block();
-                        const int issued = (int)s_flags[2];
+                        const int issued = __shfl_sync(0xffffffffu, (int)s_flags[2], 0);
                         for (; i < issued && ok; i++) {
-                            ok = mbar_wait(bar_full + 8 * s, par);
+                            ok = mbar_wait_warp(bar_full + 8 * s, par);
                             if (++s == NS) { s = 0; par ^= 1u; }
                         }
+                        halted = true;
                         break;
                     }
                     ok = w == 0;
                 } else {
-                    ok = mbar_wait(bar_full + 8 * s, par);
+                    ok = mbar_wait_warp(bar_full + 8 * s, par);
                 }
                 if (!ok) break;
 #ifdef REEF_DEBUG_AIDS
                 if (tr && i == 0) P.trace[4] = clock64();          // first K block landed
                 if (tr && i == nkb - 1) P.trace[5] = clock64();    // last K block landed
 #endif
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t da = umma_desc_sw128(st), db = umma_desc_sw128(st + TC_A_BYTES);
-                // one tcgen05.mma covers K = 8 tf32 = 32 bytes.  (Skipping the steps of a ragged last channel block
-                // that hold only zero fill was tried: the extra branch in this loop cost every launch 1.3 %.)
+                const uint64_t db = da + (uint64_t)(TC_A_BYTES >> 4);
+                // one tcgen05.mma covers K = 8 tf32 = 32 bytes
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < TC_BK / 8; k++)
-                    umma_tf32(tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(bar_empty + 8 * s);   // frees the stage once these MMAs have read it
-                if (++s == NS) { s = 0; par ^= 1u; }
+                    for (int k = 0; k < TC_BK / 8; k++)
+                        umma_tf32(tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    if (i + NS < nkb) umma_commit(bar_empty + 8 * s);   // frees the stage, where it is refilled, once these MMAs have read it
+                    if (i == nkb - 1) umma_commit(bar_acc);
+                }
+                __syncwarp();
+                da += (uint64_t)(stage_bytes >> 4);
+                if (++s == NS) { s = 0; par ^= 1u; da = umma_desc_sw128(base); }
             }
-            if (ok) umma_commit(bar_acc);
-            else s_flags[1] = 1;
+            // stopped early: the accumulator barrier completes when the multiplications issued so far have
+            if (BE && halted && ok && elect_one()) umma_commit(bar_acc);
+            __syncwarp();
+            if (!ok && lane == 0) s_flags[1] = 1;
         }
-        __syncwarp();   // lanes 1..31 of the two role warps park here instead of spinning beside their lane 0
+        __syncwarp();
         if (warp != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
         // the first two residual rows of this warp's pass over its pixel rows (rows jb + warp + 8u): requested now, used
         // after the exchange
@@ -395,7 +463,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             rpre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
             const int jr = warp + 8 * u;
             if (has_res && cvalid && jr < je - jb)
-                rpre[u] = __ldg(reinterpret_cast<const float4*>(P.res + (size_t)(pix0 + jb + jr) * P.co + co));
+                rpre[u] = ld_activation(P.res + (size_t)(pix0 + jb + jr) * P.co + co);
         }
 
         // ---------------- epilogue: all eight warps ----------------
@@ -403,64 +471,50 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         __syncthreads();
         if (tid == 0) tc_stamp(P, 6);   // accumulator complete
-        // cluster barrier #1 (arrive here, wait after staging): every rank has finished its main loop, so its
-        // stage ring is free to receive exchange data
-        // (best-effort flavour: with release semantics, the peers read this CTA's abort word behind the barrier)
-        const bool my_abort = BE && s_flags[0] != 0;   // final: producer and MMA thread are past their loops
-        if (S > 1) {
-            // (best-effort flavour: with release semantics, the peers read this CTA's abort word behind the barrier.
-            // Nothing may be written into a peer's shared memory before this barrier: only behind it is every CTA
-            // of the cluster known to have started.)
-            if (BE) cluster_arrive();
-            else cluster_arrive_relaxed();
-        }
+        const bool my_abort = BE && s_flags[0] != 0;   // final: producer and MMA warp are past their loops
         if (!ok || s_flags[1]) {
             ok = false;
             if (tid == 0 && P.error_word) *reinterpret_cast<volatile int*>(P.error_word) = 1;
         }
-        // Phase A — eight warps move the accumulator tile TMEM -> registers -> shared memory as
-        // stage[pixel][channel] (warp w reads TMEM lanes 32*(w%4).., its hardware quadrant, and the column
-        // chunks of parity w/4).  The stage ring is free by now and is reused for this.
-        // Phase B — the tile is finished pixel row by pixel row with 128-bit accesses: one warp per pixel,
-        // a lane owns 4 consecutive output channels; it sums the K-split partials of all cluster ranks in
-        // rank order 0..S-1 through distributed shared memory (S = 1: its own tile), adds the residual,
-        // applies bias | gamma,beta and ReLU, and stores one coalesced 512-byte row per warp.
+        // Phase A — eight warps move the accumulator tile TMEM -> registers -> shared memory as stage[pixel][channel]
+        // (warp w reads TMEM lanes 32*(w%4).., its hardware quadrant, and every other 16 columns, by w/4).  The stage ring
+        // is free by now and is reused for this.
+        // Phase B — the tile is finished pixel row by pixel row with 128-bit accesses: one warp per pixel, a lane owns 4
+        // consecutive output channels.  With a K split, rank q finishes rows [q*cpc, (q+1)*cpc) and reads every rank's
+        // partial of them from its shared memory; 128-bit remote loads, 16 in flight per lane, take half the time of a
+        // bulk copy per peer into a receive area (1800 cycles from its issue to the owner's barrier).
         const int quad = warp & 3, half = warp >> 2;
         const int row = quad * 32 + lane;              // TMEM lane == output channel within the tile
         const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
         float* stage = reinterpret_cast<float*>(smem);
         if (ok && !my_abort) {
-            for (int j0 = half * 32; j0 < n_lim; j0 += 64) {
+            for (int j0 = half * 16; j0 < n_lim; j0 += 64) {
                 uint32_t r[32];
-                tmem_ld32_nowait(taddr + j0, r);
+                tmem_ld16_nowait(taddr + j0, r);
+                if (j0 + 32 < n_lim) tmem_ld16_nowait(taddr + j0 + 32, r + 16);
                 tmem_ld_wait();
                 float* dst = stage + j0 * TC_BM + row;
-                if (j0 + 32 <= n_lim) {   // a full chunk: no per-column test
 #pragma unroll
-                    for (int j = 0; j < 32; j++) dst[j * TC_BM] = __uint_as_float(r[j]);
-                } else {
+                for (int j = 0; j < 16; j++)
+                    if (j0 + j < n_lim) dst[j * TC_BM] = __uint_as_float(r[j]);
+                if (j0 + 32 < n_lim) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (j0 + j < n_lim) dst[j * TC_BM] = __uint_as_float(r[j]);
+                    for (int j = 0; j < 16; j++)
+                        if (j0 + 32 + j < n_lim) dst[(32 + j) * TC_BM] = __uint_as_float(r[16 + j]);
                 }
             }
         }
         if (tid == 0) tc_stamp(P, 7);   // accumulator tile staged in shared memory
-        // K-split exchange: rank q finishes pixel rows [q*cpc, (q+1)*cpc).  Every rank sends the rows owned
-        // by each peer with ONE bulk shared-memory-to-shared-memory copy per peer (the copy engine moves the
-        // bytes and completes the owner's mbarrier); remote loads from distributed shared memory proved an
-        // order of magnitude slower here.  Owners then read only their own shared memory.
-        float* recv = stage + P.recv_offset_floats;    // recv[slot][cpc_max][128]; sender q uses slot q - (q > owner)
         // The accumulator is out of tensor memory once every warp has passed the barrier below, so the allocating
         // warp frees it there and not at the very end: nothing is then left to do between a CTA's last store and
         // its exit, which is what the next kernel of the stream waits for.
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         bool abort_all = my_abort;
         if (S > 1) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // staged tile -> visible to the copy engine
-            __syncthreads();      // the whole tile is staged
+            // cluster barrier #1: every rank's tile is staged.  (Nothing is written into a peer's shared memory, and a
+            // peer's is not read before this barrier: only behind it is every CTA of the cluster known to have started.)
+            cluster_sync_all();
             if (warp == 1) tmem_free(tmem, (uint32_t)P.tmem_cols);
-            cluster_wait();       // barrier #1: all peers are past their main loops (and their barriers are armed)
             if (tid == 0) tc_stamp(P, 3);
             if (BE) {
                 // every rank learns whether ANY rank of the cluster stopped for the preempt flag: one thread per rank
@@ -470,70 +524,26 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(f) : "r"(mapa_shared(smem_u32((const void*)&s_flags[0]), (uint32_t)tid)) : "memory");
                 abort_all = __syncthreads_or((int)f) != 0;
             }
-            if (!abort_all) {
-                if (tid < S && tid != split) {   // one thread per peer: the copies are issued side by side
-                    const int q = tid;
-                    const int qb = min(q * cpc, n_lim), qe = min(qb + cpc, n_lim);
-                    const uint32_t bytes = (uint32_t)((qe - qb) * TC_BM * 4);
-                    if (bytes != 0) {
-                        const int slot = split < q ? split : split - 1;   // the owner keeps no slot for itself
-                        const uint32_t dst = mapa_shared(smem_u32(recv + (size_t)slot * P.cpc_max * TC_BM), (uint32_t)q);
-                        const uint32_t rbar = mapa_shared(bar_red, (uint32_t)q);
-                        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                     ::"r"(dst), "r"(smem_u32(stage + (size_t)qb * TC_BM)), "r"(bytes), "r"(rbar)
-                                     : "memory");
-                    }
-                }
-                if (!mbar_wait(bar_red, 0)) {
-                    ok = false;
-                    if (tid == 0 && P.error_word) *reinterpret_cast<volatile int*>(P.error_word) = 1;
-                }
-            }
-            // cluster barrier #2 (arrive here, wait before leaving): once all ranks have received what they are
-            // owed (and, best-effort flavour, have read each other's abort words), nobody reads a peer's shared
-            // memory any more and every CTA may exit
-            cluster_arrive();
         } else {
             __syncthreads();
             if (warp == 1) tmem_free(tmem, (uint32_t)P.tmem_cols);
         }
-
-        if (tid == 0) tc_stamp(P, 8);   // exchange complete
-        // Four pixel rows per warp are in flight at a time (all partial and residual loads issued before the
-        // first use): with one or two warps per scheduler the loop is latency-bound, not bandwidth-bound.
+        if (tid == 0) tc_stamp(P, 8);
         if (ok && cvalid && !abort_all) {
-            constexpr int RB = 4;
-            if (S == 1) {
-                for (int jbase = jb + warp; jbase < je; jbase += 8 * RB) {
-                    float4 v[RB], rv[RB];
-#pragma unroll
-                    for (int u = 0; u < RB; u++) {
-                        const int j = jbase + 8 * u;
-                        rv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (j < je) {
-                            v[u] = *reinterpret_cast<const float4*>(stage + j * TC_BM + cbase);
-                            if (has_res) rv[u] = (u < 2 && jbase == jb + warp) ? rpre[u & 1] : __ldg(reinterpret_cast<const float4*>(P.res + (size_t)(pix0 + j) * P.co + co));
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < RB; u++) {
-                        const int j = jbase + 8 * u;
-                        if (j < je) {
-                            const float4 o = tc_epilogue4(v[u], rv[u], sc, sh, lo, rnd, gelu);
-                            *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + j) * P.ocs + P.ooff + co) = o;
-                            if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + j) * P.co + co) = tc_preact(o, b2, rnd);
-                        }
-                    }
-                }
-            } else {
-                // partial of rank q for row j: own rows come from the staged tile, the others from recv[q]
-                if (S <= 4)
-                    tc_finish_split<4, 4>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, gelu, has_res, b2, rpre);
-                else
-                    tc_finish_split<2, TC_MAX_SPLITS>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd,
-                                                      gelu, has_res, b2, rpre);
-            }
+            const uint32_t st = smem_u32(stage);
+#define TC_FINISH(RB, SMAX)                                                                                                            \
+    do {                                                                                                                               \
+        if (gelu) tc_finish_rows<RB, SMAX, true>(P, st, S, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, has_res, b2, rpre);         \
+        else tc_finish_rows<RB, SMAX, false>(P, st, S, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, has_res, b2, rpre);             \
+    } while (0)
+            if (S == 1) TC_FINISH(4, 1);
+            else if (S == 2) TC_FINISH(4, 2);
+            else if (S <= 4) TC_FINISH(4, 4);
+            else TC_FINISH(2, TC_MAX_SPLITS);
+#undef TC_FINISH
         }
+        // cluster barrier #2: nobody reads a peer's shared memory any more, every CTA may exit
+        if (S > 1) cluster_arrive_relaxed();
         if (S > 1) cluster_wait();      // barrier #2
         if (tid == 0) tc_stamp(P, 9);   // rows finished
         if (BE && abort_all && tid == 0 && P.stamps != nullptr) {

@@ -363,10 +363,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_chain_kernel(const
                         }
                     }
                 } else if (S <= 4) {
-                    tc_finish_split<4, 4, true>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, gelu, has_res, b2, nullptr);
+                    tc_finish_split<4, 4>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, gelu, has_res, b2);
                 } else {
-                    tc_finish_split<2, TC_MAX_SPLITS, true>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, gelu,
-                                                            has_res, b2, nullptr);
+                    tc_finish_split<2, TC_MAX_SPLITS>(P, stage, recv, S, split, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, gelu,
+                                                            has_res, b2);
                 }
             }
             // this CTA's rows of layer L are in global memory: publish (every thread orders its own stores first)

@@ -137,7 +137,7 @@ __device__ __forceinline__ bool body_im2col_nchw(const KTask& t, int vb, unsigne
             const int off = s_off[k], dyx = s_dyx[k];
             const int iy = y0 + (dyx >> 16), ix = x0 + (dyx & 0xffff);
             float x = 0.f;
-            if (off >= 0 && iy >= 0 && iy < p.hi && ix >= 0 && ix < p.wi) x = __ldg(in + base + off) + s_bias[k];
+            if (off >= 0 && iy >= 0 && iy < p.hi && ix >= 0 && ix < p.wi) x = in[base + off] + s_bias[k];
             uint32_t u;
             asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
             v[e] = __uint_as_float(u);
@@ -426,7 +426,7 @@ __device__ __forceinline__ bool body_dense(const KTask& t, int vb, unsigned char
 #pragma unroll
                 for (int j = 0; j < kDenseVec; j++) {       // requested before the wait
                     xv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if ((tid + j * kThreads) * 4 < kc) xv[j] = __ldg(reinterpret_cast<const float4*>(x + k0) + tid + j * kThreads);
+                    if ((tid + j * kThreads) * 4 < kc) xv[j] = *(reinterpret_cast<const float4*>(x + k0) + tid + j * kThreads);
                 }
                 if (flag != nullptr) {
                     const int w = dense_mbar_wait_abortable(bar_full + 8 * s, par, ctl, st);

@@ -71,6 +71,64 @@ __device__ __forceinline__ int mbar_wait_abortable(uint32_t bar, uint32_t parity
     }
     return 1;
 }
+// The waits of a whole warp: every lane polls, the warp leaves together (the votes keep its control flow, and with it the
+// addresses and descriptors of what it issues next, warp-uniform).
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+    unsigned long long t0 = 0;
+    for (int i = 0; i < (1 << 26); i++) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+        if ((i & 255) == 255) {   // give up after one second of wall time
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return false;
+        }
+    }
+    return false;
+}
+// 0 = phase complete, 1 = wait expired, 2 = `abort_word` became non-zero (see mbar_wait_abortable)
+__device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word) {
+    unsigned long long t0 = 0;
+    for (int i = 0; i < (1 << 26); i++) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return 0;
+        if (__any_sync(0xffffffffu, *abort_word != 0)) return 2;
+        if ((i & 255) == 255) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return 1;
+        }
+    }
+    return 1;
+}
+// Activations of an earlier kernel: a volatile load stays behind griddepcontrol.wait.  (__ldg promises memory that never
+// changes, and the compiler did move such loads above the wait.)
+__device__ __forceinline__ float4 ld_activation(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -113,6 +171,11 @@ __device__ __forceinline__ float4 ld_dsmem_v4(uint32_t addr) {
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ float4 ld_smem_v4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ void st_dsmem_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
@@ -151,6 +214,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
 // 32 columns of one TMEM lane per thread; the wait is separate so that several loads can be in flight
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
     asm volatile(
