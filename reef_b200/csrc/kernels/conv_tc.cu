@@ -1,6 +1,7 @@
 // Host side of the tcgen05 convolution: tile/split planning, TMA tensor maps, cluster launch.
 #include "conv_tc.cuh"
 
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -12,29 +13,28 @@ namespace reef {
 static int ceil_div_i(int a, int b) { return (a + b - 1) / b; }
 
 // ---- planning (needs no GPU) --------------------------------------------------------------------
-// One candidate plan: pixel tiles of at most `cap` pixels.
-static int tc_plan_cap(const ConvP& p, int cap, TcPlan* pl) {
+// One candidate plan: pixel tiles of at most `cap` pixels, K split over `want` ranks (0: the default of a name that fixes
+// only its tile cap).
+static int tc_plan_cap(const ConvP& p, int cap, int want, TcPlan* pl) {
     memset(pl, 0, sizeof(*pl));
     pl->spatial = (p.kh * p.kw > 1 || p.sh > 1 || p.ph || p.pw) ? 1 : 0;
     pl->xsplit = 1;
     pl->xw = p.wo;
     if (pl->spatial && p.wo > cap) {
-        // rows wider than a tile: cut every row into xsplit equal pieces
-        int xs = ceil_div_i(p.wo, cap);
-        while (xs <= p.wo && p.wo % xs != 0) xs++;
-        if (xs > p.wo || p.wo / xs < 8) return REEF_NOT_FOUND;
-        pl->xsplit = xs;
-        pl->xw = p.wo / xs;
+        // rows wider than a tile: every row is cut into pieces of about the same width, the last one ragged
+        pl->xw = ceil_div_i(p.wo, ceil_div_i(p.wo, cap));
+        if (pl->xw < 8) return REEF_NOT_FOUND;
+        pl->xsplit = ceil_div_i(p.wo, pl->xw);
         pl->rows = 1;
         pl->n_valid = pl->xw;
-        pl->n_tiles = p.ho * xs;
+        pl->n_tiles = p.ho * pl->xsplit;
     } else if (pl->spatial) {
         int best = 1;
         const int rmax = cap / p.wo;
         const int lim = rmax < p.ho ? rmax : p.ho;
         for (int r = 1; r <= lim; r++)
             if (p.ho % r == 0) best = r;               // largest divisor of Ho that fits the tile
-        if (best * 2 <= lim) best = lim;               // no useful divisor: ragged last tile
+        if (best * 2 <= lim) best = ceil_div_i(p.ho, ceil_div_i(p.ho, lim));   // no useful divisor: ragged last tile
         pl->rows = best;
         pl->n_valid = best * p.wo;
         pl->n_tiles = ceil_div_i(p.ho, best);
@@ -51,11 +51,11 @@ static int tc_plan_cap(const ConvP& p, int cap, TcPlan* pl) {
     pl->m_tiles = ceil_div_i(p.co, TC_BM);
     pl->cblocks = ceil_div_i(p.ci, TC_BK);   // a ragged last channel block reads zeros beyond Cin (TMA out-of-bounds fill)
     pl->kb_total = p.kh * p.kw * pl->cblocks;
-    // split K over a cluster until about 128 CTAs are in flight, keeping >= 2 K blocks per CTA
+    // default: split K over a cluster until about 128 CTAs are in flight, keeping >= 2 K blocks per CTA
     const int base = pl->m_tiles * pl->n_tiles;
     int s = 1;
-    if (p.plan_splits > 0) {
-        while (s < p.plan_splits && s < TC_MAX_SPLITS && pl->kb_total >= s * 2) s *= 2;
+    if (want > 0) {
+        while (s < want && s < TC_MAX_SPLITS && pl->kb_total >= s * 2) s *= 2;
     } else {
         while (s < TC_MAX_SPLITS && base * s * 2 <= 128 && pl->kb_total >= 2 * (s * 2)) s *= 2;
     }
@@ -86,13 +86,34 @@ static int tc_plan_cap(const ConvP& p, int cap, TcPlan* pl) {
     return REEF_SUCC;
 }
 
-// ---- planning (needs no GPU) --------------------------------------------------------------------
-// Default plan (names without a tuned plan): tile caps are tried from large to small; the first plan that fits
-// shared memory and puts at least 48 CTAs in flight wins, else the feasible plan with the most CTAs.  A batch-1
-// layer is bound by what one SM can pull from L2 (about 85 GB/s per CTA measured): more CTAs shorten every
-// CTA's load stream, at the price of re-reading weights from L2; where the balance lies depends on the shape
-// (ResNet's 14x14 layers are fastest at 112-128 CTAs, BERT's 128-token matmuls at 48-96), so the resource
-// generator writes measured plans into the kernel names (tp = tile cap, ts = K splits; reef_b200/tune.py).
+// Estimated SM cycles of one launch under a plan, up to a constant.  A batch-1 layer is a short chain of latencies beside
+// a load stream, so neither the fewest bytes nor the most CTAs is right for every shape:
+//   * the main loop is the slowest of: the multiplications of a rank's K blocks; all CTAs' bytes at what L2 delivers
+//     (7000 B/clk, weights re-read by every pixel tile); the layer's weights, cold in HBM, at what the loads in flight
+//     sustain (720 B/clk).  Where two are close they add up (a 4-norm);
+//   * a turn of the ring costs a memory round trip, so a deep ring of small tiles gains;
+//   * staging the accumulator, the cluster's barrier and remote reads, the residual and GELU rows of a rank, and a second
+//     CTA on an SM (it delays the early start of the next kernel) each take their share.
+// The constants were fitted on a B200, for the choice rather than the time: first to 4400 launches timed by themselves (471
+// layers of ResNet, Inception, VGG, DenseNet and BERT at odd and even sizes, weights cold: on layers left out of the fit the
+// choice is within 3 % of the best of the ~10 candidates, where the largest tiles that put 48 CTAs in flight lost 9 %), then
+// to 7200 replays of 20 whole models under different plans, where the weights of the next layer already load beside this one.
+static float tc_plan_cycles(const ConvP& p, const TcPlan& c) {
+    auto pow4 = [](float x) { return x * x * x * x; };
+    const float kb = (float)c.kb_per_split, bytes = TC_A_BYTES + 128.f * c.n_valid;
+    const float ctas = (float)c.splits * c.n_tiles * c.m_tiles;
+    const float weights = 4.f * p.co * p.ci * p.kh * p.kw;
+    const float row_turns = (float)ceil_div_i(c.cpc_max, 8);   // turns of eight warps, a pixel row each
+    float t = sqrtf(sqrtf(pow4(kb * 75.f) + pow4(ctas * kb * bytes / 7000.f) + pow4(weights / 720.f)));
+    t += 760.f * kb / c.stages + 25.f * c.n_valid + ctas;
+    if (c.splits > 1) t += 450.f + 38.f * c.splits;
+    if (p.ep & EP_RES) t += 300.f * row_turns;
+    if (p.ep & EP_GELU) t += 300.f * row_turns;
+    return t + 1570.f * (ceil_div_i((int)ctas, 148) - 1);
+}
+
+// The plan of a layer: of the tile caps and K splits that fit, the one with the least estimated time.  A kernel name can fix
+// a measured plan instead (tp = tile cap, ts = K splits, written by the resource generator; reef_b200/tune.py).
 int tc_plan(const ConvP& p, TcPlan* pl) {
     if (p.nchw || (p.ci & 3) || p.ci < 4 || p.sh != p.sw || (p.sh != 1 && p.sh != 2)) return REEF_NOT_FOUND;
     if ((p.ics & 3) || (p.ioff & 3) || (p.ocs & 3) || (p.ooff & 3) || (p.co & 3)) return REEF_NOT_FOUND;
@@ -100,25 +121,24 @@ int tc_plan(const ConvP& p, TcPlan* pl) {
     if (p.plan_cap > 0) {
         // tile cap fixed by the kernel name (a tuned plan): that candidate or nothing
         if (p.plan_cap < 8 || p.plan_cap > 208) return REEF_NOT_FOUND;
-        return tc_plan_cap(p, p.plan_cap, pl);
+        return tc_plan_cap(p, p.plan_cap, p.plan_splits, pl);
     }
-    static const int caps[] = {208, 160, 112, 96, 64, 48, 32};
     TcPlan best;
-    int best_ctas = 0;
-    for (int cap : caps) {
-        TcPlan c;
-        if (tc_plan_cap(p, cap, &c) != REEF_SUCC) continue;
-        const int ctas = c.splits * c.n_tiles * c.m_tiles;
-        if (ctas > best_ctas && ctas <= 148) {
-            best = c;
-            best_ctas = ctas;
-        } else if (best_ctas == 0) {
-            best = c;
-            best_ctas = ctas;
+    float best_cycles = 0.f;
+    for (int cap : {208, 160, 128, 112, 96, 80, 64, 48, 32, 24, 16})
+        for (int want = 1; want <= TC_MAX_SPLITS; want *= 2) {
+            const int fixed = p.plan_splits;   // a name may fix the splits alone: as many of them as K allows
+            if (fixed > 0 && want > 1) break;
+            TcPlan c;
+            if (tc_plan_cap(p, cap, fixed > 0 ? fixed : want, &c) != REEF_SUCC) continue;
+            if (fixed == 0 && c.splits != want) continue;
+            const float cycles = tc_plan_cycles(p, c);
+            if (best_cycles == 0.f || cycles < best_cycles) {
+                best = c;
+                best_cycles = cycles;
+            }
         }
-        if (best_ctas >= 48) break;
-    }
-    if (best_ctas == 0) return REEF_NOT_FOUND;
+    if (best_cycles == 0.f) return REEF_NOT_FOUND;
     *pl = best;
     return REEF_SUCC;
 }

@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     // spatial tiles: tile_n -> (row group ty, row piece tx); tx > 0 only where a row is wider than a tile
     const int tile_y = P.xsplit > 1 ? tile_n / P.xsplit : tile_n, tile_x = P.xsplit > 1 ? tile_n - tile_y * P.xsplit : 0;
     const int pix0 = P.spatial ? tile_y * P.rows * P.wo + tile_x * P.xw : tile_n * P.n_valid;
-    const int n_lim = min(P.n_valid, P.ptot - pix0);   // columns of this tile that are real pixels
+    // columns of this tile that are real pixels
+    const int n_lim = P.xsplit > 1 ? min(P.xw, P.wo - tile_x * P.xw) : min(P.n_valid, P.ptot - pix0);
     const int cpc = (n_lim + S - 1) / S;               // pixel rows one rank finishes
     const int jb = min(split * cpc, n_lim), je = min(jb + cpc, n_lim);
     // best-effort flavour: what this CTA saw at entry.  Nothing is loaded then; the cluster agrees at its first barrier.

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_chain_kernel(const
             const int nkb = valid ? kb_end - kb_begin : 0;
             const int tile_y = P.xsplit > 1 ? tile_n / P.xsplit : tile_n, tile_x = P.xsplit > 1 ? tile_n - tile_y * P.xsplit : 0;
             const int pix0 = P.spatial ? tile_y * P.rows * P.wo + tile_x * P.xw : tile_n * P.n_valid;
-            const int n_lim = valid ? min(P.n_valid, P.ptot - pix0) : 0;
+            const int n_lim = !valid ? 0 : P.xsplit > 1 ? min(P.xw, P.wo - tile_x * P.xw) : min(P.n_valid, P.ptot - pix0);
             const int cpc = (n_lim + S - 1) / S;
             const int jb = min(split * cpc, n_lim), je = min(jb + cpc, n_lim);
             if (S > 1 && valid && tid == 0) mbar_expect_tx(bar_red, (uint32_t)((S - 1) * (je - jb) * TC_BM * 4));

@@ -34,7 +34,7 @@ struct TcParams {
     int ocs, ooff;
     int spatial;             // 0: flat [P][C] view, tile = n_valid consecutive pixels; 1: tile = rows x Wo
     int wo, rows;            // spatial: output width, rows per tile
-    int xsplit, xw;          // spatial: a row is cut into xsplit tiles of xw pixels (rows == 1), else xsplit == 1
+    int xsplit, xw;          // spatial: a row is cut into xsplit tiles of xw pixels (rows == 1, the last one ragged), else xsplit == 1
     int n_valid;             // pixels per tile
     int n_mma;               // UMMA N (multiple of 16, >= n_valid)
     int tmem_cols;           // power of two >= n_mma
