@@ -155,8 +155,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         if (p.ho < 1 || p.wo < 1 || (p.ocs & 3) || p.ocs < p.ktot || p.ocs > kIm2colMaxKp || (double)p.ptot * p.ocs > 5e8) goto bad;
         p.nchw = 1;
         t.family = F_IM2COL_NCHW;
-        s->dyn_smem = (uint32_t)(p.ocs * 12);
-        t.nblocks = ceil_div(p.ptot * (p.ocs / 4), kIm2colPerBlock);
+        t.nblocks = ceil_div(p.ptot, im2col_pixels_per_block(p.ocs));
         s->nargs = 3;
         s->bytes = 4.0 * ((double)p.ci * p.hi * p.wi + (double)p.ptot * p.ocs + p.ci);
         return REEF_SUCC;
