@@ -640,6 +640,7 @@ constexpr int min_blocks(int family) { return family == F_CONV_SIMT || family ==
 template <int F>
 __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_plain(const __grid_constant__ KTask t) {
     if (F == F_LAYERNORM) prefetch_layernorm(t);
+    if (F == F_DENSE) prefetch_dense(t, blockIdx.x);
     pdl_prologue();
     run_body<F>(t, blockIdx.x, reef_dyn_smem, nullptr);
 }
@@ -651,6 +652,7 @@ template <int F>
 __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_constant__ KTask t, const int* __restrict__ flag,
                                                  int* __restrict__ task_slot) {
     if (F == F_LAYERNORM) prefetch_layernorm(t);
+    if (F == F_DENSE) prefetch_dense(t, blockIdx.x);
     pdl_prologue();
     // ONE thread reads the flag and the block takes one decision: were every thread to read it for itself, a flag
     // that goes up between the reads of two warps would let part of a block leave and the rest run the body with
