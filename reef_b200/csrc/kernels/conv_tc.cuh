@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         }
         if (P.task_slot != nullptr && ok && !abort_all) {
             __syncthreads();
-            if (tid == 0) red_release_gpu_add(P.task_slot, 1);
+            if (tid == 0) red_relaxed_gpu_add(P.task_slot, 1);
         }
     }
 

@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_plain(const __grid_
 
 // Best-effort flavour (reference wrapper: script/best_effort_kernel.py:22-33): leave at once when
 // the preempt flag is up; bodies poll it again at their loop heads; a block that ran to the end
-// (all of its stores issued, fenced) adds one to the kernel's completion counter.
+// (all of its stores issued) adds one to the kernel's completion counter.
 template <int F>
 __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_constant__ KTask t, const int* __restrict__ flag,
                                                  int* __restrict__ task_slot) {
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_con
     const int stopped = __syncthreads_or(done ? 0 : 1);
     if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
         if (!stopped) {
-            red_release_gpu_add(task_slot, 1);
+            red_relaxed_gpu_add(task_slot, 1);
         } else {
             preempt_stamp_leave();
         }
