@@ -109,8 +109,17 @@ def run_kernel(name: str, bufs: list, acc64: bool = False) -> None:
         # kh*kw*c and where a tap falls into the padding
         bufs[0][:] = im2col_nchw(bufs[1], bufs[2], a).reshape(-1)
     elif op == "fused_add_nn_relu":
-        L.reef_oracle_fused_add_nn_relu(_p(bufs[0]), _p(bufs[1]), _p(bufs[2]), i32(a["c"]), i32(a["n"]),
-                                        i32(a.get("ics", a["c"])), i32(a.get("ioff", 0)))
+        c, n, ocs, ooff = a["c"], a["n"], a.get("ocs", a["c"]), a.get("ooff", 0)
+        out = bufs[0] if ocs == c else np.empty(c * n, np.float32)
+        L.reef_oracle_fused_add_nn_relu(_p(out), _p(bufs[1]), _p(bufs[2]), i32(c), i32(n), i32(a.get("ics", c)), i32(a.get("ioff", 0)))
+        if ocs != c:
+            bufs[0][:n * ocs].reshape(n, ocs)[:, ooff:ooff + c] = out.reshape(n, c)
+    elif op == "reef_conv2d_preact":
+        # the same without a residual, both outputs channel slices: bufs = in, weight, out, bias2, out2
+        run_kernel("fused_nn_conv2d__" + name.split("__", 1)[1], bufs[:3], acc64)
+        co, ptot = a["co"], ((a["hi"] + 2 * a["ph"] - a["kh"]) // a["sh"] + 1) * ((a["wi"] + 2 * a["pw"] - a["kw"]) // a["sw"] + 1)
+        ocs, pcs, poff = a.get("ocs", co), a.get("pcs", co), a.get("poff", 0)
+        run_kernel(f"fused_add_nn_relu__c{co}_n{ptot}_ics{ocs}_ioff{a.get('ooff', 0)}_ocs{pcs}_ooff{poff}", [bufs[4], bufs[2], bufs[3]], acc64)
     elif op == "reef_conv2d_add_preact":
         # one launch in the product; here the two reference kernels it stands for, one after the other
         # (fused_nn_conv2d_add, then fused_add_nn_relu of the next unit): bufs = in, weight, out, residual, bias2, out2

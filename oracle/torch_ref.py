@@ -107,9 +107,10 @@ class TorchExecutor:
 
             def f():
                 x = t[args[1]].view(a["n"], ics)[:, ioff:ioff + a["c"]]
-                t[args[0]][:] = torch.relu(x + t[args[2]][None, :]).reshape(-1)
+                o = a.get("ooff", 0)
+                t[args[0]].view(a["n"], -1)[:, o:o + a["c"]] = torch.relu(x + t[args[2]][None, :])
             return f
-        if op.startswith("fused_nn_conv2d") or op == "reef_conv2d_add_preact":
+        if op.startswith("fused_nn_conv2d") or op in ("reef_conv2d_add_preact", "reef_conv2d_preact"):
             return self._conv(op, a, args)
         if op in ("fused_nn_max_pool2d", "fused_nn_max_pool2d_add_nn_relu", "fused_nn_avg_pool2d"):
             c, hi, wi = a["c"], a["hi"], a["wi"]
@@ -202,7 +203,7 @@ class TorchExecutor:
 
     def _conv(self, op, a, args):
         t = self.t
-        tail = "_add" if op == "reef_conv2d_add_preact" else op[len("fused_nn_conv2d"):]
+        tail = {"reef_conv2d_add_preact": "_add", "reef_conv2d_preact": ""}.get(op, op[len("fused_nn_conv2d"):])
         relu = tail.endswith("_nn_relu")
         if relu:
             tail = tail[:-8]
@@ -232,6 +233,9 @@ class TorchExecutor:
             t[args[2]].view(-1, ocs)[:, ooff:ooff + co] = y2
             if op == "reef_conv2d_add_preact":   # second output: the next unit's pre-activation
                 t[args[5]][:] = torch.relu(y2 + t[args[4]][None, :]).reshape(-1)
+            elif op == "reef_conv2d_preact":
+                o = a.get("poff", 0)
+                t[args[4]].view(y2.shape[0], -1)[:, o:o + co] = torch.relu(y2 + t[args[3]][None, :])
         return f
 
 

@@ -252,6 +252,7 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
     P->beta = (p.ep & EP_GB) ? (const float*)a[p.i_beta] : nullptr;
     P->out2 = (p.ep & EP_DUAL) ? (float*)a[p.i_out2] : nullptr;
     P->bias2 = (p.ep & EP_DUAL) ? (const float*)a[p.i_bias2] : nullptr;
+    P->pcs = p.pcs; P->poff = p.poff;
     rc = tc_error_word(&P->error_word);
     if (rc != REEF_SUCC) return rc;
     P->co = p.co; P->ci = p.ci; P->ptot = p.ptot; P->ocs = p.ocs; P->ooff = p.ooff;

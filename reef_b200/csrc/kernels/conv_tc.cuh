@@ -158,7 +158,7 @@ __device__ __forceinline__ void tc_finish_rows(const TcParams& P, uint32_t stage
                     o = tc_epilogue4(v, rv[u], sc, sh, lo, rnd, false);
                 }
                 *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + jb + jr) * P.ocs + P.ooff + co) = o;
-                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.co + co) = tc_preact(o, b2, rnd);
+                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.pcs + P.poff + co) = tc_preact(o, b2, rnd);
             }
         }
     }
@@ -202,7 +202,7 @@ __device__ __forceinline__ void tc_finish_split(const TcParams& P, const float* 
                     if (q < S) { v.x += part[u][q].x; v.y += part[u][q].y; v.z += part[u][q].z; v.w += part[u][q].w; }
                 const float4 o = tc_epilogue4(v, rv[u], sc, sh, lo, rnd, gelu);
                 *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + jb + jr) * P.ocs + P.ooff + co) = o;
-                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.co + co) = tc_preact(o, b2, rnd);
+                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.pcs + P.poff + co) = tc_preact(o, b2, rnd);
             }
         }
     }

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_chain_kernel(const
                             if (j < je) {
                                 const float4 o = tc_epilogue4(v[u], rv[u], sc, sh, lo, rnd, gelu);
                                 *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + j) * P.ocs + P.ooff + co) = o;
-                                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + j) * P.co + co) = tc_preact(o, b2, rnd);
+                                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + j) * P.pcs + P.poff + co) = tc_preact(o, b2, rnd);
                             }
                         }
                     }

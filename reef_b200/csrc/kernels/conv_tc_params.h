@@ -23,7 +23,7 @@ struct TcParams {
     const float* bias;
     const float* gamma;
     const float* beta;
-    float* out2;             // second output [P][Cout] = relu(out + bias2), else nullptr
+    float* out2;             // second output = relu(out + bias2), channel stride pcs, offset poff; else nullptr
     const float* bias2;
     const int* preempt_flag; // best-effort flavour, else nullptr
     int* task_slot;
@@ -31,7 +31,7 @@ struct TcParams {
     long long* trace;        // optional: 16 SM-clock stamps of block (0,0) (phase trace), else nullptr
     unsigned long long* stamps;   // optional: {first flag observation, last leave} in %globaltimer ns, else nullptr
     int co, ci, ptot;
-    int ocs, ooff;
+    int ocs, ooff, pcs, poff;
     int spatial;             // 0: flat [P][C] view, tile = n_valid consecutive pixels; 1: tile = rows x Wo
     int wo, rows;            // spatial: output width, rows per tile
     int xsplit, xw;          // spatial: a row is cut into xsplit tiles of xw pixels (rows == 1, the last one ragged), else xsplit == 1

@@ -165,7 +165,9 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         if (!a.need("c", &p.c) || !a.need("n", &p.n)) goto bad;
         p.ics = (int)a.get("ics", p.c);
         p.ioff = (int)a.get("ioff", 0);
-        if ((p.c | p.ics | p.ioff) & 3) goto bad;
+        p.ocs = (int)a.get("ocs", p.c);
+        p.ooff = (int)a.get("ooff", 0);
+        if ((p.c | p.ics | p.ioff | p.ocs | p.ooff) & 3) goto bad;
         t.family = F_BIAS_RELU;
         t.nblocks = ceil_div(p.c * p.n, kEltPerBlock);
         s->nargs = 3;
@@ -315,10 +317,12 @@ static int build_spec(const std::string& name, KernelSpec* s) {
     // reef_conv2d_add_preact: conv + residual written to `out`, and relu(out + bias2) written to `out2` by the
     // same epilogue: the reference's fused_nn_conv2d_add followed by the next unit's fused_add_nn_relu
     // (resource/resnet152/resnet152.cu:340-363 and :2-12) in one launch.  args: in, weight, out, residual, bias2, out2.
-    if (op == "reef_conv2d_add_preact" || op.rfind("fused_nn_conv2d", 0) == 0) {
-        const bool preact = op == "reef_conv2d_add_preact";
+    // reef_conv2d_preact: the same without a residual, both outputs channel slices (DenseNet).  args: in, weight, out, bias2,
+    // out2; pcs / poff = channel stride and offset of out2.
+    if (op == "reef_conv2d_add_preact" || op == "reef_conv2d_preact" || op.rfind("fused_nn_conv2d", 0) == 0) {
+        const bool preact = op.rfind("reef_", 0) == 0, with_res = op == "reef_conv2d_add_preact";
         ConvP& p = t.p.conv;
-        std::string tail = preact ? std::string("_add") : op.substr(strlen("fused_nn_conv2d"));
+        std::string tail = preact ? std::string(with_res ? "_add" : "") : op.substr(strlen("fused_nn_conv2d"));
         p.ep = 0;
         p.i_res = p.i_bias = p.i_gamma = p.i_beta = p.i_bias2 = p.i_out2 = -1;
         bool relu = false;
@@ -345,9 +349,8 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         if (relu) p.ep |= EP_RELU;
         if (preact) {
             p.ep |= EP_DUAL;
-            p.i_bias2 = 4;
-            p.i_out2 = 5;
-            nargs = 6;
+            p.i_bias2 = nargs++;
+            p.i_out2 = nargs++;
         }
         if (!a.need("ci", &p.ci) || !a.need("hi", &p.hi) || !a.need("wi", &p.wi) || !a.need("co", &p.co) ||
             !a.need("kh", &p.kh) || !a.need("kw", &p.kw) || !a.need("sh", &p.sh) || !a.need("sw", &p.sw) ||
@@ -356,12 +359,13 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         p.nchw = (int)a.get("nchw", 0);
         p.ics = (int)a.get("ics", p.ci); p.ioff = (int)a.get("ioff", 0);
         p.ocs = (int)a.get("ocs", p.co); p.ooff = (int)a.get("ooff", 0);
+        p.pcs = (int)a.get("pcs", p.co); p.poff = (int)a.get("poff", 0);
         p.ho = (p.hi + 2 * p.ph - p.kh) / p.sh + 1;
         p.wo = (p.wi + 2 * p.pw - p.kw) / p.sw + 1;
         p.ktot = p.kh * p.kw * p.ci;
         p.ptot = p.ho * p.wo;
         if (p.ho <= 0 || p.wo <= 0) goto bad;
-        if ((p.co | p.ocs | p.ooff) & 3) goto bad;
+        if ((p.co | p.ocs | p.ooff | p.pcs | p.poff) & 3) goto bad;
         if (!p.nchw && (p.ci % 16) == 0 && ((p.ics | p.ioff) & 3)) goto bad;
         s->nargs = nargs;
         // algorithmic work counts the real input channels (cr: the 3-channel model input is padded to 4)
@@ -371,8 +375,8 @@ static int build_spec(const std::string& name, KernelSpec* s) {
                           ((p.ep & EP_RES) ? 2.0 : 1.0) + p.co * ((p.ep & EP_GB) ? 2.0 : ((p.ep & EP_BIAS) ? 1.0 : 0.0)));
         if (preact) s->bytes += 4.0 * ((double)p.co * p.ptot + p.co);
         int impl = (int)a.get("v", 0);
-        if (preact && (impl != 1 || p.ocs != p.co || p.ooff != 0)) {
-            set_error("reef_conv2d_add_preact exists as the tensor-core variant (_v1) with a dense output only: " + name);
+        if (preact && (impl != 1 || (with_res && (p.ocs != p.co || p.ooff != 0 || p.pcs != p.co || p.poff != 0)))) {
+            set_error(op + " exists as the tensor-core variant (_v1), with dense outputs where it adds a residual: " + name);
             return REEF_NOT_FOUND;
         }
         if (impl == 0) {
@@ -431,7 +435,7 @@ static void fill_arg_bytes(KernelSpec* s) {
             b[2] = f4(t.p.conv.ci);
             break;
         case F_BIAS_RELU:
-            b[0] = f4((double)t.p.elt.c * t.p.elt.n);
+            b[0] = f4((double)(t.p.elt.n - 1) * t.p.elt.ocs + t.p.elt.ooff + t.p.elt.c);
             b[1] = f4((double)(t.p.elt.n - 1) * t.p.elt.ics + t.p.elt.ioff + t.p.elt.c);
             b[2] = f4(t.p.elt.c);
             break;
@@ -489,7 +493,7 @@ static void fill_arg_bytes(KernelSpec* s) {
             if (p.i_gamma >= 0) b[p.i_gamma] = f4(p.co);
             if (p.i_beta >= 0) b[p.i_beta] = f4(p.co);
             if (p.i_bias2 >= 0) b[p.i_bias2] = f4(p.co);
-            if (p.i_out2 >= 0) b[p.i_out2] = f4((double)p.ptot * p.co);
+            if (p.i_out2 >= 0) b[p.i_out2] = f4((double)(p.ptot - 1) * p.pcs + p.poff + p.co);
             break;
         }
         default:
@@ -511,6 +515,7 @@ ArgUse arg_use(const KernelSpec& s, int arg) {
             out = 2;
             break;
         case F_BIAS_RELU:
+            if (arg == 0) slice(t.p.elt.ooff, t.p.elt.c, t.p.elt.ocs);
             if (arg == 1) slice(t.p.elt.ioff, t.p.elt.c, t.p.elt.ics);
             break;
         case F_GLOBAL_AVG_POOL:
@@ -534,6 +539,7 @@ ArgUse arg_use(const KernelSpec& s, int arg) {
             out2 = t.p.conv.i_out2;
             if (arg == 0 && !t.p.conv.nchw) slice(t.p.conv.ioff, t.p.conv.ci, t.p.conv.ics);
             if (arg == 2) slice(t.p.conv.ooff, t.p.conv.co, t.p.conv.ocs);
+            if (arg == out2) slice(t.p.conv.poff, t.p.conv.co, t.p.conv.pcs);
             break;
         default:
             break;   // the other families write their first argument

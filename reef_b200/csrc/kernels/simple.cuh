@@ -152,7 +152,7 @@ __device__ __forceinline__ bool body_im2col_nchw(const KTask& t, int vb, unsigne
 }
 
 // ---- fused_add_nn_relu, channels-last (reference: resource/resnet152/resnet152.cu:4056-4066) ---
-// args: out, in, bias.  out[p][c] = max(in[p*ics+ioff+c] + bias[c], 0); c, ics, ioff multiples of 4.
+// args: out, in, bias.  out[p*ocs+ooff+c] = max(in[p*ics+ioff+c] + bias[c], 0); c, strides and offsets multiples of 4.
 __device__ __forceinline__ bool body_bias_relu(const KTask& t, int vb, unsigned char*, const int*) {
     const EltP& p = t.p.elt;
     float* out = (float*)t.a[0];
@@ -170,7 +170,7 @@ __device__ __forceinline__ bool body_bias_relu(const KTask& t, int vb, unsigned 
             float4 b = *reinterpret_cast<const float4*>(bias + cc);
             v.x = fmaxf(v.x + b.x, 0.f); v.y = fmaxf(v.y + b.y, 0.f);
             v.z = fmaxf(v.z + b.z, 0.f); v.w = fmaxf(v.w + b.w, 0.f);
-            *reinterpret_cast<float4*>(out + (size_t)pix * p.c + cc) = v;
+            *reinterpret_cast<float4*>(out + (size_t)pix * p.ocs + p.ooff + cc) = v;
         }
     }
     return true;

@@ -9,6 +9,7 @@ family                                 args (storage indices, in order)
 =====================================  ==========================================
 fused_add                              out, in, bias            (NCHW, model input)
 fused_add_nn_relu                      out, in, bias            (NHWC)
+reef_conv2d_preact                     in, W, out, bias2, out2  (out2 = relu(out + bias2); channel slices)
 fused_nn_conv2d                        in, W, out
 fused_nn_conv2d_nn_relu                in, W, out
 fused_nn_conv2d_add                    in, W, out, residual
@@ -282,15 +283,39 @@ class Builder:
                       [out.idx, x.idx, self.g.param(bias)])
         return out
 
-    def bias_relu_slice(self, x: Tensor, bias) -> Tensor:
-        """relu(x + bias) on a channel slice view (DenseNet pre-activation)."""
-        out = self.new_act(x.h, x.w, x.c)
+    def bias_relu_slice(self, x: Tensor, bias, out: Tensor | None = None) -> Tensor:
+        """relu(x + bias) on a channel slice view (DenseNet pre-activation), into a slice view where `out` is given."""
+        if out is None:
+            out = self.new_act(x.h, x.w, x.c)
         attrs = dict(c=x.c, n=x.h * x.w)
         if x.cstride != x.c or x.coff:
             attrs["ics"] = x.cstride
             attrs["ioff"] = x.coff
+        if out.cstride != out.c or out.coff:
+            attrs["ocs"] = out.cstride
+            attrs["ooff"] = out.coff
         self.g.kernel(kname("fused_add_nn_relu", **attrs), [out.idx, x.idx, self.g.param(bias)])
         return out
+
+    def conv_append(self, x: Tensor, co: int, k: int, pad: int, buf: Tensor, coff: int, bias, *, weight, w_gain: float) -> Tensor:
+        """DenseNet: a convolution whose `co` channels join the `coff` channels already in the concat buffer, and
+        relu(concatenation + bias), the next layer's pre-activation, as a tensor of its own.  The channels that were there
+        before are activated by a kernel that depends on nothing recent (it runs beside this layer's convolutions), the new
+        ones by the convolution's epilogue: no elementwise kernel stands between two layers.  Without the tensor-core
+        variant: the convolution, then one fused_add_nn_relu, as in the reference's graphs."""
+        out, old = self.slice_of(buf, coff, co), self.slice_of(buf, 0, coff)
+        attrs = dict(ci=x.c, hi=x.h, wi=x.w, co=co, kh=k, kw=k, sh=1, sw=1, ph=pad, pw=pad)
+        act = None
+        tail = dict(ocs=out.cstride, ooff=out.coff, pcs=coff + co, poff=coff)
+        if x.cstride == x.c and not x.coff and self.pick_conv_impl("reef_conv2d_preact", {**attrs, **tail}) == 1:
+            act = self.new_act(buf.h, buf.w, coff + co)
+            self.bias_relu_slice(old, bias[:coff], self.slice_of(act, 0, coff))
+            op = kname("reef_conv2d_preact", **attrs, **tail, v=1)
+            args = [x.idx, self.g.param(round_tf32(weight * np.float32(w_gain))), buf.idx, self.g.param(bias[coff:]), act.idx]
+            self.g.kernel(kname("reef_conv2d_preact", **attrs, **tail, v=1, **tuned_plan(op)), args)
+            return act
+        self.conv(x, co, k, 1, pad, out=out, weight=weight, w_gain=w_gain)
+        return self.bias_relu_slice(self.slice_of(buf, 0, coff + co), bias)
 
     def global_avg_pool(self, x: Tensor) -> Tensor:
         assert x.cstride == x.c and x.coff == 0

@@ -59,6 +59,8 @@ def _arg_sizes(op: str, a: dict):
     tail = op[len("fused_nn_conv2d"):] if op.startswith("fused_nn_conv2d") else None
     if op == "reef_conv2d_add_preact":
         extra = [("temp", p * co), ("param", co), ("temp", p * co)]
+    elif op == "reef_conv2d_preact":
+        extra = [("param", co), ("temp", p * a.get("pcs", co))]
     elif tail in ("", "_nn_relu"):
         extra = []
     elif tail == "_add_nn_relu":
