@@ -221,7 +221,11 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
         // channels, and channels beyond Cin (Cin not a multiple of 32) come back as zeros
         cuuint64_t dims[3] = {(cuuint64_t)p.ci, (cuuint64_t)(p.kh * p.kw), (cuuint64_t)p.co};
         cuuint64_t strides[2] = {(cuuint64_t)p.ci * 4, (cuuint64_t)p.ktot * 4};
-        cuuint32_t box[3] = {TC_BK, 1, TC_BM};
+        // Fewer output channels than a tile has rows: only they are copied (in whole 8-row groups of the swizzle).  The
+        // other rows of the operand keep what the shared memory held; their sums end in lanes that nobody reads.
+        const cuuint32_t rows = p.co < TC_BM ? (cuuint32_t)ceil_div_i(p.co, 8) * 8 : TC_BM;
+        P->load_bytes = (int)rows * TC_BK * 4 + pl.b_bytes;
+        cuuint32_t box[3] = {TC_BK, 1, rows};
         rc = encode(&P->tm_w, wgt, 3, dims, strides, box);
         if (rc != REEF_SUCC) return rc;
     }
@@ -267,7 +271,6 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
     if (p.ep & EP_RELU) P->ep |= TC_EP_RELU;
     if (p.ep & EP_GELU) P->ep |= TC_EP_GELU;
     if (p.round_tf32) P->ep |= TC_EP_ROUND;
-    P->b_bytes = pl.b_bytes;
     P->cb_magic = (unsigned)((0x100000000ull + (unsigned long long)pl.cblocks - 1) / (unsigned long long)pl.cblocks);
     for (int ky = 0; ky < p.kh; ky++)
         for (int kx = 0; kx < p.kw; kx++) {

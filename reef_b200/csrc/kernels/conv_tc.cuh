@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         // descriptors are warp-uniform (uniform registers), one elected lane executes each instruction.  As code of a
         // single thread every instruction had its operands moved into uniform registers first: 540 cycles per K block in
         // the multiplication loop, whatever the tile's width.
-        const uint32_t tx = TC_A_BYTES + (uint32_t)P.b_bytes;
+        const uint32_t tx = (uint32_t)P.load_bytes;
         const int first = nkb < NS ? nkb : NS;
         // filter tap and channel block of the next K block to refill, carried along (2^32 / 1 does not fit the magic: one
         // channel block per tap is a copy)

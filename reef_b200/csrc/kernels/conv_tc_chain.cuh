@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_chain_kernel(const
             if (S > 1 && valid && tid == 0) mbar_expect_tx(bar_red, (uint32_t)((S - 1) * (je - jb) * TC_BM * 4));
 
             const int m0 = tile_m * TC_BM;
-            const uint32_t tx = TC_A_BYTES + (uint32_t)P.b_bytes;
+            const uint32_t tx = (uint32_t)P.load_bytes;
             const int first = nkb < NS ? nkb : NS;
             auto tap_of = [&](int kb) { return P.cblocks == 1 ? kb : (int)__umulhi((unsigned)kb, P.cb_magic); };
             auto load_a = [&](int i, int s) {

@@ -16,7 +16,7 @@ constexpr int TC_MAX_SPLITS = 8;
 constexpr int TC_SMEM_CAP = 112 * 1024;
 
 struct TcParams {
-    CUtensorMap tm_w;        // weights  dims (Cin, taps, Cout), box (32, 1, 128)
+    CUtensorMap tm_w;        // weights  dims (Cin, taps, Cout), box (32, 1, up to 128)
     CUtensorMap tm_x[4];     // activations, one per stride sub-lattice (ry*s + rx)
     float* out;
     const float* res;
@@ -42,7 +42,7 @@ struct TcParams {
     int cblocks;             // Cin / 32
     int kb_total, kb_per_split, splits;
     int ep;                  // EP_* bits
-    int b_bytes;             // bytes TMA delivers per B stage (box size)
+    int load_bytes;          // bytes TMA delivers per K block (both boxes)
     int stages;              // ring depth of this launch
     int region_bytes;        // data region of shared memory: max(stage ring, staging tile + exchange area)
     int recv_offset_floats;  // exchange area offset inside the region, in floats
