@@ -120,6 +120,8 @@ REEF_HOST_API int reef_sched_wait_task(reef_scheduler_t s, uint32_t tid);
 /* Host-side failure injection for tests: the next `n` kernel launches of model `mid` return an error without
  * reaching the device. */
 REEF_HOST_API int reef_sched_inject_launch_failures(reef_scheduler_t s, uint32_t mid, int n);
+/* The same for the next `n` launches of the copy that leaves the output in pinned host memory at the end of a pass. */
+REEF_HOST_API int reef_sched_inject_mirror_failures(reef_scheduler_t s, uint32_t mid, int n);
 typedef struct {
     int state;                 /* 0 Init, 1 Waiting, 2 Executing, 3 Finish */
     int preempted, padded, padded_to_complete;

@@ -407,6 +407,10 @@ class REEFScheduler:
         """Host-side failure injection: the next ``n`` kernel launches of model ``mid`` return an error."""
         _check(self._lib.reef_sched_inject_launch_failures(self._h, C.c_uint32(mid), C.c_int(n)), "inject_launch_failures")
 
+    def inject_mirror_failures(self, mid: int, n: int):
+        """Host-side failure injection: the next ``n`` copies of the output into its pinned mirror are refused."""
+        _check(self._lib.reef_sched_inject_mirror_failures(self._h, C.c_uint32(mid), C.c_int(n)), "inject_mirror_failures")
+
     def get_task(self, tid: int) -> TaskInfo:
         info = TaskInfo()
         _check(self._lib.reef_sched_task_info(self._h, C.c_uint32(tid), C.byref(info)), "get_task")

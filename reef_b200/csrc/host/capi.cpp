@@ -342,6 +342,9 @@ int reef_sched_task_info(reef_scheduler_t s, uint32_t tid, reef_task_info_t* inf
 int reef_sched_inject_launch_failures(reef_scheduler_t s, uint32_t mid, int n) {
     return s->sched->inject_launch_failures(mid, n);
 }
+int reef_sched_inject_mirror_failures(reef_scheduler_t s, uint32_t mid, int n) {
+    return s->sched->inject_mirror_failures(mid, n);
+}
 int reef_sched_set_wait_sync(reef_scheduler_t s, int v) { s->sched->set_wait_sync(v != 0); return Succ; }
 int reef_sched_set_be_stream_cap(reef_scheduler_t s, int v) { s->sched->set_be_stream_cap(v); return Succ; }
 int reef_sched_use_mapped_flag(reef_scheduler_t s) { return s->sched->use_mapped_flag(); }

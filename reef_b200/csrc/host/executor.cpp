@@ -178,6 +178,11 @@ Status ExecutorBase::init_host_buffers() {
 
 Status ExecutorBase::launch_output_mirror(GPUStream_t stream) {
     if (!mirror) return Status::Succ;
+    if (fail_mirrors > 0) {
+        fail_mirrors--;
+        err_ = "injected launch failure of the output mirror";
+        return Status::Fail;
+    }
     if (mirror_kernel) {
         void* args[2] = {&mirror_args[0], &mirror_args[1]};
         GPU_RETURN_STATUS(reef_launch(mirror_kernel, mirror_dims, mirror_smem, stream, args));
@@ -519,6 +524,7 @@ Status HybridExecutor::launch_dispatch(int rt_idx, HybridExecutor* be, int be_id
 }
 
 Status HybridExecutor::launch_pad_piece(int idx, int block_offset, int block_num, int occupancy, GPUStream_t stream) {
+    drop_output_mirror();
     RETURN_STATUS(order_input(stream));
     int rc = reef_dispatch(nullptr, nullptr, kernels[idx], raw_args[idx].data(), block_offset, block_num, 0, occupancy,
                            task_slot_base + (size_t)idx * 4, dispatch_ctrl, dispatch_ctrl, stream, stream);
@@ -628,6 +634,7 @@ Status HybridExecutor::launch_preempt_segment(int k, GPUStream_t stream, bool si
 
 Status HybridExecutor::launch_pad_segment(int seg, GPUStream_t stream) {
     if (seg < 0 || seg >= (int)pad_segments.size()) RETURN_STATUS(Status::OutOfRange);
+    drop_output_mirror();
     RETURN_STATUS(order_input(stream));
     GPU_RETURN_STATUS(reef_graph_launch(pad_segments[seg], stream));
     return Status::Succ;
@@ -847,12 +854,12 @@ Status HybridExecutor::schedule_edges(std::vector<int>* from, std::vector<int>* 
 }
 
 Status HybridExecutor::execute_graph(GPUStream_t stream) {
+    drop_output_mirror();
     if (fail_launches > 0 && graph != nullptr && graph_stream == stream) {   // injected failure of a graph replay
         fail_launches--;
         err_ = "injected graph launch failure";
         return Status::Fail;
     }
-    drop_output_mirror();
     RETURN_STATUS(order_input(stream));   // before a capture begins: the wait is no part of the graph
     if (graph_stream != stream) {
         // The first pass on a stream launches kernel by kernel: capturing and instantiating a graph takes milliseconds,

@@ -66,6 +66,8 @@ public:
     // Failure injection on the host: the next `n` kernel launches of this executor return Status::Fail without
     // reaching the device (how the tests exercise the failed-task path; no GPU fault is involved).
     void inject_launch_failures(int n) { fail_launches = n; }
+    // the same for the next `n` launches of the output mirror (launch_output_mirror)
+    void inject_mirror_failures(int n) { fail_mirrors = n; }
 
     // The output tensor of a complete run, already in host memory: every full pass ends with a copy of "output" into a
     // pinned mirror on the pass's own stream, so that get_output behind the pass is a plain memcpy.  `launch` enqueues
@@ -112,6 +114,7 @@ protected:
     GPUDevicePtr_t mirror_args[2] = {0, 0};
     std::atomic<bool> mirror_fresh{false};
     int fail_launches = 0;
+    int fail_mirrors = 0;
     std::string err_;
 };
 

@@ -321,6 +321,12 @@ Status REEFScheduler::inject_launch_failures(ModelID mid, int n) {
     return Status::Succ;
 }
 
+Status REEFScheduler::inject_mirror_failures(ModelID mid, int n) {
+    if (mid >= model_pool_size.load()) return Status::OutOfRange;
+    model_pool[mid]->executor.inject_mirror_failures(n);
+    return Status::Succ;
+}
+
 // The device error word is read after a task's stream has been synchronised (or seen drained): non-zero means a
 // bounded wait of some kernel expired since the last look, so what ran since then did not produce valid output.
 bool REEFScheduler::device_error_seen(const char* where) {
@@ -750,7 +756,7 @@ void REEFScheduler::advance_padded(Task* be_task, TaskQueue* q, int blocks, bool
     if (side_launch) {
         // its last blocks are on the best-effort stream: the task completes when that stream has drained,
         // which the best-effort branch of the loop sees through the window
-        be_exe.launch_output_mirror(q->stream);   // (a refused launch leaves get_output to copy for itself)
+        be_exe.launch_output_mirror(q->stream);   // (refused: the mirror stays dropped and get_output copies for itself)
         reef_event_t ev;
         if (!q->free_events.empty()) {
             ev = q->free_events.back();
@@ -1162,6 +1168,9 @@ void REEFScheduler::execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr
 
     if (st == TaskState::Init || st == TaskState::Waiting) {
         if (st == TaskState::Init) task->start = std::chrono::system_clock::now();
+        // what the mirror holds is the request before's (or of a pass that was preempted behind its last launch), until
+        // this pass has ended with a copy
+        exe.drop_output_mirror();
         if (preempted) {
             reset_preempt_flag_async();
             preempted = false;

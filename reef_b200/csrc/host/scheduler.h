@@ -163,6 +163,8 @@ public:
     const std::string& error() const { return err_; }
     // host-side failure injection for tests: the next n kernel launches of model `mid` return an error
     Status inject_launch_failures(ModelID mid, int n);
+    // the same for the copy of the output into the pinned mirror that ends a pass
+    Status inject_mirror_failures(ModelID mid, int n);
 
 private:
     struct Model {

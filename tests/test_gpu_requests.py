@@ -57,6 +57,48 @@ def test_scheduler_request(tmp_path, kind, n):
     s.close()
 
 
+@pytest.mark.parametrize("kernels", [1, 3, 4, 6])
+def test_refused_output_mirror_of_a_padded_task(gen, tmp_path, kernels):
+    """A best-effort task that goes out as padding beside a real-time request ends with the copy of its output into the
+    pinned mirror.  Where that copy is refused the task is served all the same, and get_output must not hand out the
+    answer of the request before (the copy is refused on the host; nothing fails on the device)."""
+    n = 5000
+    g = Graph("copies")
+    src = g.input("data", n)
+    for i in range(kernels):
+        dst = g.add_storage("output" if i == kernels - 1 else "null", n)
+        g.kernel(kname("fused_nn_batch_flatten", n=n), [dst, src])
+        src = dst
+    base, rt_base = g.write(str(tmp_path), capi.plan_fn), gen("resnet18_64")
+    s = capi.REEFScheduler(capi.REEFScheduler.REEF, 0)
+    s.set_pad_slowdown_target(0)      # no rate limit: whatever fits goes out as padding
+    be = s.load_model_files(base + ".json", base + ".profile.json")
+    rt = s.load_model_files(rt_base + ".json", rt_base + ".profile.json", rt_base + ".param")
+    s.bind_model_queue(s.create_queue(capi.REEFScheduler.BestEffortQueue), be)
+    s.bind_model_queue(s.create_queue(capi.REEFScheduler.RealTimeQueue), rt)
+    s.set_input(rt, np.zeros(3 * 64 * 64, np.float32))
+    s.run()
+    rng = np.random.default_rng(kernels)
+    refused = 0
+    for i in range(40):
+        x = rng.normal(0, 1, n).astype(np.float32)
+        s.set_input(be, x)
+        s.inject_mirror_failures(be, i % 2)
+        # the second real-time request finds the best-effort task waiting and pads with it
+        first, t, second = s.new_task(rt), s.new_task(be), s.new_task(rt)
+        for task in (first, second):
+            s.wait_task(task)
+        try:
+            s.wait_task(t)
+        except capi.ReefError:      # not padded: the refused copy fails the task
+            assert i % 2 and not s.get_task(t).padded_to_complete
+            continue
+        refused += i % 2 and s.get_task(t).padded_to_complete
+        assert np.array_equal(s.get_output(be), x), f"request {i}: output of an earlier request"
+    assert refused > 0
+    s.close()
+
+
 @pytest.mark.parametrize("kernels", [1, 7, 8, 9, 16, 17])
 def test_best_effort_segments(tmp_path, kernels):
     """Schedules shorter than, equal to and just beyond a segment of the best-effort window, with the GPU to themselves
