@@ -176,6 +176,17 @@ Status ExecutorBase::init_host_buffers() {
     return Status::Succ;
 }
 
+Status ExecutorBase::issue_mirror(GPUStream_t stream) {
+    if (!mirror) return Status::Succ;
+    if (mirror_kernel) {
+        void* args[2] = {&mirror_args[0], &mirror_args[1]};
+        GPU_RETURN_STATUS(reef_launch(mirror_kernel, mirror_dims, mirror_smem, stream, args));
+    } else {
+        GPU_RETURN_STATUS(reef_memcpy_d2h_async(mirror, mirror_args[1], mirror_bytes, stream));
+    }
+    return Status::Succ;
+}
+
 Status ExecutorBase::launch_output_mirror(GPUStream_t stream) {
     if (!mirror) return Status::Succ;
     if (fail_mirrors > 0) {
@@ -183,12 +194,7 @@ Status ExecutorBase::launch_output_mirror(GPUStream_t stream) {
         err_ = "injected launch failure of the output mirror";
         return Status::Fail;
     }
-    if (mirror_kernel) {
-        void* args[2] = {&mirror_args[0], &mirror_args[1]};
-        GPU_RETURN_STATUS(reef_launch(mirror_kernel, mirror_dims, mirror_smem, stream, args));
-    } else {
-        GPU_RETURN_STATUS(reef_memcpy_d2h_async(mirror, mirror_args[1], mirror_bytes, stream));
-    }
+    RETURN_STATUS(issue_mirror(stream));
     mirror_fresh.store(true, std::memory_order_relaxed);
     return Status::Succ;
 }
@@ -384,6 +390,10 @@ Status ExecutorBase::launch_kernel(int i, GPUStream_t stream) {
         return Status::Fail;
     }
     RETURN_STATUS(order_input(stream));
+    return issue_kernel(i, stream);
+}
+
+Status ExecutorBase::issue_kernel(int i, GPUStream_t stream) {
     int rc = reef_launch(kernels[i], model->kernels[i].launch_params, kernel_smem[i], stream, raw_args[i].data());
     if (rc != REEF_SUCC) err_ = reef_last_error();
     GPU_RETURN_STATUS(rc);
@@ -498,6 +508,10 @@ Status HybridExecutor::launch_preempt_kernel(int i, GPUStream_t stream) {
         return Status::Fail;
     }
     RETURN_STATUS(order_input(stream));
+    return issue_preempt_kernel(i, stream);
+}
+
+Status HybridExecutor::issue_preempt_kernel(int i, GPUStream_t stream) {
     int rc = reef_launch_be(kernels[i], model->kernels[i].launch_params, kernel_smem[i], stream, preempt_flag,
                             task_slot_base + (size_t)i * 4, raw_args[i].data());
     if (rc != REEF_SUCC) err_ = reef_last_error();
@@ -526,6 +540,10 @@ Status HybridExecutor::launch_dispatch(int rt_idx, HybridExecutor* be, int be_id
 Status HybridExecutor::launch_pad_piece(int idx, int block_offset, int block_num, int occupancy, GPUStream_t stream) {
     drop_output_mirror();
     RETURN_STATUS(order_input(stream));
+    return issue_pad_piece(idx, block_offset, block_num, occupancy, stream);
+}
+
+Status HybridExecutor::issue_pad_piece(int idx, int block_offset, int block_num, int occupancy, GPUStream_t stream) {
     int rc = reef_dispatch(nullptr, nullptr, kernels[idx], raw_args[idx].data(), block_offset, block_num, 0, occupancy,
                            task_slot_base + (size_t)idx * 4, dispatch_ctrl, dispatch_ctrl, stream, stream);
     if (rc != REEF_SUCC) err_ = reef_last_error();
@@ -533,9 +551,10 @@ Status HybridExecutor::launch_pad_piece(int idx, int block_offset, int block_num
     return Status::Succ;
 }
 
+// What is captured is issued as it is (issue_*): a set_input that another thread makes meanwhile belongs to no graph — its
+// event, recorded outside the capture, would invalidate the capture — and launches of the graph are ordered behind it.
 Status HybridExecutor::build_pad_segments() {
     if (!pad_segments.empty()) return Status::Succ;
-    RETURN_STATUS(wait_input());   // a wait on another stream's event must not be captured
     GPUStream_t cap = nullptr;
     GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
     const int n = (int)num_kernels();
@@ -548,7 +567,7 @@ Status HybridExecutor::build_pad_segments() {
         for (int k = k0; k < std::min(n, k0 + kPadSegment) && st == Status::Succ; k++) {
             const KernelArg& a = trans_args[k];
             const int occ = a.resource.tensor_core ? 1 : std::max(1, std::min(2, a.resource.max_blocks_per_sm));
-            st = launch_pad_piece(k, 0, a.block_num, occ, cap);
+            st = issue_pad_piece(k, 0, a.block_num, occ, cap);
         }
         reef_graph_t g = nullptr;
         int rc = reef_graph_end(cap, &g);
@@ -569,7 +588,6 @@ Status HybridExecutor::build_pad_segments() {
 
 Status HybridExecutor::build_be_segments() {
     if (!be_segments.empty()) return Status::Succ;
-    RETURN_STATUS(wait_input());
     std::vector<int> from, to;
     RETURN_STATUS(schedule_edges(&from, &to));
     GPUStream_t cap = nullptr;
@@ -582,8 +600,8 @@ Status HybridExecutor::build_be_segments() {
             break;
         }
         const int k1 = std::min(n, k0 + kBeSegment);
-        for (int k = k0; k < k1 && st == Status::Succ; k++) st = launch_preempt_kernel(k, cap);
-        if (st == Status::Succ && k1 == n) st = launch_output_mirror(cap);
+        for (int k = k0; k < k1 && st == Status::Succ; k++) st = issue_preempt_kernel(k, cap);
+        if (st == Status::Succ && k1 == n) st = issue_mirror(cap);
         // branches side by side inside a segment, too; the segments follow one another on the stream
         std::vector<int> seg_from, seg_to;
         for (size_t e = 0; e < from.size(); e++)
@@ -600,7 +618,6 @@ Status HybridExecutor::build_be_segments() {
         else if (g) reef_graph_destroy(g);
     }
     reef_stream_destroy(cap);
-    drop_output_mirror();
     if (st != Status::Succ) {
         for (auto g : be_segments) reef_graph_destroy(g);
         be_segments.clear();
@@ -676,11 +693,11 @@ Status HybridExecutor::build_chains(int clusters) {
 }
 
 // the schedule in order: a chain launch for every run that has one, a plain launch for every other kernel
-Status HybridExecutor::launch_schedule(GPUStream_t stream, bool use_chains) {
-    RETURN_STATUS(order_input(stream));
+Status HybridExecutor::launch_schedule(GPUStream_t stream, bool capturing) {
+    if (!capturing) RETURN_STATUS(order_input(stream));
     size_t ci = 0;
     for (size_t i = 0; i < num_kernels();) {
-        if (use_chains && ci < chains.size() && chains[ci].begin == (int)i) {
+        if (ci < chains.size() && chains[ci].begin == (int)i) {
             int rc = reef_chain_launch(chains[ci].handle, stream);
             if (rc != REEF_SUCC) {
                 err_ = reef_last_error();
@@ -690,7 +707,7 @@ Status HybridExecutor::launch_schedule(GPUStream_t stream, bool use_chains) {
             ci++;
             continue;
         }
-        Status st = ExecutorBase::launch_kernel((int)i, stream);
+        Status st = capturing ? issue_kernel((int)i, stream) : ExecutorBase::launch_kernel((int)i, stream);
         if (st != Status::Succ) return st;
         i++;
     }
@@ -808,7 +825,7 @@ Status HybridExecutor::execute_preempt_resume_chained(int delay_us, int clusters
 Status HybridExecutor::execute_chained(GPUStream_t stream) {
     if (stream == nullptr) stream = s;
     drop_output_mirror();
-    RETURN_STATUS(launch_schedule(stream, true));
+    RETURN_STATUS(launch_schedule(stream, false));
     RETURN_STATUS(launch_output_mirror(stream));
     GPU_RETURN_STATUS(reef_stream_sync(stream));
     return Status::Succ;
@@ -855,18 +872,17 @@ Status HybridExecutor::schedule_edges(std::vector<int>* from, std::vector<int>* 
 
 Status HybridExecutor::execute_graph(GPUStream_t stream) {
     drop_output_mirror();
-    if (fail_launches > 0 && graph != nullptr && graph_stream == stream) {   // injected failure of a graph replay
+    if (fail_launches > 0 && graph_stream == stream) {   // injected failure of a graph replay
         fail_launches--;
         err_ = "injected graph launch failure";
         return Status::Fail;
     }
-    RETURN_STATUS(order_input(stream));   // before a capture begins: the wait is no part of the graph
     if (graph_stream != stream) {
         // The first pass on a stream launches kernel by kernel: capturing and instantiating a graph takes milliseconds,
         // which a request should not wait for before it is known that more of them follow.
         if (graph) reef_graph_destroy(graph);
         graph = nullptr;
-        RETURN_STATUS(launch_schedule(stream, true));
+        RETURN_STATUS(launch_schedule(stream, false));
         RETURN_STATUS(launch_output_mirror(stream));
         graph_stream = stream;
         return Status::Succ;
@@ -874,7 +890,7 @@ Status HybridExecutor::execute_graph(GPUStream_t stream) {
     if (graph == nullptr) {
         GPU_RETURN_STATUS(reef_graph_begin(stream));
         Status st = launch_schedule(stream, true);
-        if (st == Status::Succ) st = launch_output_mirror(stream);
+        if (st == Status::Succ) st = issue_mirror(stream);
         std::vector<int> from, to;
         const bool relaxed = st == Status::Succ && chains.empty() && schedule_edges(&from, &to) == Status::Succ;
         int rc = relaxed ? reef_graph_end_relaxed(stream, from.data(), to.data(), from.size(), &graph) : reef_graph_end(stream, &graph);
@@ -887,6 +903,7 @@ Status HybridExecutor::execute_graph(GPUStream_t stream) {
             return st != Status::Succ ? st : Status::Fail;
         }
     }
+    RETURN_STATUS(order_input(stream));
     GPU_RETURN_STATUS(reef_graph_launch(graph, stream));
     if (mirror) mirror_fresh.store(true, std::memory_order_relaxed);   // the graph ends with the copy
     return Status::Succ;

@@ -89,6 +89,9 @@ protected:
     size_t storage_bytes(size_t idx) const;
     Status init_host_buffers();
     Status wait_input();
+    // the bare launches, as a capture records them: no order behind an input, no failure injection, no note of the mirror
+    Status issue_kernel(int kernel_offset, GPUStream_t stream);
+    Status issue_mirror(GPUStream_t stream);
 
     std::vector<GPUDevicePtr_t> storage;            // one device pointer per storage entry (views into one arena)
     std::vector<GPUFunction_t> kernels;             // per kernel call
@@ -248,7 +251,9 @@ protected:
         reef_chain_t handle;
     };
     std::vector<Chain> chains;
-    Status launch_schedule(GPUStream_t stream, bool use_chains);
+    Status launch_schedule(GPUStream_t stream, bool capturing);
+    Status issue_preempt_kernel(int kernel_offset, GPUStream_t stream);
+    Status issue_pad_piece(int idx, int block_offset, int block_num, int occupancy, GPUStream_t stream);
     // which launches of the schedule (and, as number num_kernels(), of the output mirror behind it) have to wait for
     // which others
     Status schedule_edges(std::vector<int>* from, std::vector<int>* to);

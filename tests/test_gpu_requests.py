@@ -1,6 +1,7 @@
 """Requests through host memory: staged input, output mirror, graph replay behind the first pass.  A one-kernel model that
 copies its input makes every byte of the way visible; sizes straddle the two-piece split of the staging copy, the limit
 between the mirror's copy kernel and the copy engine, and the limit of the pinned buffers."""
+import threading
 
 import numpy as np
 import pytest
@@ -97,6 +98,49 @@ def test_refused_output_mirror_of_a_padded_task(gen, tmp_path, kernels):
         assert np.array_equal(s.get_output(be), x), f"request {i}: output of an earlier request"
     assert refused > 0
     s.close()
+
+
+@pytest.mark.parametrize("kind", [capi.REEFScheduler.RealTimeQueue, capi.REEFScheduler.BestEffortQueue])
+def test_input_set_while_graphs_are_captured(gen, kind):
+    """A pipelined client stages inputs all the time.  One that arrives while a graph of the model is captured (by its first
+    requests, or when it is bound) is no part of the capture: every request is served, and the input staged last counts."""
+    base = gen("inception_v3_139")
+    n = 3 * 139 * 139
+    rng = np.random.default_rng(6)
+    last = rng.normal(0, 1, n).astype(np.float32)
+    want = None
+    for _ in range(6):
+        s = capi.REEFScheduler(capi.REEFScheduler.REEF, 0)
+        mid = s.load_model_files(base + ".json", base + ".profile.json", base + ".param")
+        q = s.create_queue(kind)
+        s.run()
+        stop, failed = threading.Event(), []
+
+        def stage():
+            x = rng.normal(0, 1, n).astype(np.float32)
+            while not stop.is_set():
+                try:
+                    s.set_input(mid, x)
+                except capi.ReefError as e:
+                    failed.append(e)
+                    return
+
+        client = threading.Thread(target=stage)
+        client.start()
+        try:
+            s.bind_model_queue(q, mid)
+            for _ in range(6):
+                s.wait_task(s.new_task(mid))
+        finally:
+            stop.set()
+            client.join()
+        assert not failed
+        s.set_input(mid, last)
+        s.wait_task(s.new_task(mid))
+        out = s.get_output(mid)
+        want = out if want is None else want
+        assert np.array_equal(out, want)
+        s.close()
 
 
 @pytest.mark.parametrize("kernels", [1, 7, 8, 9, 16, 17])
