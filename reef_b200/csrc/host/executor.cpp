@@ -200,13 +200,18 @@ Status ExecutorBase::launch_output_mirror(GPUStream_t stream) {
 }
 
 Status ExecutorBase::order_input(GPUStream_t stream) {
-    if (!input_pending.load(std::memory_order_acquire)) return Status::Succ;
+    // taken before the event is looked at: an input that another thread stages from here on is pending again, for the next
+    // launch, and never cleared unseen
+    if (!input_pending.exchange(false, std::memory_order_acq_rel)) return Status::Succ;
     if (stream != input_stream) {
         int pending = 1;
-        GPU_RETURN_STATUS(reef_event_query(input_ev, &pending));
-        if (pending) GPU_RETURN_STATUS(reef_stream_wait_event(stream, input_ev));
+        reef_status rc = reef_event_query(input_ev, &pending);
+        if (rc == REEF_SUCC && pending) rc = reef_stream_wait_event(stream, input_ev);
+        if (rc != REEF_SUCC) {
+            input_pending.store(true, std::memory_order_release);
+            return Status::Fail;
+        }
     }
-    input_pending.store(false, std::memory_order_release);
     return Status::Succ;
 }
 
