@@ -558,10 +558,8 @@ Status HybridExecutor::issue_pad_piece(int idx, int block_offset, int block_num,
 
 // What is captured is issued as it is (issue_*): a set_input that another thread makes meanwhile belongs to no graph — its
 // event, recorded outside the capture, would invalidate the capture — and launches of the graph are ordered behind it.
-Status HybridExecutor::build_pad_segments() {
+Status HybridExecutor::build_pad_segments(GPUStream_t cap) {
     if (!pad_segments.empty()) return Status::Succ;
-    GPUStream_t cap = nullptr;
-    GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
     const int n = (int)num_kernels();
     Status st = Status::Succ;
     for (int k0 = 0; k0 < n && st == Status::Succ; k0 += kPadSegment) {
@@ -583,7 +581,6 @@ Status HybridExecutor::build_pad_segments() {
         if (st == Status::Succ) pad_segments.push_back(g);
         else if (g) reef_graph_destroy(g);
     }
-    reef_stream_destroy(cap);
     if (st != Status::Succ) {
         for (auto g : pad_segments) reef_graph_destroy(g);
         pad_segments.clear();
@@ -591,12 +588,10 @@ Status HybridExecutor::build_pad_segments() {
     return st;
 }
 
-Status HybridExecutor::build_be_segments() {
+Status HybridExecutor::build_be_segments(GPUStream_t cap) {
     if (!be_segments.empty()) return Status::Succ;
     std::vector<int> from, to;
     RETURN_STATUS(schedule_edges(&from, &to));
-    GPUStream_t cap = nullptr;
-    GPU_RETURN_STATUS(reef_stream_create(&cap, 0));
     const int n = (int)num_kernels();
     Status st = Status::Succ;
     for (int k0 = 0; k0 < n && st == Status::Succ; k0 += kBeSegment) {
@@ -622,7 +617,6 @@ Status HybridExecutor::build_be_segments() {
         if (st == Status::Succ) be_segments.push_back(g);
         else if (g) reef_graph_destroy(g);
     }
-    reef_stream_destroy(cap);
     if (st != Status::Succ) {
         for (auto g : be_segments) reef_graph_destroy(g);
         be_segments.clear();

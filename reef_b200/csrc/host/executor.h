@@ -163,14 +163,16 @@ public:
     // Padding segments: the kernel list cut into runs of kPadSegment kernels, each run captured once as a CUDA
     // graph of whole-kernel pieces (one launch and one completion event for the run; inside it the kernels keep
     // their programmatic dependencies).  Segment g covers kernels [g*kPadSegment, (g+1)*kPadSegment).
+    // They are captured on `cap`, a stream with nothing on it: a graph's kernels keep the priority and the SM partition of
+    // the stream that they were captured on, wherever the graph is launched.
     static const int kPadSegment = 4;
-    Status build_pad_segments();
+    Status build_pad_segments(GPUStream_t cap);
     bool has_pad_segments() const { return !pad_segments.empty(); }
     Status launch_pad_segment(int seg, GPUStream_t stream);
     // Best-effort segments: the same cut into runs of kBeSegment kernels for the best-effort flavour (every kernel still
     // polls the flag and counts into its slot).  A task at full speed is fed one graph launch and one event per run.
     static const int kBeSegment = 16;
-    Status build_be_segments();
+    Status build_be_segments(GPUStream_t cap);
     Status launch_preempt_segment(int kernel_offset, GPUStream_t stream, bool single, int* last);
     bool has_tensor_core_kernels() const { return has_tc; }
     // Persistent chains: every run of two or more consecutive tensor-core convolution / matmul kernels of the

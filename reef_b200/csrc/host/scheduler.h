@@ -207,7 +207,9 @@ private:
         std::vector<int> preempted_kernels;   // kernels that were in flight at the last preemption (diagnostics)
     };
 
+    Status make_stream(bool rt, executor::GPUStream_t* stream);
     Status create_task_queue(std::shared_ptr<TaskQueue>& ret, bool rt);
+    Status capture_graphs(Model& model);
     void loop_body();
     void execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr<TaskQueue>& tqueue);
     void execute_rt_task(std::shared_ptr<Task>& task);
