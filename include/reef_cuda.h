@@ -99,6 +99,8 @@ REEF_API reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g);
  * it touches memory, so an order that follows from other edges needs none of its own. */
 REEF_API reef_status reef_graph_end_relaxed(reef_stream_t s, const int* from, const int* to, size_t num_edges, reef_graph_t* g);
 REEF_API reef_status reef_graph_launch(reef_graph_t g, reef_stream_t s);
+/* brings the graph to the device ahead of its first launch, which otherwise does it; returns when it is there */
+REEF_API reef_status reef_graph_upload(reef_graph_t g, reef_stream_t s);
 REEF_API reef_status reef_graph_destroy(reef_graph_t g);
 
 /* ---- kernel registry ---------------------------------------------------------------------- */

@@ -515,6 +515,11 @@ reef_status reef_graph_launch(reef_graph_t g, reef_stream_t s) {
     add_launches(h->kernels);
     return REEF_SUCC;
 }
+reef_status reef_graph_upload(reef_graph_t g, reef_stream_t s) {
+    CK(cudaGraphUpload(((reef_graph_s*)g)->exec, (cudaStream_t)s));
+    CK(cudaStreamSynchronize((cudaStream_t)s));
+    return REEF_SUCC;
+}
 reef_status reef_graph_destroy(reef_graph_t g) {
     reef_graph_s* h = (reef_graph_s*)g;
     if (!h) return REEF_SUCC;

@@ -213,8 +213,11 @@ public:
     // small kernels: 77 us kernel by kernel, 67 us)
     Status execute(GPUStream_t stream = nullptr);
     // the whole kernel list on `stream`: launched kernel by kernel the first time, then captured as a CUDA graph and
-    // replayed
+    // replayed.  build_graph captures it ahead of the first pass, for launches on `stream`, on a stream `cap` of the same
+    // kind with nothing on it: a server's requests then never wait for a capture.
     Status execute_graph(GPUStream_t stream);
+    Status build_graph(GPUStream_t cap, GPUStream_t stream);
+    bool has_graph(GPUStream_t stream) const { return graph != nullptr && graph_stream == stream; }
     // every kernel through the dispatcher without a best-effort partner, then sync
     Status execute_dispatch(GPUStream_t stream = nullptr);
     // best-effort run, flag raised after delay_us, resumed from the first incomplete kernel until done

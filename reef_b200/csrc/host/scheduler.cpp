@@ -232,22 +232,22 @@ Status REEFScheduler::bind_model_queue(const QueueID& qid, const ModelID& mid) {
             return Status::Fail;
         }
     }
-    if (qid != rt_queue_id) return capture_graphs(*model_pool[mid]);
-    return Status::Succ;
+    return capture_graphs(*model_pool[mid], qid == rt_queue_id);
 }
 
-// The graphs of a best-effort model, captured before its requests come: the segments of its window and, under dynamic
-// kernel padding, its padding segments.  On a stream of their own, since the queue's may be at work for another model; of
-// the queue's kind, since a captured kernel keeps the priority and the SM partition of the stream of its capture (segments
-// captured on any other stream ran on every SM: ResNet-50 with 16 SMs set aside for best-effort work 5300 inf/s, as
-// without a partition, where single launches gave 690).
-Status REEFScheduler::capture_graphs(Model& model) {
+// The graphs of a model, captured before its requests come: the whole pass of a real-time model, the window segments and
+// (under dynamic kernel padding) the padding segments of a best-effort one.  On a stream of their own, since the queue's
+// may be at work for another model; of the queue's kind, since a captured kernel keeps the priority and the SM partition of
+// the stream of its capture (segments captured on any other stream ran on every SM: ResNet-50 with 16 SMs set aside for
+// best-effort work 5300 inf/s, as without a partition, where single launches gave 690).
+Status REEFScheduler::capture_graphs(Model& model, bool rt) {
     auto& exe = model.executor;
+    if (rt && (rt_queue.get() == nullptr || !(rt_graph || mode == ScheduleMode::REEF))) return Status::Succ;
     executor::GPUStream_t cap = nullptr;
-    RETURN_STATUS(make_stream(false, &cap));
-    const char* what = "best-effort segments: ";
-    Status st = exe.build_be_segments(cap);
-    if (st == Status::Succ && mode == ScheduleMode::REEF) {
+    RETURN_STATUS(make_stream(rt, &cap));
+    const char* what = rt ? "real-time graph: " : "best-effort segments: ";
+    Status st = rt ? exe.build_graph(cap, rt_queue->stream) : exe.build_be_segments(cap);
+    if (st == Status::Succ && !rt && mode == ScheduleMode::REEF) {
         what = "padding segments: ";
         st = exe.build_pad_segments(cap);
     }
@@ -719,6 +719,8 @@ void REEFScheduler::execute_rt_task(std::shared_ptr<Task>& task) {
     if (n_rt_tasks > 0) rt_pause_ns[n_rt_tasks % 4] = ns_since(last_rt_finish);
     auto& exe = task->model->executor;
     bool ok = true;
+    // a model that was never bound (it has the real-time queue by default) gets its graph here, before any clock below runs
+    if (!exe.has_graph(rt_queue->stream)) capture_graphs(*task->model, true);
     if (mode == ScheduleMode::REEF && any_be_waiting() && side_padding_needed(exe)) {
         // the graph goes out first; the best-effort streams are preempted while it starts up
         ok = timeline_padding(task);

@@ -209,7 +209,7 @@ private:
 
     Status make_stream(bool rt, executor::GPUStream_t* stream);
     Status create_task_queue(std::shared_ptr<TaskQueue>& ret, bool rt);
-    Status capture_graphs(Model& model);
+    Status capture_graphs(Model& model, bool rt);
     void loop_body();
     void execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr<TaskQueue>& tqueue);
     void execute_rt_task(std::shared_ptr<Task>& task);

@@ -305,3 +305,30 @@ def test_best_effort_segments_stay_in_their_partition(gen):
         s.shutdown()
         s.close()
     assert rate[16] < rate[0] / 2, rate
+
+
+@pytest.mark.parametrize("bound", [True, False])
+def test_real_time_graph_is_captured_before_the_first_request(gen, bound):
+    """Binding a model to the real-time queue captures its graph: the first request replays it already (a model that was
+    never bound captures it ahead of its first request's clock).  Seen through an injected failure, which says whether it
+    hit the replay of a graph or the launch of a kernel."""
+    base = gen("resnet18_64")
+    x = seeded_input(3 * 64 * 64, seed=13)
+    s = S(S.REEF)
+    s.run()
+    rt = s.load_model_files(base + ".json", base + ".profile.json", base + ".param")
+    if bound:
+        s.bind_model_queue(s.create_queue(S.RealTimeQueue), rt)
+    s.set_input(rt, x)
+    s.inject_launch_failures(rt, 1)
+    with pytest.raises(capi.ReefError):
+        s.wait_task(s.new_task(rt))
+    assert "graph launch failure" in s._err()
+    outs = []
+    for _ in range(3):
+        s.wait_task(s.new_task(rt))
+        outs.append(s.get_output(rt))
+    assert rel_err(outs[0], _oracle_out(base, x)) < tol_for(base)
+    assert all(np.array_equal(o, outs[0]) for o in outs)
+    s.shutdown()
+    s.close()
