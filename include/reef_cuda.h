@@ -96,8 +96,11 @@ REEF_API reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g);
  * from[e] == i and to[e] == j for some e (indices in capture order, from < to), so that independent branches of a model
  * run side by side.  An edge between two kernels is a programmatic one (the later kernel's prologue overlaps the earlier
  * kernel, as between neighbours of the captured stream); every kernel of this library waits for its predecessors before
- * it touches memory, so an order that follows from other edges needs none of its own. */
-REEF_API reef_status reef_graph_end_relaxed(reef_stream_t s, const int* from, const int* to, size_t num_edges, reef_graph_t* g);
+ * it touches memory, so an order that follows from other edges needs none of its own.  num_launches = the launches that
+ * the edges count: a capture of more or fewer nodes (a launch that issued two, an empty one) is refused, since every later
+ * index would name the wrong one. */
+REEF_API reef_status reef_graph_end_relaxed(reef_stream_t s, size_t num_launches, const int* from, const int* to, size_t num_edges,
+                                            reef_graph_t* g);
 REEF_API reef_status reef_graph_launch(reef_graph_t g, reef_stream_t s);
 /* brings the graph to the device ahead of its first launch, which otherwise does it; returns when it is there */
 REEF_API reef_status reef_graph_upload(reef_graph_t g, reef_stream_t s);

@@ -447,9 +447,18 @@ reef_status reef_graph_end(reef_stream_t s, reef_graph_t* g) {
     return graph_instantiate(graph, g);
 }
 // The captured chain of nodes in order, its edges replaced by the given ones.
-static reef_status graph_relax(cudaGraph_t graph, const int* from, const int* to, size_t num_edges) {
+static reef_status graph_relax(cudaGraph_t graph, size_t num_launches, const int* from, const int* to, size_t num_edges) {
     size_t n = 0, roots = 1;
     CK(cudaGraphGetNodes(graph, nullptr, &n));
+    if (n != num_launches) {
+        set_error("reef_graph_end_relaxed: " + std::to_string(n) + " nodes captured where the edges count " + std::to_string(num_launches) + " launches");
+        return REEF_FAIL;
+    }
+    for (size_t e = 0; e < num_edges; e++)
+        if (from[e] < 0 || from[e] >= to[e] || (size_t)to[e] >= n) {
+            set_error("reef_graph_end_relaxed: edge outside the captured launches");
+            return REEF_OUT_OF_RANGE;
+        }
     if (n < 2) return REEF_SUCC;
     std::vector<cudaGraphNode_t> order(n), a, b;
     std::vector<cudaGraphEdgeData> edge;
@@ -481,10 +490,6 @@ static reef_status graph_relax(cudaGraph_t graph, const int* from, const int* to
     b.clear();
     edge.clear();
     for (size_t e = 0; e < num_edges; e++) {
-        if (from[e] < 0 || from[e] >= to[e] || (size_t)to[e] >= n) {
-            set_error("reef_graph_end_relaxed: edge outside the captured launches");
-            return REEF_OUT_OF_RANGE;
-        }
         cudaGraphEdgeData d;
         memset(&d, 0, sizeof(d));
         if (kernel[from[e]] && kernel[to[e]]) {
@@ -498,11 +503,12 @@ static reef_status graph_relax(cudaGraph_t graph, const int* from, const int* to
     if (num_edges) CK(cudaGraphAddDependencies_v2(graph, a.data(), b.data(), edge.data(), num_edges));
     return REEF_SUCC;
 }
-reef_status reef_graph_end_relaxed(reef_stream_t s, const int* from, const int* to, size_t num_edges, reef_graph_t* g) {
+reef_status reef_graph_end_relaxed(reef_stream_t s, size_t num_launches, const int* from, const int* to, size_t num_edges,
+                                   reef_graph_t* g) {
     *g = nullptr;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamEndCapture((cudaStream_t)s, &graph));
-    reef_status rc = graph_relax(graph, from, to, num_edges);
+    reef_status rc = graph_relax(graph, num_launches, from, to, num_edges);
     if (rc != REEF_SUCC) {
         cudaGraphDestroy(graph);
         return rc;

@@ -610,7 +610,8 @@ Status HybridExecutor::build_be_segments(GPUStream_t cap) {
                 seg_to.push_back(to[e] - k0);
             }
         reef_graph_t g = nullptr;
-        if (reef_graph_end_relaxed(cap, seg_from.data(), seg_to.data(), seg_from.size(), &g) != REEF_SUCC) {
+        const size_t launches = (size_t)(k1 - k0) + (k1 == n && mirror ? 1 : 0);
+        if (reef_graph_end_relaxed(cap, launches, seg_from.data(), seg_to.data(), seg_from.size(), &g) != REEF_SUCC) {
             err_ = reef_last_error();
             st = Status::Fail;
         }
@@ -879,7 +880,7 @@ Status HybridExecutor::build_graph(GPUStream_t cap, GPUStream_t stream) {
     if (st == Status::Succ) st = issue_mirror(cap);
     std::vector<int> from, to;
     const bool relaxed = st == Status::Succ && chains.empty() && schedule_edges(&from, &to) == Status::Succ;
-    int rc = relaxed ? reef_graph_end_relaxed(cap, from.data(), to.data(), from.size(), &graph) : reef_graph_end(cap, &graph);
+    int rc = relaxed ? reef_graph_end_relaxed(cap, num_kernels() + (mirror ? 1 : 0), from.data(), to.data(), from.size(), &graph) : reef_graph_end(cap, &graph);
     if (st != Status::Succ || rc != REEF_SUCC) {
         // a launch failed while capturing: what was captured is a partial graph and must never be replayed
         if (rc != REEF_SUCC && st == Status::Succ) err_ = reef_last_error();

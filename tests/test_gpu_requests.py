@@ -1,6 +1,7 @@
 """Requests through host memory: staged input, output mirror, graph replay behind the first pass.  A one-kernel model that
 copies its input makes every byte of the way visible; sizes straddle the two-piece split of the staging copy, the limit
 between the mirror's copy kernel and the copy engine, and the limit of the pinned buffers."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -203,3 +204,35 @@ def test_branches_side_by_side(gen, model):
     assert capi.device_error() == 0
     s.close()
     e.close()
+
+
+def test_relaxed_graph_counts_its_launches():
+    """The edges of a relaxed graph are indices of launches: a capture with another number of nodes than launches, or an
+    edge beyond them, is refused (here on a capture of three 4-byte memsets)."""
+    lib = capi.cuda_lib()
+    assert lib.reef_gpu_init(C.c_int(0)) == capi.SUCC
+    stream, buf = C.c_void_p(), C.c_uint64()
+    assert lib.reef_stream_create(C.byref(stream), C.c_int(0)) == capi.SUCC
+    assert lib.reef_malloc(C.byref(buf), C.c_size_t(12)) == capi.SUCC
+
+    def end(launches, edges):
+        assert lib.reef_graph_begin(stream) == capi.SUCC
+        for i in range(3):
+            assert lib.reef_memset_async(C.c_uint64(buf.value + 4 * i), C.c_int(i + 1), C.c_size_t(4), stream) == capi.SUCC
+        graph = C.c_void_p()
+        a, b = ((C.c_int * len(edges))(*[e[i] for e in edges]) for i in (0, 1))
+        rc = lib.reef_graph_end_relaxed(stream, C.c_size_t(launches), a, b, C.c_size_t(len(edges)), C.byref(graph))
+        return rc, graph
+
+    for launches, edges, status in ((2, [(0, 1)], capi.FAIL), (4, [(0, 1), (1, 2)], capi.FAIL), (3, [(0, 3)], capi.OUT_OF_RANGE),
+                                    (3, [(1, 1)], capi.OUT_OF_RANGE), (3, [(-1, 1)], capi.OUT_OF_RANGE)):
+        rc, graph = end(launches, edges)
+        assert rc == status and not graph.value
+    rc, graph = end(3, [(0, 2)])
+    assert rc == capi.SUCC and lib.reef_graph_launch(graph, stream) == capi.SUCC
+    assert lib.reef_stream_sync(stream) == capi.SUCC
+    got = np.zeros(12, np.uint8)
+    assert lib.reef_memcpy_d2h(got.ctypes.data_as(C.c_void_p), buf, C.c_size_t(12)) == capi.SUCC
+    assert got.tolist() == [1] * 4 + [2] * 4 + [3] * 4
+    for rc in (lib.reef_graph_destroy(graph), lib.reef_free(buf), lib.reef_stream_destroy(stream)):
+        assert rc == capi.SUCC
