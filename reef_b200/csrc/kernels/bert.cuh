@@ -349,6 +349,35 @@ __device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned 
     if (row0 + row < S) {
         const float inv = 1.0f / sum;
         o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+        if (split_sum_lost((o.x + o.y) + (o.z + o.w))) {
+            // by fp32 multiply-adds: the row's largest score, then its probabilities and their sum over the values
+            const float* q = base + (size_t)(row0 + row) * 3 * H;
+            float high = ninf, total = 0.f;
+            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (int pass = 0; pass < 2; pass++)
+#pragma unroll 1
+                for (int key = 0; key < S; key++) {
+                    const float* kv = base + (size_t)key * 3 * H + H;
+                    float sc = 0.f;
+#pragma unroll 1
+                    for (int i = 0; i < kAttD; i++) sc = fmaf(q[i], kv[i], sc);
+                    sc = mask && mask[key] == 0.f ? ninf : sc * scale;
+                    if (pass == 0) {
+                        high = fmaxf(high, sc);
+                        continue;
+                    }
+                    const float pr = sc == ninf ? 0.f : expf(sc - high);
+                    const float4 v = *reinterpret_cast<const float4*>(kv + H + d0);
+                    total += pr;
+                    e.x = fmaf(pr, v.x, e.x); e.y = fmaf(pr, v.y, e.y); e.z = fmaf(pr, v.z, e.z); e.w = fmaf(pr, v.w, e.w);
+                }
+            const float by = 1.0f / total;
+            if (split_sum_lost(o.x)) o.x = e.x * by;
+            if (split_sum_lost(o.y)) o.y = e.y * by;
+            if (split_sum_lost(o.z)) o.z = e.z * by;
+            if (split_sum_lost(o.w)) o.w = e.w * by;
+        }
         *reinterpret_cast<float4*>(out + (size_t)(row0 + row) * H + head * kAttD + d0) = o;
     }
     return true;

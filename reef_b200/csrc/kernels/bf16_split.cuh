@@ -2,11 +2,20 @@
 // values (8 + 8 + 8 significand bits), a product of two values the sum of nine bf16 products, each of them exact in fp32.
 // Six of the nine are computed; the three left out together stay below 2^-26 of |a b|, under half of what one fp32
 // rounding loses.
+//
+// That holds for the values that three bf16 values can carry.  bf16 has the exponents of fp32, but from 3.3962e38 on a
+// finite value (up to 3.4028e38) rounds to infinity, and the remainders of an infinity are NaN, also where fp32 instructions
+// would give infinity.  A sum with such an operand always ends as infinity or NaN: whoever computes sums this way looks at
+// each result once and repeats it with fp32 instructions where it is not finite (split_sum_lost).  At the other end, of
+// |x| below 2^-110 what lies under 2^-134 is dropped.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace reef {
+
+// an operand was beyond what bf16 carries, or the sum itself is not finite
+__device__ __forceinline__ bool split_sum_lost(float x) { return !(fabsf(x) <= 3.402823466e38f); }
 
 // x = the exact sum of three bf16 values, two values of x at a time (first in the lower half)
 struct Bf16Triple {

@@ -239,6 +239,27 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
             const float4 x = *reinterpret_cast<const float4*>(src + (size_t)g * TP * PROW);
             v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
         }
+        if (split_sum_lost((v.x + v.y) + (v.z + v.w))) {
+            // by fp32 multiply-adds over the taps inside the image (co is a multiple of four, p.co too)
+            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int oy = op / p.wo, iy0 = oy * p.sh - p.ph, ix0 = (op - oy * p.wo) * p.sw - p.pw;
+            const float* w = wgt + (size_t)co * p.ktot;
+#pragma unroll 1
+            for (int k = 0; k < p.ktot; k++, w++) {
+                const int tap = k / p.ci, ch = k - tap * p.ci, ty = tap / p.kw;
+                const int iy = iy0 + ty, ix = ix0 + tap - ty * p.kw;
+                if (iy < 0 || iy >= p.hi || ix < 0 || ix >= p.wi) continue;
+                const float x = in[p.nchw ? (ch * p.hi + iy) * p.wi + ix : (iy * p.wi + ix) * p.ics + p.ioff + ch];
+                e.x = fmaf(x, w[0], e.x);
+                e.y = fmaf(x, w[p.ktot], e.y);
+                e.z = fmaf(x, w[2 * p.ktot], e.z);
+                e.w = fmaf(x, w[3 * p.ktot], e.w);
+            }
+            if (split_sum_lost(v.x)) v.x = e.x;
+            if (split_sum_lost(v.y)) v.y = e.y;
+            if (split_sum_lost(v.z)) v.z = e.z;
+            if (split_sum_lost(v.w)) v.w = e.w;
+        }
         float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
         if (p.ep & EP_GB) {
             sc = *reinterpret_cast<const float4*>((const float*)t.a[p.i_gamma] + co);
