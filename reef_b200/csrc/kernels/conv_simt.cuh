@@ -233,6 +233,15 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
         const int c4 = item % (TC / 4), row = item / (TC / 4);       // row: pixel within the block
         const int sub = row / TP, op = tile_p * (8 / KG) * TP + row, co = c0 + c4 * 4;
         if (op >= p.ptot || co >= p.co) continue;
+        float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.ep & EP_GB) {
+            sc = *reinterpret_cast<const float4*>((const float*)t.a[p.i_gamma] + co);
+            sh = *reinterpret_cast<const float4*>((const float*)t.a[p.i_beta] + co);
+        } else if (p.ep & EP_BIAS) {
+            sh = *reinterpret_cast<const float4*>((const float*)t.a[p.i_bias] + co);
+        }
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (res) r = *reinterpret_cast<const float4*>(res + (size_t)op * p.co + co);
         const float* src = ring + (size_t)(sub * KG * TP + row - sub * TP) * PROW + c4 * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int g = 0; g < KG; g++) {                               // fixed order: deterministic
@@ -260,15 +269,6 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
             if (split_sum_lost(v.z)) v.z = e.z;
             if (split_sum_lost(v.w)) v.w = e.w;
         }
-        float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p.ep & EP_GB) {
-            sc = *reinterpret_cast<const float4*>((const float*)t.a[p.i_gamma] + co);
-            sh = *reinterpret_cast<const float4*>((const float*)t.a[p.i_beta] + co);
-        } else if (p.ep & EP_BIAS) {
-            sh = *reinterpret_cast<const float4*>((const float*)t.a[p.i_bias] + co);
-        }
-        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (res) r = *reinterpret_cast<const float4*>(res + (size_t)op * p.co + co);
         v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
         if (p.ep & EP_GB) {
             // explicit fused multiply-add: the three flavours of this body are compiled in different
