@@ -145,22 +145,32 @@ def test_model_totals_match_the_published_architectures(libs, tmp_path):
     assert t50["tensor_core_kernels"] == 53 and t50["hbm_floor_us_nominal"] > t50["tf32_floor_us_nominal"]
 
 
-def test_tuned_plan_table_is_consistent(libs):
-    """Every measured plan in the table resolves in the registry, keeps the family's argument count, and is what
-    the generator writes into the schedule; REEF_UNTUNED keeps the bare names."""
+def test_tuned_plan_table_is_consistent(libs, tmp_path, monkeypatch):
+    """Every measured plan in a table that the tuner has written resolves in the registry, keeps the family's argument
+    count, and is what the generator writes into the schedule; REEF_UNTUNED keeps the bare names.  (No table is shipped:
+    the planner's own choice is within what replays vary by for every layer that was tuned.)"""
     import json
     import os
     from reef_b200 import capi, resources, tune
+    from reef_b200.resources import graph
     from reef_b200.resources.graph import tuned_plan
-    path = os.path.join(os.path.dirname(resources.__file__), "tuned_plans.json")
+    path = str(tmp_path / "tuned_plans.json")
+    names = ["fused_nn_conv2d_add_nn_relu__ci%d_hi%d_wi%d_co%d_kh3_kw3_sh1_sw1_ph1_pw1_v1" % s
+             for s in ((128, 56, 56, 256), (512, 14, 14, 512), (96, 35, 35, 96), (64, 61, 83, 64))]
+    tune._write_table({"plans": dict(zip(names, ([96, 2], [64, 8], [48, 4], [112, 1]))),
+                       "measured_us": {n: [6.0, 5.0] for n in names}, "models_ms": {}}, path)
     table = json.load(open(path))
-    assert table["plans"], "the committed table holds the measured plans"
+    assert table["plans"], "the table holds the measured plans"
+    monkeypatch.setattr(graph, "_TUNED", table["plans"])
     for name, (tp, ts) in table["plans"].items():
         assert name in table["measured_us"] and table["measured_us"][name][1] <= table["measured_us"][name][0]
         d0, _, n0 = capi.kernel_plan(name)
         d1, smem, n1 = capi.kernel_plan(f"{name}_tp{tp}_ts{ts}")
         assert n0 == n1 and smem <= 112 * 1024 and d1[3] == 256
         assert tuned_plan(name) == dict(tp=tp, ts=ts)
+        monkeypatch.setenv("REEF_UNTUNED", "1")
+        assert tuned_plan(name) == {}
+        monkeypatch.delenv("REEF_UNTUNED")
     # candidates(): the default plan first, then distinct (grid, shared memory) alternatives within 24..300 CTAs
     c = tune.candidates("fused_nn_conv2d_add_nn_relu__ci256_hi14_wi14_co256_kh3_kw3_sh1_sw1_ph1_pw1_v1")
     assert c[0][0] is None and len(c) > 4 and len({(g, s) for _, g, s in c[1:]}) == len(c) - 1
