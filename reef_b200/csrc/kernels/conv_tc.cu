@@ -69,7 +69,9 @@ static int tc_plan_cap(const ConvP& p, int cap, int want, TcPlan* pl) {
     // Shared memory: at most TC_SMEM_CAP per CTA, so that two CTAs fit one SM (a real-time kernel beside the
     // early-launched prologue of its successor, or beside a best-effort kernel).  The stage ring is reused by
     // the epilogue for the staged accumulator tile (one 512-byte row per pixel) and, with a K split, the
-    // exchange area recv[S-1][cpc_max][128].
+    // exchange area recv[S-1][cpc_max][128].  That area is the chain kernel's (conv_tc_chain.cuh); the launches of one layer
+    // read their partials from distributed shared memory and leave it unused.  It counts for both all the same: a chain
+    // gives its layers' results bit for bit, so a layer has one plan, and it must fit either kernel.
     const int budget = TC_SMEM_CAP - 1024 - 256;   // alignment slack and control words
     const int stage_bytes = TC_A_BYTES + pl->n_mma * 128;
     pl->stages = pl->kb_per_split < TC_MAX_STAGES ? pl->kb_per_split : TC_MAX_STAGES;

@@ -36,8 +36,6 @@ namespace reef {
 
 enum : int { TC_EP_RES = 1, TC_EP_BIAS = 2, TC_EP_GB = 4, TC_EP_RELU = 8, TC_EP_ROUND = 16, TC_EP_GELU = 32 };
 
-// Branch-free form of (+residual) (+bias | *gamma+beta) (ReLU): r = 0, sc = 1, sh = 0, lo = -inf stand in for
-// the absent terms (v + 0 and fma(v, 1, b) are exact, so this equals the conditional form bit for bit).
 // exact-erf GELU (reference: resource/bert/bert.cu:167-173).  Not inlined here on purpose: inlined, the compiler turned
 // the uniform `if (gelu)` of the epilogue into straight-line code and every layer paid for erff on each element
 // (0.5 us per launch on the row-finishing loop).  Where a whole loop is for GELU layers (tc_finish_rows) it is inlined:
@@ -45,23 +43,8 @@ enum : int { TC_EP_RES = 1, TC_EP_BIAS = 2, TC_EP_GB = 4, TC_EP_RELU = 8, TC_EP_
 __device__ __forceinline__ float tc_gelu_inline(float v) { return v * (0.5f * erff(v * 0.70710678118654752440f) + 0.5f); }
 static __device__ __noinline__ float tc_gelu(float v) { return tc_gelu_inline(v); }
 
-__device__ __forceinline__ float tc_epilogue(float v, float r, float sc, float sh, float lo, bool rnd, bool gelu = false) {
-    if (gelu) {
-        // matmul + bias -> GELU -> (+residual)
-        v = tc_gelu(v + sh) + r;
-    } else {
-        v = fmaxf(fmaf(v + r, sc, sh), lo);
-    }
-    if (rnd) {
-        // The tensor core reads only the upper 19 bits of an fp32 operand (truncation, a bias toward zero).
-        // Rounding the stored activation to the nearest TF32 value makes the consumer's truncation exact.
-        uint32_t u;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
-        v = __uint_as_float(u);
-    }
-    return v;
-}
-
+// The tensor core reads only the upper 19 bits of an fp32 operand (truncation, a bias toward zero).  Rounding the stored
+// activation to the nearest TF32 value makes the consumer's truncation exact.
 __device__ __forceinline__ float4 tc_round4(float4 o) {
     uint32_t u;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.x)); o.x = __uint_as_float(u);
@@ -71,7 +54,10 @@ __device__ __forceinline__ float4 tc_round4(float4 o) {
     return o;
 }
 
-// the same on the 4 channels of a lane at once: one uniform branch per pixel row instead of one per element
+// Branch-free form of (+residual) (+bias | *gamma+beta) (ReLU): r = 0, sc = 1, sh = 0, lo = -inf stand in for
+// the absent terms (v + 0 and fma(v, 1, b) are exact, so this equals the conditional form bit for bit).
+// The 4 channels of a lane at once: one uniform branch per pixel row instead of one per element.  With GELU: matmul + bias ->
+// GELU -> (+residual).
 __device__ __forceinline__ float4 tc_epilogue4(float4 v, float4 r, float4 sc, float4 sh, float lo, bool rnd, bool gelu) {
     float4 o;
     if (gelu) {
@@ -81,28 +67,14 @@ __device__ __forceinline__ float4 tc_epilogue4(float4 v, float4 r, float4 sc, fl
         o.x = fmaxf(fmaf(v.x + r.x, sc.x, sh.x), lo); o.y = fmaxf(fmaf(v.y + r.y, sc.y, sh.y), lo);
         o.z = fmaxf(fmaf(v.z + r.z, sc.z, sh.z), lo); o.w = fmaxf(fmaf(v.w + r.w, sc.w, sh.w), lo);
     }
-    if (rnd) {
-        uint32_t u;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.x)); o.x = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.y)); o.y = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.z)); o.z = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(o.w)); o.w = __uint_as_float(u);
-    }
-    return o;
+    return rnd ? tc_round4(o) : o;
 }
 
 // second output of the dual epilogue: relu(o + b2), rounded like the first when the layer rounds
 __device__ __forceinline__ float4 tc_preact(float4 o, float4 b2, bool rnd) {
     float4 r;
     r.x = fmaxf(o.x + b2.x, 0.f); r.y = fmaxf(o.y + b2.y, 0.f); r.z = fmaxf(o.z + b2.z, 0.f); r.w = fmaxf(o.w + b2.w, 0.f);
-    if (rnd) {
-        uint32_t u;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(r.x)); r.x = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(r.y)); r.y = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(r.z)); r.z = __uint_as_float(u);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(r.w)); r.w = __uint_as_float(u);
-    }
-    return r;
+    return rnd ? tc_round4(r) : r;
 }
 
 

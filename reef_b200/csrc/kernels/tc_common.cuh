@@ -53,31 +53,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
-// The same wait for the best-effort flavour's MMA thread: it also gives up when `abort_word` (shared memory, written
-// by the TMA producer of the same CTA when it saw the preempt flag) becomes non-zero.  0 = phase complete,
-// 1 = wait expired, 2 = abort requested.
-__device__ __forceinline__ int mbar_wait_abortable(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word) {
-    unsigned long long t0 = 0;
-    for (int i = 0; i < (1 << 26); i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return 0;
-        if (*abort_word) return 2;
-        if ((i & 255) == 255) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > 1000000000ull) return 1;
-        }
-    }
-    return 1;
-}
 // The waits of a whole warp: every lane polls, the warp leaves together (the votes keep its control flow, and with it the
 // addresses and descriptors of what it issues next, warp-uniform).
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
@@ -104,7 +79,8 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
-// 0 = phase complete, 1 = wait expired, 2 = `abort_word` became non-zero (see mbar_wait_abortable)
+// The wait of the best-effort flavour's MMA warp also gives up when `abort_word` (shared memory, written by the TMA producer
+// of the same CTA when it saw the preempt flag) becomes non-zero.  0 = phase complete, 1 = wait expired, 2 = abort requested.
 __device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word) {
     unsigned long long t0 = 0;
     for (int i = 0; i < (1 << 26); i++) {
@@ -168,11 +144,6 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
 }
 // volatile keeps the load behind the cluster barrier (also a volatile asm); no "memory" clobber, so the
 // loads of one reduction batch are issued back to back and overlap
-__device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ float4 ld_dsmem_v4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
@@ -212,15 +183,6 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
