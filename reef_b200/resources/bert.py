@@ -80,10 +80,12 @@ def build_bert(*, name: str = "bert_base", layers: int = 12, hidden: int = 768, 
     for li in range(layers):
         att_attrs = dict(s=seq, heads=heads, d=hidden // heads)
         att_tc = False
-        # The exact-fp32 attention is the faster one while its blocks (16 query rows of a head each) fit the 148 SMs at once
-        # (12 heads of 128 tokens: 5.7 us against 7.8 us); with more heads than that the TF32 kernel's single block per
-        # head is, where the registry has the shape (<= 128 tokens).
-        if conv_impl != "simt" and heads * (-(-seq // 16)) > 148:
+        # The exact-fp32 attention while its blocks (16 query rows of a head each) are resident all at once: one to an SM up
+        # to 148 (12 heads of 128 tokens: 5.3 us, TF32 7.2), two beyond (24 heads of 128 tokens, 192 blocks: 7.0 and 7.8;
+        # the widest loss is 32 heads of 96 tokens, 7.0 and 6.5).  From 297 blocks on it takes a second turn and the TF32
+        # kernel's single block per head is faster (40 heads of 128 tokens, 320 blocks: 10.7 and 8.1; 64 heads: 13.4 and
+        # 7.5), where the registry has the shape (<= 128 tokens).
+        if conv_impl != "simt" and heads * (-(-seq // 16)) > 2 * 148:
             try:
                 capi.kernel_plan(kname("reef_attention", **att_attrs, v=1))
                 att_attrs["v"] = 1

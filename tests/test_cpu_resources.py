@@ -181,6 +181,15 @@ def test_tuned_plan_table_is_consistent(libs, tmp_path, monkeypatch):
         [("temp", 64 * 128), ("param", 128), ("temp", 64 * 128)]
 
 
+@pytest.mark.parametrize("heads,seq,tc", [(12, 128, False), (19, 128, False), (37, 128, False), (38, 113, True), (38, 129, False)])
+def test_attention_kernel_of_a_bert(libs, heads, seq, tc):
+    """TF32 attention from 297 blocks of 16 query rows on and up to 128 tokens, exact fp32 attention otherwise."""
+    from reef_b200.resources.bert import build_bert
+    b = build_bert(layers=1, hidden=64 * heads, heads=heads, ffn=64, vocab=8, seq=seq)
+    names = [k["name"] for k in b.g.kernels if k["name"].startswith("reef_attention")]
+    assert len(names) == 1 and names[0].endswith("_v1") == tc
+
+
 def test_estimate_slot_usage(libs, tmp_path):
     from reef_b200 import estimate, resources
     d = resources.generate("resnet18_64", str(tmp_path))
