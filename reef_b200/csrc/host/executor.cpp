@@ -1,6 +1,8 @@
 #include "executor.h"
 
+#ifdef __SSE2__
 #include <emmintrin.h>
+#endif
 
 #include <algorithm>
 #include <chrono>
@@ -262,8 +264,11 @@ Status ExecutorBase::set_input(const std::string& key, const void* value, size_t
 static const size_t kStageSplit = 128u << 10;
 // Host copy into the staging area.  Large pieces bypass the caches (streaming stores): lines left dirty in a core's
 // cache are snooped by the copy engine, and the next request's memcpy into them ran at half speed (602 KB: 26 us
-// against 21 us).  The staging area and the pieces are 64-byte aligned.
+// against 21 us).  The staging area and the pieces are 64-byte aligned.  (x86; a plain copy on other hosts.)
 static void stage_copy(unsigned char* dst, const unsigned char* src, size_t n) {
+#ifndef __SSE2__
+    memcpy(dst, src, n);
+#else
     if (n < (64u << 10)) {
         memcpy(dst, src, n);
         return;
@@ -279,6 +284,7 @@ static void stage_copy(unsigned char* dst, const unsigned char* src, size_t n) {
     }
     memcpy(dst + i, src + i, n - i);
     _mm_sfence();
+#endif
 }
 
 Status ExecutorBase::set_input(int idx, const void* value, size_t len) {
