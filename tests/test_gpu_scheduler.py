@@ -332,3 +332,47 @@ def test_real_time_graph_is_captured_before_the_first_request(gen, bound):
     assert all(np.array_equal(o, outs[0]) for o in outs)
     s.shutdown()
     s.close()
+
+
+@pytest.mark.parametrize("mode", [S.REEF, S.Reset, S.WaitPreempt])
+@pytest.mark.parametrize("model", ["inception_v3_139", "densenet121_64"])
+def test_preempted_inside_a_segment_of_a_branching_model(gen, model, mode):
+    """A best-effort task alone on the GPU is fed whole segments, whose branches run side by side: when a real-time request
+    comes out of a long pause, kernels later in the schedule may be complete while an earlier one is not.  Preempted at
+    many points (restarted from the segment, or in WaitPreempt mode from the first kernel whose counter is short), the
+    output is bit for bit that of an uninterrupted pass."""
+    base, rt_base = gen(model), gen("resnet18_64")
+    s = S(mode)
+    s.run()
+    rt = s.load_model_files(rt_base + ".json", rt_base + ".profile.json", rt_base + ".param")
+    be = s.load_model_files(base + ".json", base + ".profile.json", base + ".param")
+    s.bind_model_queue(s.create_queue(S.RealTimeQueue), rt)
+    s.bind_model_queue(s.create_queue(S.BestEffortQueue), be)
+    n = s.get_data_size(be, "data") // 4
+    x = seeded_input(n, seed=14)
+    s.set_input(rt, seeded_input(3 * 64 * 64, seed=15))
+    s.set_input(be, x)
+    s.wait_task(s.new_task(be))
+    want = s.get_output(be)
+    s.wait_task(s.new_task(rt))
+    rt_want = s.get_output(rt)
+    preempted = 0
+    for i in range(40):
+        time.sleep(0.03)        # no real-time request is expected any more: the window holds whole segments
+        s.set_input(be, np.zeros(n, np.float32) if i % 2 else x)
+        t_be = s.new_task(be)
+        t0 = time.perf_counter()
+        while time.perf_counter() - t0 < 15e-6 * i:
+            pass
+        t_rt = s.new_task(rt)
+        s.wait_task(t_rt)
+        s.wait_task(t_be)
+        preempted += s.get_task(t_be).preempted
+        assert np.array_equal(s.get_output(rt), rt_want)
+        if i % 2 == 0:
+            assert np.array_equal(s.get_output(be), want), f"preempted after {15 * i} us"
+    print(model, mode, "preempted", preempted, "of 40")
+    assert preempted > 0
+    assert capi.device_error() == 0
+    s.shutdown()
+    s.close()
