@@ -738,7 +738,7 @@ void REEFScheduler::execute_rt_task(std::shared_ptr<Task>& task) {
                 ok = false;
             }
             if (reef_stream_sync(rt_queue->stream) != REEF_SUCC) ok = false;
-            if (ok) task->model->add_alone_sample((double)ns_since(t0));
+            if (ok) task->model->baseline.add_alone((double)ns_since(t0));
         } else if (exe.execute_to((int)exe.num_kernels(), rt_queue->stream) != Status::Succ) {
             err_ = "real-time launch failed: " + exe.error();
             ok = false;
@@ -1060,11 +1060,11 @@ bool REEFScheduler::timeline_padding(std::shared_ptr<Task>& rt_task) {
     const uint64_t window_ns = ns_since(t0);
     pad_trace.window_ns += window_ns;
     if (probe) {
-        rt_model.add_alone_sample((double)window_ns);
+        rt_model.baseline.add_probe((double)window_ns);
     } else if (drain_only) {
     } else if (pad_target > 0 && model_ns > 0) {
         // slowdown controller: one multiplicative step per window on the kernel rate
-        const double baseline = rt_model.alone_ns() > 0.0 ? rt_model.alone_ns() : 1.02 * model_ns;
+        const double baseline = rt_model.baseline.ns() > 0.0 ? rt_model.baseline.ns() : 1.02 * model_ns;
         const double ratio = (double)window_ns / baseline;
         pad_ratio_ema = pad_ratio_ema == 0.0 ? ratio : 0.8 * pad_ratio_ema + 0.2 * ratio;
         if (pad_ratio_ema > 1.0 + pad_target) pad_rate *= 0.97;

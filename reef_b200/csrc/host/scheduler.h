@@ -23,6 +23,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "baseline.h"
 #include "common.h"
 #include "executor.h"
 #include "threadsafe_queue.h"
@@ -170,19 +171,8 @@ private:
     struct Model {
         executor::HybridExecutor executor;
         QueueID qid;
-        // real-time models: host-observed duration of an unpadded graph replay (ns), the baseline of the padding
-        // slowdown controller = the smallest of the last four samples (anything that disturbs a sample makes it
-        // longer).  Sampled by every replay that runs without best-effort work and by unpadded probe windows.
-        double alone_samples[4] = {0, 0, 0, 0};
-        uint32_t alone_count = 0;
+        ReplayBaseline baseline;    // real-time models: host-observed duration of unpadded graph replays
         uint32_t pad_windows = 0;
-        void add_alone_sample(double ns) { alone_samples[alone_count++ % 4] = ns; }
-        double alone_ns() const {
-            double m = 0.0;
-            for (double v : alone_samples)
-                if (v > 0.0 && (m == 0.0 || v < m)) m = v;
-            return m;
-        }
     };
     static const uint32_t kPadProbePeriod = 64;
     struct InFlight {
