@@ -804,15 +804,18 @@ bool REEFScheduler::side_padding_needed(HybridExecutor& rt_exe) {
 // Dynamic kernel padding when a tensor-core (cluster) kernel is involved on either side.  Such kernels are
 // not hosted by the logical-block dispatcher, so the padding is done in space and time by separate launches:
 //  * the real-time task replays its CUDA graph on the high-priority stream (full speed, no per-kernel host
-//    work).  Its kernels release their successor only after their own dependency wait, so at most two grids
-//    of the chain are resident: the running one and the prologue of the next;
+//    work).  Its kernels release their successors only after their own dependency wait, so that of each branch at
+//    most two grids are resident: the running one and the prologue of the next;
 //  * while it runs, this thread issues best-effort PIECES (block ranges of a queue's head kernel, whole
 //    kernels where they fit) on that queue's own low-priority stream, up to `pad_depth` per stream so that the
 //    stream never idles for a launch round trip.  Pieces of one stream run one after the other;
 //  * space is accounted in SM slots (two tensor-core CTAs fit one SM): the streams with pieces out may
 //    together occupy what the real-time kernels of the next `pad_window` positions leave free (position =
 //    elapsed time mapped onto the measured latency profile; reference policy scheduler.cpp:566-595 restated
-//    for a free-running real-time stream);
+//    for a free-running real-time stream).  Positions are counted in schedule order, a kernel and the next, also
+//    where the graph runs branches side by side: an estimate, which the rate limit corrects.  (Laid out along the
+//    graph's own edges, with all branches counted, the same target gave less: Inception-v3 over VGG-16 and
+//    DenseNet-201 255 best-effort inf/s instead of 270, ResNet-152 over 4 ResNet-152 520 instead of 655);
 //  * a queue that has issued `pad_quantum` pieces drains and yields, so every best-effort client advances.
 // Pieces are launched in the plain flavour (they do not poll the preempt flag; they are short and sized to the
 // free slots) and count into the task's completion slots.
