@@ -376,3 +376,25 @@ def test_preempted_inside_a_segment_of_a_branching_model(gen, model, mode):
     assert capi.device_error() == 0
     s.shutdown()
     s.close()
+
+
+def test_bound_graph_of_persistent_chains(gen):
+    """A real-time model whose tensor-core layers run as persistent chains: captured when it is bound, on another stream
+    than it is launched on; results are those of the launches, bit for bit."""
+    base = gen("resnet18_64")
+    x = seeded_input(3 * 64 * 64, seed=17)
+    outs = []
+    for clusters in (-1, 0):
+        s = S(S.REEF)
+        s.set_rt_chains(clusters)
+        s.run()
+        rt = s.load_model_files(base + ".json", base + ".profile.json", base + ".param")
+        s.bind_model_queue(s.create_queue(S.RealTimeQueue), rt)
+        for _ in range(3):
+            s.set_input(rt, x)
+            s.wait_task(s.new_task(rt))
+            outs.append(s.get_output(rt))
+        s.shutdown()
+        s.close()
+    assert all(np.array_equal(o, outs[0]) for o in outs)
+    assert capi.device_error() == 0
