@@ -69,15 +69,15 @@ static int tc_plan_cap(const ConvP& p, int cap, int want, TcPlan* pl) {
     // Shared memory: at most TC_SMEM_CAP per CTA, so that two CTAs fit one SM (a real-time kernel beside the
     // early-launched prologue of its successor, or beside a best-effort kernel).  The stage ring is reused by
     // the epilogue for the staged accumulator tile (one 512-byte row per pixel) and, with a K split, the
-    // exchange area recv[S-1][cpc_max][128].  That area is the chain kernel's (conv_tc_chain.cuh); the launches of one layer
-    // read their partials from distributed shared memory and leave it unused.  It counts for both all the same: a chain
+    // exchange area recv[S-1][cpc_max][128].  Both are the chain kernel's (conv_tc_chain.cuh); the launches of one layer
+    // stage nothing and have a receive area of their own (tc_place_recv).  They count for both all the same: a chain
     // gives its layers' results bit for bit, so a layer has one plan, and it must fit either kernel.
     const int budget = TC_SMEM_CAP - 1024 - 256;   // alignment slack and control words
     const int stage_bytes = TC_A_BYTES + pl->n_mma * 128;
     pl->stages = pl->kb_per_split < TC_MAX_STAGES ? pl->kb_per_split : TC_MAX_STAGES;
     while (pl->stages > 1 && pl->stages * stage_bytes > budget) pl->stages--;
     if (pl->stages * stage_bytes > budget || (pl->stages < 2 && pl->kb_per_split > 1)) return REEF_NOT_FOUND;
-    const int ring = pl->stages * stage_bytes;
+    int ring = pl->stages * stage_bytes;
     pl->cpc_max = ceil_div_i(pl->n_valid, pl->splits);
     pl->recv_offset_floats = pl->n_valid * TC_BM;
     const int epi = pl->n_valid * 512 + (pl->splits > 1 ? (pl->splits - 1) * pl->cpc_max * 512 : 0);
@@ -85,6 +85,29 @@ static int tc_plan_cap(const ConvP& p, int cap, int want, TcPlan* pl) {
     pl->region_bytes = ring > epi ? ring : epi;
     pl->region_bytes = ((pl->region_bytes + 127) / 128) * 128;
     pl->smem = 1024 + pl->region_bytes + 256;   // alignment slack + data region + control words
+    return REEF_SUCC;
+}
+
+// Where a plan's receive area goes (see TcParams::recv_offset).  Apart from the ring the peers may store into it at any time, over
+// the ring only behind a cluster barrier that stands between the accumulator and the exchange (0.25 us): apart wherever shared
+// memory has room for both, if need be with a stage less (3x3, 256 channels, 14x14: 4.5 us over five stages, 4.3 apart from four).
+// `earlier`: no more shared memory than the plan took when partials were read from the peers' staging tiles; schedules written
+// then state that size, and load with it.
+static int tc_place_recv(TcPlan* pl, bool earlier) {
+    const int budget = earlier ? pl->region_bytes : TC_SMEM_CAP - 1024 - 256;
+    const int stage_bytes = TC_A_BYTES + pl->n_mma * 128;
+    int ring = pl->stages * stage_bytes;
+    pl->gpc = ceil_div_i(ceil_div_i(pl->n_valid, 4), pl->splits);
+    const int recv = pl->splits > 1 ? pl->splits * pl->gpc * TC_BM * 16 : 0;
+    if (recv > budget) return REEF_NOT_FOUND;
+    if (!earlier && ring + recv > budget && pl->stages > 2 && ring - stage_bytes + recv <= budget) {
+        pl->stages--;
+        ring -= stage_bytes;
+    }
+    pl->recv_late = ring + recv > budget;
+    pl->recv_offset = pl->recv_late ? 0 : ring;
+    if (pl->recv_offset + recv > pl->region_bytes) pl->region_bytes = (pl->recv_offset + recv + 127) / 128 * 128;
+    pl->smem = 1024 + pl->region_bytes + 256;
     return REEF_SUCC;
 }
 
@@ -123,7 +146,8 @@ int tc_plan(const ConvP& p, TcPlan* pl) {
     if (p.plan_cap > 0) {
         // tile cap fixed by the kernel name (a tuned plan): that candidate or nothing
         if (p.plan_cap < 8 || p.plan_cap > 208) return REEF_NOT_FOUND;
-        return tc_plan_cap(p, p.plan_cap, p.plan_splits, pl);
+        const int rc = tc_plan_cap(p, p.plan_cap, p.plan_splits, pl);
+        return rc == REEF_SUCC ? tc_place_recv(pl, p.plan_earlier != 0) : rc;
     }
     TcPlan best;
     float best_cycles = 0.f;
@@ -142,7 +166,7 @@ int tc_plan(const ConvP& p, TcPlan* pl) {
         }
     if (best_cycles == 0.f) return REEF_NOT_FOUND;
     *pl = best;
-    return REEF_SUCC;
+    return tc_place_recv(pl, p.plan_earlier != 0);
 }
 
 // ---- tensor maps ---------------------------------------------------------------------------------
@@ -287,6 +311,10 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
     P->region_bytes = pl.region_bytes;
     P->recv_offset_floats = pl.recv_offset_floats;
     P->cpc_max = pl.cpc_max;
+    P->gpc = pl.gpc;
+    P->gpc_magic = (unsigned)((65536 + pl.gpc - 1) / pl.gpc);
+    P->recv_offset = pl.recv_offset;
+    P->recv_late = pl.recv_late;
     P->n_tiles = pl.n_tiles;
     P->tile_begin = 0;
     P->pdl = 1;
@@ -422,7 +450,7 @@ int tc_func_attrs(const TcPlan& pl, cudaFuncAttributes* fa, int* occ) {
         set_error(std::string("cudaFuncGetAttributes(conv_tc): ") + cudaGetErrorString(e));
         return REEF_FAIL;
     }
-    // shared memory (plus the 1 KB the hardware reserves per CTA) and 124 registers x 256 threads: two at most
+    // shared memory (plus the 1 KB the hardware reserves per CTA) and 128 registers x 256 threads: two at most
     const int by_smem = (228 * 1024) / (pl.smem + 1024);
     *occ = by_smem < 1 ? 1 : (by_smem > 2 ? 2 : by_smem);
     return REEF_SUCC;

@@ -10,17 +10,20 @@
 //
 // Batch-1 convolutions are tiny GEMMs (N = 49..3136 pixels), far too few tiles for 148 SMs and too
 // many weight bytes per tile for one SM's load bandwidth, so K is split across a thread-block
-// CLUSTER (1..8 CTAs).  Each CTA accumulates its K range in TMEM, parks the partial tile in its own
-// shared memory, and after a cluster barrier every CTA sums a slice of the tile over all ranks through
-// distributed shared memory in rank order 0..S-1 — a fixed order, so results are bit-reproducible (no
-// float atomics, no global scratch, no counters to reset when a best-effort run is preempted and re-run).
+// CLUSTER (1..8 CTAs).  Each CTA accumulates its K range in TMEM and owns a share of the tile's pixels; it
+// stores the other ranks' pixels of its partial tile straight from registers into their shared memory
+// (st.async, counted by the receiver's mbarrier) and sums its own share over the ranks in rank order 0..S-1 —
+// a fixed order, so results are bit-reproducible (no float atomics, no global scratch, no counters to reset when
+// a best-effort run is preempted and re-run).
 //
-// One warp issues TMA, one warp issues tcgen05.mma, all eight warps run the epilogue
-// (tcgen05.ld -> +residual -> +bias | *gamma+beta -> ReLU -> coalesced 512-byte rows, four output
-// channels per lane).  What bounds it: a launch of a few microseconds is a chain of latencies (hand-over from
-// the previous grid 1.7 us, first K block 0.3 us, cluster barrier 0.6 us, rows 1 us) around a main loop that
-// takes about 57 bytes a clock into an SM.  Issue by whole warps and the remote-load epilogue took the replay
-// of ResNet-152 from 827 to 760 us, Inception-v3's from 377 to 338 us, BERT's (128 tokens) from 593 to 560 us.
+// One warp issues TMA, one warp issues tcgen05.mma, all eight warps run the exchange and the epilogue
+// (tcgen05.ld -> +residual -> +bias | *gamma+beta -> ReLU -> stores), a thread being one output channel throughout,
+// as tensor memory has it.  What bounds it: a launch of a few microseconds is a chain of latencies (hand-over from
+// the previous grid and first K block 1.4 us, multiplications 160 cycles per K block, exchange 0.4-0.9 us) beside a
+// load stream that takes about 57 bytes a clock into an SM.  Reading the partials out of the peers' staged tiles between
+// two cluster barriers took 1.2 us for 28 pixels over eight ranks where the stores take 0.4, 1.7 against 0.8 for 64
+// pixels; together with multiplications issued at the tensor core's pace: 1x1 1024 -> 256 at 14x14 4.41 -> 3.09 us, 3x3
+// 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us.
 // Every mbarrier wait is bounded: on expiry the kernel records an error word,
 // skips further waits, still joins every cluster barrier, frees its TMEM and returns.
 #pragma once
@@ -87,52 +90,109 @@ __device__ __forceinline__ void tc_stamp(const TcParams& P, int slot) {
 __device__ __forceinline__ void tc_stamp(const TcParams&, int) {}
 #endif
 
-// Finishes the pixel rows [jb, je) this CTA owns: row jb + i of the accumulator is summed over the staged tiles of the
-// cluster's ranks 0..S-1 in rank order (a fixed order: bit-reproducible), read from distributed shared memory; then the
-// epilogue, and a 512-byte row is stored.  A warp takes every 8th row and RB of them at a time, RB * SMAX 128-bit loads per
-// lane in flight (16: the kernel is built for two CTAs per SM, so a thread has 128 registers).
-template <int RB, int SMAX, bool GELU>
-__device__ __forceinline__ void tc_finish_rows(const TcParams& P, uint32_t stage, int S, int jb, int je, int warp, int cbase, int co, int pix0,
-                                               float4 sc, float4 sh, float lo, bool rnd, bool has_res, float4 b2, const float4* rpre) {
-    uint32_t src[SMAX];
+__device__ __forceinline__ float tc_round1(float v) {
+    uint32_t u;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
+    return __uint_as_float(u);
+}
+
+// What a thread finishes pixel groups (of four) with: output channel `co`, every other group of the rank's
+// share.  With two warps on a scheduler a hundred instructions of a warp are 0.2 us and more, so what can be worked
+// out ahead of the last wait is, and everything per pixel is predicated.
+struct TcShare {
+    uint32_t out, out2, res;   // element of the first group's first pixel; eight pixels further per turn
+    int count, left;           // groups; pixels from the first group to the end of the share (0: no such channel)
+    float sc, sh, b2;          // scale and shift (bias), shift of the second output
+    float rpre[2][4];          // residual of the first two groups
+};
+
+// Finishes the groups of a share.  The sum of a group over the cluster's ranks 0..S-1 in rank order (a fixed order:
+// bit-reproducible) comes from the receive area, `src` being the place of this channel and the first group in the slot of rank 0;
+// without a K split it comes from tensor memory, `src` being the first group's column.  Stores and residual loads are 128
+// contiguous bytes per warp and pixel.  U groups at a time, so that their loads overlap.
+template <int S, int U, bool GELU>
+__device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_t src) {
+    const uint32_t slot_bytes = (uint32_t)P.gpc * (TC_BM * 16);
+    const uint32_t ocs = (uint32_t)P.ocs, pcs = (uint32_t)P.pcs, rcs = (uint32_t)P.co;
+    const bool has_res = P.res != nullptr;
+#pragma unroll 1
+    for (int k0 = 0; k0 < w.count; k0 += U) {
+        float v[U][4], r[U][4];
+        uint32_t own[U][4];
+        float4 part[U][S];
 #pragma unroll
-    for (int q = 0; q < SMAX; q++) {
-        const uint32_t own = stage + (uint32_t)(jb * TC_BM + cbase) * 4u;
-        src[q] = SMAX == 1 ? own : mapa_shared(own, (uint32_t)(q < S ? q : 0));
-    }
-    for (int jbase = warp; jbase < je - jb; jbase += 8 * RB) {
-        float4 part[RB][SMAX], rv[RB];
+        for (int u = 0; u < U; u++) {
+            const bool more = u == 0 || k0 + u < w.count;   // (the share's last turn may be short: a group of it is read again)
+            if (S == 1) {
+                tmem_ld4_nowait(src + (more ? (uint32_t)u * 8u : 0u), own[u]);
+            } else {
 #pragma unroll
-        for (int u = 0; u < RB; u++) {
-            const int jr = jbase + 8 * u;   // row within this CTA's share
-            rv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (jr < je - jb) {
-#pragma unroll
-                for (int q = 0; q < SMAX; q++)
-                    if (q < S) part[u][q] = SMAX == 1 ? ld_smem_v4(src[q] + (uint32_t)jr * TC_BM * 4u) : ld_dsmem_v4(src[q] + (uint32_t)jr * TC_BM * 4u);
-                if (has_res) rv[u] = (u < 2 && jbase == warp) ? rpre[u & 1] : ld_activation(P.res + (size_t)(pix0 + jb + jr) * P.co + co);
+                for (int q = 0; q < S; q++) part[u][q] = ld_smem_v4(src + (more ? (uint32_t)u * (2 * TC_BM * 16) : 0u) + (uint32_t)q * slot_bytes);
             }
         }
+        if (has_res) {
 #pragma unroll
-        for (int u = 0; u < RB; u++) {
-            const int jr = jbase + 8 * u;
-            if (jr < je - jb) {
-                float4 v = part[u][0];
+            for (int u = 0; u < U; u++)
 #pragma unroll
-                for (int q = 1; q < SMAX; q++)   // fixed rank order: deterministic sum
-                    if (q < S) { v.x += part[u][q].x; v.y += part[u][q].y; v.z += part[u][q].z; v.w += part[u][q].w; }
-                float4 o;
-                if (GELU) {
-                    o.x = tc_gelu_inline(v.x + sh.x) + rv[u].x; o.y = tc_gelu_inline(v.y + sh.y) + rv[u].y;
-                    o.z = tc_gelu_inline(v.z + sh.z) + rv[u].z; o.w = tc_gelu_inline(v.w + sh.w) + rv[u].w;
-                    if (rnd) o = tc_round4(o);
-                } else {
-                    o = tc_epilogue4(v, rv[u], sc, sh, lo, rnd, false);
+                for (int i = 0; i < 4; i++)
+                    r[u][i] = ld_activation_if((k0 + u >= 2) && 8 * u + i < w.left, P.res + (w.res + (uint32_t)(8 * u + i) * rcs));
+            if (k0 < 2) {
+#pragma unroll
+                for (int u = 0; u < (U < 2 ? U : 2); u++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) r[u][i] = k0 == 0 ? w.rpre[u][i] : w.rpre[1][i];
+            }
+        }
+        if (S == 1) {
+            tmem_ld_wait();
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    asm volatile("" : "+r"(own[u][i]));   // (used behind the wait)
+                    v[u][i] = __uint_as_float(own[u][i]);
                 }
-                *reinterpret_cast<float4*>(P.out + (size_t)(pix0 + jb + jr) * P.ocs + P.ooff + co) = o;
-                if (P.out2 != nullptr) *reinterpret_cast<float4*>(P.out2 + (size_t)(pix0 + jb + jr) * P.pcs + P.poff + co) = tc_preact(o, b2, rnd);
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                v[u][0] = part[u][0].x; v[u][1] = part[u][0].y; v[u][2] = part[u][0].z; v[u][3] = part[u][0].w;
+#pragma unroll
+                for (int q = 1; q < S; q++) { v[u][0] += part[u][q].x; v[u][1] += part[u][q].y; v[u][2] += part[u][q].z; v[u][3] += part[u][q].w; }
             }
         }
+        // (uniform branches around whole turns: an absent term costs nothing)
+#define TC_EACH(EXPR)                        \
+    do {                                     \
+        _Pragma("unroll") for (int u = 0; u < U; u++) _Pragma("unroll") for (int i = 0; i < 4; i++) v[u][i] = (EXPR); \
+    } while (0)
+        if (GELU) TC_EACH(tc_gelu_inline(v[u][i] + w.sh));
+        if (has_res) TC_EACH(v[u][i] + r[u][i]);
+        if (!GELU) {
+            if (P.ep & TC_EP_GB) TC_EACH(fmaf(v[u][i], w.sc, w.sh));
+            else TC_EACH(v[u][i] + w.sh);
+        }
+        if (P.ep & TC_EP_RELU) TC_EACH(fmaxf(v[u][i], 0.f));
+        if (P.ep & TC_EP_ROUND) TC_EACH(tc_round1(v[u][i]));
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (8 * u + i < w.left) P.out[w.out + (uint32_t)(8 * u + i) * ocs] = v[u][i];
+        if (P.out2 != nullptr) {
+            TC_EACH(fmaxf(v[u][i] + w.b2, 0.f));
+            if (P.ep & TC_EP_ROUND) TC_EACH(tc_round1(v[u][i]));
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (8 * u + i < w.left) P.out2[w.out2 + (uint32_t)(8 * u + i) * pcs] = v[u][i];
+        }
+#undef TC_EACH
+        src += S == 1 ? 8u * U : 2u * U * (TC_BM * 16);
+        w.left -= 8 * U;
+        w.out += 8 * U * ocs;
+        w.out2 += 8 * U * pcs;
+        w.res += 8 * U * rcs;
     }
 }
 
@@ -182,10 +242,10 @@ __device__ __forceinline__ void tc_finish_split(const TcParams& P, const float* 
 
 // BE = best-effort flavour (reference wrapper contract: script/best_effort_kernel.py:22-33, with the polls the
 // reference gets for free from killing wavefronts): the preempt flag is read at block entry and, by the TMA producer,
-// at the head of its refill loop (every 4th K block).  A CTA that saw the flag stops loading, lets the tensor core
-// finish what has landed, and takes part in every cluster barrier; at the first barrier the ranks of a cluster
-// exchange what they saw, and if any rank stopped, ALL ranks skip the exchange, the stores and the completion counter —
-// the kernel is idempotent, so it is simply launched again later.  The real-time flavour carries none of this.
+// at the head of its refill loop (every 4th K block).  A CTA that saw the flag stops loading and lets the tensor core
+// finish what has landed; it takes part in the exchange all the same, each rank sending along what it saw, and if any
+// rank stopped, ALL ranks skip the stores and the completion counter — the kernel is idempotent, so it is simply
+// launched again later.  The real-time flavour carries none of this.
 template <bool BE>
 __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __grid_constant__ TcParams P) {
     extern __shared__ __align__(16) unsigned char tc_smem_raw[];
@@ -197,10 +257,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     // the control words sit behind the data region (stage ring, reused by the epilogue's staging + exchange area)
     const uint32_t ctrl = base + (uint32_t)P.region_bytes;
     const int NS = P.stages;   // ring depth of this launch (<= TC_MAX_STAGES)
-    const uint32_t bar_full = ctrl, bar_empty = ctrl + 8 * TC_MAX_STAGES, bar_acc = ctrl + 16 * TC_MAX_STAGES;
+    const uint32_t bar_full = ctrl, bar_empty = ctrl + 8 * TC_MAX_STAGES, bar_acc = ctrl + 16 * TC_MAX_STAGES, bar_recv = bar_acc + 8;
     volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + P.region_bytes + 16 * TC_MAX_STAGES + 16);
-    volatile uint32_t* s_flags = s_tmem + 1;    // [0] abort (preempt flag seen by this CTA), [1] wait expired,
-                                                //  [2] K blocks whose loads were issued when the producer stopped
+    volatile uint32_t* s_flags = s_tmem + 1;    // [0] abort (preempt flag seen by this CTA), [1] K blocks whose loads were issued when
+                                                //  the producer stopped, [2..9] what the ranks of the cluster saw (best-effort flavour)
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be warp-uniform)
@@ -217,21 +277,36 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     const int kb_end = min(kb_begin + P.kb_per_split, P.kb_total);
     const int nkb = kb_end - kb_begin;
 
+    // spatial tiles: tile_n -> (row group ty, row piece tx); tx > 0 only where a row is wider than a tile
+    const int tile_y = P.xsplit > 1 ? tile_n / P.xsplit : tile_n, tile_x = P.xsplit > 1 ? tile_n - tile_y * P.xsplit : 0;
+    const int pix0 = P.spatial ? tile_y * P.rows * P.wo + tile_x * P.xw : tile_n * P.n_valid;
+    const int m0 = tile_m * TC_BM;
+    // columns of this tile that are real pixels, and its real output channels
+    const int n_lim = P.xsplit > 1 ? min(P.xw, P.wo - tile_x * P.xw) : min(P.n_valid, P.ptot - pix0);
+    const int co_lim = min(TC_BM, P.co - m0);
+    // the share of this rank: pixel groups (of four) [grp0, grp0 + mg)
+    const int groups = (n_lim + 3) >> 2, gpc = P.gpc;
+    const int grp0 = split * gpc, mg = max(0, min(gpc, groups - grp0));
+    const uint32_t recv_bytes = (uint32_t)((S - 1) * (mg * co_lim * 16 + (BE ? 4 : 0)));   // from the other ranks
+
     if (tid == 0) {
         for (int s = 0; s < NS; s++) {
             mbar_init(bar_full + 8 * s, 1);
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_acc, 1);
+        mbar_init(bar_recv, 1);
         s_flags[0] = (uint32_t)(flag0 != 0);
         s_flags[1] = 0;
-        s_flags[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (recv_bytes != 0) mbar_expect_tx(bar_recv, recv_bytes);
         asm volatile("prefetch.tensormap [%0];" ::"l"(&P.tm_w) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&P.tm_x[0]) : "memory");
     }
-    if (warp == 1) {
+    // The warp that allocates tensor memory frees it: one of the half that has fewer groups to finish (none, often)
+    const int awarp = S > 1 && (grp0 & 1) == 0 ? 5 : 1;
+    if (warp == awarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)s_tmem)),
                      "r"((uint32_t)P.tmem_cols)
                      : "memory");
@@ -242,19 +317,14 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *s_tmem;
     if (tid == 0) tc_stamp(P, 1);   // set-up done (barriers, TMEM)
+    // "my receive area may be written": where it is apart from the stage ring, from here on (the barrier's latency then hides
+    // behind the main loop); where it lies over the ring, behind the accumulator
+    if (S > 1 && !P.recv_late) cluster_arrive();
 
-    // spatial tiles: tile_n -> (row group ty, row piece tx); tx > 0 only where a row is wider than a tile
-    const int tile_y = P.xsplit > 1 ? tile_n / P.xsplit : tile_n, tile_x = P.xsplit > 1 ? tile_n - tile_y * P.xsplit : 0;
-    const int pix0 = P.spatial ? tile_y * P.rows * P.wo + tile_x * P.xw : tile_n * P.n_valid;
-    // columns of this tile that are real pixels
-    const int n_lim = P.xsplit > 1 ? min(P.xw, P.wo - tile_x * P.xw) : min(P.n_valid, P.ptot - pix0);
-    const int cpc = (n_lim + S - 1) / S;               // pixel rows one rank finishes
-    const int jb = min(split * cpc, n_lim), je = min(jb + cpc, n_lim);
     // best-effort flavour: what this CTA saw at entry.  Nothing is loaded then; the cluster agrees at its first barrier.
     const bool abort0 = BE && s_flags[0] != 0;
 
     {
-        const int m0 = tile_m * TC_BM;
         // ---------------- TMA producer, part 1: fill the ring (no waits) ----------------
         // Warp 0 refills the ring and warp 1 issues the multiplications as whole warps: control flow, addresses and
         // descriptors are warp-uniform (uniform registers), one elected lane executes each instruction.  As code of a
@@ -314,25 +384,24 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         }
         __syncwarp();
 
-        // epilogue parameters of this lane's 4 output channels: model constants, requested right after the first loads so
-        // that their latency is long gone when the accumulator is ready
-        const int cbase = lane * 4;
-        const int co = m0 + cbase;
-        const bool cvalid = co < P.co;
-        float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 b2 = make_float4(0.f, 0.f, 0.f, 0.f);
+        // warp w reads TMEM lanes 32*(w%4).., its hardware quadrant: a thread is output channel `row` of the tile.  Its epilogue
+        // parameters are model constants, requested right after the first loads, so that their latency is long gone when the
+        // accumulator is ready.
+        const int quad = warp & 3, half = warp >> 2;
+        const int row = quad * 32 + lane;
+        const int co = m0 + row;
+        const bool cvalid = row < co_lim;
+        TcShare w;
+        w.sc = 1.f; w.sh = 0.f; w.b2 = 0.f;
         if (cvalid) {
             if (P.ep & TC_EP_GB) {
-                sc = __ldg(reinterpret_cast<const float4*>(P.gamma + co));
-                sh = __ldg(reinterpret_cast<const float4*>(P.beta + co));
+                w.sc = ld_param(P.gamma + co);
+                w.sh = ld_param(P.beta + co);
             } else if (P.ep & TC_EP_BIAS) {
-                sh = __ldg(reinterpret_cast<const float4*>(P.bias + co));
+                w.sh = ld_param(P.bias + co);
             }
-            if (P.bias2 != nullptr) b2 = __ldg(reinterpret_cast<const float4*>(P.bias2 + co));
+            if (P.bias2 != nullptr) w.b2 = ld_param(P.bias2 + co);
         }
-        const float lo = (P.ep & TC_EP_RELU) ? 0.f : -__int_as_float(0x7f800000);
-        const bool has_res = (P.ep & TC_EP_RES) != 0;
-        const bool rnd = (P.ep & TC_EP_ROUND) != 0;
         const bool gelu = (P.ep & TC_EP_GELU) != 0;
 
         if (warp == 0) {
@@ -368,156 +437,176 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 if (++s == NS) { s = 0; par ^= 1u; }
             }
             if (BE && stop && lane == 0) {
-                s_flags[2] = (uint32_t)issued;     // first how far the loads got, then the request to stop
+                s_flags[1] = (uint32_t)issued;     // first how far the loads got, then the request to stop
                 __threadfence_block();
                 s_flags[0] = 1;
             }
-            if (!ok && lane == 0) s_flags[1] = 1;
+            // (a wait that expired here leaves the multiplications, and with them the accumulator's barrier, incomplete)
         } else if (warp == 1) {
             // ---------------- MMA issuer ----------------
+            // The next stage's barrier is looked at before this stage's multiplications are issued, and those are predicated
+            // on the issuing lane instead of branched around: the loop then runs at the tensor core's pace (umma_tf32_if).
             bool ok = true, halted = false;
-            const uint32_t idesc = umma_idesc_tf32(P.n_mma);
+            const uint32_t idesc = umma_idesc_tf32(P.n_mma), lead = elect_one() ? 1u : 0u;
 #ifdef REEF_DEBUG_AIDS
             const bool tr = lane == 0 && P.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
 #endif
             int s = 0;
             uint32_t par = 0;
             uint64_t da = umma_desc_sw128(base);
+            bool ready = false;
             for (int i = 0; i < nkb; i++) {
-                if (BE) {
-                    const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0]);
-                    if (w == 2) {
-                        // The producer stopped.  Loads it had issued may still be in flight: they must have landed
-                        // before this CTA leaves or reuses its shared memory, so their barriers are awaited (bounded)
-                        // without multiplying.
-                        __threadfence_block();
-                        const int issued = __shfl_sync(0xffffffffu, (int)s_flags[2], 0);
-                        for (; i < issued && ok; i++) {
-                            ok = mbar_wait_warp(bar_full + 8 * s, par);
-                            if (++s == NS) { s = 0; par ^= 1u; }
+                if (!ready) {
+                    if (BE) {
+                        const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0]);
+                        if (w == 2) {
+                            // The producer stopped.  Loads it had issued may still be in flight: they must have landed
+                            // before this CTA leaves or reuses its shared memory, so their barriers are awaited (bounded)
+                            // without multiplying.
+                            __threadfence_block();
+                            const int issued = __shfl_sync(0xffffffffu, (int)s_flags[1], 0);
+                            for (; i < issued && ok; i++) {
+                                ok = mbar_wait_warp(bar_full + 8 * s, par);
+                                if (++s == NS) { s = 0; par ^= 1u; }
+                            }
+                            halted = true;
+                            break;
                         }
-                        halted = true;
-                        break;
+                        ok = w == 0;
+                    } else {
+                        ok = mbar_wait_warp(bar_full + 8 * s, par);
                     }
-                    ok = w == 0;
-                } else {
-                    ok = mbar_wait_warp(bar_full + 8 * s, par);
+                    if (!ok) break;
                 }
-                if (!ok) break;
 #ifdef REEF_DEBUG_AIDS
                 if (tr && i == 0) P.trace[4] = clock64();          // first K block landed
                 if (tr && i == nkb - 1) P.trace[5] = clock64();    // last K block landed
 #endif
+                const int s2 = s + 1 == NS ? 0 : s + 1;
+                const uint32_t par2 = s2 == 0 ? par ^ 1u : par;
+                const bool next = mbar_test(bar_full + 8 * s2, par2);
                 const uint64_t db = da + (uint64_t)(TC_A_BYTES >> 4);
                 // one tcgen05.mma covers K = 8 tf32 = 32 bytes
-                if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TC_BK / 8; k++)
-                        umma_tf32(tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                    if (i + NS < nkb) umma_commit(bar_empty + 8 * s);   // frees the stage, where it is refilled, once these MMAs have read it
-                    if (i == nkb - 1) umma_commit(bar_acc);
-                }
-                __syncwarp();
-                da += (uint64_t)(stage_bytes >> 4);
-                if (++s == NS) { s = 0; par ^= 1u; da = umma_desc_sw128(base); }
+                for (int k = 0; k < TC_BK / 8; k++)
+                    umma_tf32_if(lead, tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                if (i + NS < nkb) umma_commit_if(lead, bar_empty + 8 * s);   // frees the stage, where it is refilled, once these MMAs have read it
+                ready = __all_sync(0xffffffffu, next);
+                da = s2 == 0 ? umma_desc_sw128(base) : da + (uint64_t)(stage_bytes >> 4);
+                s = s2;
+                par = par2;
             }
-            // stopped early: the accumulator barrier completes when the multiplications issued so far have
-            if (BE && halted && ok && elect_one()) umma_commit(bar_acc);
-            __syncwarp();
-            if (!ok && lane == 0) s_flags[1] = 1;
+            // complete, or stopped early: the accumulator's barrier completes when the multiplications issued so far have
+            if (ok) umma_commit_if(lead, bar_acc);
         }
         __syncwarp();
         if (warp != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-        // the first two residual rows of this warp's pass over its pixel rows (rows jb + warp + 8u): requested now, used
-        // after the exchange
-        float4 rpre[2];
+        // this half's groups of the share: every other one
+        const int gfirst = grp0 + ((grp0 ^ half) & 1);
+        w.count = max(0, (grp0 + mg - gfirst + 1) >> 1);
+        w.left = cvalid && w.count > 0 ? min(n_lim, (grp0 + mg) * 4) - gfirst * 4 : 0;
+        w.out = (uint32_t)((pix0 + gfirst * 4) * P.ocs + P.ooff + co);
+        w.out2 = (uint32_t)((pix0 + gfirst * 4) * P.pcs + P.poff + co);
+        w.res = (uint32_t)((pix0 + gfirst * 4) * P.co + co);
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            rpre[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            const int jr = warp + 8 * u;
-            if (has_res && cvalid && jr < je - jb)
-                rpre[u] = ld_activation(P.res + (size_t)(pix0 + jb + jr) * P.co + co);
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) w.rpre[u][i] = ld_activation_if(P.res != nullptr && 8 * u + i < w.left, P.res + (w.res + (uint32_t)((8 * u + i) * P.co)));
+
+        // The exchange: this half's groups of the tile leave tensor memory four at a time for the owner's shared memory, slot `split`
+        // there; an own group goes into the own slot (the thread that finishes a group is the one that put it there).  The next
+        // rank's leave first, so that the ranks do not all store to the same one.  Where a turn's groups go is worked out ahead of
+        // it, for the first turn ahead of the accumulator.
+        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16), recv = base + (uint32_t)P.recv_offset;
+        const int turns = (groups - half + 1) >> 1;
+        int rot = (grp0 + mg - half + 1) >> 1;
+        if (rot >= turns) rot = 0;
+        uint32_t col[4], dst[4], bar[4];   // bar = 0: an own group; dst = 0: none
+        auto route = [&](int t0) {
+            const uint32_t place = (uint32_t)P.recv_offset + (uint32_t)(split * gpc * TC_BM + row) * 16u;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int t = t0 + u, g = half + 2 * (t >= turns ? 0 : t + rot < turns ? t + rot : t + rot - turns);
+                const int owner = (int)(((uint32_t)g * P.gpc_magic) >> 16);
+                const uint32_t off = place + (uint32_t)(g - owner * gpc) * (TC_BM * 16), peer = owner == split ? base : mapa_shared(base, (uint32_t)owner);
+                col[u] = taddr + (uint32_t)g * 4u;
+                dst[u] = cvalid && t < turns ? peer + off : 0u;
+                bar[u] = owner != split && dst[u] != 0 ? peer + (bar_recv - base) : 0u;
+            }
+        };
+        if (S > 1) {
+            route(0);
+            if (!P.recv_late) cluster_wait();           // every rank's receive area may be written
         }
 
-        // ---------------- epilogue: all eight warps ----------------
-        bool ok = mbar_wait(bar_acc, 0);
+        // ---------------- exchange and epilogue: all eight warps ----------------
+        bool ok = mbar_wait_warp(bar_acc, 0);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        __syncthreads();
+        // best-effort flavour: behind this barrier the producer and the MMA warp are past their loops, the flag word is final
+        if (BE) __syncthreads();
+        bool abort_all = BE && s_flags[0] != 0;
         if (tid == 0) tc_stamp(P, 6);   // accumulator complete
-        const bool my_abort = BE && s_flags[0] != 0;   // final: producer and MMA warp are past their loops
-        if (!ok || s_flags[1]) {
-            ok = false;
-            if (tid == 0 && P.error_word) *reinterpret_cast<volatile int*>(P.error_word) = 1;
-        }
-        // Phase A — eight warps move the accumulator tile TMEM -> registers -> shared memory as stage[pixel][channel]
-        // (warp w reads TMEM lanes 32*(w%4).., its hardware quadrant, and every other 16 columns, by w/4).  The stage ring
-        // is free by now and is reused for this.
-        // Phase B — the tile is finished pixel row by pixel row with 128-bit accesses: one warp per pixel, a lane owns 4
-        // consecutive output channels.  With a K split, rank q finishes rows [q*cpc, (q+1)*cpc) and reads every rank's
-        // partial of them from its shared memory; 128-bit remote loads, 16 in flight per lane, take half the time of a
-        // bulk copy per peer into a receive area (1800 cycles from its issue to the owner's barrier).
-        const int quad = warp & 3, half = warp >> 2;
-        const int row = quad * 32 + lane;              // TMEM lane == output channel within the tile
-        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
-        float* stage = reinterpret_cast<float*>(smem);
-        if (ok && !my_abort) {
-            for (int j0 = half * 16; j0 < n_lim; j0 += 64) {
-                uint32_t r[32];
-                tmem_ld16_nowait(taddr + j0, r);
-                if (j0 + 32 < n_lim) tmem_ld16_nowait(taddr + j0 + 32, r + 16);
-                tmem_ld_wait();
-                float* dst = stage + j0 * TC_BM + row;
+        if (S > 1) {
+            if (P.recv_late) {
+                cluster_arrive_relaxed();   // (what it orders, the reads of the ring, was seen complete through the accumulator's barrier)
+                cluster_wait();
+            }
+            if (tid == 0) tc_stamp(P, 3);
+            // (A rank that gave up sends what it has: the receivers count bytes, and nobody stores the result of a failed or
+            // preempted launch.)
+            if (quad * 32 < co_lim) {
+#pragma unroll 1
+                for (int t0 = 0; t0 < turns;) {
+                    uint32_t v[4][4];
 #pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (j0 + j < n_lim) dst[j * TC_BM] = __uint_as_float(r[j]);
-                if (j0 + 32 < n_lim) {
+                    for (int u = 0; u < 4; u++) tmem_ld4_nowait(col[u], v[u]);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (j0 + 32 + j < n_lim) dst[(32 + j) * TC_BM] = __uint_as_float(r[16 + j]);
+                    for (int u = 0; u < 4; u++) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) asm volatile("" : "+r"(v[u][i]));   // (used behind the wait)
+                        st_async_v4_if(bar[u] != 0, dst[u], bar[u], v[u]);
+                        st_smem_v4_if(bar[u] == 0 && dst[u] != 0, dst[u], v[u]);
+                    }
+                    t0 += 4;
+                    if (t0 < turns) route(t0);
                 }
             }
-        }
-        if (tid == 0) tc_stamp(P, 7);   // accumulator tile staged in shared memory
-        // The accumulator is out of tensor memory once every warp has passed the barrier below, so the allocating
-        // warp frees it there and not at the very end: nothing is then left to do between a CTA's last store and
-        // its exit, which is what the next kernel of the stream waits for.
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        bool abort_all = my_abort;
-        if (S > 1) {
-            // cluster barrier #1: every rank's tile is staged.  (Nothing is written into a peer's shared memory, and a
-            // peer's is not read before this barrier: only behind it is every CTA of the cluster known to have started.)
-            cluster_sync_all();
-            if (warp == 1) tmem_free(tmem, (uint32_t)P.tmem_cols);
-            if (tid == 0) tc_stamp(P, 3);
-            if (BE) {
-                // every rank learns whether ANY rank of the cluster stopped for the preempt flag: one thread per rank
-                // reads that rank's abort word through distributed shared memory; all ranks compute the same OR
-                uint32_t f = 0;
-                if (tid < S)
-                    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(f) : "r"(mapa_shared(smem_u32((const void*)&s_flags[0]), (uint32_t)tid)) : "memory");
-                abort_all = __syncthreads_or((int)f) != 0;
+            // the accumulator is out of tensor memory
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (warp != awarp) {
+                asm volatile("bar.arrive 1, 256;" ::: "memory");
+            } else if (w.count == 0) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                tmem_free(tmem, (uint32_t)P.tmem_cols);
             }
-        } else {
-            __syncthreads();
-            if (warp == 1) tmem_free(tmem, (uint32_t)P.tmem_cols);
+            if (BE && tid < S && tid != split) {
+                const uint32_t peer = mapa_shared(base, (uint32_t)tid);
+                st_async_u32(peer + (smem_u32((const void*)&s_flags[2]) - base) + (uint32_t)split * 4u, peer + (bar_recv - base), abort_all || !ok ? 1u : 0u);
+            }
+            if (tid == 0) tc_stamp(P, 7);   // shares sent
+            if (recv_bytes != 0 && !mbar_wait_cluster_warp(bar_recv, 0)) ok = false;
+            if (BE) {
+                // every rank has the words of all the others: all take the same exit
+                for (int q = 0; q < S; q++)
+                    if (q != split && s_flags[2 + q] != 0) abort_all = true;
+            }
         }
-        if (tid == 0) tc_stamp(P, 8);
-        if (ok && cvalid && !abort_all) {
-            const uint32_t st = smem_u32(stage);
-#define TC_FINISH(RB, SMAX)                                                                                                            \
-    do {                                                                                                                               \
-        if (gelu) tc_finish_rows<RB, SMAX, true>(P, st, S, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, has_res, b2, rpre);         \
-        else tc_finish_rows<RB, SMAX, false>(P, st, S, jb, je, warp, cbase, co, pix0, sc, sh, lo, rnd, has_res, b2, rpre);             \
+        if (!ok && P.error_word) *reinterpret_cast<volatile int*>(P.error_word) = 1;
+        if (tid == 0) tc_stamp(P, 8);       // shares received
+        if (ok && !abort_all && quad * 32 < co_lim) {
+            const uint32_t src = S == 1 ? taddr + (uint32_t)gfirst * 4u : recv + (uint32_t)((gfirst - grp0) * TC_BM + row) * 16u;
+#define TC_FINISH(S_, U_)                                   \
+    do {                                                    \
+        if (gelu) tc_finish<S_, U_, true>(P, w, src);       \
+        else tc_finish<S_, U_, false>(P, w, src);           \
     } while (0)
-            if (S == 1) TC_FINISH(4, 1);
-            else if (S == 2) TC_FINISH(4, 2);
-            else if (S <= 4) TC_FINISH(4, 4);
-            else TC_FINISH(2, TC_MAX_SPLITS);
+            if (S == 8) TC_FINISH(8, 1);
+            else if (S == 4) TC_FINISH(4, 1);
+            else if (S == 2) TC_FINISH(2, 2);
+            else TC_FINISH(1, 2);
 #undef TC_FINISH
         }
-        // cluster barrier #2: nobody reads a peer's shared memory any more, every CTA may exit
-        if (S > 1) cluster_arrive_relaxed();
-        if (S > 1) cluster_wait();      // barrier #2
         if (tid == 0) tc_stamp(P, 9);   // rows finished
         if (BE && abort_all && tid == 0 && P.stamps != nullptr) {
             // measurement only: when this block saw the preempt flag and left (device clock)
@@ -526,9 +615,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             atomicMin(&P.stamps[0], t);
             atomicMax(&P.stamps[1], t);
         }
-        if (P.task_slot != nullptr && ok && !abort_all) {
-            __syncthreads();
-            if (tid == 0) red_relaxed_gpu_add(P.task_slot, 1);
+        if (P.task_slot != nullptr && __syncthreads_and(ok && !abort_all) && tid == 0) red_relaxed_gpu_add(P.task_slot, 1);
+        // (A rank leaves without waiting for its peers: what it sent them is on its way, and nobody reads its shared memory.)
+        if (S == 1) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (warp != awarp) asm volatile("bar.arrive 1, 256;" ::: "memory");
+        }
+        if (warp == awarp && !(S > 1 && w.count == 0)) {
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            tmem_free(tmem, (uint32_t)P.tmem_cols);
         }
     }
 

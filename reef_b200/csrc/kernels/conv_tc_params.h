@@ -45,8 +45,12 @@ struct TcParams {
     int load_bytes;          // bytes TMA delivers per K block (both boxes)
     int stages;              // ring depth of this launch
     int region_bytes;        // data region of shared memory: max(stage ring, staging tile + exchange area)
-    int recv_offset_floats;  // exchange area offset inside the region, in floats
-    int cpc_max;             // pixel rows a rank finishes at most = ceil(n_valid / splits)
+    int recv_offset_floats;  // chain kernel: exchange area offset inside the region, in floats
+    int cpc_max;             // chain kernel: pixel rows a rank finishes at most = ceil(n_valid / splits)
+    int gpc;                 // pixel groups (of four) a rank finishes at most = ceil(ceil(n_valid / 4) / splits)
+    unsigned gpc_magic;      // ceil(2^16 / gpc): owner of a group = group * gpc_magic >> 16
+    int recv_offset;         // receive area [splits][gpc][128 channels][4 pixels] inside the region, in bytes
+    int recv_late;           // it lies over the stage ring: written once every rank's accumulator is complete
     int n_tiles;             // pixel tiles; linear tile index = tile_m * n_tiles + tile_n
     int tile_begin;          // first tile of this launch (dynamic kernel padding launches sub-ranges)
     unsigned cb_magic;       // ceil(2^32 / cblocks): tap = umulhi(kb, cb_magic) without an integer division

@@ -302,6 +302,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
             p.round_tf32 = (int)a.get("rt", 0);   // outputs feed LayerNorm / attention in fp32: no TF32 rounding
             p.plan_cap = (int)a.get("tp", 0);
             p.plan_splits = (int)a.get("ts", 0);
+            p.plan_earlier = (int)a.get("pv", 0) == 1;
             if (tc_plan(p, &s->tc) != REEF_SUCC) goto bad;
             t.family = F_CONV_TC;
             t.nblocks = s->tc.splits * s->tc.n_tiles * s->tc.m_tiles;
@@ -389,6 +390,7 @@ static int build_spec(const std::string& name, KernelSpec* s) {
             p.round_tf32 = (int)a.get("rt", 1);
             p.plan_cap = (int)a.get("tp", 0);       // tuned plan carried by the name: tile cap and K splits
             p.plan_splits = (int)a.get("ts", 0);
+            p.plan_earlier = (int)a.get("pv", 0) == 1;
             if (tc_plan(p, &s->tc) != REEF_SUCC) {
                 set_error("shape not supported by the tensor-core convolution: " + name);
                 return REEF_NOT_FOUND;

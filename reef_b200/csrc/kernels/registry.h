@@ -20,6 +20,7 @@ struct TcPlan {
     int n_tiles, m_tiles, cblocks, kb_total, kb_per_split, splits;
     int b_bytes, smem;
     int region_bytes, recv_offset_floats, cpc_max, stages;
+    int gpc, recv_offset, recv_late;
     int xsplit, xw;
 };
 

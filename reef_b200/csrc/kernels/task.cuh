@@ -56,6 +56,7 @@ struct ConvP {
     int i_bias2, i_out2;     // EP_DUAL: second output out2 = relu(out + bias2) (the next unit's pre-activation)
     int pcs, poff;           // channel stride and offset of the second output
     int plan_cap, plan_splits;   // tensor-core variant: tile cap / K splits fixed by the name (tp, ts), 0 = planner's choice
+    int plan_earlier;            // tensor-core variant: the plan that earlier versions wrote into schedules (pv1)
 };
 
 struct PoolP {

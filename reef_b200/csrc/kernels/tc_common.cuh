@@ -95,11 +95,58 @@ __device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t p
     }
     return 1;
 }
+// One look, without the suspension that try_wait may take: for a look ahead at a barrier that may be far from complete.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// The bounded wait of a whole warp for data that the other CTAs of the cluster have stored (st_async): acquire at cluster scope.
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity) {
+    unsigned long long t0 = 0;
+    for (int i = 0; i < (1 << 26); i++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (__all_sync(0xffffffffu, done != 0)) return true;
+        if ((i & 255) == 255) {   // give up after one second of wall time
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return false;
+        }
+    }
+    return false;
+}
 // Activations of an earlier kernel: a volatile load stays behind griddepcontrol.wait.  (__ldg promises memory that never
 // changes, and the compiler did move such loads above the wait.)
 __device__ __forceinline__ float4 ld_activation(const float* p) {
     float4 v;
     asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+// A model constant, requested where this stands: a plain load may be moved down to its first use, behind the waits.
+__device__ __forceinline__ float ld_param(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+// The same for one value under a per-lane condition.  Predicated: as a branch around the instruction each of them cost about 30
+// cycles of a launch's tail.
+__device__ __forceinline__ float ld_activation_if(bool c, const float* p) {
+    float v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(p), "r"((int)c));
     return v;
 }
 // one lane of a converged warp
@@ -142,17 +189,26 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// volatile keeps the load behind the cluster barrier (also a volatile asm); no "memory" clobber, so the
-// loads of one reduction batch are issued back to back and overlap
-__device__ __forceinline__ float4 ld_dsmem_v4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ float4 ld_smem_v4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
+}
+// Store into the shared memory of a CTA of the cluster, counted in bytes by that CTA's mbarrier.  The source is registers: the
+// sender may leave at once, and the receiver is alive until its barrier has seen every byte.
+__device__ __forceinline__ void st_async_v4_if(bool c, uint32_t addr, uint32_t bar, const uint32_t* v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+                 "@q st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n\t}"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar), "r"((int)c)
+                 : "memory");
+}
+__device__ __forceinline__ void st_smem_v4_if(bool c, uint32_t addr, const uint32_t* v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n\t}"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"((int)c)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_u32(uint32_t addr, uint32_t bar, uint32_t v) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void st_dsmem_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
@@ -180,15 +236,32 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same as code of a whole warp: `lead` is non-zero in the one lane that issues.  Predicated, so that the warp's control flow
+// stays uniform and the descriptors in uniform registers: the tensor core is then fed at its own rate, (4096 + 32 N) / 128 cycles
+// per instruction (operand reads from shared memory: 160 cycles per K block of four at N = 32, 192 at 64, 256 at 128).  A branch
+// around the instructions, and a look at the barrier between them, cost 307 / 320 / 332.
+__device__ __forceinline__ void umma_tf32_if(uint32_t lead, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t lead, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(bar), "r"(lead)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 // 32 columns of one TMEM lane per thread; the wait is separate so that several loads can be in flight
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {

@@ -277,3 +277,31 @@ def test_generated_schedules_pass_the_storage_size_check(gen, libs, model):
         base = gen(model)
     err = C.create_string_buffer(512)
     assert L.reef_model_check((base + ".json").encode(), err, C.c_size_t(512)) == capi.SUCC, err.value
+
+
+EARLIER_PLANS = [   # kernel name, cluster x tiles and shared memory that earlier versions wrote into schedules
+    ("fused_nn_conv2d_add_nn_relu__ci1024_hi14_wi14_co256_kh1_kw1_sh1_sw1_ph0_pw0_v1", [8, 14], 83200),
+    ("fused_nn_conv2d_add_nn_relu__ci64_hi56_wi56_co64_kh3_kw3_sh1_sw1_ph1_pw1_v1", [2, 56], 99584),
+    ("fused_nn_conv2d_add_nn_relu__ci64_hi17_wi17_co64_kh3_kw3_sh1_sw1_ph1_pw1_v1_tp64_ts2", [2, 6], 99584),
+    ("reef_matmul_nt_bias__m128_n2304_k768_v1", [2, 72], 103680),
+]
+
+
+@pytest.mark.parametrize("name,grid,smem", EARLIER_PLANS, ids=[n[:60] for n, _, _ in EARLIER_PLANS])
+def test_schedules_of_earlier_versions_load_with_the_plan_they_state(libs, tmp_path, name, grid, smem):
+    L = capi.host_lib()
+    err = C.create_string_buffer(512)
+    nargs = capi.kernel_plan(name)[2]
+    big = 1 << 24
+
+    def check(dims, shared):
+        path = tmp_path / "one.json"
+        path.write_text(json.dumps({"storage": [{"name": "temp", "size": big, "stype": "float32"}] * nargs,
+                                    "kernels": [{"name": name, "launch_params": dims + [1, 256, 1, 1], "args": list(range(nargs))}],
+                                    "args": [], "shared_memory": {name: shared}}))
+        return L.reef_model_check(str(path).encode(), err, C.c_size_t(512))
+
+    assert check(grid, smem) == capi.SUCC, err.value
+    assert check(capi.kernel_plan(name)[0][:2], capi.kernel_plan(name)[1]) == capi.SUCC, err.value
+    assert check(grid, 60000) != capi.SUCC and b"shared_memory" in err.value
+    assert check([grid[0], grid[1] + 1], smem) != capi.SUCC and b"launch_params" in err.value
