@@ -34,8 +34,13 @@ __device__ __forceinline__ bool body_embedding(const KTask& t, int vb, unsigned 
 
 // ---- LayerNorm of x (+ residual): mean, two-pass variance, (x-mu)/sqrt(var+1e-12)*gamma+beta ------------------
 // (reference: bert.cu:175-204,338-342,352-379; eps at :201).  args: out, x, [residual], gamma, beta.
-// One warp per row, the row lives in registers (h <= 1024, h % 128 == 0), warp-shuffle reductions.
-constexpr int kLnRowsPerBlock = 8;
+// A row lives in registers, at most two 128-bit values a lane (h <= 1024, h % 128 == 0): one, two or four warps share a row, so that
+// many SMs take part and every load of a launch is in flight at once.  What bounds a launch is its latency: the hand-over, one trip
+// to L2 and two reductions.  A warp to a row of 768 kept its 12 to 24 loads in a chain of branches and eight rows on an SM:
+// 128 rows 3.49 -> 1.86 us, 384 rows 3.59 -> 2.06 us a launch; a replay of BERT-base 490 -> 440 us at 128 tokens, 773 -> 718 us
+// at 384.
+__host__ __device__ inline int ln_warps_per_row(int h) { return h <= 256 ? 1 : h <= 512 ? 2 : 4; }
+constexpr int kLnRowsPerBlock = 8;   // with one warp to a row; schedules of earlier versions have it for every width
 // gamma and beta are model constants: they are asked into L2 before the wait for the previous kernel.  A model's weights have
 // flushed them out since its last pass, and behind the reductions their trip from HBM would stand on the critical path
 // (0.5 us a launch: BERT-base at 128 tokens 531 -> 518 us a replay).
@@ -48,53 +53,65 @@ __device__ __forceinline__ void prefetch_layernorm(const KTask& t) {
     }
 }
 __device__ __forceinline__ bool body_layernorm(const KTask& t, int vb, unsigned char*, const int*) {
-    const int rows = t.p.raw[0], h = t.p.raw[1], has_res = t.p.raw[2];
+    __shared__ float sums[2][8];
+    const int rows = t.p.raw[0], h = t.p.raw[1], has_res = t.p.raw[2], rows_per_block = t.p.raw[3];
     float* out = (float*)t.a[0];
     const float* x = (const float*)t.a[1];
     const float* res = has_res ? (const float*)t.a[2] : nullptr;
     const float* gamma = (const float*)t.a[has_res ? 3 : 2];
     const float* beta = (const float*)t.a[has_res ? 4 : 3];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int row = vb * kLnRowsPerBlock + warp;
-    if (row >= rows) return true;
-    const int n4 = h >> 7;   // float4 per lane
-    float4 v[8];
-    float sum = 0.f;
+    const int W = ln_warps_per_row(h), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int part = warp & (W - 1), sub = warp / W;          // this warp's share of its row, its row among the block's
+    // the sum over a row: its warps' sums in their order
+    auto row_sum = [&](float v, float* s) {
+        v = warp_sum(v);
+        if (W == 1) return v;
+        if (lane == 0) s[warp] = v;
+        __syncthreads();
+        float all = s[sub * W];
+        for (int q = 1; q < W; q++) all += s[sub * W + q];
+        return all;
+    };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    int c[2];
+    bool in[2];
+    float4 g[2], b[2];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        if (i < n4) {
-            const int c = (i * 32 + lane) * 4;
-            v[i] = *reinterpret_cast<const float4*>(x + (size_t)row * h + c);
-            if (res) {
-                const float4 r = *reinterpret_cast<const float4*>(res + (size_t)row * h + c);
-                v[i].x += r.x; v[i].y += r.y; v[i].z += r.z; v[i].w += r.w;
-            }
-            sum += v[i].x + v[i].y + v[i].z + v[i].w;
-        }
+    for (int i = 0; i < 2; i++) {
+        c[i] = ((i * W + part) * 32 + lane) * 4;
+        in[i] = c[i] < h;
+        g[i] = in[i] ? *reinterpret_cast<const float4*>(gamma + c[i]) : zero;
+        b[i] = in[i] ? *reinterpret_cast<const float4*>(beta + c[i]) : zero;
     }
-    const float mu = warp_sum(sum) / (float)h;
-    float sq = 0.f;
+    __syncthreads();                           // a persistent caller's previous block is out of the sums
+    for (int r0 = 0; r0 < rows_per_block; r0 += 8 / W) {
+        const int row = vb * rows_per_block + r0 + sub;
+        const size_t at = (size_t)row * h;
+        float4 v[2], r[2];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        if (i < n4) {
-            const float a = v[i].x - mu, b = v[i].y - mu, c = v[i].z - mu, d = v[i].w - mu;
-            sq += a * a + b * b + c * c + d * d;
+        for (int i = 0; i < 2; i++) {
+            const bool there = in[i] && row < rows;
+            v[i] = there ? *reinterpret_cast<const float4*>(x + at + c[i]) : zero;
+            r[i] = there && res ? *reinterpret_cast<const float4*>(res + at + c[i]) : zero;
         }
-    }
-    const float rstd = 1.0f / sqrtf(warp_sum(sq) / (float)h + 1e-12f);
+        float sum = 0.f, sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        if (i < n4) {
-            const int c = (i * 32 + lane) * 4;
-            const float4 g = *reinterpret_cast<const float4*>(gamma + c);
-            const float4 b = *reinterpret_cast<const float4*>(beta + c);
-            float4 o;
-            o.x = (v[i].x - mu) * rstd * g.x + b.x;
-            o.y = (v[i].y - mu) * rstd * g.y + b.y;
-            o.z = (v[i].z - mu) * rstd * g.z + b.z;
-            o.w = (v[i].w - mu) * rstd * g.w + b.w;
-            *reinterpret_cast<float4*>(out + (size_t)row * h + c) = o;
+        for (int i = 0; i < 2; i++) {
+            v[i].x += r[i].x; v[i].y += r[i].y; v[i].z += r[i].z; v[i].w += r[i].w;
+            sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
         }
+        const float mu = row_sum(sum, sums[0]) / (float)h;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            v[i].x -= mu; v[i].y -= mu; v[i].z -= mu; v[i].w -= mu;
+            if (in[i]) sq += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+        }
+        const float rstd = 1.0f / sqrtf(row_sum(sq, sums[1]) / (float)h + 1e-12f);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            if (in[i] && row < rows)
+                *reinterpret_cast<float4*>(out + at + c[i]) = make_float4(v[i].x * rstd * g[i].x + b[i].x, v[i].y * rstd * g[i].y + b[i].y,
+                                                                          v[i].z * rstd * g[i].z + b[i].z, v[i].w * rstd * g[i].w + b[i].w);
     }
     return true;
 }

@@ -247,7 +247,8 @@ static int build_spec(const std::string& name, KernelSpec* s) {
         if (!a.need("rows", &rows) || !a.need("h", &h) || (h % 128) != 0 || h > 1024) goto bad;
         t.p.raw[0] = rows; t.p.raw[1] = h; t.p.raw[2] = op == "reef_add_layernorm";
         t.family = F_LAYERNORM;
-        t.nblocks = ceil_div(rows, kLnRowsPerBlock);
+        t.p.raw[3] = (int)a.get("pv", 0) == 1 ? kLnRowsPerBlock : kLnRowsPerBlock / ln_warps_per_row(h);
+        t.nblocks = ceil_div(rows, t.p.raw[3]);
         s->nargs = t.p.raw[2] ? 5 : 4;
         s->bytes = 4.0 * ((2.0 + t.p.raw[2]) * rows * h + 2.0 * h);
         return REEF_SUCC;
