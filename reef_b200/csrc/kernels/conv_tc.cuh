@@ -103,7 +103,7 @@ struct TcShare {
     uint32_t out, out2, res;   // element of the first group's first pixel; eight pixels further per turn
     int count, left;           // groups; pixels from the first group to the end of the share (0: no such channel)
     float sc, sh, b2;          // scale and shift (bias), shift of the second output
-    float rpre[2][4];          // residual of the first two groups
+    float rpre[2][4];          // residual of the next two groups
 };
 
 // Finishes the groups of a share.  The sum of a group over the cluster's ranks 0..S-1 in rank order (a fixed order:
@@ -130,18 +130,15 @@ __device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_
                 for (int q = 0; q < S; q++) part[u][q] = ld_smem_v4(src + (more ? (uint32_t)u * (2 * TC_BM * 16) : 0u) + (uint32_t)q * slot_bytes);
             }
         }
-        if (has_res) {
+        if (has_res) {   // this turn's was requested two groups ago; the next one's travels beside this turn
 #pragma unroll
             for (int u = 0; u < U; u++)
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-                    r[u][i] = ld_activation_if((k0 + u >= 2) && 8 * u + i < w.left, P.res + (w.res + (uint32_t)(8 * u + i) * rcs));
-            if (k0 < 2) {
-#pragma unroll
-                for (int u = 0; u < (U < 2 ? U : 2); u++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) r[u][i] = k0 == 0 ? w.rpre[u][i] : w.rpre[1][i];
-            }
+                for (int i = 0; i < 4; i++) {
+                    r[u][i] = w.rpre[u][i];
+                    if (U == 1) w.rpre[0][i] = w.rpre[1][i];
+                    w.rpre[U == 1 ? 1 : u][i] = ld_activation_if(8 * (u + 2) + i < w.left, P.res + (w.res + (uint32_t)(8 * (u + 2) + i) * rcs));
+                }
         }
         if (S == 1) {
             tmem_ld_wait();
