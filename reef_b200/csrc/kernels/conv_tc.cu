@@ -111,19 +111,38 @@ static int tc_place_recv(TcPlan* pl, bool earlier) {
     return REEF_SUCC;
 }
 
-// Estimated SM cycles of one launch under a plan, up to a constant.  A batch-1 layer is a short chain of latencies beside
+// Estimated SM cycles of one launch under a placed plan, up to a constant.  A batch-1 layer is a short chain of latencies beside
 // a load stream, so neither the fewest bytes nor the most CTAs is right for every shape:
 //   * the main loop is the slowest of: the multiplications of a rank's K blocks; all CTAs' bytes at what L2 delivers
-//     (7000 B/clk, weights re-read by every pixel tile); the layer's weights, cold in HBM, at what the loads in flight
-//     sustain (720 B/clk).  Where two are close they add up (a 4-norm);
-//   * a turn of the ring costs a memory round trip, so a deep ring of small tiles gains;
-//   * staging the accumulator, the cluster's barrier and remote reads, the residual and GELU rows of a rank, and a second
-//     CTA on an SM (it delays the early start of the next kernel) each take their share.
-// The constants were fitted on a B200, for the choice rather than the time: first to 4400 launches timed by themselves (471
-// layers of ResNet, Inception, VGG, DenseNet and BERT at odd and even sizes, weights cold: on layers left out of the fit the
-// choice is within 3 % of the best of the ~10 candidates, where the largest tiles that put 48 CTAs in flight lost 9 %), then
-// to 7200 replays of 20 whole models under different plans, where the weights of the next layer already load beside this one.
+//     (weights re-read by every pixel tile); the layer's weights, cold in HBM.  Where two are close they add up (a 4-norm);
+//   * K blocks beyond the ring wait for their refill, and a deep ring of small tiles gains;
+//   * the exchange of a K split costs its latency and the bytes that distributed shared memory takes, 15 a clock and SM; the
+//     cluster barrier of a receive area over the ring;
+//   * each turn of the two halves of a CTA over its pixel groups, more with a residual, a second output or GELU;
+//   * a second CTA on an SM (it delays the early start of the next kernel), and every CTA a little.
+// The constants were fitted on a B200, for the choice rather than the time: first to 6660 launches timed by themselves (316
+// layers of ResNet, Inception, VGG, DenseNet and BERT at odd and even sizes, weights cold: on layers left out of the fit the choice
+// is within 3 % of the best of a layer's ~20 plans, where the estimate for the staged exchange loses 7 %), then to 3655 replays of
+// each of 21 whole models under different plans, where branches share the SMs and the next layer's weights load beside this
+// one: 1.1 % faster over the models again (Inception-v3 5 %).
 static float tc_plan_cycles(const ConvP& p, const TcPlan& c) {
+    auto pow4 = [](float x) { return x * x * x * x; };
+    const float kb = (float)c.kb_per_split, rows = (float)(p.co < TC_BM ? ceil_div_i(p.co, 8) * 8 : TC_BM);
+    const float bytes = 128.f * (rows + c.n_valid), ctas = (float)c.splits * c.n_tiles * c.m_tiles;
+    const float weights = 4.f * p.co * p.ci * p.kh * p.kw;
+    const float mma = 189.f + 0.273f * c.n_mma;
+    float t = sqrtf(sqrtf(pow4(kb * (mma > 2.f * c.n_mma ? mma : 2.f * c.n_mma)) + pow4(ctas * kb * bytes / 22500.f) + pow4(weights / 4460.f)));
+    t += (411.f * (c.kb_per_split - c.stages) + 67.f * kb) / c.stages;
+    if (c.splits > 1)
+        t += 1210.f + 51.f * c.recv_late + 0.317f * c.n_valid * (p.co < TC_BM ? p.co : TC_BM) * (c.splits - 1) / c.splits;
+    const int groups = ceil_div_i(c.n_valid, 4), turns = ceil_div_i(c.gpc < groups ? c.gpc : groups, 2);
+    t += turns * (606.f + (p.ep & EP_RES ? 203.f : 0.f) + (p.ep & EP_DUAL ? 106.f : 0.f) + (p.ep & EP_GELU ? 211.f : 0.f));
+    return t + 0.79f * c.n_valid + 15.2f * ctas + 1760.f * (ceil_div_i((int)ctas, 148) - 1);
+}
+
+// The estimate that chose plans when partials were read from the peers' staging tiles.  Schedules written then state its choice and
+// load with it (see ConvP::plan_earlier).
+static float tc_plan_cycles_earlier(const ConvP& p, const TcPlan& c) {
     auto pow4 = [](float x) { return x * x * x * x; };
     const float kb = (float)c.kb_per_split, bytes = TC_A_BYTES + 128.f * c.n_valid;
     const float ctas = (float)c.splits * c.n_tiles * c.m_tiles;
@@ -151,22 +170,27 @@ int tc_plan(const ConvP& p, TcPlan* pl) {
     }
     TcPlan best;
     float best_cycles = 0.f;
-    for (int cap : {208, 160, 128, 112, 96, 80, 64, 48, 32, 24, 16})
+    const bool earlier = p.plan_earlier != 0;
+    for (int cap : {208, 160, 128, 112, 96, 80, 64, 56, 48, 40, 32, 24, 16, 8}) {
+        if (earlier && (cap == 56 || cap == 40 || cap == 8)) continue;
         for (int want = 1; want <= TC_MAX_SPLITS; want *= 2) {
             const int fixed = p.plan_splits;   // a name may fix the splits alone: as many of them as K allows
             if (fixed > 0 && want > 1) break;
             TcPlan c;
             if (tc_plan_cap(p, cap, fixed > 0 ? fixed : want, &c) != REEF_SUCC) continue;
             if (fixed == 0 && c.splits != want) continue;
-            const float cycles = tc_plan_cycles(p, c);
+            float cycles = tc_plan_cycles_earlier(p, c);   // (its ring was not yet shared with a receive area)
+            if (tc_place_recv(&c, earlier) != REEF_SUCC) continue;
+            if (!earlier) cycles = tc_plan_cycles(p, c);
             if (best_cycles == 0.f || cycles < best_cycles) {
                 best = c;
                 best_cycles = cycles;
             }
         }
+    }
     if (best_cycles == 0.f) return REEF_NOT_FOUND;
     *pl = best;
-    return tc_place_recv(pl, p.plan_earlier != 0);
+    return REEF_SUCC;
 }
 
 // ---- tensor maps ---------------------------------------------------------------------------------

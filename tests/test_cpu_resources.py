@@ -284,6 +284,8 @@ EARLIER_PLANS = [   # kernel name, cluster x tiles and shared memory that earlie
     ("fused_nn_conv2d_add_nn_relu__ci64_hi56_wi56_co64_kh3_kw3_sh1_sw1_ph1_pw1_v1", [2, 56], 99584),
     ("fused_nn_conv2d_add_nn_relu__ci64_hi17_wi17_co64_kh3_kw3_sh1_sw1_ph1_pw1_v1_tp64_ts2", [2, 6], 99584),
     ("reef_matmul_nt_bias__m128_n2304_k768_v1", [2, 72], 103680),
+    ("reef_matmul_nt_bias_gelu__m384_n3072_k768_v1", [2, 120], 107776),
+    ("fused_nn_conv2d_add_nn_relu__ci512_hi14_wi14_co512_kh3_kw3_sh1_sw1_ph1_pw1_v1", [8, 16], 99584),
     ("reef_layernorm__rows128_h768", [16, 1], 0),
 ]
 
