@@ -214,13 +214,16 @@ __device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned 
     } else if (k_begin < k_end) {
         load_k(k_begin);
     }
-    int buf = 0;
+    int buf = 0, f = flag != nullptr ? ld_flag(flag) : 0;
 #pragma unroll 1
     for (int k0 = k_begin; k0 < k_end; k0 += kAttChunk) {
-        // best-effort flavour: loop-head poll of the preempt flag
-        if (flag != nullptr && __any_sync(0xffffffffu, ld_flag(flag))) {
-            stopped = true;
-            break;
+        // best-effort flavour: loop-head poll of the preempt flag, asked for a step ahead
+        if (flag != nullptr && k0 > k_begin) {
+            if (__any_sync(0xffffffffu, f)) {
+                stopped = true;
+                break;
+            }
+            f = ld_flag(flag);
         }
         if (STAGED) {
             stage(k0 + kAttChunk, 1, mine_s + (buf ^ 1) * 4096, false);

@@ -175,12 +175,13 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
         if (kt < slices) load(s);
         commit();
     }
-    int stage = 0, fill = STAGES - 1;
+    int stage = 0, fill = STAGES - 1, f = 0;
     for (int i0 = group, n = 0; i0 < slices; i0 += KG, n++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncwarp();                          // slice landed for every lane; the stage before it is free for every lane
-        // best-effort flavour: loop-head poll of the preempt flag, every 8th slice of a warp
-        if (flag != nullptr && (n & 7) == 7 && __any_sync(0xffffffffu, ld_flag(flag))) {
+        // best-effort flavour: loop-head poll of the preempt flag, every 8th slice of a warp, asked for four slices ahead
+        if (flag != nullptr && (n & 7) == 3) f = ld_flag(flag);
+        if (flag != nullptr && (n & 7) == 7 && __any_sync(0xffffffffu, f)) {
             stopped = true;
             break;
         }

@@ -407,8 +407,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // running one is resident early (programmatic dependent launch) and made its entry poll long before its
             // predecessor finished, possibly before the flag went up.  Its first loads are out (their barriers were
             // armed for both operands, so the activation loads had to follow the weight loads); it issues no more, and
-            // the MMA warp only waits for those to land.
-            if (BE && !stop) stop = __any_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(P.preempt_flag) != 0);
+            // the MMA warp only waits for those to land.  Every look is taken four K blocks after its load was issued: waited
+            // for in place, the trip to L2 stood between the multiplications (0.6 us a launch, 1.6 in BERT's matmuls).
+            int f = 0;
+            if (BE) f = *reinterpret_cast<const volatile int*>(P.preempt_flag);
             for (int i = first; i < nkb && ok && !stop; i++) {
                 // coordinates are worked out ahead of the wait for a free stage: the per-tap sub-lattice and offsets come from a
                 // host table
@@ -420,13 +422,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                     c2 = tile_y * P.rows + P.tap_qy[t];
                 }
                 if (++cb == P.cblocks) { cb = 0; tap++; }
-                // loop-head poll of the preempt flag (every 4th K block): the load is issued before the wait for a
-                // free stage and looked at after it, so its latency hides behind the wait
-                int f = 0;
-                if (BE && (i & 3) == 0) f = *reinterpret_cast<const volatile int*>(P.preempt_flag);
                 ok = mbar_wait_warp(bar_empty + 8 * s, par);
                 if (!ok) break;
-                if (BE && __any_sync(0xffffffffu, f != 0)) { stop = true; break; }
+                if (BE && ((i - first) & 3) == 3) {   // loop-head poll of the preempt flag
+                    if (__any_sync(0xffffffffu, f != 0)) { stop = true; break; }
+                    f = *reinterpret_cast<const volatile int*>(P.preempt_flag);
+                }
                 const uint32_t dst = base + s * stage_bytes, bar = bar_full + 8 * s;
                 mbar_expect_tx_if(lead, bar, tx);
                 tma_load_3d_if(lead, dst, &P.tm_w, bar, c0, t, m0);
@@ -435,6 +436,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 issued++;
                 if (++s == NS) { s = 0; par ^= 1u; }
             }
+            if (BE && !stop) stop = __any_sync(0xffffffffu, f != 0);
             if (BE && stop && lane == 0) {
                 s_flags[1] = (uint32_t)issued;     // first how far the loads got, then the request to stop
                 __threadfence_block();
@@ -551,6 +553,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 cluster_wait();
             }
             if (tid == 0) tc_stamp(P, 3);
+            // what this rank saw, to every other rank (ahead of the shares: the slowest store is the last)
+            if (BE && warp == 7 && lane < S && lane != split) {
+                const uint32_t peer = mapa_shared(base, (uint32_t)lane);
+                st_async_u32(peer + (smem_u32((const void*)&s_flags[2]) - base) + (uint32_t)split * 4u, peer + (bar_recv - base), abort_all || !ok ? 1u : 0u);
+            }
+            __syncwarp();
             // (A rank that gave up sends what it has: the receivers count bytes, and nobody stores the result of a failed or
             // preempted launch.)
             if (quad * 32 < co_lim) {
@@ -579,16 +587,11 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 tmem_free(tmem, (uint32_t)P.tmem_cols);
             }
-            if (BE && tid < S && tid != split) {
-                const uint32_t peer = mapa_shared(base, (uint32_t)tid);
-                st_async_u32(peer + (smem_u32((const void*)&s_flags[2]) - base) + (uint32_t)split * 4u, peer + (bar_recv - base), abort_all || !ok ? 1u : 0u);
-            }
             if (tid == 0) tc_stamp(P, 7);   // shares sent
             if (recv_bytes != 0 && !mbar_wait_cluster_warp(bar_recv, 0)) ok = false;
             if (BE) {
                 // every rank has the words of all the others: all take the same exit
-                for (int q = 0; q < S; q++)
-                    if (q != split && s_flags[2 + q] != 0) abort_all = true;
+                if (__any_sync(0xffffffffu, lane < S && lane != split && s_flags[2 + lane] != 0)) abort_all = true;
             }
         }
         if (!ok && P.error_word) *reinterpret_cast<volatile int*>(P.error_word) = 1;

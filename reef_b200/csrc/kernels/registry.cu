@@ -662,11 +662,14 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_con
                                                  int* __restrict__ task_slot) {
     if (F == F_LAYERNORM) prefetch_layernorm(t);
     if (F == F_DENSE) prefetch_dense(t, blockIdx.x);
-    pdl_prologue();
     // ONE thread reads the flag and the block takes one decision: were every thread to read it for itself, a flag
     // that goes up between the reads of two warps would let part of a block leave and the rest run the body with
-    // threads missing (wrong partial sums counted as a complete block, barriers short of arrivals).
-    if (__syncthreads_or(threadIdx.x == 0 ? ld_flag(flag) : 0)) {
+    // threads missing (wrong partial sums counted as a complete block, barriers short of arrivals).  It is read ahead of
+    // the wait for the previous kernel, so that its trip to L2 (0.4 us) is not on the way to the body: a flag that goes up
+    // during that wait is seen by the body's polls or by the next kernel of the stream, which starts behind this wait.
+    const int up = threadIdx.x == 0 ? ld_flag(flag) : 0;
+    pdl_prologue();
+    if (__syncthreads_or(up)) {
         if (threadIdx.x == 0) preempt_stamp_leave();
         return;
     }

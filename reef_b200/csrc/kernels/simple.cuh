@@ -426,6 +426,9 @@ __device__ __forceinline__ bool body_dense(const KTask& t, int vb, unsigned char
         if (warp == 0)
             for (int st = 0; st < first; st++) issue(st);
         int issued = first;        // meaningful in warp 0 only
+        // best-effort flavour: the preempt flag is asked for at every refill and looked at with the next one, 32 KB of weights
+        // later (waited for in place, its trip to L2 held the ring: 25088 -> 4096 79 us instead of 71)
+        int f = flag != nullptr && tid == 0 ? ld_flag(flag) : 0;
         bool ok = true;
         float acc[kDenseRG];
         int st = 0;
@@ -480,7 +483,7 @@ __device__ __forceinline__ bool body_dense(const KTask& t, int vb, unsigned char
                 if (warp == 0 && st + kDenseStages < nst && !(flag != nullptr && ctl[0])) {
                     int go = 1;
                     if (lane == 0) {
-                        if (flag != nullptr && ld_flag(flag)) {              // loop-head poll of the preempt flag
+                        if (f != 0) {                                        // loop-head poll of the preempt flag
                             ctl[1] = issued;                                 // first how far the copies got, then the request
                             __threadfence_block();
                             ctl[0] = 1;
@@ -489,6 +492,7 @@ __device__ __forceinline__ bool body_dense(const KTask& t, int vb, unsigned char
                             ctl[2] = 1;
                             go = 0;
                         }
+                        if (flag != nullptr) f = ld_flag(flag);
                     }
                     go = __shfl_sync(0xffffffffu, go, 0);
                     if (go) {
