@@ -347,6 +347,17 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
 
 static bool g_attr_set[16] = {false};
 
+// The number of K splits is a template parameter: the exchange and the sums are straight code behind the accumulator.
+typedef void (*tc_kernel_fn)(TcParams);
+static tc_kernel_fn tc_kernel(bool be, int splits) {
+    switch (splits) {
+        case 1: return be ? reef_conv_tc_kernel<true, 1> : reef_conv_tc_kernel<false, 1>;
+        case 2: return be ? reef_conv_tc_kernel<true, 2> : reef_conv_tc_kernel<false, 2>;
+        case 4: return be ? reef_conv_tc_kernel<true, 4> : reef_conv_tc_kernel<false, 4>;
+        default: return be ? reef_conv_tc_kernel<true, 8> : reef_conv_tc_kernel<false, 8>;
+    }
+}
+
 #ifdef REEF_DEBUG_AIDS
 static long long* g_trace[16] = {nullptr};
 // Phase trace of the tensor-core convolution (development builds only): when enabled, block (0,0) of every launch
@@ -394,8 +405,8 @@ int tc_prepare_device() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 16 && !g_attr_set[dev]) {
-        const void* fns[2] = {(const void*)reef_conv_tc_kernel<false>, (const void*)reef_conv_tc_kernel<true>};
-        for (const void* fn : fns) {
+        for (int i = 0; i < 8; i++) {
+            const void* fn = (const void*)tc_kernel(i & 1, 1 << (i >> 1));
             cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
             if (e == cudaSuccess)   // the whole unified L1/shared array as shared memory, so that two CTAs are resident
                 e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -459,8 +470,7 @@ int tc_launch(const TcParams& P0, const TcPlan& pl, cudaStream_t st, const int* 
     cfg.numAttrs = na;
     // the best-effort flavour (flag polls at block entry and at the producer's loop head) is its own instantiation:
     // the real-time flavour carries no poll
-    cudaError_t e = flag != nullptr ? cudaLaunchKernelEx(&cfg, reef_conv_tc_kernel<true>, P)
-                                    : cudaLaunchKernelEx(&cfg, reef_conv_tc_kernel<false>, P);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, tc_kernel(flag != nullptr, pl.splits), P);
     if (e != cudaSuccess) {
         set_error(std::string("cudaLaunchKernelEx(conv_tc): ") + cudaGetErrorString(e));
         return REEF_FAIL;
@@ -469,7 +479,7 @@ int tc_launch(const TcParams& P0, const TcPlan& pl, cudaStream_t st, const int* 
 }
 
 int tc_func_attrs(const TcPlan& pl, cudaFuncAttributes* fa, int* occ) {
-    cudaError_t e = cudaFuncGetAttributes(fa, (const void*)reef_conv_tc_kernel<false>);
+    cudaError_t e = cudaFuncGetAttributes(fa, (const void*)tc_kernel(false, pl.splits));
     if (e != cudaSuccess) {
         set_error(std::string("cudaFuncGetAttributes(conv_tc): ") + cudaGetErrorString(e));
         return REEF_FAIL;

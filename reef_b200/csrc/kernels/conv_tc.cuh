@@ -243,7 +243,7 @@ __device__ __forceinline__ void tc_finish_split(const TcParams& P, const float* 
 // finish what has landed; it takes part in the exchange all the same, each rank sending along what it saw, and if any
 // rank stopped, ALL ranks skip the stores and the completion counter — the kernel is idempotent, so it is simply
 // launched again later.  The real-time flavour carries none of this.
-template <bool BE>
+template <bool BE, int S>
 __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __grid_constant__ TcParams P) {
     extern __shared__ __align__(16) unsigned char tc_smem_raw[];
     // stage buffers need 1024-byte alignment (swizzle atom); carve barriers behind them
@@ -269,7 +269,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     const int split = blockIdx.x;
     const int tile = P.tile_begin + (int)blockIdx.y;
     const int tile_n = tile % P.n_tiles, tile_m = tile / P.n_tiles;
-    const int S = P.splits;
     const int kb_begin = split * P.kb_per_split;
     const int kb_end = min(kb_begin + P.kb_per_split, P.kb_total);
     const int nkb = kb_end - kb_begin;
@@ -598,16 +597,9 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         if (tid == 0) tc_stamp(P, 8);       // shares received
         if (ok && !abort_all && quad * 32 < co_lim) {
             const uint32_t src = S == 1 ? taddr + (uint32_t)gfirst * 4u : recv + (uint32_t)((gfirst - grp0) * TC_BM + row) * 16u;
-#define TC_FINISH(S_, U_)                                   \
-    do {                                                    \
-        if (gelu) tc_finish<S_, U_, true>(P, w, src);       \
-        else tc_finish<S_, U_, false>(P, w, src);           \
-    } while (0)
-            if (S == 8) TC_FINISH(8, 1);
-            else if (S == 4) TC_FINISH(4, 1);
-            else if (S == 2) TC_FINISH(2, 2);
-            else TC_FINISH(1, 2);
-#undef TC_FINISH
+            constexpr int U = S <= 2 ? 2 : 1;
+            if (gelu) tc_finish<S, U, true>(P, w, src);
+            else tc_finish<S, U, false>(P, w, src);
         }
         if (tid == 0) tc_stamp(P, 9);   // rows finished
         if (BE && abort_all && tid == 0 && P.stamps != nullptr) {
