@@ -201,51 +201,69 @@ __device__ __forceinline__ bool body_copy(const KTask& t, int vb, unsigned char*
 // avg: count-include-pad multiplies by 1/k^2 (reference: resource/inception/inception.cu:578-587)
 // args: in, out[, bias].  One thread = 4 channels of one output pixel; vblock = 256 such items.
 constexpr int kPoolItemsPerBlock = kThreads;
+__device__ __forceinline__ void pool_add(bool max, float4& acc, float4 v) {
+    if (max) {
+        acc.x = fmaxf(acc.x, v.x); acc.y = fmaxf(acc.y, v.y); acc.z = fmaxf(acc.z, v.z); acc.w = fmaxf(acc.w, v.w);
+    } else {
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+}
+// K = 2, 3: a window of the usual sizes.  All of its values are requested at once, from places clamped into the input (a value
+// from outside the window's part of the input is replaced by the neutral one): the taps as branches were K * K trips to L2 one after
+// the other.  K = 0: any size, tap by tap.  3x3 over 112x112x64 3.06 -> 1.96 us, over
+// 17x17x768 3.09 -> 1.86 us a launch; a replay of Inception-v3 289 -> 282 us.
+template <bool MAX, int K>
+__device__ __forceinline__ void pool_window(const PoolP& p, const float* in, int oy, int ox, float4& acc, int& cnt) {
+    const float4 neutral = acc;
+    const int y0 = oy * p.s - p.p, x0 = ox * p.s - p.p;
+    if (K > 0) {
+        float4 v[K == 0 ? 1 : K * K];
+#pragma unroll
+        for (int ky = 0; ky < K; ky++)
+#pragma unroll
+            for (int kx = 0; kx < K; kx++)
+                v[ky * K + kx] = *reinterpret_cast<const float4*>(in + (size_t)(min(max(y0 + ky, 0), p.hi - 1) * p.wi + min(max(x0 + kx, 0), p.wi - 1)) * p.ics);
+#pragma unroll
+        for (int ky = 0; ky < K; ky++)
+#pragma unroll
+            for (int kx = 0; kx < K; kx++) {
+                const bool there = (unsigned)(y0 + ky) < (unsigned)p.hi && (unsigned)(x0 + kx) < (unsigned)p.wi;
+                pool_add(MAX, acc, there ? v[ky * K + kx] : neutral);
+                cnt += there ? 1 : 0;
+            }
+    } else {
+        for (int ky = 0; ky < p.k; ky++)
+            for (int kx = 0; kx < p.k; kx++)
+                if ((unsigned)(y0 + ky) < (unsigned)p.hi && (unsigned)(x0 + kx) < (unsigned)p.wi) {
+                    pool_add(MAX, acc, *reinterpret_cast<const float4*>(in + (size_t)((y0 + ky) * p.wi + x0 + kx) * p.ics));
+                    cnt++;
+                }
+    }
+}
 template <bool MAX>
 __device__ __forceinline__ bool body_pool(const KTask& t, int vb, unsigned char*, const int*) {
     const PoolP& p = t.p.pool;
-    const float* in = (const float*)t.a[0];
-    float* out = (float*)t.a[1];
-    const float* bias = p.has_bias ? (const float*)t.a[2] : nullptr;
-    const int c4 = p.c >> 2;
-    const int total = p.ho * p.wo * c4;
-#pragma unroll 1
-    for (int it = 0; it < kPoolItemsPerBlock / kThreads; it++) {
-        int i = vb * kPoolItemsPerBlock + it * kThreads + threadIdx.x;
-        if (i >= total) break;
-        int pix = i / c4, cc = (i - pix * c4) << 2;
-        int oy = pix / p.wo, ox = pix - oy * p.wo;
-        float4 acc = MAX ? make_float4(-3.402823e38f, -3.402823e38f, -3.402823e38f, -3.402823e38f)
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
-        int cnt = 0;
-        for (int ky = 0; ky < p.k; ky++) {
-            int iy = oy * p.s + ky - p.p;
-            if (iy < 0 || iy >= p.hi) continue;
-            for (int kx = 0; kx < p.k; kx++) {
-                int ix = ox * p.s + kx - p.p;
-                if (ix < 0 || ix >= p.wi) continue;
-                float4 v = *reinterpret_cast<const float4*>(in + ((size_t)iy * p.wi + ix) * p.ics + p.ioff + cc);
-                if (MAX) {
-                    acc.x = fmaxf(acc.x, v.x); acc.y = fmaxf(acc.y, v.y);
-                    acc.z = fmaxf(acc.z, v.z); acc.w = fmaxf(acc.w, v.w);
-                } else {
-                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                }
-                cnt++;
-            }
+    const int c4 = p.c >> 2, i = vb * kPoolItemsPerBlock + (int)threadIdx.x;
+    if (i >= p.ho * p.wo * c4) return true;
+    const int pix = i / c4, cc = (i - pix * c4) << 2, oy = pix / p.wo, ox = pix - oy * p.wo;
+    const float* in = (const float*)t.a[0] + p.ioff + cc;
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (MAX && p.has_bias) b = *reinterpret_cast<const float4*>((const float*)t.a[2] + cc);
+    float4 acc = MAX ? make_float4(-3.402823e38f, -3.402823e38f, -3.402823e38f, -3.402823e38f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    int cnt = 0;
+    if (p.k == 3) pool_window<MAX, 3>(p, in, oy, ox, acc, cnt);
+    else if (p.k == 2) pool_window<MAX, 2>(p, in, oy, ox, acc, cnt);
+    else pool_window<MAX, 0>(p, in, oy, ox, acc, cnt);
+    if (MAX) {
+        if (p.has_bias) {
+            acc.x = fmaxf(acc.x + b.x, 0.f); acc.y = fmaxf(acc.y + b.y, 0.f);
+            acc.z = fmaxf(acc.z + b.z, 0.f); acc.w = fmaxf(acc.w + b.w, 0.f);
         }
-        if (MAX) {
-            if (bias) {
-                float4 b = *reinterpret_cast<const float4*>(bias + cc);
-                acc.x = fmaxf(acc.x + b.x, 0.f); acc.y = fmaxf(acc.y + b.y, 0.f);
-                acc.z = fmaxf(acc.z + b.z, 0.f); acc.w = fmaxf(acc.w + b.w, 0.f);
-            }
-        } else {
-            float sc = p.cip ? 1.0f / (float)(p.k * p.k) : 1.0f / (float)(cnt > 0 ? cnt : 1);
-            acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
-        }
-        *reinterpret_cast<float4*>(out + (size_t)pix * p.ocs + p.ooff + cc) = acc;
+    } else {
+        const float sc = p.cip ? 1.0f / (float)(p.k * p.k) : 1.0f / (float)(cnt > 0 ? cnt : 1);
+        acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
     }
+    *reinterpret_cast<float4*>((float*)t.a[1] + (size_t)pix * p.ocs + p.ooff + cc) = acc;
     return true;
 }
 
