@@ -276,8 +276,6 @@ __device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned 
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
             const float mnew = fmaxf(m[r], top);
-            const float corr = mnew == ninf ? 1.f : expf(m[r] - mnew);
-            m[r] = mnew;
             float add = 0.f;
 #pragma unroll
             for (int j = 0; j < 2; j++)
@@ -286,12 +284,18 @@ __device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned 
                     s[j][e] = s[j][e] == ninf ? 0.f : expf(s[j][e] - mnew);
                     add += s[j][e];
                 }
-            l[r] = l[r] * corr + add;
+            if (k0 > k_begin) {   // (the first step has nothing to rescale)
+                const float corr = mnew == ninf ? 1.f : expf(m[r] - mnew);
+                l[r] = l[r] * corr + add;
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                ctx[j][2 * r] *= corr;
-                ctx[j][2 * r + 1] *= corr;
+                for (int j = 0; j < 8; j++) {
+                    ctx[j][2 * r] *= corr;
+                    ctx[j][2 * r + 1] *= corr;
+                }
+            } else {
+                l[r] = add;
             }
+            m[r] = mnew;
         }
         Bf16Triple p[4];
 #pragma unroll
@@ -352,16 +356,18 @@ __device__ __forceinline__ bool attention_rows(const KTask& t, int vb, unsigned 
                     make_float4(ctx[4 * q][2 * r + h], ctx[4 * q + 1][2 * r + h], ctx[4 * q + 2][2 * r + h], ctx[4 * q + 3][2 * r + h]);
     }
     __syncthreads();
+    // sixteen lanes share a row: each works out the factor of one warp's part, the others have it from there
     const int row = threadIdx.x >> 4, d0 = (threadIdx.x & 15) * 4;
-    float top = ninf;
+    const float mw = ml[(lane & 7) * ROWS + row];
+    float top = mw;
 #pragma unroll
-    for (int w = 0; w < 8; w++) top = fmaxf(top, ml[w * ROWS + row]);
+    for (int q = 1; q < 8; q <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, q));
+    const float fw = mw == ninf ? 0.f : expf(mw - top);
     float sum = 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < 8; w++) {          // fixed order: deterministic
-        const float mw = ml[w * ROWS + row];
-        const float f = mw == ninf ? 0.f : expf(mw - top);
+        const float f = __shfl_sync(0xffffffffu, fw, (lane & 16) + w);
         sum = fmaf(f, ml[(8 + w) * ROWS + row], sum);
         const float4 x = *reinterpret_cast<const float4*>(part + (w * ROWS + row) * kAttRowStride + d0);
         o.x = fmaf(f, x.x, o.x); o.y = fmaf(f, x.y, o.y); o.z = fmaf(f, x.z, o.z); o.w = fmaf(f, x.w, o.w);
