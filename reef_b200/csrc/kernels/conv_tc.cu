@@ -179,7 +179,7 @@ int tc_plan(const ConvP& p, TcPlan* pl) {
             TcPlan c;
             if (tc_plan_cap(p, cap, fixed > 0 ? fixed : want, &c) != REEF_SUCC) continue;
             if (fixed == 0 && c.splits != want) continue;
-            float cycles = tc_plan_cycles_earlier(p, c);   // (its ring was not yet shared with a receive area)
+            float cycles = earlier ? tc_plan_cycles_earlier(p, c) : 0.f;   // (its ring was not yet shared with a receive area)
             if (tc_place_recv(&c, earlier) != REEF_SUCC) continue;
             if (!earlier) cycles = tc_plan_cycles(p, c);
             if (best_cycles == 0.f || cycles < best_cycles) {
