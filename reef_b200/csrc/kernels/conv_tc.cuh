@@ -41,7 +41,7 @@ enum : int { TC_EP_RES = 1, TC_EP_BIAS = 2, TC_EP_GB = 4, TC_EP_RELU = 8, TC_EP_
 
 // exact-erf GELU (reference: resource/bert/bert.cu:167-173).  Not inlined here on purpose: inlined, the compiler turned
 // the uniform `if (gelu)` of the epilogue into straight-line code and every layer paid for erff on each element
-// (0.5 us per launch on the row-finishing loop).  Where a whole loop is for GELU layers (tc_finish_rows) it is inlined:
+// (0.5 us per launch on the row-finishing loop).  Where a whole loop is for GELU layers (tc_finish<.., true>) it is inlined:
 // the calls made BERT's 768 -> 3072 matmul at 384 tokens spend 8 us on finishing its rows.
 __device__ __forceinline__ float tc_gelu_inline(float v) { return v * (0.5f * erff(v * 0.70710678118654752440f) + 0.5f); }
 static __device__ __noinline__ float tc_gelu(float v) { return tc_gelu_inline(v); }

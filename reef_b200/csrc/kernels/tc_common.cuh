@@ -129,21 +129,15 @@ __device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t pa
     }
     return false;
 }
-// Activations of an earlier kernel: a volatile load stays behind griddepcontrol.wait.  (__ldg promises memory that never
-// changes, and the compiler did move such loads above the wait.)
-__device__ __forceinline__ float4 ld_activation(const float* p) {
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
 // A model constant, requested where this stands: a plain load may be moved down to its first use, behind the waits.
 __device__ __forceinline__ float ld_param(const float* p) {
     float v;
     asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
-// The same for one value under a per-lane condition.  Predicated: as a branch around the instruction each of them cost about 30
-// cycles of a launch's tail.
+// An activation of an earlier kernel, under a per-lane condition: a volatile load stays behind griddepcontrol.wait (__ldg
+// promises memory that never changes, and the compiler did move such loads above the wait).  Predicated: as a branch around
+// the instruction each of them cost about 30 cycles of a launch's tail.
 __device__ __forceinline__ float ld_activation_if(bool c, const float* p) {
     float v;
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.f32 %0, [%1];\n\t}" : "=f"(v) : "l"(p), "r"((int)c));
