@@ -23,12 +23,14 @@ struct Bf16Triple {
 };
 __device__ __forceinline__ Bf16Triple bf16_split(float x, float y) {
     Bf16Triple r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.h) : "f"(y), "f"(x));
-    x -= __uint_as_float(r.h << 16);
-    y -= __uint_as_float(r.h & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.m) : "f"(y), "f"(x));
-    x -= __uint_as_float(r.m << 16);
-    y -= __uint_as_float(r.m & 0xffff0000u);
+    // x - h as h * -1 + x with a bf16 operand: no unpacking (two instructions a value less), and exact, as the subtraction is
+    // (ResNet-50 at 193x193 in fp32, a replay: 564 -> 549 us)
+    asm("{\n\t.reg .b16 p, q, n;\n\tmov.b16 n, 0xBF80;\n\tcvt.rn.bf16x2.f32 %0, %2, %1;\n\tmov.b32 {p, q}, %0;\n\t"
+        "fma.rn.f32.bf16 %1, p, n, %1;\n\tfma.rn.f32.bf16 %2, q, n, %2;\n\t}"
+        : "=&r"(r.h), "+f"(x), "+f"(y));
+    asm("{\n\t.reg .b16 p, q, n;\n\tmov.b16 n, 0xBF80;\n\tcvt.rn.bf16x2.f32 %0, %2, %1;\n\tmov.b32 {p, q}, %0;\n\t"
+        "fma.rn.f32.bf16 %1, p, n, %1;\n\tfma.rn.f32.bf16 %2, q, n, %2;\n\t}"
+        : "=&r"(r.m), "+f"(x), "+f"(y));
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.l) : "f"(y), "f"(x));
     return r;
 }
@@ -36,6 +38,12 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the same from zero: no registers to clear
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // d[i] = the product of fragments a and b[i], N of them side by side (the multiplications into one accumulator depend on one

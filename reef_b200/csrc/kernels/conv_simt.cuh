@@ -21,9 +21,13 @@
 // run on their own through a private ring of cp.async stages, no block barrier in the loop; the KG partial tiles meet in
 // shared memory, summed in a fixed order.  A lane's K positions in a fragment are four consecutive ones (the order inside
 // a slice is free as long as both operands agree), so an operand row is read with one 128-bit load.
-// Measured, 3x3 256 -> 256 at 13x13: 133 -> 13.6 us; 3x3 512 -> 512 at 7x7: 261 -> 18.3 us; ResNet-50 at 193x193, a request:
-// 3.39 -> 0.64 ms.
+// What is left: a block alone on its SM keeps the tensor cores busy a quarter of the time, two of them half of it, and issue
+// 82 % of what the schedulers can; so every instruction of a slice counts (ResNet-50 at 193x193: addresses per tap instead of
+// per slice, and no clearing of accumulators, 585 -> 564 us a replay; ResNet-18 at 64x64 168 -> 153).
+// Measured, 3x3 256 -> 256 at 13x13: 133 us by fp32 instructions, 13.9, now 12.4; 3x3 512 -> 512 at 7x7: 261, 19.5, 16.7.
 #pragma once
+#include <type_traits>
+
 #include "bf16_split.cuh"
 #include "task.cuh"
 
@@ -88,7 +92,9 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
 
     // Loader: this lane copies chunk lane % 4 of rows lane / 4 + 8 i (four lanes read the 64 bytes of a row).  Per pixel
     // row the offset of its first tap, and the taps inside the image: FAST, one bit per filter row and column, else the
-    // position of the first tap.  Rows beyond the last pixel repeat it (their results are not stored).
+    // position of the first tap.  Rows beyond the last pixel or channel repeat the last one (their results are not stored).
+    // What a slice needs beyond one address per row is worked out where the tap changes: with it done for every slice, and
+    // the zeroing and adding of accumulators, a warp issued 358 instructions a slice, of which 156 multiply and split.
     const int lrow = lane >> 2, lk = (lane & 3) * 4;
     int off[TP / 8];
     int in_y[TP / 8], in_x[TP / 8];
@@ -101,46 +107,51 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
         in_y[i] = FAST ? taps_inside(iy, p.hi, p.kh) : iy;
         in_x[i] = FAST ? taps_inside(ix, p.wi, p.kw) : ix;
     }
-    const float* wrow = wgt + (size_t)(c0 + lrow) * p.ktot + lk;
-    const int wlast = p.co - 1 - c0 - lrow, wstep = 8 * p.ktot;   // rows further than wlast are beyond the last channel
+    unsigned woff[TC / 8];                     // rows of the weights, in elements from the block's first
+#pragma unroll
+    for (int j = 0; j < TC / 8; j++) woff[j] = (unsigned)(min(c0 + lrow + 8 * j, p.co - 1) - c0) * (unsigned)p.ktot;
+    const int ktot = p.ktot, ci = p.ci, kstep = KG * CBK;
     // slice kt = group, group + KG, ...: tap and channel of this lane's chunk are carried along
-    int kt = group, cb = group * CBK + lk, ky = 0, kx = 0;
-    auto settle = [&]() {
-        while (cb >= p.ci) {
-            cb -= p.ci;
+    int k = group * CBK + lk, cb = k, ky = 0, kx = 0;
+    const float* wslice = wgt + (size_t)c0 * ktot + k;
+    int tap_off[TP / 8], tap_in[TP / 8];       // this lane's pixels under the current tap: offset, 16 (bytes) or 0 outside
+    auto settle = [&](bool first) {
+        if (!first && cb < ci) return;
+        while (cb >= ci) {
+            cb -= ci;
             if (++kx == p.kw) {
                 kx = 0;
                 ky++;
             }
         }
+        const int d = (ky * p.wi + kx) * p.ics, y = min(ky, 31);   // (behind the last slice: no tap is bit 31)
+#pragma unroll
+        for (int i = 0; i < TP / 8; i++) {
+            const bool v = in_y[i] >> y & in_x[i] >> kx & 1;
+            tap_off[i] = v ? off[i] + d : 0;
+            tap_in[i] = v ? 16 : 0;
+        }
     };
-    if (FAST) settle();
+    if (FAST) settle(true);
     auto load = [&](int stage) {
         const uint32_t a = mine_s + (uint32_t)(stage * STAGE + lrow * CROW + lk) * 4;
-        const int k = kt * CBK;
         if (FAST) {
-            const bool kin = k + lk < p.ktot;
-            const int d = (ky * p.wi + kx) * p.ics + cb;
+            const bool kin = k < ktot;
 #pragma unroll
-            for (int i = 0; i < TP / 8; i++) {
-                const bool v = kin && (in_y[i] >> ky & in_x[i] >> kx & 1);
-                const float* src = in + (v ? off[i] + d : 0);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a + i * 8 * CROW * 4), "l"(src), "r"(v ? 16 : 0) : "memory");
-            }
-            const float* src = wrow + k;
+            for (int i = 0; i < TP / 8; i++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a + i * 8 * CROW * 4), "l"(in + tap_off[i] + cb), "r"(kin ? tap_in[i] : 0) : "memory");
+            const float* src = kin ? wslice : wgt;
 #pragma unroll
-            for (int j = 0; j < TC / 8; j++, src += wstep)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a + (TP + j * 8) * CROW * 4), "l"(kin && 8 * j <= wlast ? src : wgt),
-                             "r"(kin && 8 * j <= wlast ? 16 : 0)
-                             : "memory");
-            cb += KG * CBK;
-            settle();
+            for (int j = 0; j < TC / 8; j++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a + (TP + j * 8) * CROW * 4), "l"(src + woff[j]), "r"(kin ? 16 : 0) : "memory");
+            cb += kstep;
+            settle(false);
         } else {
 #pragma unroll 1
             for (int e = 0; e < 4; e++) {
-                const int ke = k + lk + e;
-                const bool kin = ke < p.ktot;
-                const int tp = ke / p.ci, c = ke - tp * p.ci;
+                const int ke = k + e;
+                const bool kin = ke < ktot;
+                const int tp = ke / ci, c = ke - tp * ci;
                 const int dy = tp / p.kw, dx = tp - dy * p.kw;
                 const int d = p.nchw ? (c * p.hi + dy) * p.wi + dx : (dy * p.wi + dx) * p.ics + c;
 #pragma unroll
@@ -149,15 +160,14 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
                     const bool v = kin && iy >= 0 && iy < p.hi && ix >= 0 && ix < p.wi;
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(a + (i * 8 * CROW + e) * 4), "l"(in + (v ? off[i] + d : 0)), "r"(v ? 4 : 0) : "memory");
                 }
-                const float* src = wrow + k + e;
+                const float* src = kin ? wslice + e : wgt;
 #pragma unroll
-                for (int j = 0; j < TC / 8; j++, src += wstep)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(a + ((TP + j * 8) * CROW + e) * 4),
-                                 "l"(kin && 8 * j <= wlast ? src : wgt), "r"(kin && 8 * j <= wlast ? 4 : 0)
-                                 : "memory");
+                for (int j = 0; j < TC / 8; j++)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(a + ((TP + j * 8) * CROW + e) * 4), "l"(src + woff[j]), "r"(kin ? 4 : 0) : "memory");
             }
         }
-        kt += KG;
+        k += kstep;
+        wslice += kstep;
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
@@ -170,23 +180,25 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
     const int g = lane >> 2, c = lane & 3;
     bool stopped = false;
     __syncthreads();                           // a persistent caller's previous tile is out of the ring
+    int loaded = group;                        // the slice that `load` fetches next
 #pragma unroll
     for (int s = 0; s < STAGES - 1; s++) {
-        if (kt < slices) load(s);
+        if (loaded < slices) load(s);
+        loaded += KG;
         commit();
     }
     int stage = 0, fill = STAGES - 1, f = 0;
-    for (int i0 = group, n = 0; i0 < slices; i0 += KG, n++) {
+    auto turn = [&] {                          // the next slice has landed and the stage before it is free, for every lane
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncwarp();                          // slice landed for every lane; the stage before it is free for every lane
-        // best-effort flavour: loop-head poll of the preempt flag, every 8th slice of a warp, asked for four slices ahead
-        if (flag != nullptr && (n & 7) == 3) f = ld_flag(flag);
-        if (flag != nullptr && (n & 7) == 7 && __any_sync(0xffffffffu, f)) {
-            stopped = true;
-            break;
-        }
-        if (kt < slices) load(fill);
+        __syncwarp();
+    };
+    auto refill = [&] {
+        if (loaded < slices) load(fill);
+        loaded += KG;
         commit();
+        if (++fill == STAGES) fill = 0;
+    };
+    auto multiply = [&](auto even) {
         // (rows of 64 bytes without padding: the eight lanes of a 128-bit load's quarter read two rows = all 32 banks)
         const float* a = mine + stage * STAGE + g * CROW + c * 4;
         const float4 x0 = *reinterpret_cast<const float4*>(a), x1 = *reinterpret_cast<const float4*>(a + 8 * CROW);
@@ -200,19 +212,36 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
             mma_bf16(small[j], a0.m, a1.m, a2.m, a3.m, b0.m, b1.m);
             mma_bf16(small[j], a0.m, a1.m, a2.m, a3.m, b0.h, b1.h);
             mma_bf16(small[j], a0.h, a1.h, a2.h, a3.h, b0.m, b1.m);
-            mma_bf16(big[j], a0.h, a1.h, a2.h, a3.h, b0.h, b1.h);
-        }
-        if (n & 1) {
-#pragma unroll
-            for (int j = 0; j < NT; j++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    sum[j][e] += big[j][e];
-                    big[j][e] = 0.f;
-                }
+            if (even.value) mma_bf16_zero(big[j], a0.h, a1.h, a2.h, a3.h, b0.h, b1.h);
+            else mma_bf16(big[j], a0.h, a1.h, a2.h, a3.h, b0.h, b1.h);
         }
         if (++stage == STAGES) stage = 0;
-        if (++fill == STAGES) fill = 0;
+    };
+    // two slices at a time, whose large products are added up before they join the sum
+    for (int i0 = group, n = 0; i0 < slices; i0 += 2 * KG, n++) {
+        turn();
+        refill();
+        multiply(std::true_type());
+        if (i0 + KG >= slices) break;
+        turn();
+        // best-effort flavour: loop-head poll of the preempt flag, every 8th slice of a warp, asked for four slices ahead
+        if (flag != nullptr && (n & 3) == 1) f = ld_flag(flag);
+        if (flag != nullptr && (n & 3) == 3 && __any_sync(0xffffffffu, f)) {
+            stopped = true;
+            break;
+        }
+        refill();
+        multiply(std::false_type());
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) sum[j][e] += big[j][e];
+    }
+    if (slices <= group || ((slices - group + KG - 1) / KG & 1) == 0) {   // every slice's large products are in the sum
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) big[j][e] = 0.f;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     if (__syncthreads_or(stopped)) return false;
