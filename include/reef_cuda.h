@@ -120,6 +120,8 @@ REEF_API reef_status reef_module_get_kernel(reef_module_t mod, const char* name,
  * "launch_params" (reference: model.cpp:35-37) and the dynamic shared memory in bytes as stored in
  * "shared_memory".  Needs no GPU; the resource generator calls it so json and registry agree. */
 REEF_API reef_status reef_kernel_plan(const char* name, uint32_t dims[6], uint32_t* dyn_smem, int* num_args);
+/* the same of a kernel that is resolved already: nothing is planned again */
+REEF_API reef_status reef_kernel_geometry(reef_kernel_t k, uint32_t dims[6], uint32_t* dyn_smem, int* num_args);
 /* Algorithmic work of one launch of a kernel name: floating-point operations and bytes that must move
  * (weights + inputs + outputs (+ residual, + second output) + per-channel parameters), and whether the name
  * selects the tensor-core kernel.  Needs no GPU; no reference counterpart (roofline bookkeeping). */

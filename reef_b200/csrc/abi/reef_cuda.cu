@@ -561,16 +561,23 @@ reef_status reef_module_get_kernel(reef_module_t mod, const char* name, reef_ker
     *k = h;
     return REEF_SUCC;
 }
-reef_status reef_kernel_plan(const char* name, uint32_t dims[6], uint32_t* dyn_smem, int* num_args) {
-    KernelSpec s;
-    int rc = plan_kernel(name, &s);
-    if (rc != REEF_SUCC) return rc;
+static void geometry_of(const KernelSpec& s, uint32_t dims[6], uint32_t* dyn_smem, int* num_args) {
     for (int i = 0; i < 3; i++) {
         dims[i] = s.grid[i];
         dims[3 + i] = s.block[i];
     }
     if (dyn_smem) *dyn_smem = s.dyn_smem;
     if (num_args) *num_args = s.nargs;
+}
+reef_status reef_kernel_plan(const char* name, uint32_t dims[6], uint32_t* dyn_smem, int* num_args) {
+    KernelSpec s;
+    int rc = plan_kernel(name, &s);
+    if (rc == REEF_SUCC) geometry_of(s, dims, dyn_smem, num_args);
+    return rc;
+}
+reef_status reef_kernel_geometry(reef_kernel_t k, uint32_t dims[6], uint32_t* dyn_smem, int* num_args) {
+    if (!k || !dims) return REEF_FAIL;
+    geometry_of(k->spec, dims, dyn_smem, num_args);
     return REEF_SUCC;
 }
 reef_status reef_kernel_cost(const char* name, double* flops, double* bytes, int* tensor_core) {

@@ -62,7 +62,7 @@ Status ExecutorBase::resolve_kernels(const Model& m, GPUModule_t mod, std::vecto
         for (int earlier = 0; earlier < 2 && !(dims_fit && smem_fits); earlier++) {
             const std::string name = ki.name + (earlier ? "_pv1" : "");
             int rc = reef_module_get_kernel(mod, name.c_str(), &k);
-            if (rc == REEF_SUCC) rc = reef_kernel_plan(name.c_str(), dims, &smem, &nargs);
+            if (rc == REEF_SUCC) rc = reef_kernel_geometry(k, dims, &smem, &nargs);
             if (rc != REEF_SUCC) {
                 *err = reef_last_error();
                 return (Status)rc;
