@@ -74,8 +74,8 @@ __device__ __forceinline__ int taps_inside(int first, int n, int taps) {
 
 // 16 pixels x 8 NT channels per warp.  FAST: channels-last input whose 16-byte chunks lie in one tap each; else (planar
 // input, odd channel counts) element by element.
-template <int NT, int STAGES, bool FAST>
-__device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, float* ring, const int* flag) {
+template <int NT, int STAGES, bool FAST, class Enter>
+__device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, float* ring, const int* flag, Enter enter) {
     constexpr int TP = CTP, TC = 8 * NT, CROW = CBK, STAGE = (TP + TC) * CROW;
     static_assert(8 * STAGES * STAGE * 4 <= kConvSimtRing && 8 * TP * (TC + 4) * 4 <= kConvSimtRing, "ring too small");
     const ConvP& p = t.p.conv;
@@ -179,6 +179,7 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
         for (int e = 0; e < 4; e++) sum[j][e] = big[j][e] = small[j][e] = 0.f;
     const int g = lane >> 2, c = lane & 3;
     bool stopped = false;
+    if (!enter()) return false;
     __syncthreads();                           // a persistent caller's previous tile is out of the ring
     int loaded = group;                        // the slice that `load` fetches next
 #pragma unroll
@@ -324,12 +325,13 @@ __device__ __forceinline__ bool conv_simt_tile_body(const KTask& t, int vb, floa
     return true;
 }
 
-__device__ __forceinline__ bool body_conv_simt(const KTask& t, int vb, unsigned char* smem_raw, const int* flag) {
+template <class Enter>
+__device__ __forceinline__ bool body_conv_simt(const KTask& t, int vb, unsigned char* smem_raw, const int* flag, Enter enter) {
     float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
     const ConvP& p = t.p.conv;
-    if (!conv_simt_fast(p)) return conv_simt_tile_body<4, 3, false>(t, vb, ring, flag);
-    if (p.tile_c == 32) return conv_simt_tile_body<4, 4, true>(t, vb, ring, flag);
-    return conv_simt_tile_body<2, 4, true>(t, vb, ring, flag);
+    if (!conv_simt_fast(p)) return conv_simt_tile_body<4, 3, false>(t, vb, ring, flag, enter);
+    if (p.tile_c == 32) return conv_simt_tile_body<4, 4, true>(t, vb, ring, flag, enter);
+    return conv_simt_tile_body<2, 4, true>(t, vb, ring, flag, enter);
 }
 
 }  // namespace reef

@@ -570,15 +570,16 @@ int plan_kernel(const char* name, KernelSpec* s) {
 // ------------------------------------------------------------------------------------------
 // device flavours
 // ------------------------------------------------------------------------------------------
-template <int F>
-__device__ __forceinline__ bool run_body(const KTask& t, int vb, unsigned char* smem, const int* flag) {
+template <int F, class Enter>
+__device__ __forceinline__ bool run_body(const KTask& t, int vb, unsigned char* smem, const int* flag, Enter enter) {
+    if (F == F_CONV_SIMT) return body_conv_simt(t, vb, smem, flag, enter);
+    if (!enter()) return false;
     if (F == F_MOCK_ADD) return body_mock<false>(t, vb, smem, flag);
     if (F == F_MOCK_MUL) return body_mock<true>(t, vb, smem, flag);
     if (F == F_FUSED_ADD_NCHW) return body_fused_add_nchw(t, vb, smem, flag);
     if (F == F_NCHW_TO_NHWC4) return body_nchw_to_nhwc4(t, vb, smem, flag);
     if (F == F_IM2COL_NCHW) return body_im2col_nchw(t, vb, smem, flag);
     if (F == F_BIAS_RELU) return body_bias_relu(t, vb, smem, flag);
-    if (F == F_CONV_SIMT) return body_conv_simt(t, vb, smem, flag);
     if (F == F_MAX_POOL) return body_pool<true>(t, vb, smem, flag);
     if (F == F_AVG_POOL) return body_pool<false>(t, vb, smem, flag);
     if (F == F_GLOBAL_AVG_POOL) return body_gap(t, vb, smem, flag);
@@ -595,38 +596,28 @@ __device__ __forceinline__ bool run_body(const KTask& t, int vb, unsigned char* 
 // (not inlined: the dispatcher calls it for either kind, and two copies of every body spilled)
 __device__ __noinline__ bool run_any(const KTask& t, int vb, unsigned char* smem, const int* flag) {
     switch (t.family) {
-        case F_MOCK_ADD: return run_body<F_MOCK_ADD>(t, vb, smem, flag);
-        case F_MOCK_MUL: return run_body<F_MOCK_MUL>(t, vb, smem, flag);
-        case F_FUSED_ADD_NCHW: return run_body<F_FUSED_ADD_NCHW>(t, vb, smem, flag);
-        case F_NCHW_TO_NHWC4: return run_body<F_NCHW_TO_NHWC4>(t, vb, smem, flag);
-        case F_IM2COL_NCHW: return run_body<F_IM2COL_NCHW>(t, vb, smem, flag);
-        case F_BIAS_RELU: return run_body<F_BIAS_RELU>(t, vb, smem, flag);
-        case F_CONV_SIMT: return run_body<F_CONV_SIMT>(t, vb, smem, flag);
-        case F_MAX_POOL: return run_body<F_MAX_POOL>(t, vb, smem, flag);
-        case F_AVG_POOL: return run_body<F_AVG_POOL>(t, vb, smem, flag);
-        case F_GLOBAL_AVG_POOL: return run_body<F_GLOBAL_AVG_POOL>(t, vb, smem, flag);
-        case F_COPY: return run_body<F_COPY>(t, vb, smem, flag);
-        case F_DENSE: return run_body<F_DENSE>(t, vb, smem, flag);
-        case F_SOFTMAX: return run_body<F_SOFTMAX>(t, vb, smem, flag);
-        case F_EMBEDDING: return run_body<F_EMBEDDING>(t, vb, smem, flag);
-        case F_LAYERNORM: return run_body<F_LAYERNORM>(t, vb, smem, flag);
+        case F_MOCK_ADD: return run_body<F_MOCK_ADD>(t, vb, smem, flag, EnterAlways());
+        case F_MOCK_MUL: return run_body<F_MOCK_MUL>(t, vb, smem, flag, EnterAlways());
+        case F_FUSED_ADD_NCHW: return run_body<F_FUSED_ADD_NCHW>(t, vb, smem, flag, EnterAlways());
+        case F_NCHW_TO_NHWC4: return run_body<F_NCHW_TO_NHWC4>(t, vb, smem, flag, EnterAlways());
+        case F_IM2COL_NCHW: return run_body<F_IM2COL_NCHW>(t, vb, smem, flag, EnterAlways());
+        case F_BIAS_RELU: return run_body<F_BIAS_RELU>(t, vb, smem, flag, EnterAlways());
+        case F_CONV_SIMT: return run_body<F_CONV_SIMT>(t, vb, smem, flag, EnterAlways());
+        case F_MAX_POOL: return run_body<F_MAX_POOL>(t, vb, smem, flag, EnterAlways());
+        case F_AVG_POOL: return run_body<F_AVG_POOL>(t, vb, smem, flag, EnterAlways());
+        case F_GLOBAL_AVG_POOL: return run_body<F_GLOBAL_AVG_POOL>(t, vb, smem, flag, EnterAlways());
+        case F_COPY: return run_body<F_COPY>(t, vb, smem, flag, EnterAlways());
+        case F_DENSE: return run_body<F_DENSE>(t, vb, smem, flag, EnterAlways());
+        case F_SOFTMAX: return run_body<F_SOFTMAX>(t, vb, smem, flag, EnterAlways());
+        case F_EMBEDDING: return run_body<F_EMBEDDING>(t, vb, smem, flag, EnterAlways());
+        case F_LAYERNORM: return run_body<F_LAYERNORM>(t, vb, smem, flag, EnterAlways());
         case F_ATTENTION:           // (the staged form for either: the dispatcher has 128 registers; same results bit for bit)
-        case F_ATTENTION_STAGED: return run_body<F_ATTENTION_STAGED>(t, vb, smem, flag);
+        case F_ATTENTION_STAGED: return run_body<F_ATTENTION_STAGED>(t, vb, smem, flag, EnterAlways());
         default: return true;
     }
 }
 
 extern __shared__ __align__(16) unsigned char reef_dyn_smem[];
-
-// Programmatic dependent launch: this kernel waits for its predecessor's results before touching memory (a
-// no-op for an ordinary launch) and only then lets its successor start its prologue.  Releasing the successor
-// before the wait would let a chain of kernels run ahead without bound: every grid's blocks would become
-// resident, release the next grid and park at their wait, until the SMs are full of parked blocks and a
-// best-effort kernel on another stream finds no room.  In this order at most two grids of a chain are resident.
-__device__ __forceinline__ void pdl_prologue() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // Device-side preemption stamps (optional, measurement only): when the host has armed the two words with
 // reef_preempt_stamps_arm, the first best-effort block that sees the preempt flag up records %globaltimer into word
@@ -650,8 +641,7 @@ template <int F>
 __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_plain(const __grid_constant__ KTask t) {
     if (F == F_LAYERNORM) prefetch_layernorm(t);
     if (F == F_DENSE) prefetch_dense(t, blockIdx.x);
-    pdl_prologue();
-    run_body<F>(t, blockIdx.x, reef_dyn_smem, nullptr);
+    run_body<F>(t, blockIdx.x, reef_dyn_smem, nullptr, EnterPlain());
 }
 
 // Best-effort flavour (reference wrapper: script/best_effort_kernel.py:22-33): leave at once when
@@ -662,18 +652,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F)) k_be(const __grid_con
                                                  int* __restrict__ task_slot) {
     if (F == F_LAYERNORM) prefetch_layernorm(t);
     if (F == F_DENSE) prefetch_dense(t, blockIdx.x);
-    // ONE thread reads the flag and the block takes one decision: were every thread to read it for itself, a flag
-    // that goes up between the reads of two warps would let part of a block leave and the rest run the body with
-    // threads missing (wrong partial sums counted as a complete block, barriers short of arrivals).  It is read ahead of
-    // the wait for the previous kernel, so that its trip to L2 (0.4 us) is not on the way to the body: a flag that goes up
-    // during that wait is seen by the body's polls or by the next kernel of the stream, which starts behind this wait.
-    const int up = threadIdx.x == 0 ? ld_flag(flag) : 0;
-    pdl_prologue();
-    if (__syncthreads_or(up)) {
-        if (threadIdx.x == 0) preempt_stamp_leave();
-        return;
-    }
-    const bool done = run_body<F>(t, blockIdx.x, reef_dyn_smem, flag);
+    const EnterBestEffort enter = {threadIdx.x == 0 ? ld_flag(flag) : 0};
+    const bool done = run_body<F>(t, blockIdx.x, reef_dyn_smem, flag, enter);
     // a body may stop at a loop head in some of its warps only (the GEMV polls per warp): the block counts as
     // complete only when every thread ran to the end
     const int stopped = __syncthreads_or(done ? 0 : 1);
