@@ -171,7 +171,7 @@ public:
     Status launch_pad_segment(int seg, GPUStream_t stream);
     // Best-effort segments: the same cut into runs of kBeSegment kernels for the best-effort flavour (every kernel still
     // polls the flag and counts into its slot).  A task at full speed is fed one graph launch and one event per run.
-    static const int kBeSegment = 24;
+    static const int kBeSegment = 16;
     Status build_be_segments(GPUStream_t cap);
     Status launch_preempt_segment(int kernel_offset, GPUStream_t stream, bool single, int* last);
     bool has_tensor_core_kernels() const { return has_tc; }

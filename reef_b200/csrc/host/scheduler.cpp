@@ -1244,11 +1244,10 @@ void REEFScheduler::execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr
     // see the flag and leave before the stream is idle, about 3 us per kernel and stream (4 clients, ResNet-152: a
     // preemption drains in 17 us with two kernels in flight, 42 us with two segments of four, 67 us with two of eight).
     // When none is to be expected nobody waits for a drain, and an entry is a whole segment: one graph launch and one
-    // event for 24 kernels keep the stream busy where the host could not, and branches run side by side inside it
-    // (DenseNet-201, one client: 2.5 ms a pass kernel by kernel; segments of 16 / 24 / 32 kernels 1.017 / 0.963 / 0.969 ms,
-    // ResNet-152 0.672 / 0.660 / 0.651: a boundary costs 3-5 us, and past 24 kernels little of that is left).  Longer ones
-    // are a burden on a real-time request that comes out of a long pause and meets them whole (ResNet-18 every 50 ms beside
-    // either client: 121-124 / 122-125 / 122-126 us).  A window of one, or wait_sync, asks for quick drains: single kernels.
+    // event for sixteen kernels keep the stream busy where the host could not, and branches run side by side inside it
+    // (DenseNet-201, one client: 2.5 ms a pass kernel by kernel; segments of 8 / 16 / 32 kernels 1.29 / 1.18 / 1.13 ms).
+    // Longer ones are a burden on a real-time request that comes out of a long pause (ResNet-18 every 50 ms beside that
+    // client: 153 / 156 / 169 us).  A window of one, or wait_sync, asks for quick drains: single kernels.
     const bool shallow = wait_sync || be_stream_device_queue_cap < 2 || rt_expected();
     while (task->launch_offset < num_kernels && (int)tqueue->inflight.size() < be_stream_device_queue_cap) {
         int last = task->launch_offset;
