@@ -23,7 +23,7 @@
 // a slice is free as long as both operands agree), so an operand row is read with one 128-bit load.
 // What is left: a block alone on its SM keeps the tensor cores busy a quarter of the time, two of them half of it, and issue
 // 82 % of what the schedulers can; so every instruction of a slice counts (ResNet-50 at 193x193: addresses per tap instead of
-// per slice, and no clearing of accumulators, 585 -> 564 us a replay; ResNet-18 at 64x64 168 -> 153).
+// per slice, and no clearing of accumulators, 585 -> 564 us a replay; with the shorter split 549, with the set-up ahead of the wait 521; ResNet-18 at 64x64 168 -> 140).
 // Measured, 3x3 256 -> 256 at 13x13: 133 us by fp32 instructions, 13.9, now 12.4; 3x3 512 -> 512 at 7x7: 261, 19.5, 16.7.
 #pragma once
 #include <type_traits>
@@ -41,6 +41,7 @@ constexpr int kConvSimtSmem = kConvSimtRing + 128;
 // Channels of the warp tile and K groups of a shape: the least time by what was measured.  One block on an SM takes 0.57 us
 // per slice of eight 16x32 tiles and 0.41 us of 16x16 (splitting operands into bf16 is most of it), blocks that share an SM
 // overlap by a sixth; launch, prologue and epilogue take 3.5 us, every further block of an SM half a microsecond.
+// (A slice takes 0.47 and 0.35 us by now; the ratio, which decides, is what it was.)
 struct ConvSimtTile {
     int tc, kg;
 };

@@ -23,7 +23,8 @@
 // load stream that takes about 57 bytes a clock into an SM.  Reading the partials out of the peers' staged tiles between
 // two cluster barriers took 1.2 us for 28 pixels over eight ranks where the stores take 0.4, 1.7 against 0.8 for 64
 // pixels; together with multiplications issued at the tensor core's pace: 1x1 1024 -> 256 at 14x14 4.41 -> 3.09 us, 3x3
-// 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us.
+// 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us (573, 826
+// and 282 with the steps that are told beside the code below).
 // Every mbarrier wait is bounded: on expiry the kernel records an error word,
 // skips further waits, still joins every cluster barrier, frees its TMEM and returns.
 #pragma once
