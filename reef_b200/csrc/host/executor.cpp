@@ -947,12 +947,6 @@ Status HybridExecutor::execute_dispatch(GPUStream_t stream) {
     return Status::Succ;
 }
 
-static void busy_wait_us(int us) {
-    auto t0 = std::chrono::steady_clock::now();
-    while (std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count() < us) {
-    }
-}
-
 Status HybridExecutor::execute_preempt_resume(int delay_us, int* restarts, int* first_incomplete, int* first_count) {
     GPUStream_t flag_stream;
     GPU_RETURN_STATUS(reef_stream_create(&flag_stream, 1));
@@ -966,12 +960,26 @@ Status HybridExecutor::execute_preempt_resume(int delay_us, int* restarts, int* 
     reset_task_slots(s, 0);
     Status st = Status::Succ;
     while (from < n) {
-        for (int i = from; i < n && st == Status::Succ; i++) st = launch_preempt_kernel(i, s);
-        if (st != Status::Succ) break;
+        // The flag goes up `delay` after the first launch, while the others are still being issued where that takes longer:
+        // a host that issues no faster than the kernels run would else raise it behind the last one.
         const bool preempt = rounds < 8;
+        const auto delay = std::chrono::microseconds(delay_us << std::min(rounds, 6));
+        const auto t0 = std::chrono::steady_clock::now();
+        bool raised = false;
+        for (int i = from; i < n && st == Status::Succ; i++) {
+            st = launch_preempt_kernel(i, s);
+            if (preempt && !raised && std::chrono::steady_clock::now() - t0 >= delay) {
+                reef_write32_async(flag_stream, preempt_flag, 1);
+                raised = true;
+            }
+        }
+        if (st != Status::Succ) break;
         if (preempt) {
-            busy_wait_us(delay_us << std::min(rounds, 6));
-            reef_write32_async(flag_stream, preempt_flag, 1);
+            if (!raised) {
+                while (std::chrono::steady_clock::now() - t0 < delay) {
+                }
+                reef_write32_async(flag_stream, preempt_flag, 1);
+            }
             reef_stream_sync(flag_stream);
         }
         if (reef_preempt_wait(s, 5000000) != REEF_SUCC) { st = Status::Timeout; break; }
