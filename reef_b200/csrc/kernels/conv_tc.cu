@@ -342,6 +342,9 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
     P->n_tiles = pl.n_tiles;
     P->tile_begin = 0;
     P->pdl = 1;
+#ifdef REEF_DEBUG_AIDS
+    P->withheld_rank = P->withheld_load = -1;
+#endif
     return REEF_SUCC;
 }
 

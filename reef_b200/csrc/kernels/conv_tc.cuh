@@ -25,8 +25,9 @@
 // pixels; together with multiplications issued at the tensor core's pace: 1x1 1024 -> 256 at 14x14 4.41 -> 3.09 us, 3x3
 // 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us (573, 826
 // and 282 with the steps that are told beside the code below).
-// Every mbarrier wait is bounded: on expiry the kernel records an error word,
-// skips further waits, still joins every cluster barrier, frees its TMEM and returns.
+// Every mbarrier wait is bounded.  One that expires sets a word of the CTA that ends its other waits; the CTA then sends what it has,
+// stays until nothing can be stored into its shared memory any more (peers' shares, its own loads; bounded again), records the
+// error word, frees its TMEM and returns.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -87,8 +88,11 @@ __device__ __forceinline__ float4 tc_preact(float4 o, float4 b2, bool rnd) {
 __device__ __forceinline__ void tc_stamp(const TcParams& P, int slot) {
     if (P.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0) P.trace[slot] = clock64();
 }
+// the load of one K block of one rank that is announced and never made: what waits for it gives up
+__device__ __forceinline__ bool tc_withheld(const TcParams& P, int i) { return blockIdx.y == 0 && P.withheld_rank == (int)blockIdx.x && P.withheld_load == i; }
 #else
 __device__ __forceinline__ void tc_stamp(const TcParams&, int) {}
+__device__ __forceinline__ bool tc_withheld(const TcParams&, int) { return false; }
 #endif
 
 __device__ __forceinline__ float tc_round1(float v) {
@@ -259,6 +263,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + P.region_bytes + 16 * TC_MAX_STAGES + 16);
     volatile uint32_t* s_flags = s_tmem + 1;    // [0] abort (preempt flag seen by this CTA), [1] K blocks whose loads were issued when
                                                 //  the producer stopped, [2..9] what the ranks of the cluster saw (best-effort flavour)
+    volatile uint32_t* gave_up = s_flags + 10;  // a wait of this CTA expired
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be warp-uniform)
@@ -295,6 +300,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         mbar_init(bar_recv, 1);
         s_flags[0] = (uint32_t)(flag0 != 0);
         s_flags[1] = 0;
+        *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (recv_bytes != 0) mbar_expect_tx(bar_recv, recv_bytes);
@@ -339,7 +345,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 const int kb = kb_begin + lane, t = P.cblocks == 1 ? kb : (int)__umulhi((unsigned)kb, P.cb_magic);
                 bc0 = (kb - t * P.cblocks) * TC_BK;
                 mbar_expect_tx(bar_full + 8 * lane, tx);
-                tma_load_3d(base + lane * stage_bytes, &P.tm_w, bar_full + 8 * lane, bc0, t, m0);
+                if (!tc_withheld(P, lane)) tma_load_3d(base + lane * stage_bytes, &P.tm_w, bar_full + 8 * lane, bc0, t, m0);
                 if (P.spatial) {
                     bmap = &P.tm_x[P.tap_map[t]];
                     bc1 = tile_x * P.xw + P.tap_qx[t];
@@ -360,7 +366,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // in this order at most two grids of a chain are resident and the other SM slots stay free for
             // best-effort kernels.  One thread per CTA executing the instruction counts for the CTA.
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            if (lane < first && !abort0) {
+            if (lane < first && !abort0 && !tc_withheld(P, lane)) {
                 const uint32_t bdst = base + lane * stage_bytes + TC_A_BYTES;
                 if (P.spatial) tma_load_3d(bdst, bmap, bar_full + 8 * lane, bc0, bc1, bc2);
                 else tma_load_2d(bdst, bmap, bar_full + 8 * lane, bc0, bc1);
@@ -422,7 +428,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                     c2 = tile_y * P.rows + P.tap_qy[t];
                 }
                 if (++cb == P.cblocks) { cb = 0; tap++; }
-                ok = mbar_wait_warp(bar_empty + 8 * s, par);
+                ok = mbar_wait_warp(bar_empty + 8 * s, par, gave_up);
                 if (!ok) break;
                 if (BE && ((i - first) & 3) == 3) {   // loop-head poll of the preempt flag
                     if (__any_sync(0xffffffffu, f != 0)) { stop = true; break; }
@@ -430,18 +436,21 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 }
                 const uint32_t dst = base + s * stage_bytes, bar = bar_full + 8 * s;
                 mbar_expect_tx_if(lead, bar, tx);
-                tma_load_3d_if(lead, dst, &P.tm_w, bar, c0, t, m0);
-                if (P.spatial) tma_load_3d_if(lead, dst + TC_A_BYTES, &P.tm_x[map], bar, c0, c1, c2);
-                else tma_load_2d_if(lead, dst + TC_A_BYTES, &P.tm_x[0], bar, c0, c1);
+                if (!tc_withheld(P, i)) {
+                    tma_load_3d_if(lead, dst, &P.tm_w, bar, c0, t, m0);
+                    if (P.spatial) tma_load_3d_if(lead, dst + TC_A_BYTES, &P.tm_x[map], bar, c0, c1, c2);
+                    else tma_load_2d_if(lead, dst + TC_A_BYTES, &P.tm_x[0], bar, c0, c1);
+                }
                 issued++;
                 if (++s == NS) { s = 0; par ^= 1u; }
             }
             if (BE && !stop) stop = __any_sync(0xffffffffu, f != 0);
+            if (lane == 0) s_flags[1] = (uint32_t)issued;     // first how far the loads got, then the request to stop
             if (BE && stop && lane == 0) {
-                s_flags[1] = (uint32_t)issued;     // first how far the loads got, then the request to stop
                 __threadfence_block();
                 s_flags[0] = 1;
             }
+            __syncwarp();
             // (a wait that expired here leaves the multiplications, and with them the accumulator's barrier, incomplete)
         } else if (warp == 1) {
             // ---------------- MMA issuer ----------------
@@ -459,7 +468,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             for (int i = 0; i < nkb; i++) {
                 if (!ready) {
                     if (BE) {
-                        const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0]);
+                        const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0], gave_up);
                         if (w == 2) {
                             // The producer stopped.  Loads it had issued may still be in flight: they must have landed
                             // before this CTA leaves or reuses its shared memory, so their barriers are awaited (bounded)
@@ -467,7 +476,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                             __threadfence_block();
                             const int issued = __shfl_sync(0xffffffffu, (int)s_flags[1], 0);
                             for (; i < issued && ok; i++) {
-                                ok = mbar_wait_warp(bar_full + 8 * s, par);
+                                ok = mbar_wait_warp(bar_full + 8 * s, par, gave_up);
                                 if (++s == NS) { s = 0; par ^= 1u; }
                             }
                             halted = true;
@@ -475,7 +484,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                         }
                         ok = w == 0;
                     } else {
-                        ok = mbar_wait_warp(bar_full + 8 * s, par);
+                        ok = mbar_wait_warp(bar_full + 8 * s, par, gave_up);
                     }
                     if (!ok) break;
                 }
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         }
 
         // ---------------- exchange and epilogue: all eight warps ----------------
-        bool ok = mbar_wait_warp(bar_acc, 0);
+        bool ok = mbar_wait_warp(bar_acc, 0, gave_up);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // best-effort flavour: behind this barrier the producer and the MMA warp are past their loops, the flag word is final
         if (BE) __syncthreads();
@@ -559,8 +568,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 st_async_u32(peer + (smem_u32((const void*)&s_flags[2]) - base) + (uint32_t)split * 4u, peer + (bar_recv - base), abort_all || !ok ? 1u : 0u);
             }
             __syncwarp();
-            // (A rank that gave up sends what it has: the receivers count bytes, and nobody stores the result of a failed or
-            // preempted launch.)
+            // (A rank that gave up sends what it has: the receivers count bytes.  The result of a preempted launch is stored by
+            // none of them, that of a failed one means nothing: the error word says so.)
             if (quad * 32 < co_lim) {
 #pragma unroll 1
                 for (int t0 = 0; t0 < turns;) {
@@ -588,7 +597,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 tmem_free(tmem, (uint32_t)P.tmem_cols);
             }
             if (tid == 0) tc_stamp(P, 7);   // shares sent
-            if (recv_bytes != 0 && !mbar_wait_cluster_warp(bar_recv, 0)) ok = false;
+            // A rank whose shares are there leaves by itself: nothing more will be stored into its shared memory.  One that gave
+            // up stays until every warp of the cluster is past its stores, each of them after bounded waits, and these
+            // have landed.  (Only then does anybody wait for this barrier; to arrive costs nothing that could be measured.)
+            cluster_arrive_relaxed();
+            if (recv_bytes != 0 && !mbar_wait_cluster_warp(bar_recv, 0, gave_up)) {
+                ok = false;
+                cluster_wait();
+                mbar_wait_cluster_warp(bar_recv, 0, nullptr);
+            }
             if (BE) {
                 // every rank has the words of all the others: all take the same exit
                 if (__any_sync(0xffffffffu, lane < S && lane != split && s_flags[2 + lane] != 0)) abort_all = true;
@@ -619,6 +636,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         if (warp == awarp && !(S > 1 && w.count == 0)) {
             asm volatile("bar.sync 1, 256;" ::: "memory");
             tmem_free(tmem, (uint32_t)P.tmem_cols);
+        }
+        // a CTA that gave up leaves no load behind that could still write into its shared memory (one limit for all of them)
+        if (!ok && warp == 0) {
+            const int issued = (int)s_flags[1];
+            bool landed = true;
+            for (int i = max(0, issued - NS); i < issued && landed; i++) landed = mbar_wait_warp(bar_full + 8 * (i % NS), (uint32_t)(i / NS) & 1u, nullptr);
         }
     }
 

@@ -31,30 +31,15 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Bounded wait: returns false when the phase did not complete within the iteration limit.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    unsigned long long t0 = 0;
-    for (int i = 0; i < (1 << 26); i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((i & 255) == 255) {   // give up after one second of wall time
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > 1000000000ull) return false;
-        }
-    }
-    return false;
+// Every wait is bounded: it gives up after this time (one second; the test of what follows an expired wait takes less).
+#ifndef REEF_WAIT_LIMIT_NS
+#define REEF_WAIT_LIMIT_NS 1000000000
+#endif
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
-// The waits of a whole warp: every lane polls, the warp leaves together (the votes keep its control flow, and with it the
-// addresses and descriptors of what it issues next, warp-uniform).
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -66,34 +51,67 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+// The same for data that the other CTAs of the cluster have stored (st_async): acquire at cluster scope.
+__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// The wait of one thread: false when it gave up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     unsigned long long t0 = 0;
     for (int i = 0; i < (1 << 26); i++) {
-        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
-        if ((i & 255) == 255) {   // give up after one second of wall time
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (mbar_try(bar, parity)) return true;
+        if ((i & 255) == 255) {
+            const unsigned long long t = global_ns();
             if (t0 == 0) t0 = t;
-            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return false;
+            else if (t - t0 > REEF_WAIT_LIMIT_NS) return false;
         }
     }
     return false;
 }
-// The wait of the best-effort flavour's MMA warp also gives up when `abort_word` (shared memory, written by the TMA producer
-// of the same CTA when it saw the preempt flag) becomes non-zero.  0 = phase complete, 1 = wait expired, 2 = abort requested.
-__device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word) {
+// The waits of a whole warp: every lane polls, the warp leaves together (the votes keep its control flow, and with it the
+// addresses and descriptors of what it issues next, warp-uniform).  `gave_up` (shared memory, or null) is what the waits of a CTA
+// share: one that expires sets it, and all others end with it instead of sitting out a limit each.
+__device__ __forceinline__ bool wait_is_over(uint32_t tries, unsigned long long& t0, volatile uint32_t* gave_up) {
+    if (gave_up != nullptr && __any_sync(0xffffffffu, *gave_up != 0)) return true;
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    if (__all_sync(0xffffffffu, t - t0 > REEF_WAIT_LIMIT_NS) || tries >= 1u << 26) {
+        if (gave_up != nullptr) *gave_up = 1;
+        return true;
+    }
+    return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
     unsigned long long t0 = 0;
-    for (int i = 0; i < (1 << 26); i++) {
+    for (uint32_t i = 0;; i++) {
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return false;
+    }
+}
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
+    unsigned long long t0 = 0;
+    for (uint32_t i = 0;; i++) {
+        if (__all_sync(0xffffffffu, mbar_try_cluster(bar, parity))) return true;
+        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return false;
+    }
+}
+// The wait of the best-effort flavour's MMA warp also ends when `abort_word` (shared memory, written by the TMA producer
+// of the same CTA when it saw the preempt flag) becomes non-zero.  0 = phase complete, 1 = gave up, 2 = abort requested.
+__device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word, volatile uint32_t* gave_up) {
+    unsigned long long t0 = 0;
+    for (uint32_t i = 0;; i++) {
         if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return 0;
         if (__any_sync(0xffffffffu, *abort_word != 0)) return 2;
-        if ((i & 255) == 255) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return 1;
-        }
+        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return 1;
     }
-    return 1;
 }
 // One look, without the suspension that try_wait may take: for a look ahead at a barrier that may be far from complete.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -106,28 +124,6 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity)
         : "memory");
     return done != 0;
-}
-// The bounded wait of a whole warp for data that the other CTAs of the cluster have stored (st_async): acquire at cluster scope.
-__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity) {
-    unsigned long long t0 = 0;
-    for (int i = 0; i < (1 << 26); i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (__all_sync(0xffffffffu, done != 0)) return true;
-        if ((i & 255) == 255) {   // give up after one second of wall time
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (__all_sync(0xffffffffu, t - t0 > 1000000000ull)) return false;
-        }
-    }
-    return false;
 }
 // A model constant, requested where this stands: a plain load may be moved down to its first use, behind the waits.
 __device__ __forceinline__ float ld_param(const float* p) {
