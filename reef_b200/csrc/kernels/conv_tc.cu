@@ -343,7 +343,7 @@ int tc_build_params(const ConvP& p, const TcPlan& pl, void* const* a, TcParams* 
     P->tile_begin = 0;
     P->pdl = 1;
 #ifdef REEF_DEBUG_AIDS
-    P->withheld_rank = P->withheld_load = -1;
+    P->withheld_rank = P->withheld_load = -1;   // (no delay either)
 #endif
     return REEF_SUCC;
 }

@@ -25,9 +25,9 @@
 // pixels; together with multiplications issued at the tensor core's pace: 1x1 1024 -> 256 at 14x14 4.41 -> 3.09 us, 3x3
 // 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us (573, 826
 // and 282 with the steps that are told beside the code below).
-// Every mbarrier wait is bounded.  One that expires sets a word of the CTA that ends its other waits; the CTA then sends what it has,
-// stays until nothing can be stored into its shared memory any more (peers' shares, its own loads; bounded again), records the
-// error word, frees its TMEM and returns.
+// Every mbarrier wait is bounded.  A warp that gave up skips its further waits and sends what it has; the CTA stays until nothing can be
+// stored into its shared memory any more (peers' shares, its own loads; bounded again), records the error word, frees its TMEM
+// and returns.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -90,9 +90,15 @@ __device__ __forceinline__ void tc_stamp(const TcParams& P, int slot) {
 }
 // the load of one K block of one rank that is announced and never made: what waits for it gives up
 __device__ __forceinline__ bool tc_withheld(const TcParams& P, int i) { return blockIdx.y == 0 && P.withheld_rank == (int)blockIdx.x && P.withheld_load == i; }
+// ... and sends its shares this much later
+__device__ __forceinline__ void tc_withheld_delay(const TcParams& P) {
+    if (P.withheld_delay_ns > 0 && blockIdx.y == 0 && P.withheld_rank == (int)blockIdx.x)
+        for (const unsigned long long t = global_ns(); global_ns() - t < (unsigned long long)P.withheld_delay_ns;) __nanosleep(1000);
+}
 #else
 __device__ __forceinline__ void tc_stamp(const TcParams&, int) {}
 __device__ __forceinline__ bool tc_withheld(const TcParams&, int) { return false; }
+__device__ __forceinline__ void tc_withheld_delay(const TcParams&) {}
 #endif
 
 __device__ __forceinline__ float tc_round1(float v) {
@@ -263,7 +269,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + P.region_bytes + 16 * TC_MAX_STAGES + 16);
     volatile uint32_t* s_flags = s_tmem + 1;    // [0] abort (preempt flag seen by this CTA), [1] K blocks whose loads were issued when
                                                 //  the producer stopped, [2..9] what the ranks of the cluster saw (best-effort flavour)
-    volatile uint32_t* gave_up = s_flags + 10;  // a wait of this CTA expired
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (known to be warp-uniform)
@@ -300,7 +305,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         mbar_init(bar_recv, 1);
         s_flags[0] = (uint32_t)(flag0 != 0);
         s_flags[1] = 0;
-        *gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (recv_bytes != 0) mbar_expect_tx(bar_recv, recv_bytes);
@@ -323,6 +327,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
     // "my receive area may be written": where it is apart from the stage ring, from here on (the barrier's latency then hides
     // behind the main loop); where it lies over the ring, behind the accumulator
     if (S > 1 && !P.recv_late) cluster_arrive();
+
+    bool ok = true;                             // no wait of this warp has expired; one that has ends the others
 
     // best-effort flavour: what this CTA saw at entry.  Nothing is loaded then; the cluster agrees at its first barrier.
     const bool abort0 = BE && s_flags[0] != 0;
@@ -400,7 +406,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // ---------------- TMA producer, part 2: refill stages as the MMAs release them ----------------
             // (stage index and phase parity are carried along: a division by the runtime ring depth per K block
             // is dozens of cycles on this critical path)
-            bool ok = true;
             int s = first == NS ? 0 : first;      // first < NS only when nkb < NS, and then this loop does not run
             uint32_t par = 0;                      // parity of the "empty" phase awaited: ((i / NS) - 1) & 1
             int issued = abort0 ? 0 : first;       // K blocks whose loads are out
@@ -428,7 +433,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                     c2 = tile_y * P.rows + P.tap_qy[t];
                 }
                 if (++cb == P.cblocks) { cb = 0; tap++; }
-                ok = mbar_wait_warp(bar_empty + 8 * s, par, gave_up);
+                ok = mbar_wait_warp(bar_empty + 8 * s, par);
                 if (!ok) break;
                 if (BE && ((i - first) & 3) == 3) {   // loop-head poll of the preempt flag
                     if (__any_sync(0xffffffffu, f != 0)) { stop = true; break; }
@@ -456,7 +461,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // ---------------- MMA issuer ----------------
             // The next stage's barrier is looked at before this stage's multiplications are issued, and those are predicated
             // on the issuing lane instead of branched around: the loop then runs at the tensor core's pace (umma_tf32_if).
-            bool ok = true, halted = false;
+            bool halted = false;
             const uint32_t idesc = umma_idesc_tf32(P.n_mma), lead = elect_one() ? 1u : 0u;
 #ifdef REEF_DEBUG_AIDS
             const bool tr = lane == 0 && P.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
@@ -468,7 +473,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             for (int i = 0; i < nkb; i++) {
                 if (!ready) {
                     if (BE) {
-                        const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0], gave_up);
+                        const int w = mbar_wait_abortable_warp(bar_full + 8 * s, par, &s_flags[0]);
                         if (w == 2) {
                             // The producer stopped.  Loads it had issued may still be in flight: they must have landed
                             // before this CTA leaves or reuses its shared memory, so their barriers are awaited (bounded)
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                             __threadfence_block();
                             const int issued = __shfl_sync(0xffffffffu, (int)s_flags[1], 0);
                             for (; i < issued && ok; i++) {
-                                ok = mbar_wait_warp(bar_full + 8 * s, par, gave_up);
+                                ok = mbar_wait_warp(bar_full + 8 * s, par);
                                 if (++s == NS) { s = 0; par ^= 1u; }
                             }
                             halted = true;
@@ -484,7 +489,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                         }
                         ok = w == 0;
                     } else {
-                        ok = mbar_wait_warp(bar_full + 8 * s, par, gave_up);
+                        ok = mbar_wait_warp(bar_full + 8 * s, par);
                     }
                     if (!ok) break;
                 }
@@ -550,7 +555,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         }
 
         // ---------------- exchange and epilogue: all eight warps ----------------
-        bool ok = mbar_wait_warp(bar_acc, 0, gave_up);
+        ok = ok && mbar_wait_warp(bar_acc, 0);
+        tc_withheld_delay(P);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // best-effort flavour: behind this barrier the producer and the MMA warp are past their loops, the flag word is final
         if (BE) __syncthreads();
@@ -601,10 +607,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
             // up stays until every warp of the cluster is past its stores, each of them after bounded waits, and these
             // have landed.  (Only then does anybody wait for this barrier; to arrive costs nothing that could be measured.)
             cluster_arrive_relaxed();
-            if (recv_bytes != 0 && !mbar_wait_cluster_warp(bar_recv, 0, gave_up)) {
-                ok = false;
-                cluster_wait();
-                mbar_wait_cluster_warp(bar_recv, 0, nullptr);
+            if (recv_bytes != 0) {
+                ok = ok && mbar_wait_cluster_warp(bar_recv, 0);
+                if (!ok) {
+                    cluster_wait();
+                    mbar_wait_cluster_warp(bar_recv, 0);
+                }
             }
             if (BE) {
                 // every rank has the words of all the others: all take the same exit
@@ -641,7 +649,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         if (!ok && warp == 0) {
             const int issued = (int)s_flags[1];
             bool landed = true;
-            for (int i = max(0, issued - NS); i < issued && landed; i++) landed = mbar_wait_warp(bar_full + 8 * (i % NS), (uint32_t)(i / NS) & 1u, nullptr);
+            for (int i = max(0, issued - NS); i < issued && landed; i++) landed = mbar_wait_warp(bar_full + 8 * (i % NS), (uint32_t)(i / NS) & 1u);
         }
     }
 

@@ -58,7 +58,7 @@ struct TcParams {
     signed char tap_qx[64];  // ... and the tap's offset on that sub-lattice, so that the input coordinate
     signed char tap_qy[64];  //     stride*x + kx - pw becomes (x + qx) on map (ry*stride + rx)
 #ifdef REEF_DEBUG_AIDS
-    int withheld_rank, withheld_load;   // this rank announces this K block's load and never makes it (-1: none)
+    int withheld_rank, withheld_load, withheld_delay_ns;   // this rank announces this K block's load and never makes it (-1: none)
 #endif
     int pdl;                 // programmatic dependent launch: weights are fetched before the grid dependency wait
 };

@@ -77,40 +77,34 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 // The waits of a whole warp: every lane polls, the warp leaves together (the votes keep its control flow, and with it the
-// addresses and descriptors of what it issues next, warp-uniform).  `gave_up` (shared memory, or null) is what the waits of a CTA
-// share: one that expires sets it, and all others end with it instead of sitting out a limit each.
-__device__ __forceinline__ bool wait_is_over(uint32_t tries, unsigned long long& t0, volatile uint32_t* gave_up) {
-    if (gave_up != nullptr && __any_sync(0xffffffffu, *gave_up != 0)) return true;
+// addresses and descriptors of what it issues next, warp-uniform).
+__device__ __forceinline__ bool wait_is_over(uint32_t tries, unsigned long long& t0) {
     const unsigned long long t = global_ns();
     if (t0 == 0) t0 = t;
-    if (__all_sync(0xffffffffu, t - t0 > REEF_WAIT_LIMIT_NS) || tries >= 1u << 26) {
-        if (gave_up != nullptr) *gave_up = 1;
-        return true;
-    }
-    return false;
+    return __all_sync(0xffffffffu, t - t0 > REEF_WAIT_LIMIT_NS) || tries >= 1u << 26;
 }
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
     unsigned long long t0 = 0;
     for (uint32_t i = 0;; i++) {
         if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
-        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return false;
+        if ((i & 255) == 255 && wait_is_over(i, t0)) return false;
     }
 }
-__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint32_t bar, uint32_t parity) {
     unsigned long long t0 = 0;
     for (uint32_t i = 0;; i++) {
         if (__all_sync(0xffffffffu, mbar_try_cluster(bar, parity))) return true;
-        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return false;
+        if ((i & 255) == 255 && wait_is_over(i, t0)) return false;
     }
 }
 // The wait of the best-effort flavour's MMA warp also ends when `abort_word` (shared memory, written by the TMA producer
 // of the same CTA when it saw the preempt flag) becomes non-zero.  0 = phase complete, 1 = gave up, 2 = abort requested.
-__device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word, volatile uint32_t* gave_up) {
+__device__ __forceinline__ int mbar_wait_abortable_warp(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_word) {
     unsigned long long t0 = 0;
     for (uint32_t i = 0;; i++) {
         if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return 0;
         if (__any_sync(0xffffffffu, *abort_word != 0)) return 2;
-        if ((i & 255) == 255 && wait_is_over(i, t0, gave_up)) return 1;
+        if ((i & 255) == 255 && wait_is_over(i, t0)) return 1;
     }
 }
 // One look, without the suspension that try_wait may take: for a look ahead at a barrier that may be far from complete.

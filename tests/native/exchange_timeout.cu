@@ -8,9 +8,9 @@ unsigned long long* preempt_stamps_ptr() { return nullptr; }
 }  // namespace reef
 
 // out[m][n] = x[m][k] * w[n][k]^T by tiles of `cap` pixels and `splits` ranks; rank `rank` of the first tile never gets its
-// K block `load` (-1: it does).  plan[3] = {ranks, pixel tiles x channel tiles, K blocks of a rank}, slot = CTAs that counted themselves
+// K block `load` (-1: it does) and, once it has given up, sends its shares `delay_ms` later.  plan[4] = {ranks, pixel tiles x channel tiles, K blocks of a rank, receive area over the ring}, slot = CTAs that counted themselves
 // complete, error = the device error word, cleared again.
-extern "C" __attribute__((visibility("default"))) int exchange_run(int m, int n, int k, int cap, int splits, int best_effort, int rank, int load, const float* x,
+extern "C" __attribute__((visibility("default"))) int exchange_run(int m, int n, int k, int cap, int splits, int best_effort, int rank, int load, int delay_ms, const float* x,
                                                                    const float* w, float* out, int* plan, int* slot, int* error, float* ms) {
     using namespace reef;
     ConvP p;
@@ -20,7 +20,7 @@ extern "C" __attribute__((visibility("default"))) int exchange_run(int m, int n,
     p.plan_cap = cap; p.plan_splits = splits;
     TcPlan pl;
     if (tc_plan(p, &pl) != REEF_SUCC) return 1;
-    plan[0] = pl.splits; plan[1] = pl.n_tiles * pl.m_tiles; plan[2] = pl.kb_per_split;
+    plan[0] = pl.splits; plan[1] = pl.n_tiles * pl.m_tiles; plan[2] = pl.kb_per_split; plan[3] = pl.recv_late;
     float *dx, *dw, *dout;
     int* words;   // preempt flag, completion counter
     if (cudaMalloc(&dx, 4ull * m * k) || cudaMalloc(&dw, 4ull * n * k) || cudaMalloc(&dout, 4ull * m * n) || cudaMalloc(&words, 8)) return 2;
@@ -32,6 +32,7 @@ extern "C" __attribute__((visibility("default"))) int exchange_run(int m, int n,
     if (tc_prepare_device() != REEF_SUCC || tc_build_params(p, pl, args, &P) != REEF_SUCC) return 4;
     P.withheld_rank = rank;
     P.withheld_load = load;
+    P.withheld_delay_ns = delay_ms * 1000000;
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);

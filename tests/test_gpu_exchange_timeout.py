@@ -38,9 +38,10 @@ CASES = [  # pixels, output channels, K, tile cap, ranks, rank that waits, its K
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("delay", [0, 2 * LIMIT_MS])      # in the second case the peers give up long before its shares come
 @pytest.mark.parametrize("best_effort", [0, 1])
 @pytest.mark.parametrize("case", CASES, ids=["%d_%d_%d_ts%d_rank%d_load%d" % (c[:3] + c[4:]) for c in CASES])
-def test_a_wait_of_the_exchange_that_expires(case, best_effort):
+def test_a_wait_of_the_exchange_that_expires(case, best_effort, delay):
     m, n, k, cap, splits, rank, load = case
     lib = C.CDLL(_library())
     rng = np.random.default_rng(m)
@@ -48,25 +49,29 @@ def test_a_wait_of_the_exchange_that_expires(case, best_effort):
     want = x.astype(np.float64) @ w.astype(np.float64).T
     f32 = lambda a: a.ctypes.data_as(C.POINTER(C.c_float))      # noqa: E731
 
-    def run(rank, load):
-        out, plan, slot, error, ms = np.zeros((m, n), np.float32), (C.c_int * 3)(), C.c_int(), C.c_int(), C.c_float()
-        rc = lib.exchange_run(m, n, k, cap, splits, best_effort, rank, load, f32(x), f32(w), f32(out), plan, C.byref(slot), C.byref(error), C.byref(ms))
+    def run(rank, load, delay=0):
+        out, plan, slot, error, ms = np.zeros((m, n), np.float32), (C.c_int * 4)(), C.c_int(), C.c_int(), C.c_float()
+        rc = lib.exchange_run(m, n, k, cap, splits, best_effort, rank, load, delay, f32(x), f32(w), f32(out), plan, C.byref(slot), C.byref(error), C.byref(ms))
         assert rc == 0
         return out, list(plan), slot.value, error.value, ms.value
 
     def good():
-        out, (ranks, tiles, blocks), slot, error, _ = run(-1, -1)
+        out, (ranks, tiles, blocks, _), slot, error, _ = run(-1, -1)
         assert ranks == splits and load < blocks
         assert error == 0 and slot == ranks * tiles
         assert np.abs(out - want).max() <= TF32_TOL * np.abs(want).max()
         return out
 
     before = good()
-    _, (ranks, tiles, _), slot, error, ms = run(rank, load)
+    _, (ranks, tiles, _, over_ring), slot, error, ms = run(rank, load, delay)
     print(case, "best-effort" if best_effort else "plain", f"ended after {ms:.1f} ms, {slot} of {ranks * tiles} CTAs complete")
     assert error == 1
-    assert slot < ranks * tiles
-    # the wait that expires, then the peers' shares and the own loads at most, each with a limit of its own
-    assert LIMIT_MS <= ms <= 3.5 * LIMIT_MS
+    groups = -(-min(m, cap) // 4)
+    receivers = -(-groups // -(-groups // ranks))      # ranks with a share
+    # CTAs that cannot have counted themselves complete when it comes too late (over the ring, a barrier holds all ranks until it does)
+    late = receivers + (rank >= receivers) if delay and not over_ring else 1
+    assert slot <= ranks * tiles - late
+    # the wait that expires, the peers' shares and the own loads, each with a limit of its own
+    assert LIMIT_MS + delay <= ms <= 3.5 * LIMIT_MS + delay
     for _ in range(3):
         assert np.array_equal(good(), before)
