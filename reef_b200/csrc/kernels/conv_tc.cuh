@@ -111,7 +111,8 @@ __device__ __forceinline__ float tc_round1(float v) {
 // share.  With two warps on a scheduler a hundred instructions of a warp are 0.2 us and more, so what can be worked
 // out ahead of the last wait is, and everything per pixel is predicated.
 struct TcShare {
-    uint32_t out, out2, res;   // element of the first group's first pixel; eight pixels further per turn
+    float *out, *out2;         // this channel of the first group's first pixel; eight pixels further per turn.  Pointers: a slice of a
+    const float* res;          // wide buffer may lie beyond 2^32 elements
     int count, left;           // groups; pixels from the first group to the end of the share (0: no such channel)
     float sc, sh, b2;          // scale and shift (bias), shift of the second output
     float rpre[2][4];          // residual of the next two groups
@@ -124,7 +125,7 @@ struct TcShare {
 template <int S, int U, bool GELU>
 __device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_t src) {
     const uint32_t slot_bytes = (uint32_t)P.gpc * (TC_BM * 16);
-    const uint32_t ocs = (uint32_t)P.ocs, pcs = (uint32_t)P.pcs, rcs = (uint32_t)P.co;
+    const size_t ocs = (size_t)P.ocs, pcs = (size_t)P.pcs, rcs = (size_t)P.co;
     const bool has_res = P.res != nullptr;
 #pragma unroll 1
     for (int k0 = 0; k0 < w.count; k0 += U) {
@@ -148,7 +149,7 @@ __device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_
                 for (int i = 0; i < 4; i++) {
                     r[u][i] = w.rpre[u][i];
                     if (U == 1) w.rpre[0][i] = w.rpre[1][i];
-                    w.rpre[U == 1 ? 1 : u][i] = ld_activation_if(8 * (u + 2) + i < w.left, P.res + (w.res + (uint32_t)(8 * (u + 2) + i) * rcs));
+                    w.rpre[U == 1 ? 1 : u][i] = ld_activation_if(8 * (u + 2) + i < w.left, w.res + (8 * (u + 2) + i) * rcs);
                 }
         }
         if (S == 1) {
@@ -185,7 +186,7 @@ __device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_
         for (int u = 0; u < U; u++)
 #pragma unroll
             for (int i = 0; i < 4; i++)
-                if (8 * u + i < w.left) P.out[w.out + (uint32_t)(8 * u + i) * ocs] = v[u][i];
+                if (8 * u + i < w.left) w.out[(8 * u + i) * ocs] = v[u][i];
         if (P.out2 != nullptr) {
             TC_EACH(fmaxf(v[u][i] + w.b2, 0.f));
             if (P.ep & TC_EP_ROUND) TC_EACH(tc_round1(v[u][i]));
@@ -193,7 +194,7 @@ __device__ __forceinline__ void tc_finish(const TcParams& P, TcShare& w, uint32_
             for (int u = 0; u < U; u++)
 #pragma unroll
                 for (int i = 0; i < 4; i++)
-                    if (8 * u + i < w.left) P.out2[w.out2 + (uint32_t)(8 * u + i) * pcs] = v[u][i];
+                    if (8 * u + i < w.left) w.out2[(8 * u + i) * pcs] = v[u][i];
         }
 #undef TC_EACH
         src += S == 1 ? 8u * U : 2u * U * (TC_BM * 16);
@@ -520,13 +521,13 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
         const int gfirst = grp0 + ((grp0 ^ half) & 1);
         w.count = max(0, (grp0 + mg - gfirst + 1) >> 1);
         w.left = cvalid && w.count > 0 ? min(n_lim, (grp0 + mg) * 4) - gfirst * 4 : 0;
-        w.out = (uint32_t)((pix0 + gfirst * 4) * P.ocs + P.ooff + co);
-        w.out2 = (uint32_t)((pix0 + gfirst * 4) * P.pcs + P.poff + co);
-        w.res = (uint32_t)((pix0 + gfirst * 4) * P.co + co);
+        w.out = P.out + ((size_t)(pix0 + gfirst * 4) * P.ocs + P.ooff + co);
+        w.out2 = P.out2 + ((size_t)(pix0 + gfirst * 4) * P.pcs + P.poff + co);
+        w.res = P.res + ((size_t)(pix0 + gfirst * 4) * P.co + co);
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) w.rpre[u][i] = ld_activation_if(P.res != nullptr && 8 * u + i < w.left, P.res + (w.res + (uint32_t)((8 * u + i) * P.co)));
+            for (int i = 0; i < 4; i++) w.rpre[u][i] = ld_activation_if(P.res != nullptr && 8 * u + i < w.left, w.res + (size_t)(8 * u + i) * P.co);
 
         // The exchange: this half's groups of the tile leave tensor memory four at a time for the owner's shared memory, slot `split`
         // there; an own group goes into the own slot (the thread that finishes a group is the one that put it there).  The next
