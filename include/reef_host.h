@@ -76,6 +76,9 @@ REEF_HOST_API int reef_executor_execute_preempt_resume(reef_executor_t e, int de
                                                        int* first_count);
 /* Completion counters (task slots) and logical block counts per kernel, n entries each. */
 REEF_HOST_API int reef_executor_task_slots(reef_executor_t e, int* slots, int* block_nums, size_t n);
+/* The completion counters as the first preemption of the last reef_executor_execute_preempt_resume found them (all zero if there
+ * was none).  A counter says something only up to the first short one: see HybridExecutor::get_be_kernel_offset. */
+REEF_HOST_API int reef_executor_preempted_slots(reef_executor_t e, int* slots, size_t n);
 /* Average milliseconds of `iters` executions after `warmup` (mode: 0 raw launches, 1 graph, 2 best-effort). */
 REEF_HOST_API int reef_executor_time(reef_executor_t e, int mode, int warmup, int iters, float* avg_ms);
 /* Average milliseconds of one replay of a CUDA graph holding only the model's tensor-core kernels, in schedule

@@ -276,6 +276,13 @@ class HybridExecutor:
                self._err())
         return (restarts.value, first.value, count.value) if with_count else (restarts.value, first.value)
 
+    def preempted_slots(self):
+        """Completion counters as the first preemption of the last ``execute_preempt_resume`` found them."""
+        n = self.num_kernels()
+        slots = (C.c_int * n)()
+        _check(self._lib.reef_executor_preempted_slots(self._h, slots, C.c_size_t(n)), "preempted_slots")
+        return list(slots)
+
     def task_slots(self):
         n = self.num_kernels()
         slots = (C.c_int * n)()

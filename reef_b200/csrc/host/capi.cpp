@@ -165,6 +165,12 @@ int reef_executor_task_slots(reef_executor_t e, int* slots, int* block_nums, siz
     }
     return Succ;
 }
+int reef_executor_preempted_slots(reef_executor_t e, int* slots, size_t n) {
+    if (n < e->exe.num_kernels()) return OutOfRange;
+    const std::vector<int>& found = e->exe.preempted_slots();
+    for (size_t i = 0; i < e->exe.num_kernels(); i++) slots[i] = i < found.size() ? found[i] : 0;
+    return Succ;
+}
 int reef_executor_time(reef_executor_t e, int mode, int warmup, int iters, float* avg_ms) {
     reef_event_t a, b;
     if (reef_event_create(&a) != REEF_SUCC || reef_event_create(&b) != REEF_SUCC) return Fail;

@@ -511,7 +511,6 @@ void HybridExecutor::copy_be_kernel_offset(GPUStream_t stream) {
 }
 
 int HybridExecutor::get_be_kernel_offset(int begin) {
-    // first kernel whose completion counter is short of its logical block count
     for (size_t i = begin; i < num_kernels(); i++)
         if (task_slots_host[i] < trans_args[i].block_num) return (int)i;
     return (int)num_kernels();
@@ -955,6 +954,7 @@ Status HybridExecutor::execute_preempt_resume(int delay_us, int* restarts, int* 
     drop_output_mirror();
     if (first_incomplete) *first_incomplete = -1;
     if (first_count) *first_count = -1;
+    preempted_slots_.clear();
     GPU_RETURN_STATUS(reef_write32_async(flag_stream, preempt_flag, 0));
     GPU_RETURN_STATUS(reef_stream_sync(flag_stream));
     reset_task_slots(s, 0);
@@ -993,6 +993,7 @@ Status HybridExecutor::execute_preempt_resume(int delay_us, int* restarts, int* 
         if (k >= n) break;
         if (rounds == 0 && first_incomplete) *first_incomplete = k;
         if (rounds == 0 && first_count) *first_count = task_slots_host[k];
+        if (rounds == 0) preempted_slots_.assign(task_slots_host, task_slots_host + n);
         reset_task_slots(s, k);
         from = k;
         rounds++;

@@ -150,7 +150,11 @@ public:
     Status reset_task_slot_async(int kernel_offset, GPUStream_t stream);
     void reset_task_slots(GPUStream_t stream, int from_kernel = 0);
     void copy_be_kernel_offset(GPUStream_t stream);
+    // Where a preempted run restarts: the first kernel from `begin` on whose counter is short of its block count.  What the
+    // counters behind it say means nothing: a block decides whether to run from a look at the flag that was taken ahead of its
+    // wait for the kernel before, so a kernel behind one that left early may run whole, over partial data, and count every block.
     int get_be_kernel_offset(int begin);
+    const std::vector<int>& preempted_slots() const { return preempted_slots_; }
 
     Status launch_preempt_kernel(int kernel_offset, GPUStream_t stream);
     // dispatcher launch of kernel `rt_idx`, padded with logical blocks of `be`'s kernel `be_idx`
@@ -245,6 +249,7 @@ protected:
     GPUDevicePtr_t task_slot_base = 0;
     GPUDevicePtr_t dispatch_ctrl = 0;
     int* task_slots_host = nullptr;
+    std::vector<int> preempted_slots_;   // counters found by the first preemption of execute_preempt_resume
     bool has_tc = false;
     std::shared_ptr<ModelProfile> model_profile;
     reef_graph_t graph = nullptr;

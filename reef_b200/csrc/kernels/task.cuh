@@ -123,7 +123,9 @@ struct EnterPlain {
 // that goes up between the reads of two warps would let part of a block leave and the rest run the body with
 // threads missing (wrong partial sums counted as a complete block, barriers short of arrivals).  It is read ahead of
 // the wait for the previous kernel, so that its trip to L2 (0.4 us) is not on the way to the body: a flag that goes up
-// during that wait is seen by the body's polls or by the next kernel of the stream, which starts behind this wait.
+// during that wait is seen by the body's polls or by the next kernel of the stream, which starts behind this wait.  A body without
+// polls then runs whole behind a kernel that left early, over partial data, and counts its block: the run is
+// resumed from the first short counter, and what later counters say means nothing.
 struct EnterBestEffort {
     int up;                 // what thread 0 read, 0 elsewhere
     __device__ __forceinline__ bool operator()() const {

@@ -17,7 +17,7 @@ __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
 }
 
 // The completion counter of a best-effort kernel, issued by one thread behind a CTA barrier.  It says that the block ran to its
-// end and is read behind the kernel's end only (a copy on its stream), which publishes all stores: with release semantics the
+// end, over whole data if every kernel before it has a full counter too (HybridExecutor::get_be_kernel_offset), and is read behind the kernel's end only (a copy on its stream), which publishes all stores: with release semantics the
 // thread waited for the CTA's stores to reach L2 first, in every block between its last store and its exit.
 __device__ __forceinline__ void red_relaxed_gpu_add(int* p, int v) {
     asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
