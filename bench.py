@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Benchmark of the REEF executor kernel path on B200.
 
-Workload (BASELINE.json configs[2], the configuration the headline metric is quoted on): one
+Workload (the configuration the headline metric is quoted on): one
 real-time (RT) client issuing back-to-back ResNet-152 batch-1 requests while 4 best-effort (BE)
 clients run ResNet-152 batch-1 closed-loop, all on one GPU through REEFScheduler in REEF mode
 (flag preemption + dynamic kernel padding).  Synthetic, seeded weights and inputs.
@@ -36,22 +36,22 @@ sys.path.insert(0, ROOT)
 UNIT = "inf/s"
 REQS_PER_STEP = 100     # one step = this many back-to-back RT requests
 # DRAM traffic of the dominant kernel per launch, from an ncu capture of all 154 tensor-core launches of one
-# ResNet-152 pass (dram__bytes_read.sum + dram__bytes_write.sum; summary committed as
-# profiles/conv_tc_resnet152_dram.md).  A constant of that capture: it is NOT measured in a bench run.
+# ResNet-152 pass (dram__bytes_read.sum + dram__bytes_write.sum).  A constant of that capture: it is NOT measured in a
+# bench run.
 CONV_TC_TRAFFIC_PER_LAUNCH = {"c2": 2407620, "c1": 2407620}
-# BASELINE.json configs; "c2" is the configuration the headline metric is quoted on and the default
+# "c2" is the configuration the headline metric is quoted on and the default
 WORKLOADS = {
     "c0": dict(metric="resnet18_b1_inferences_per_s_rt_only", rt="resnet18", be=[],
-               desc="configs[0]: ResNet-18 b1, single RT client, no contention"),
+               desc="ResNet-18 b1, single RT client, no contention"),
     "c1": dict(metric="resnet152_b1_inferences_per_s_rt_only", rt="resnet152", be=[],
-               desc="configs[1]: ResNet-152 b1, RT-only closed-loop requests"),
+               desc="ResNet-152 b1, RT-only closed-loop requests"),
     "c2": dict(metric="resnet152_b1_inferences_per_s_rt_plus_4be", rt="resnet152", be=["resnet152"] * 4,
-               desc="configs[2]: ResNet-152 b1 RT client back-to-back + 4 BE ResNet-152 b1 closed-loop clients, REEF mode"),
+               desc="ResNet-152 b1 RT client back-to-back + 4 BE ResNet-152 b1 closed-loop clients, REEF mode"),
     "c3": dict(metric="inception_v3_b1_inferences_per_s_rt_plus_vgg16_densenet201_be", rt="inception_v3",
                be=["vgg16", "densenet201"],
-               desc="configs[3]: RT Inception-v3 b1 (299x299) + BE VGG-16 b1 + BE DenseNet-201 b1, REEF mode (kernel padding mix)"),
+               desc="RT Inception-v3 b1 (299x299) + BE VGG-16 b1 + BE DenseNet-201 b1, REEF mode (kernel padding mix)"),
     "c4": dict(metric="bert_base_s128_inferences_per_s_rt_plus_4be_resnet50", rt="bert_base", be=["resnet50"] * 4,
-               desc="configs[4]: RT BERT-base b1 seq 128 + 4 BE ResNet-50 b1 per GPU, REEF mode"),
+               desc="RT BERT-base b1 seq 128 + 4 BE ResNet-50 b1 per GPU, REEF mode"),
 }
 METRIC = WORKLOADS["c2"]["metric"]
 WORKLOAD = WORKLOADS["c2"]["desc"]
@@ -428,7 +428,7 @@ def main():
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "peak_kind": peak_kind,
                 "traffic_source": ("constant from an ncu capture of the 154 ResNet-152 launches (dram bytes read + written "
-                                   "per launch, profiles/conv_tc_resnet152_dram.md); not measured in this run"
+                                   "per launch); not measured in this run"
                                    if traffic is not None else None),
                 "kernel": "reef_conv_tc_kernel (tcgen05 TF32 convolution/matmul: the %d launches of one %s pass as a CUDA "
                           "graph of their own, timed with CUDA events over 50 replays)" % (tc_n, wl["rt"]),

@@ -37,13 +37,12 @@ __device__ __forceinline__ bool body_embedding(const KTask& t, int vb, unsigned 
 // A row lives in registers, at most two 128-bit values a lane (h <= 1024, h % 128 == 0): one, two or four warps share a row, so that
 // many SMs take part and every load of a launch is in flight at once.  What bounds a launch is its latency: the hand-over, one trip
 // to L2 and two reductions.  A warp to a row of 768 kept its 12 to 24 loads in a chain of branches and eight rows on an SM:
-// 128 rows 3.49 -> 1.86 us, 384 rows 3.59 -> 2.06 us a launch; a replay of BERT-base 490 -> 440 us at 128 tokens, 773 -> 718 us
-// at 384.
+// 128 rows 3.49 -> 1.86 us, 384 rows 3.59 -> 2.06 us a launch.
 __host__ __device__ inline int ln_warps_per_row(int h) { return h <= 256 ? 1 : h <= 512 ? 2 : 4; }
 constexpr int kLnRowsPerBlock = 8;   // with one warp to a row; schedules of earlier versions have it for every width
 // gamma and beta are model constants: they are asked into L2 before the wait for the previous kernel.  A model's weights have
 // flushed them out since its last pass, and behind the reductions their trip from HBM would stand on the critical path
-// (0.5 us a launch: BERT-base at 128 tokens 531 -> 518 us a replay).
+// (0.5 us a launch of 128 rows).
 __device__ __forceinline__ void prefetch_layernorm(const KTask& t) {
     const int h = t.p.raw[1], first = t.p.raw[2] ? 3 : 2, lines = h >> 5;
     if ((int)threadIdx.x < 2 * lines) {
@@ -131,8 +130,7 @@ __device__ __forceinline__ bool body_layernorm(const KTask& t, int vb, unsigned 
 // straight into registers (250 of them, one block per SM), the next loads travelling during either product.  Beyond that
 // what counts is how many warps hide the chains of dependent multiplications behind each other (2 us per 16 keys with one
 // block on an SM): keys and values are staged through shared memory by cp.async and two blocks share an SM.
-// Measured, 12 heads: 128 tokens 8.6 (fp32 instructions) / 7.8 (TF32, tcgen05) -> 5.7 us, 384 tokens 30.9 -> 15.4 us, 512
-// tokens 75 -> 28.8 us; error against fp64 0.3-0.5 of the fp32 instructions'.
+// Measured, 12 heads: 128 tokens 8.6 us by fp32 instructions, 7.8 in TF32 on tcgen05, 5.1 here; 384 tokens 30.9 and 14.4 us; error against fp64 0.3-0.5 of the fp32 instructions'.
 constexpr int kAttChunk = 16;                              // keys a warp takes at a time
 constexpr int kAttD = 64;
 constexpr int kAttRowStride = kAttD + 4;

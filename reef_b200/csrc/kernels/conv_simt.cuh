@@ -22,9 +22,10 @@
 // shared memory, summed in a fixed order.  A lane's K positions in a fragment are four consecutive ones (the order inside
 // a slice is free as long as both operands agree), so an operand row is read with one 128-bit load.
 // What is left: a block alone on its SM keeps the tensor cores busy a quarter of the time, two of them half of it, and issue
-// 82 % of what the schedulers can; so every instruction of a slice counts (ResNet-50 at 193x193: addresses per tap instead of
-// per slice, and no clearing of accumulators, 585 -> 564 us a replay; with the shorter split 549, with the set-up ahead of the wait 521; ResNet-18 at 64x64 168 -> 140).
-// Measured, 3x3 256 -> 256 at 13x13: 133 us by fp32 instructions, 13.9, now 12.4; 3x3 512 -> 512 at 7x7: 261, 19.5, 16.7.
+// 82 % of what the schedulers can; so every instruction of a slice counts.  Addresses are worked out per tap instead of per slice,
+// accumulators are not cleared, a remainder of the split is one multiply-add, and the set-up runs ahead of the wait for the previous
+// kernel.  Measured, 3x3 256 -> 256 at 13x13: 133 us by fp32 instructions, 13.9 before these, 11.1 with them; 3x3 512 -> 512 at
+// 7x7: 261, 19.6, 15.8.
 #pragma once
 #include <type_traits>
 
@@ -38,10 +39,9 @@ constexpr int CTP = 16;                       // pixels of a warp tile
 constexpr int kConvSimtRing = 98304;          // eight warps' stages; two blocks fit an SM
 constexpr int kConvSimtSmem = kConvSimtRing + 128;
 
-// Channels of the warp tile and K groups of a shape: the least time by what was measured.  One block on an SM takes 0.57 us
-// per slice of eight 16x32 tiles and 0.41 us of 16x16 (splitting operands into bf16 is most of it), blocks that share an SM
+// Channels of the warp tile and K groups of a shape: the least time by what was measured.  A slice of eight 16x32 tiles
+// counts as 0.57 us for one block on an SM and one of 16x16 as 0.41 (the ratio decides; splitting operands into bf16 is most of it), blocks that share an SM
 // overlap by a sixth; launch, prologue and epilogue take 3.5 us, every further block of an SM half a microsecond.
-// (A slice takes 0.47 and 0.35 us by now; the ratio, which decides, is what it was.)
 struct ConvSimtTile {
     int tc, kg;
 };

@@ -18,13 +18,12 @@
 //
 // One warp issues TMA, one warp issues tcgen05.mma, all eight warps run the exchange and the epilogue
 // (tcgen05.ld -> +residual -> +bias | *gamma+beta -> ReLU -> stores), a thread being one output channel throughout,
-// as tensor memory has it.  What bounds it: a launch of a few microseconds is a chain of latencies (hand-over from
-// the previous grid and first K block 1.4 us, multiplications 160 cycles per K block, exchange 0.4-0.9 us) beside a
-// load stream that takes about 57 bytes a clock into an SM.  Reading the partials out of the peers' staged tiles between
-// two cluster barriers took 1.2 us for 28 pixels over eight ranks where the stores take 0.4, 1.7 against 0.8 for 64
-// pixels; together with multiplications issued at the tensor core's pace: 1x1 1024 -> 256 at 14x14 4.41 -> 3.09 us, 3x3
-// 256 -> 256 5.03 -> 4.00 us, replays of ResNet-152 779 -> 604 us, DenseNet-201 994 -> 863 us, Inception-v3 320 -> 291 us (573, 826
-// and 282 with the steps that are told beside the code below).
+// as tensor memory has it.  What bounds it: a launch of a small layer is a chain of latencies (hand-over from the previous grid and
+// first K block 1.4 us, the rank's few K blocks, exchange 0.7 us, rows 0.4); a large 3x3 layer is bound by what an SM takes in, 57
+// bytes a clock of operands (3x3, 512 channels, 28x28: 646 cycles per K block of 30 KB and two CTAs on an SM, where the
+// multiplications need 240) and 16 of partial sums.  Shares stored into the owner replace partials read out of the peers'
+// staged tiles between two cluster barriers: 28 pixels over eight ranks 1.2 -> 0.4 us behind the accumulator; with
+// multiplications issued at the tensor core's pace, 1x1 1024 -> 256 at 14x14 4.4 -> 3.1 us a launch, 3x3 256 -> 256 5.0 -> 4.0.
 // Every mbarrier wait is bounded.  A warp that gave up skips its further waits and sends what it has; the CTA stays until nothing can be
 // stored into its shared memory any more (peers' shares, its own loads; bounded again), records the error word, frees its TMEM
 // and returns.
@@ -360,8 +359,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) reef_conv_tc_kernel(const __gri
                 }
             }
             // Weights of the K blocks beyond the ring: into L2, each once among the tiles that share them.  A stage freed by the
-            // multiplications is refilled from there in half the time that it takes from HBM (replays: ResNet-152 603 -> 584 us,
-            // BERT-base at 128 tokens 439 -> 425, VGG-16 267 -> 260, DenseNet-201 866 -> 848).
+            // multiplications is refilled from there in half the time that it takes from HBM (2 to 3 % of a replay of ResNet-152,
+            // BERT-base, VGG-16 or DenseNet-201).
             if (!abort0)
                 for (int i = first + lane; i < nkb; i += 32) {
                     const int kb = kb_begin + i, t = P.cblocks == 1 ? kb : (int)__umulhi((unsigned)kb, P.cb_magic);

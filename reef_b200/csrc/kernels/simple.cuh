@@ -211,7 +211,7 @@ __device__ __forceinline__ void pool_add(bool max, float4& acc, float4 v) {
 // K = 2, 3: a window of the usual sizes.  All of its values are requested at once, from places clamped into the input (a value
 // from outside the window's part of the input is replaced by the neutral one): the taps as branches were K * K trips to L2 one after
 // the other.  K = 0: any size, tap by tap.  3x3 over 112x112x64 3.06 -> 1.96 us, over
-// 17x17x768 3.09 -> 1.86 us a launch; a replay of Inception-v3 289 -> 282 us.
+// 17x17x768 3.09 -> 1.86 us a launch.
 template <bool MAX, int K>
 __device__ __forceinline__ void pool_window(const PoolP& p, const float* in, int oy, int ox, float4& acc, int& cnt) {
     const float4 neutral = acc;

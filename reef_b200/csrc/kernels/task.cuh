@@ -107,9 +107,9 @@ __device__ __forceinline__ void pdl_prologue() {
 
 // How a block enters: called once, with all threads, ahead of a body's first access to memory.  The fp32 convolution calls it
 // itself, behind what it works out from its parameters: its divisions and addresses, half a microsecond of a launch, are then out
-// of the way while the previous kernel still runs (replays: ResNet-50 at 193x193 549 -> 520 us, at 70x70 335 -> 307, ResNet-18
-// at 64x64 149 -> 140).  The other bodies have little to work out; with the same in pooling, elementwise kernels, the im2col
-// gather, LayerNorm and attention no model gained, and it is called ahead of them.  False: leave.
+// of the way while the previous kernel still runs (5 % of a replay of ResNet-50 at 193x193, 8 % at 70x70).  The other bodies have
+// little to work out: it is called ahead of them (inside pooling, elementwise kernels, the im2col gather, LayerNorm and attention no
+// model gained).  False: leave.
 struct EnterAlways {        // the dispatcher's blocks
     __device__ __forceinline__ bool operator()() const { return true; }
 };

@@ -242,9 +242,10 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t da, uint64_t
         : "memory");
 }
 // The same as code of a whole warp: `lead` is non-zero in the one lane that issues.  Predicated, so that the warp's control flow
-// stays uniform and the descriptors in uniform registers: the tensor core is then fed at its own rate, (4096 + 32 N) / 128 cycles
-// per instruction (operand reads from shared memory: 160 cycles per K block of four at N = 32, 192 at 64, 256 at 128).  A branch
-// around the instructions, and a look at the barrier between them, cost 307 / 320 / 332.
+// stays uniform and the descriptors in uniform registers: the tensor core is then fed at its own rate, measured over resident
+// operands as (4096 + 32 N) / 32 cycles per K block of four instructions up to N = 128 (operand reads from shared memory: 160 at
+// N = 32, 192 at 64, 256 at 128) and 2 N beyond.  A branch around the instructions, and a look at the barrier between them, cost 307 at
+// N = 32 and 332 at 96.
 __device__ __forceinline__ void umma_tf32_if(uint32_t lead, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
