@@ -424,7 +424,7 @@ HybridExecutor::~HybridExecutor() {
     for (auto& c : chains) reef_chain_destroy(c.handle);
     if (graph) reef_graph_destroy(graph);
     for (auto g : pad_segments) reef_graph_destroy(g);
-    for (auto g : be_segments) reef_graph_destroy(g);
+    drop_be_segments();
     if (own_flag && preempt_flag) reef_free(preempt_flag);
     if (task_slot_base) reef_free(task_slot_base);
     if (dispatch_ctrl) reef_free(dispatch_ctrl);
@@ -603,43 +603,58 @@ Status HybridExecutor::build_be_segments(GPUStream_t cap) {
     std::vector<int> from, to;
     RETURN_STATUS(schedule_edges(&from, &to));
     const int n = (int)num_kernels();
-    Status st = Status::Succ;
-    for (int k0 = 0; k0 < n && st == Status::Succ; k0 += kBeSegment) {
-        if (reef_graph_begin(cap) != REEF_SUCC) {
-            st = Status::Fail;
-            break;
-        }
-        const int k1 = std::min(n, k0 + kBeSegment);
+    // kernels [k0, k1) and, behind the last one, the output mirror
+    auto capture = [&](int k0, int k1, reef_graph_t* g) -> Status {
+        if (reef_graph_begin(cap) != REEF_SUCC) return Status::Fail;
+        Status st = Status::Succ;
         for (int k = k0; k < k1 && st == Status::Succ; k++) st = issue_preempt_kernel(k, cap);
         if (st == Status::Succ && k1 == n) st = issue_mirror(cap);
-        // branches side by side inside a segment, too; the segments follow one another on the stream
-        std::vector<int> seg_from, seg_to;
-        for (size_t e = 0; e < from.size(); e++)
-            if (from[e] >= k0 && to[e] < k1 + (k1 == n ? 1 : 0)) {
-                seg_from.push_back(from[e] - k0);
-                seg_to.push_back(to[e] - k0);
-            }
-        reef_graph_t g = nullptr;
-        const size_t launches = (size_t)(k1 - k0) + (k1 == n && mirror ? 1 : 0);
-        if (reef_graph_end_relaxed(cap, launches, seg_from.data(), seg_to.data(), seg_from.size(), &g) != REEF_SUCC) {
+        int rc;
+        if (k1 - k0 <= kPadSegment) {
+            rc = reef_graph_end(cap, g);    // a short one stays in order: its edges would take as long to work out as the rest
+        } else {
+            // branches side by side inside a segment, too; the segments follow one another on the stream
+            std::vector<int> seg_from, seg_to;
+            for (size_t e = 0; e < from.size(); e++)
+                if (from[e] >= k0 && to[e] < k1 + (k1 == n ? 1 : 0)) {
+                    seg_from.push_back(from[e] - k0);
+                    seg_to.push_back(to[e] - k0);
+                }
+            const size_t launches = (size_t)(k1 - k0) + (k1 == n && mirror ? 1 : 0);
+            rc = reef_graph_end_relaxed(cap, launches, seg_from.data(), seg_to.data(), seg_from.size(), g);
+        }
+        if (rc != REEF_SUCC) {
             err_ = reef_last_error();
             st = Status::Fail;
         }
-        if (st == Status::Succ) be_segments.push_back(g);
-        else if (g) reef_graph_destroy(g);
+        return st;
+    };
+    Status st = Status::Succ;
+    for (int k = 0; k < n && st == Status::Succ; k += kPadSegment) {
+        reef_graph_t g = nullptr;
+        const bool whole = k % kBeSegment == 0;
+        st = capture(k, std::min(n, k + (whole ? kBeSegment : kPadSegment)), &g);
+        if (whole) be_segments.push_back(g);
+        be_short_segments.push_back(whole ? nullptr : g);
     }
-    if (st != Status::Succ) {
-        for (auto g : be_segments) reef_graph_destroy(g);
-        be_segments.clear();
-    }
+    if (st != Status::Succ) drop_be_segments();
     return st;
 }
 
-// Best-effort kernels from k on: a whole segment where k stands at a segment boundary, else (a task resumed in the middle
-// of a segment, or `single`) kernel k alone.  *last = the last kernel launched.
+void HybridExecutor::drop_be_segments() {
+    for (auto* v : {&be_segments, &be_short_segments}) {
+        for (auto g : *v)
+            if (g) reef_graph_destroy(g);
+        v->clear();
+    }
+}
+
+// Best-effort kernels from k on: a whole segment where k stands at a segment boundary, a short one where it stands at a
+// boundary of those (a task resumed behind padding), else, or with `single`, kernel k alone.  *last = the last kernel launched.
 Status HybridExecutor::launch_preempt_segment(int k, GPUStream_t stream, bool single, int* last) {
     const int n = (int)num_kernels();
-    if (single || be_segments.empty() || k % kBeSegment != 0) {
+    const bool whole = k % kBeSegment == 0;
+    if (single || be_segments.empty() || k % kPadSegment != 0) {
         *last = k;
         RETURN_STATUS(launch_preempt_kernel(k, stream));
         if (k == n - 1) RETURN_STATUS(launch_output_mirror(stream));
@@ -651,8 +666,8 @@ Status HybridExecutor::launch_preempt_segment(int k, GPUStream_t stream, bool si
         return Status::Fail;
     }
     RETURN_STATUS(order_input(stream));
-    *last = std::min(n, k + kBeSegment) - 1;
-    int rc = reef_graph_launch(be_segments[k / kBeSegment], stream);
+    *last = std::min(n, k + (whole ? kBeSegment : kPadSegment)) - 1;
+    int rc = reef_graph_launch(whole ? be_segments[k / kBeSegment] : be_short_segments[k / kPadSegment], stream);
     if (rc != REEF_SUCC) err_ = reef_last_error();
     GPU_RETURN_STATUS(rc);
     if (*last == n - 1 && mirror) mirror_fresh.store(true, std::memory_order_relaxed);

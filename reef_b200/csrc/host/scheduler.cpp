@@ -1245,9 +1245,9 @@ void REEFScheduler::execute_be_task(std::shared_ptr<Task>& task, std::shared_ptr
     // preemption drains in 17 us with two kernels in flight, 42 us with two segments of four, 67 us with two of eight).
     // When none is to be expected nobody waits for a drain, and an entry is a whole segment: one graph launch and one
     // event for sixteen kernels keep the stream busy where the host could not, and branches run side by side inside it
-    // (DenseNet-201, one client: 2.5 ms a pass kernel by kernel, 1.0 by segments of 16; 24 and 32 take 5 % less).  Longer
-    // ones are a burden on who is preempted in the middle of one, since it goes on kernel by kernel to the segment's end: a
-    // real-time ResNet-18 at 300 px and four best-effort ones at 60 px are served a fifth later with segments of 24.  A window of one, or wait_sync, asks for quick drains: single kernels.
+    // (DenseNet-201, one client: 2.5 ms a pass kernel by kernel, 1.0 by segments of 16; 24 and 32 take 5 % less).  Who was
+    // padded or preempted between their boundaries reaches the next one by segments of four.  A window of one, or wait_sync, asks
+    // for quick drains: single kernels.
     const bool shallow = wait_sync || be_stream_device_queue_cap < 2 || rt_expected();
     while (task->launch_offset < num_kernels && (int)tqueue->inflight.size() < be_stream_device_queue_cap) {
         int last = task->launch_offset;
