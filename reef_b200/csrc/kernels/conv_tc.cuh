@@ -22,7 +22,7 @@
 // first K block 1.4 us, the rank's few K blocks, exchange 0.7 us, rows 0.4); a large 3x3 layer is bound by what an SM takes in, 57
 // bytes a clock of operands (3x3, 512 channels, 28x28: 646 cycles per K block of 30 KB and two CTAs on an SM, where the
 // multiplications need 240) and 16 of partial sums.  Shares stored into the owner replace partials read out of the peers'
-// staged tiles between two cluster barriers: 28 pixels over eight ranks 1.2 -> 0.4 us behind the accumulator; with
+// staged tiles between two cluster barriers: 28 pixels over eight ranks 1.65 -> 0.66 us from the accumulator to the last share; with
 // multiplications issued at the tensor core's pace, 1x1 1024 -> 256 at 14x14 4.4 -> 3.1 us a launch, 3x3 256 -> 256 5.0 -> 4.0.
 // Every mbarrier wait is bounded.  A warp that gave up skips its further waits and sends what it has; the CTA stays until nothing can be
 // stored into its shared memory any more (peers' shares, its own loads; bounded again), records the error word, frees its TMEM
